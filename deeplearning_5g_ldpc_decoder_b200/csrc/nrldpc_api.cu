@@ -477,8 +477,16 @@ void make_encode_params(const CodeParams& cp, DeviceState* st, EncodeParams* e) 
   e->symbols = cp.symbols;
   e->c0 = cp.c0;
   e->Kb = cp.K / cp.Zc;
-  for (int i = 0; i < g.nnz; ++i) e->edge[i] = (uint32_t)g.col[i] | ((uint32_t)(g.vij[cp.iLS][i] % cp.Zc) << 16);
-  for (int r = 0; r <= g.rows; ++r) e->row_off[r] = g.row_off[r];
+  e->W2 = (2 * cp.Zc + 31) / 32 + 1;
+  for (int r = 0; r < g.rows; ++r) {
+    const int cols = r < 4 ? e->Kb : e->Kb + 4;
+    for (int i = g.row_off[r]; i < g.row_off[r + 1]; ++i) {
+      if (g.col[i] >= cols) continue;
+      const uint32_t s = (uint32_t)(g.vij[cp.iLS][i] % cp.Zc);
+      e->edge[e->num_edges++] = ((uint32_t)g.col[i] * (uint32_t)e->W2 + (s >> 5)) | ((s & 31u) << 16);
+    }
+    e->row_off[r + 1] = (uint16_t)e->num_edges;
+  }
   // Core parity circulants (c_lib/ldpc_encoder.c:95-109): BG1 row 0 / row 1 at
   // base column 22, BG2 row 0 / row 2 at base column 10.
   if (cp.bgn == 1) {
@@ -491,10 +499,28 @@ void make_encode_params(const CodeParams& cp, DeviceState* st, EncodeParams* e) 
   e->crc_tab = st->crc_tab + (size_t)cp.crctype * kMaxB;
 }
 
+void set_encode_buffers(EncodeParams* e, const uint8_t* info, int64_t info_stride, int32_t num_cw, uint8_t* rm,
+                        int64_t rm_stride) {
+  e->num_cw = num_cw;
+  e->info = info;
+  e->info_stride = info_stride;
+  e->rm = rm;
+  e->rm_stride = rm_stride;
+  // a single row needs no aligned stride
+  e->info_vec = reinterpret_cast<uintptr_t>(info) % 4 == 0 && (num_cw == 1 || info_stride % 4 == 0);
+  e->rm_vec = reinterpret_cast<uintptr_t>(rm) % 4 == 0 && (num_cw == 1 || rm_stride % 4 == 0);
+}
+
+// derive_params, and A systematic bits that fit K: B is kept in 16 bits, so an A
+// near 65536 passes its size check with a B that has wrapped.
+bool derive_encode(const ldpc_in_config_t& in, CodeParams* cp) {
+  return derive_params(in, cp, true) == 0 && cp->A <= cp->K;
+}
+
 int32_t encode_one(uint8_t* infobytes, uint8_t* rm_bytes, ldpc_in_config_t* inconfig) {
   if (!inconfig) return NRLDPC_ERR_CONFIG;
   CodeParams cp;
-  if (derive_params(*inconfig, &cp, true) != 0) return NRLDPC_ERR_CONFIG;
+  if (!derive_encode(*inconfig, &cp)) return NRLDPC_ERR_CONFIG;
   std::lock_guard<std::mutex> lock(g_mu);
   DeviceState* st = nullptr;
   if (device_state(&st) != 0) return NRLDPC_ERR_CUDA;
@@ -506,12 +532,9 @@ int32_t encode_one(uint8_t* infobytes, uint8_t* rm_bytes, ldpc_in_config_t* inco
     return NRLDPC_ERR_CUDA;
   EncodeParams e;
   make_encode_params(cp, st, &e);
-  e.num_cw = 1;
-  e.info = static_cast<const uint8_t*>(st->one_info.ptr);
-  e.info_stride = in_bytes;
-  e.rm = static_cast<uint8_t*>(st->one_rm.ptr);
-  e.rm_stride = out_bytes;
-  if (launch_encode(e, s) != 0) return NRLDPC_ERR_CUDA;
+  set_encode_buffers(&e, static_cast<const uint8_t*>(st->one_info.ptr), in_bytes, 1,
+                     static_cast<uint8_t*>(st->one_rm.ptr), out_bytes);
+  if (launch_encode(e, st->num_sms, s) != 0) return NRLDPC_ERR_CUDA;
   if (cp.E > 0 && cudaMemcpyAsync(rm_bytes, st->one_rm.ptr, (cp.E + 7) / 8, cudaMemcpyDeviceToHost, s) != cudaSuccess)
     return NRLDPC_ERR_CUDA;
   if (cudaStreamSynchronize(s) != cudaSuccess) return NRLDPC_ERR_CUDA;
@@ -890,7 +913,7 @@ int32_t nrldpc_encode_batch(const uint8_t* d_info, int64_t info_stride, int32_t 
                             const ldpc_in_config_t* inconfig, uint8_t* d_rm, int64_t rm_stride, void* stream) {
   if (!inconfig || num_cw < 0) return NRLDPC_ERR_ARG;
   CodeParams cp;
-  if (derive_params(*inconfig, &cp, true) != 0) return NRLDPC_ERR_CONFIG;
+  if (!derive_encode(*inconfig, &cp)) return NRLDPC_ERR_CONFIG;
   if (num_cw == 0) return NRLDPC_OK;
   if (!d_info || !d_rm || info_stride < cp.A / 8 || rm_stride < (cp.E + 7) / 8) return NRLDPC_ERR_ARG;
   std::lock_guard<std::mutex> lock(g_mu);
@@ -898,12 +921,8 @@ int32_t nrldpc_encode_batch(const uint8_t* d_info, int64_t info_stride, int32_t 
   if (device_state(&st) != 0) return NRLDPC_ERR_CUDA;
   EncodeParams e;
   make_encode_params(cp, st, &e);
-  e.num_cw = num_cw;
-  e.info = d_info;
-  e.info_stride = info_stride;
-  e.rm = d_rm;
-  e.rm_stride = rm_stride;
-  return launch_encode(e, stream) == 0 ? NRLDPC_OK : NRLDPC_ERR_CUDA;
+  set_encode_buffers(&e, d_info, info_stride, num_cw, d_rm, rm_stride);
+  return launch_encode(e, st->num_sms, stream) == 0 ? NRLDPC_OK : NRLDPC_ERR_CUDA;
 }
 
 int32_t nrldpc_encode_batch_ncb(const uint8_t* d_info, int64_t info_stride, int32_t num_cw,
@@ -911,7 +930,7 @@ int32_t nrldpc_encode_batch_ncb(const uint8_t* d_info, int64_t info_stride, int3
                                 void* stream) {
   if (!inconfig || num_cw < 0) return NRLDPC_ERR_ARG;
   CodeParams cp;
-  if (derive_params(*inconfig, &cp, true) != 0) return NRLDPC_ERR_CONFIG;
+  if (!derive_encode(*inconfig, &cp)) return NRLDPC_ERR_CONFIG;
   if (ncb > 0 && ncb < cp.N) {
     if (ncb < cp.K - 2 * cp.Zc) return NRLDPC_ERR_CONFIG;
     // TS 38.212 Table 5.4.2.1-2 with Ncb < N
@@ -929,12 +948,8 @@ int32_t nrldpc_encode_batch_ncb(const uint8_t* d_info, int64_t info_stride, int3
   if (device_state(&st) != 0) return NRLDPC_ERR_CUDA;
   EncodeParams e;
   make_encode_params(cp, st, &e);
-  e.num_cw = num_cw;
-  e.info = d_info;
-  e.info_stride = info_stride;
-  e.rm = d_rm;
-  e.rm_stride = rm_stride;
-  return launch_encode(e, stream) == 0 ? NRLDPC_OK : NRLDPC_ERR_CUDA;
+  set_encode_buffers(&e, d_info, info_stride, num_cw, d_rm, rm_stride);
+  return launch_encode(e, st->num_sms, stream) == 0 ? NRLDPC_OK : NRLDPC_ERR_CUDA;
 }
 
 int32_t cuda_ldpc_5g_encode(uint8_t* infobytes, uint8_t* rm_bytes, ldpc_in_config_t* inconfig) {

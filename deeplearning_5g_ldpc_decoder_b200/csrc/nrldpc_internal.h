@@ -149,7 +149,13 @@ struct EncodeParams {
   int64_t info_stride;
   uint8_t* rm;              // [num_cw][rm_stride] rate-matched bytes (ceil(E/8) written)
   int64_t rm_stride;
-  uint32_t edge[kMaxNnz];   // base column in the low 16 bits, V_ij mod Zc in the high
+  int32_t info_vec, rm_vec; // rows 4-byte aligned: 32-bit loads / stores
+  int32_t W2;               // 32-bit words of a column kept twice in a row (2 Zc bits, and one word for the funnel shift)
+  int32_t num_edges;
+  // Edges into systematic columns (rows 0..3) or systematic + core columns (the
+  // other rows), row by row: the word of the doubled columns where the
+  // circulant's row 0 lies in the low 16 bits, its bit there in the high.
+  uint32_t edge[kMaxNnz];
   uint16_t row_off[kMaxRows + 1];
 };
 
@@ -230,7 +236,7 @@ struct TrainParams {
 };
 
 // Kernel launchers (defined in the .cu files).  Return a cudaError_t value.
-int launch_encode(const EncodeParams& p, void* stream);
+int launch_encode(const EncodeParams& p, int num_sms, void* stream);
 int launch_train_forward(const TrainParams& p, bool f64, int grid, int block, int smem, void* stream);
 int launch_train_backward(const TrainParams& p, bool f64, int grid, int block, int smem, void* stream);
 int occupancy_train(bool backward, bool f64, bool bg2, int block, int smem, bool alias = false);

@@ -121,7 +121,7 @@ def ldpc_encode(info: torch.Tensor, inconfig, ncb: int = 0) -> torch.Tensor:
     if info.stride(1) != 1:
         info = info.contiguous()
     n = info.shape[0]
-    out = torch.zeros((n, (cfg.E + 7) // 8), dtype=torch.uint8, device=info.device)
+    out = torch.empty((n, (cfg.E + 7) // 8), dtype=torch.uint8, device=info.device)   # every byte is written
     lib = capi.load_library()
     stream = torch.cuda.current_stream(info.device).cuda_stream
     with torch.cuda.device(info.device):

@@ -64,3 +64,31 @@ def test_encode_decode_round_trip(cuda):
     torch.cuda.synchronize()
     assert (res.status == 0).all()
     assert torch.equal(res.hardbits[:, :1053], pay)
+
+
+@pytest.mark.parametrize("bgn,A,E,rv,Qm,n,offset", [
+    (2, 8, 96, 0, 8, 3, 0),            # Zc 6 (less than a word), 12 symbols
+    (2, 40, 2112, 1, 1, 2, 1),         # repetition of a short buffer, BPSK, rows off the 4-byte grid
+    (1, 176, 32 * 6, 0, 6, 5, 0),      # Zc 10, exactly 32 symbols of 6 bits
+    (1, 704, 33 * 4, 2, 4, 4, 3),      # Zc 36 (a word and four bits), 33 symbols
+    (2, 3816, 31 * 6 * 20, 3, 6, 2, 1),   # Zc 384 of BG2, 620 symbols
+    (1, 4080, 13824, 0, 8, 17, 2),     # Zc 192: rows off the 4-byte grid
+    (1, 8424, 25344, 0, 8, 2500, 0),   # more blocks than CTAs in flight
+    (1, 8424, 65520, 2, 2, 2, 0),      # repetition at the largest block
+])
+def test_encode_word_edges_match_oracle(oracle, cuda, bgn, A, E, rv, Qm, n, offset):
+    """Partial words, partial 32-symbol steps, wraps and unaligned rows of the 32-bit encoder: exact."""
+    rng = np.random.default_rng(A + E)
+    pay = rng.integers(0, 256, size=(n, A // 8), dtype=np.uint8)
+    wide = torch.zeros((n, A // 8 + offset + 1), dtype=torch.uint8, device=cuda)
+    wide[:, offset:offset + A // 8] = torch.from_numpy(pay).to(cuda)
+    out = ldpc_encode(wide[:, offset:], (bgn, A, 1, E, rv, Qm, 0)).cpu().numpy()
+    cfg = in_config(bgn, A, 1, E, rv, Qm, 0)
+    for i in list(range(min(n, 8))) + list(range(max(n - 2, 0), n)):
+        assert np.array_equal(out[i], oracle.encode(pay[i], cfg)), i
+
+
+def test_encode_refuses_a_payload_beyond_the_code(cuda, lib):
+    """B is kept in 16 bits: A = 65520 wraps to B = 8, which no code block can carry."""
+    with pytest.raises(RuntimeError):
+        ldpc_encode(torch.zeros((1, 65520 // 8), dtype=torch.uint8, device=cuda), (1, 65520, 1, 960, 0, 2, 0))
