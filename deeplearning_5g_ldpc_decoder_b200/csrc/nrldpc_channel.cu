@@ -56,12 +56,17 @@ __constant__ Seg kQam256[4][15] = {
 };
 __constant__ int kQam256N[4] = {15, 14, 12, 8};
 
-__device__ __forceinline__ float seg_llr(const Seg* seg, int n, float r, float A, float nv) {
-  int k = 0;
-  while (k < n - 1 && !(r < __fmul_rn(seg[k].thr, A))) ++k;
-  const Seg s = seg[k];
-  const float lin = __fadd_rn(__fmul_rn(s.s, r), __fmul_rn(s.c2, A));
-  return __fdiv_rn(__fmul_rn(__fmul_rn(s.c1, A), lin), nv);
+// x / nv, correctly rounded.  kFast: from r = RN(1 / nv), two remainder steps
+// (Markstein's theorem: with a correctly rounded reciprocal and a quotient
+// within an ulp, q + r (x - q nv) in fused operations rounds correctly).  The
+// host asks for it only where neither the reciprocal nor a remainder can leave
+// the normal range.
+template <bool kFast>
+__device__ __forceinline__ float div_nv(float x, float nv, float r) {
+  if constexpr (!kFast) return __fdiv_rn(x, nv);
+  float q = __fmul_rn(x, r);
+  q = __fmaf_rn(__fmaf_rn(-q, nv, x), r, q);
+  return __fmaf_rn(__fmaf_rn(-q, nv, x), r, q);
 }
 
 __device__ __forceinline__ int16_t quantize(float llr) {
@@ -78,75 +83,160 @@ __device__ __forceinline__ uint64_t splitmix(uint64_t z) {
   return z ^ (z >> 31);
 }
 
-__device__ __forceinline__ float bsign(uint32_t b) { return b ? -1.0f : 1.0f; }
+// PAM cell of r for 2^m levels spaced 2A: the number of boundaries
+// (2 c - 2^m) A, c = 1 .. 2^m - 1, that r is not below.  The estimate from a
+// multiply is off by one at most and is settled by the boundaries themselves.
+template <int m>
+__device__ __forceinline__ int pam_cell(float r, float A, float inv_2a) {
+  constexpr int n = 1 << m;
+  int c = (int)floorf(__fmaf_rn(r, inv_2a, (float)(n / 2)));
+  c = min(max(c, 0), n - 1);
+  if (c > 0 && r < __fmul_rn((float)(2 * c - n), A)) {
+    --c;
+  } else if (c < n - 1 && !(r < __fmul_rn((float)(2 * c + 2 - n), A))) {
+    ++c;
+  }
+  return c;
+}
 
-__global__ void channel_kernel(const uint8_t* __restrict__ rm, int64_t rm_stride, int32_t num_cw, int32_t E,
-                               int32_t Qm, float nv, float sigma, float A, uint64_t seed,
-                               int16_t* __restrict__ llr, int64_t llr_stride, float* __restrict__ symbols) {
-  const int64_t nsym = E / Qm;
-  const int64_t total = nsym * (int64_t)num_cw;
-  for (int64_t g = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; g < total; g += (int64_t)gridDim.x * blockDim.x) {
-    const int64_t cw = g / nsym, s = g - cw * nsym;
-    const uint8_t* in = rm + cw * rm_stride;
-    uint32_t b[8];
-    for (int j = 0; j < Qm; ++j) {
-      const int64_t t = s * Qm + j;
-      b[j] = (in[t >> 3] >> (7 - (t & 7))) & 1u;
+constexpr int kChannelThreads = 256;
+constexpr int kGroup = 4;   // symbols per thread and step
+
+// One thread takes four consecutive symbols: their 4 Qm bits start on a nibble,
+// and their 4 Qm LLRs are one run of 8 Qm bytes, stored 16 bytes at a time
+// where rows are aligned (kVec).  Every pair's max-log line is looked up by
+// the PAM cell of the coordinate (one cell per coordinate serves all Qm / 2
+// pairs) in a shared table of 8-byte entries, at most 16 per pair, which no
+// lane pattern makes conflict; the division by the noise power, the same for
+// every LLR, is a multiplication and two remainder steps.  Bound by
+// instruction issue: the counter generator's four 64-bit products, logf, sqrtf
+// and sincospif per symbol, then about 15 instructions per LLR.
+// 2048 x 25344 LLRs, 64QAM: 286 us with one symbol per thread, a search of the
+// segments in constant memory and 2-byte stores, 107 us in this form.
+template <int Qm, bool kFast>
+__global__ void __launch_bounds__(kChannelThreads) channel_kernel(const uint8_t* __restrict__ rm, int64_t rm_stride, int32_t num_cw, int32_t E,
+                               float nv, float sigma, float A, uint64_t seed,
+                               int16_t* __restrict__ llr, int64_t llr_stride, float* __restrict__ symbols, bool vec) {
+  constexpr int m = Qm > 2 ? Qm / 2 : 1, kCells = 1 << m;
+  // per pair and cell: s c1 A and c2 A of the line (c1 A) (s r + c2 A); c1 A > 0
+  __shared__ float2 s_line[m][kCells];
+  if constexpr (Qm > 2) {
+    for (int k = threadIdx.x; k < m * kCells; k += blockDim.x) {
+      const int p = k / kCells, c = k - p * kCells;
+      const Seg* seg = Qm == 4 ? kQam16[p & 1] : Qm == 6 ? kQam64[p % 3] : kQam256[p & 3];
+      const int n = Qm == 4 ? kQam16N[p & 1] : Qm == 6 ? kQam64N[p % 3] : kQam256N[p & 3];
+      int j = 0;
+      while (j < n - 1 && seg[j].thr <= (float)(2 * c - kCells)) ++j;   // segments the cell lies above
+      s_line[p][c] = make_float2(copysignf(__fmul_rn(seg[j].c1, A), seg[j].s), __fmul_rn(seg[j].c2, A));
     }
-    float re, im;
-    if (Qm == 1) {
-      re = im = __fmul_rn(bsign(b[0]), A);
-    } else if (Qm == 2) {
-      re = __fmul_rn(bsign(b[0]), A);
-      im = __fmul_rn(bsign(b[1]), A);
-    } else if (Qm == 4) {
-      re = __fmul_rn(__fmul_rn(bsign(b[0]), __fsub_rn(2.0f, bsign(b[2]))), A);
-      im = __fmul_rn(__fmul_rn(bsign(b[1]), __fsub_rn(2.0f, bsign(b[3]))), A);
-    } else if (Qm == 6) {
-      re = __fmul_rn(__fmul_rn(bsign(b[0]), __fsub_rn(4.0f, __fmul_rn(bsign(b[2]), __fsub_rn(2.0f, bsign(b[4]))))), A);
-      im = __fmul_rn(__fmul_rn(bsign(b[1]), __fsub_rn(4.0f, __fmul_rn(bsign(b[3]), __fsub_rn(2.0f, bsign(b[5]))))), A);
+    __syncthreads();
+  }
+  const float rnv = kFast ? __frcp_rn(nv) : 0.0f;
+  const float inv_2a = 0.5f / A;
+  const uint32_t nsym = (uint32_t)(E / Qm);
+  const uint32_t groups = (nsym + kGroup - 1) / kGroup;
+  const uint64_t total = (uint64_t)groups * (uint64_t)num_cw;
+  for (uint64_t g = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; g < total; g += (uint64_t)gridDim.x * blockDim.x) {
+    const uint32_t cw = total <= 0xFFFFFFFFull ? (uint32_t)g / groups : (uint32_t)(g / groups);
+    const uint32_t gi = (uint32_t)(g - (uint64_t)cw * groups);
+    const uint32_t s0 = gi * kGroup;
+    const uint32_t left = min((uint32_t)kGroup, nsym - s0);
+    // the group's 4 Qm bits, first bit on top (bits past E are not used)
+    uint32_t word = 0u;
+    {
+      const uint8_t* in = rm + (int64_t)cw * rm_stride;
+      const uint32_t byte0 = (uint32_t)(((uint64_t)s0 * Qm) >> 3);
+      const uint32_t nbytes = (uint32_t)(((uint64_t)E + 7) >> 3);
+#pragma unroll
+      for (int j = 0; j < (4 * Qm + 7) / 8; ++j)
+        if (byte0 + j < nbytes) word |= (uint32_t)__ldg(in + byte0 + j) << (24 - 8 * j);
+      if (Qm == 1 && (gi & 1u)) word <<= 4;
+    }
+    uint32_t q[2 * Qm];   // 4 Qm int16 LLRs
+#pragma unroll
+    for (int i = 0; i < kGroup; ++i) {
+      const auto sign = [&](int j) { return (int32_t)(word << (i * Qm + j)) < 0 ? -1.0f : 1.0f; };   // 1 - 2 b_j
+      float re, im;
+      if constexpr (Qm == 1) {
+        re = im = __fmul_rn(sign(0), A);
+      } else if constexpr (Qm == 2) {
+        re = __fmul_rn(sign(0), A);
+        im = __fmul_rn(sign(1), A);
+      } else if constexpr (Qm == 4) {
+        re = __fmul_rn(__fmul_rn(sign(0), __fsub_rn(2.0f, sign(2))), A);
+        im = __fmul_rn(__fmul_rn(sign(1), __fsub_rn(2.0f, sign(3))), A);
+      } else if constexpr (Qm == 6) {
+        re = __fmul_rn(__fmul_rn(sign(0), __fsub_rn(4.0f, __fmul_rn(sign(2), __fsub_rn(2.0f, sign(4))))), A);
+        im = __fmul_rn(__fmul_rn(sign(1), __fsub_rn(4.0f, __fmul_rn(sign(3), __fsub_rn(2.0f, sign(5))))), A);
+      } else {
+        re = __fmul_rn(__fmul_rn(sign(0), __fsub_rn(8.0f, __fmul_rn(sign(2), __fsub_rn(4.0f,
+                       __fmul_rn(sign(4), __fsub_rn(2.0f, sign(6))))))), A);
+        im = __fmul_rn(__fmul_rn(sign(1), __fsub_rn(8.0f, __fmul_rn(sign(3), __fsub_rn(4.0f,
+                       __fmul_rn(sign(5), __fsub_rn(2.0f, sign(7))))))), A);
+      }
+      // Box-Muller from a counter-based generator.
+      const uint64_t z = splitmix(seed ^ splitmix(((uint64_t)cw << 32) ^ (uint64_t)(s0 + i)));
+      const float u1 = ((float)(z >> 40) + 1.0f) * (1.0f / 16777218.0f);
+      const float u2 = ((float)((z >> 16) & 0xFFFFFFu) + 1.0f) * (1.0f / 16777218.0f);
+      const float rad = sqrtf(-2.0f * logf(u1));
+      float sn, cs;
+      sincospif(2.0f * u2, &sn, &cs);
+      re = __fadd_rn(re, __fmul_rn(sigma, __fmul_rn(rad, cs)));
+      im = __fadd_rn(im, __fmul_rn(sigma, __fmul_rn(rad, sn)));
+      if (symbols && (uint32_t)i < left) {
+        float* o = symbols + 2 * ((int64_t)cw * nsym + s0 + i);
+        o[0] = re;
+        o[1] = im;
+      }
+      const auto put = [&](int j, int16_t v) {   // LLR j of symbol i
+        const int k = i * Qm + j;
+        if (k & 1) q[k >> 1] |= (uint32_t)(uint16_t)v << 16;
+        else q[k >> 1] = (uint32_t)(uint16_t)v;
+      };
+      if constexpr (Qm == 1) {
+        put(0, quantize(div_nv<kFast>(__fmul_rn(__fmul_rn(4.0f, __fadd_rn(re, im)), A), nv, rnv)));
+      } else if constexpr (Qm == 2) {
+        put(0, quantize(div_nv<kFast>(__fmul_rn(__fmul_rn(4.0f, re), A), nv, rnv)));
+        put(1, quantize(div_nv<kFast>(__fmul_rn(__fmul_rn(4.0f, im), A), nv, rnv)));
+      } else {
+        const int cr = pam_cell<m>(re, A, inv_2a), ci = pam_cell<m>(im, A, inv_2a);
+#pragma unroll
+        for (int p = 0; p < m; ++p) {
+          const float2 lr = s_line[p][cr], li = s_line[p][ci];
+          const float xr = __fmul_rn(fabsf(lr.x), __fadd_rn(__fmul_rn(copysignf(1.0f, lr.x), re), lr.y));
+          const float xi = __fmul_rn(fabsf(li.x), __fadd_rn(__fmul_rn(copysignf(1.0f, li.x), im), li.y));
+          put(2 * p, quantize(div_nv<kFast>(xr, nv, rnv)));
+          put(2 * p + 1, quantize(div_nv<kFast>(xi, nv, rnv)));
+        }
+      }
+    }
+    int16_t* out = llr + (int64_t)cw * llr_stride + (int64_t)s0 * Qm;
+    if (vec && left == kGroup) {
+      if constexpr (Qm == 1) {
+        *reinterpret_cast<uint2*>(out) = make_uint2(q[0], q[1]);
+      } else {
+#pragma unroll
+        for (int k = 0; k < Qm / 2; ++k)
+          reinterpret_cast<uint4*>(out)[k] = make_uint4(q[4 * k], q[4 * k + 1], q[4 * k + 2], q[4 * k + 3]);
+      }
     } else {
-      re = __fmul_rn(__fmul_rn(bsign(b[0]), __fsub_rn(8.0f, __fmul_rn(bsign(b[2]), __fsub_rn(4.0f,
-                     __fmul_rn(bsign(b[4]), __fsub_rn(2.0f, bsign(b[6]))))))), A);
-      im = __fmul_rn(__fmul_rn(bsign(b[1]), __fsub_rn(8.0f, __fmul_rn(bsign(b[3]), __fsub_rn(4.0f,
-                     __fmul_rn(bsign(b[5]), __fsub_rn(2.0f, bsign(b[7]))))))), A);
-    }
-    // Box-Muller from a counter-based generator.
-    const uint64_t z = splitmix(seed ^ splitmix(((uint64_t)cw << 32) ^ (uint64_t)s));
-    const float u1 = ((float)(z >> 40) + 1.0f) * (1.0f / 16777218.0f);
-    const float u2 = ((float)((z >> 16) & 0xFFFFFFu) + 1.0f) * (1.0f / 16777218.0f);
-    const float rad = sqrtf(-2.0f * logf(u1));
-    float sn, cs;
-    sincospif(2.0f * u2, &sn, &cs);
-    re = __fadd_rn(re, __fmul_rn(sigma, __fmul_rn(rad, cs)));
-    im = __fadd_rn(im, __fmul_rn(sigma, __fmul_rn(rad, sn)));
-    if (symbols) {
-      symbols[2 * g] = re;
-      symbols[2 * g + 1] = im;
-    }
-    int16_t* out = llr + cw * llr_stride + s * Qm;
-    if (Qm == 1) {
-      out[0] = quantize(__fdiv_rn(__fmul_rn(__fmul_rn(4.0f, __fadd_rn(re, im)), A), nv));
-    } else if (Qm == 2) {
-      out[0] = quantize(__fdiv_rn(__fmul_rn(__fmul_rn(4.0f, re), A), nv));
-      out[1] = quantize(__fdiv_rn(__fmul_rn(__fmul_rn(4.0f, im), A), nv));
-    } else if (Qm == 4) {
-      for (int p = 0; p < 2; ++p) {
-        out[2 * p] = quantize(seg_llr(kQam16[p], kQam16N[p], re, A, nv));
-        out[2 * p + 1] = quantize(seg_llr(kQam16[p], kQam16N[p], im, A, nv));
-      }
-    } else if (Qm == 6) {
-      for (int p = 0; p < 3; ++p) {
-        out[2 * p] = quantize(seg_llr(kQam64[p], kQam64N[p], re, A, nv));
-        out[2 * p + 1] = quantize(seg_llr(kQam64[p], kQam64N[p], im, A, nv));
-      }
-    } else {
-      for (int p = 0; p < 4; ++p) {
-        out[2 * p] = quantize(seg_llr(kQam256[p], kQam256N[p], re, A, nv));
-        out[2 * p + 1] = quantize(seg_llr(kQam256[p], kQam256N[p], im, A, nv));
-      }
+#pragma unroll
+      for (int k = 0; k < kGroup * Qm; ++k)
+        if ((uint32_t)k < left * Qm) out[k] = (int16_t)(q[k >> 1] >> (16 * (k & 1)));
     }
   }
+}
+
+template <int Qm>
+void launch_channel_qm(bool fast, int grid, cudaStream_t s, const uint8_t* rm, int64_t rm_stride, int32_t num_cw,
+                       int32_t E, float nv, float sigma, float A, uint64_t seed, int16_t* llr, int64_t llr_stride,
+                       float* symbols, bool vec) {
+  if (fast)
+    channel_kernel<Qm, true><<<grid, kChannelThreads, 0, s>>>(rm, rm_stride, num_cw, E, nv, sigma, A, seed, llr,
+                                                              llr_stride, symbols, vec);
+  else
+    channel_kernel<Qm, false><<<grid, kChannelThreads, 0, s>>>(rm, rm_stride, num_cw, E, nv, sigma, A, seed, llr,
+                                                               llr_stride, symbols, vec);
 }
 
 }  // namespace
@@ -154,15 +244,29 @@ __global__ void channel_kernel(const uint8_t* __restrict__ rm, int64_t rm_stride
 int launch_channel(const uint8_t* rm, int64_t rm_stride, int32_t num_cw, int32_t E, int32_t Qm, float nv,
                    float sigma, float A, uint64_t seed, int16_t* llr, int64_t llr_stride, float* symbols,
                    void* stream) {
-  const int64_t total = (int64_t)(E / Qm) * num_cw;
+  const int64_t groups = ((int64_t)(E / Qm) + kGroup - 1) / kGroup;
+  const int64_t total = groups * num_cw;
   if (total == 0) return 0;
   int dev = 0, sms = 0;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  const int64_t want = (total + 255) / 256;
+  const int64_t want = (total + kChannelThreads - 1) / kChannelThreads;
   const int grid = (int)(want < 16LL * sms ? want : 16LL * sms);
-  channel_kernel<<<grid, 256, 0, reinterpret_cast<cudaStream_t>(stream)>>>(rm, rm_stride, num_cw, E, Qm, nv, sigma,
-                                                                           A, seed, llr, llr_stride, symbols);
+  // Remainder-step division: with nv in this range the reciprocal is normal,
+  // quotients of the coordinates' magnitudes (below 2^32) stay finite, and the
+  // remainder of any quotient that does not quantise to 0 is normal.
+  const bool fast = nv > 0x1p-60f && nv < 0x1p60f;
+  // 8-byte runs for BPSK, 16-byte ones otherwise
+  const int align = Qm == 1 ? 8 : 16;
+  const bool vec = reinterpret_cast<uintptr_t>(llr) % align == 0 && (num_cw == 1 || (llr_stride * 2) % align == 0);
+  cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
+  switch (Qm) {
+    case 1: launch_channel_qm<1>(fast, grid, s, rm, rm_stride, num_cw, E, nv, sigma, A, seed, llr, llr_stride, symbols, vec); break;
+    case 2: launch_channel_qm<2>(fast, grid, s, rm, rm_stride, num_cw, E, nv, sigma, A, seed, llr, llr_stride, symbols, vec); break;
+    case 4: launch_channel_qm<4>(fast, grid, s, rm, rm_stride, num_cw, E, nv, sigma, A, seed, llr, llr_stride, symbols, vec); break;
+    case 6: launch_channel_qm<6>(fast, grid, s, rm, rm_stride, num_cw, E, nv, sigma, A, seed, llr, llr_stride, symbols, vec); break;
+    default: launch_channel_qm<8>(fast, grid, s, rm, rm_stride, num_cw, E, nv, sigma, A, seed, llr, llr_stride, symbols, vec); break;
+  }
   count_launch();
   return (int)cudaGetLastError();
 }

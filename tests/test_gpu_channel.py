@@ -106,3 +106,33 @@ def test_device_front_end_matches_reference_functions(cuda, reflib, Qm):
         llr, sym = channel_llrs(torch.from_numpy(rm).to(cuda), E, Qm, noise_db, seed=3, return_symbols=True)
         want = reflib.demap_symbols(sym.cpu().numpy(), Qm, noise_db)
         assert np.array_equal(llr.cpu().numpy().reshape(-1), want), noise_db
+
+
+@pytest.mark.parametrize("Qm", [1, 2, 4, 6, 8])
+@pytest.mark.parametrize("symbols,n,shift", [(1, 1, 0), (5, 3, 0), (7, 9, 1), (64, 2, 3), (4099, 5, 0), (40001, 40, 0)])
+def test_channel_edges_match_host_demapper(cuda, lib, monkeypatch, Qm, symbols, n, shift):
+    """Partial groups of four symbols, LLR rows off the 16-byte grid, every division path (a noise power whose
+    reciprocal is not in the fast range included): LLRs equal the host restatement on the reported symbols."""
+    # numpy's cast of a float beyond int64 (-200 dB) has no defined value: clip the LLR well outside the int16 range first
+    plain = channel_ref.quantize
+    monkeypatch.setattr(channel_ref, "quantize", lambda llr: plain(np.clip(llr, np.float32(-1e4), np.float32(1e4))))
+    # the noise power is the C library's powf (as in the reference); numpy's float32 power is an ulp off at -7.25 dB
+    libm = ctypes.CDLL("libm.so.6")
+    libm.powf.restype, libm.powf.argtypes = ctypes.c_float, [ctypes.c_float, ctypes.c_float]
+    amp = channel_ref.constants(Qm, 0.0)[0]
+    monkeypatch.setattr(channel_ref, "constants", lambda _, db: (
+        amp, np.float32(libm.powf(10.0, float(np.float32(db) / np.float32(10.0))))))
+    E = symbols * Qm if symbols < 40000 else symbols // 8 * Qm
+    rng = np.random.default_rng(symbols + Qm)
+    rm = torch.from_numpy(rng.integers(0, 256, size=(n, (E + 7) // 8), dtype=np.uint8)).to(cuda)
+    for noise_db in (-200.0, -21.5, -7.25, 6.0):
+        buf = torch.full((n, E + 8), 77, dtype=torch.int16, device=cuda)
+        sym = torch.zeros((n, E // Qm, 2), dtype=torch.float32, device=cuda)
+        rc = lib.nrldpc_channel_batch(rm.data_ptr(), rm.shape[1], n, E, Qm, ctypes.c_float(noise_db), 9,
+                                      buf.data_ptr() + 2 * shift, E + 8, sym.data_ptr(),
+                                      torch.cuda.current_stream().cuda_stream)
+        assert rc == 0
+        got = buf.cpu().numpy()
+        want = channel_ref.demap(sym.cpu().numpy(), Qm, noise_db).reshape(n, E)
+        assert np.array_equal(got[:, shift:shift + E], want), noise_db
+        assert (got[:, :shift] == 77).all() and (got[:, shift + E:] == 77).all()
