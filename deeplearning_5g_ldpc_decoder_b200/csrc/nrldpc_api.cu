@@ -831,35 +831,40 @@ int32_t nrldpc_decode_batch_host(const int16_t* h_llr, int64_t llr_stride, int32
   uint8_t* d_bits = static_cast<uint8_t*>(hs.bits.ptr);
   int32_t* d_stat = static_cast<int32_t*>(hs.stat.ptr);
   int32_t* d_iters = static_cast<int32_t*>(hs.iters.ptr);
+  // Copies from or to pageable memory hold the calling thread, so a chunk's
+  // decode is enqueued right after its copy in, and nothing is copied out before
+  // every decode is enqueued: with the copies out between the decodes, each
+  // chunk ran alone when the results went to pageable arrays (2048 BG1 Zc=384
+  // blocks, pinned LLRs, numpy results: 5.10 -> 3.12 ms).
   for (int k = 0; k < nchunks; ++k) {
     const int64_t c0 = cuts[k], n = cuts[k + 1] - cuts[k];
     const size_t off = (size_t)c0 * (size_t)llr_stride;
+    cudaStream_t comp = hs.comp[k & 3];
     if (cudaMemcpyAsync(d_llr + off, h_llr + off, sizeof(int16_t) * (size_t)n * (size_t)llr_stride,
                         cudaMemcpyHostToDevice, hs.copy) != cudaSuccess ||
-        cudaEventRecord(hs.h2d[k], hs.copy) != cudaSuccess)
+        cudaEventRecord(hs.h2d[k], hs.copy) != cudaSuccess || cudaStreamWaitEvent(comp, hs.h2d[k], 0) != cudaSuccess)
       return NRLDPC_ERR_CUDA;
+    const int32_t rc = decode_batch_locked(d_llr + off, llr_stride, (int32_t)n, inconfig, decoder_cfg,
+                                           d_bits + (size_t)c0 * (size_t)bits_stride, bits_stride, d_stat + c0,
+                                           d_iters + c0, nullptr, 0, nullptr, 0, comp);
+    if (rc != NRLDPC_OK) return rc;
+    if (cudaEventRecord(hs.dec[k], comp) != cudaSuccess) return NRLDPC_ERR_CUDA;
   }
   for (int k = 0; k < nchunks; ++k) {
     const int64_t c0 = cuts[k], n = cuts[k + 1] - cuts[k];
-    cudaStream_t comp = hs.comp[k & 3];
-    if (cudaStreamWaitEvent(comp, hs.h2d[k], 0) != cudaSuccess) return NRLDPC_ERR_CUDA;
-    const int32_t rc = decode_batch_locked(d_llr + (size_t)c0 * (size_t)llr_stride, llr_stride, (int32_t)n, inconfig,
-                                           decoder_cfg, d_bits + (size_t)c0 * (size_t)bits_stride, bits_stride,
-                                           d_stat + c0, d_iters + c0, nullptr, 0, nullptr, 0, comp);
-    if (rc != NRLDPC_OK) return rc;
-    if (cudaEventRecord(hs.dec[k], comp) != cudaSuccess || cudaStreamWaitEvent(hs.copy, hs.dec[k], 0) != cudaSuccess)
-      return NRLDPC_ERR_CUDA;
+    if (cudaStreamWaitEvent(hs.copy, hs.dec[k], 0) != cudaSuccess) return NRLDPC_ERR_CUDA;
     if (decoder_cfg->max_iterations > 0 &&
         cudaMemcpyAsync(h_hardbits + (size_t)c0 * (size_t)bits_stride, d_bits + (size_t)c0 * (size_t)bits_stride,
                         (size_t)n * (size_t)bits_stride, cudaMemcpyDeviceToHost, hs.copy) != cudaSuccess)
       return NRLDPC_ERR_CUDA;
-    if (h_status && cudaMemcpyAsync(h_status + c0, d_stat + c0, sizeof(int32_t) * (size_t)n, cudaMemcpyDeviceToHost,
-                                    hs.copy) != cudaSuccess)
-      return NRLDPC_ERR_CUDA;
-    if (h_iterations && cudaMemcpyAsync(h_iterations + c0, d_iters + c0, sizeof(int32_t) * (size_t)n,
-                                        cudaMemcpyDeviceToHost, hs.copy) != cudaSuccess)
-      return NRLDPC_ERR_CUDA;
   }
+  // status and iterations of all chunks: one copy each, after the last chunk's bits
+  if (h_status &&
+      cudaMemcpyAsync(h_status, d_stat, sizeof(int32_t) * (size_t)num_cw, cudaMemcpyDeviceToHost, hs.copy) != cudaSuccess)
+    return NRLDPC_ERR_CUDA;
+  if (h_iterations && cudaMemcpyAsync(h_iterations, d_iters, sizeof(int32_t) * (size_t)num_cw, cudaMemcpyDeviceToHost,
+                                      hs.copy) != cudaSuccess)
+    return NRLDPC_ERR_CUDA;
   if (cudaStreamSynchronize(hs.copy) != cudaSuccess) return NRLDPC_ERR_CUDA;
   return NRLDPC_OK;
 }
