@@ -37,6 +37,7 @@ SOURCES = [
     "nrldpc_noalloc.cu",
     "nrldpc_tb.cu",
     "nrldpc_train.cu",
+    "nrldpc_train_tape.cu",
     "nrldpc_tables.cpp",
 ]
 HEADERS = [

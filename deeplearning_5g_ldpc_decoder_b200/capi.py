@@ -132,6 +132,9 @@ EXPORTED_SYMBOLS = (
     "nrldpc_train_forward_f64",
     "nrldpc_train_backward_f64",
     "nrldpc_train_checkpoint_words",
+    "nrldpc_train_tape_floats",
+    "nrldpc_train_forward_tape",
+    "nrldpc_train_backward_tape",
     "nrldpc_set_trained_weights",
     "nrldpc_set_degree_alpha",
     "nrldpc_mixed_plan_create",
@@ -220,6 +223,13 @@ def _declare(lib: ctypes.CDLL) -> None:
     lib.nrldpc_train_checkpoint_words.argtypes = [ctypes.POINTER(LdpcInConfig), i32, i32, i32,
                                                   ctypes.POINTER(ctypes.c_int64), ctypes.POINTER(ctypes.c_int64)]
     lib.nrldpc_train_checkpoint_words.restype = i32
+    lib.nrldpc_train_tape_floats.argtypes = [ctypes.POINTER(LdpcInConfig), i32, i32, ctypes.POINTER(ctypes.c_int64)]
+    lib.nrldpc_train_tape_floats.restype = i32
+    lib.nrldpc_train_forward_tape.argtypes = [vp, i32, ctypes.POINTER(LdpcInConfig), i32, vp, vp, f32, vp, vp, vp, vp]
+    lib.nrldpc_train_forward_tape.restype = i32
+    lib.nrldpc_train_backward_tape.argtypes = [vp, i32, ctypes.POINTER(LdpcInConfig), i32, vp, vp, f32, i32, vp, vp,
+                                               vp, vp, vp, vp, vp]
+    lib.nrldpc_train_backward_tape.restype = i32
     lib.nrldpc_encode_batch_ncb.argtypes = [vp, i64, i32, ctypes.POINTER(LdpcInConfig), i32, vp, i64, vp]
     lib.nrldpc_encode_batch_ncb.restype = i32
     lib.nrldpc_tb_segment.argtypes = [ctypes.POINTER(TbDesc), ctypes.POINTER(TbInfo)]

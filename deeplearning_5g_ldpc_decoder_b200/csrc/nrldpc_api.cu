@@ -671,6 +671,82 @@ int train_backward(const void* d_llr, int32_t batch, const ldpc_in_config_t* cfg
   return launch_train_backward(p, f64, grid, block, smem_b, stream) == 0 ? NRLDPC_OK : NRLDPC_ERR_CUDA;
 }
 
+constexpr int kTapeSmemCap = 227 * 1024 - 1024;   // opt-in shared memory per block, less the static reduction buffer
+constexpr int kTapeAccCap = 16 * 1024;            // of it for the backward's alpha / beta sums
+
+// Parameters of the tape-keeping training kernels for one configuration.
+int make_tape_params(const ldpc_in_config_t* cfg, int32_t T, int32_t batch, float clip, TrainTapeParams* p) {
+  CodeParams cp;
+  if (!cfg || derive_params(*cfg, &cp, true) != 0) return NRLDPC_ERR_CONFIG;
+  if (T < 1 || batch < 0) return NRLDPC_ERR_ARG;
+  memset(p, 0, sizeof(*p));
+  const BaseGraph& g = base_graph(cp.bgn);
+  p->Zc = cp.Zc;
+  p->R = g.rows;
+  p->n = cp.lq_len;
+  p->nnz = g.nnz;
+  p->T = T;
+  p->batch = batch;
+  p->clip = clip > 0.0f ? clip : INFINITY;
+  p->tape_words = (int64_t)g.nnz * cp.Zc;
+  for (int e = 0; e < g.nnz; ++e)
+    p->edge[e] = (uint32_t)g.col[e] * (uint32_t)cp.Zc | ((uint32_t)(g.vij[cp.iLS][e] % cp.Zc) << 16);
+  for (int r = 0; r <= g.rows; ++r) p->row_off[r] = g.row_off[r];
+  return NRLDPC_OK;
+}
+
+// Code blocks per CTA (G) and CTAs per SM.  A dozen blocks with barriers of
+// their own hide each other's latency, so the smallest G wins whose CTAs keep
+// the most code blocks on an SM (G > 1 pays where Zc leaves a warp partly
+// empty), and never more than spreading the batch over the SMs needs.  Sets
+// p->G, p->acc, *block and *smem; returns the CTAs per SM.
+int pick_tape_groups(DeviceState* st, TrainTapeParams* p, bool backward, int* block, int* smem) {
+  p->acc = backward && 2 * p->T * p->R * 4 <= kTapeAccCap;
+  const int acc = p->acc ? 2 * p->T * p->R * 4 : 0;
+  const int spread = std::max(1, (p->batch + st->num_sms - 1) / std::max(1, st->num_sms));
+  const int gmax = std::max(1, std::min(kThreadsTarget / p->Zc, spread));
+  int best_g = 0, best_cw = 0, best_occ = 0;
+  for (int G = 1; G <= gmax; ++G) {
+    const int bytes = G * p->n * 4 + acc;
+    if (bytes > kTapeSmemCap) break;
+    const int blk = (G * p->Zc + 31) & ~31;
+    const uint64_t key = (backward ? 5ull : 4ull) << 56 | (uint64_t)(p->R == NRLDPC_BG2_ROWS) << 48 | (uint64_t)blk << 32 |
+                         (uint64_t)(uint32_t)bytes;
+    auto hit = st->occupancy.find(key);
+    if (hit == st->occupancy.end())
+      hit = st->occupancy.emplace(key, occupancy_train_tape(backward, p->R == NRLDPC_BG2_ROWS, blk, bytes)).first;
+    if (hit->second * G > best_cw) {
+      best_cw = hit->second * G;
+      best_g = G;
+      best_occ = hit->second;
+    }
+  }
+  if (best_g == 0) return 0;
+  p->G = best_g;
+  *block = (best_g * p->Zc + 31) & ~31;
+  *smem = best_g * p->n * 4 + acc;
+  return best_occ;
+}
+
+// Shared end of the two tape entry points (the buffers are set in p).
+int launch_tape_kernel(TrainTapeParams* p, bool backward, void* stream) {
+  std::lock_guard<std::mutex> lock(g_mu);
+  DeviceState* st = nullptr;
+  if (device_state(&st) != 0) return NRLDPC_ERR_CUDA;
+  int block, smem;
+  const int occ = pick_tape_groups(st, p, backward, &block, &smem);
+  if (occ < 1) return NRLDPC_ERR_CUDA;
+  const int items = (p->batch + p->G - 1) / p->G;
+  const int grid = std::max(1, std::min(items, occ * st->num_sms));
+  if (backward) {
+    p->carry_per_cta = (int64_t)p->G * p->tape_words;
+    Buffer& b = st->train_scratch[reinterpret_cast<cudaStream_t>(stream)];
+    if (ensure(&b, sizeof(float) * (size_t)grid * (size_t)p->carry_per_cta)) return NRLDPC_ERR_CUDA;
+    p->carry = static_cast<float*>(b.ptr);
+  }
+  return launch_train_tape(*p, backward, grid, block, smem, stream) == 0 ? NRLDPC_OK : NRLDPC_ERR_CUDA;
+}
+
 }  // namespace
 
 void count_launch() { g_launches.fetch_add(1, std::memory_order_relaxed); }
@@ -1045,6 +1121,53 @@ int32_t nrldpc_train_checkpoint_words(const ldpc_in_config_t* cfg, int32_t itera
   if (lq_elems) *lq_elems = (int64_t)iterations * batch * p.n;
   if (msg_words) *msg_words = (int64_t)iterations * batch * p.R * p.msg_words;
   return NRLDPC_OK;
+}
+
+int32_t nrldpc_train_tape_floats(const ldpc_in_config_t* cfg, int32_t iterations, int32_t batch, int64_t* floats) {
+  TrainTapeParams p;
+  const int rc = make_tape_params(cfg, iterations, batch, 0.0f, &p);
+  if (rc != NRLDPC_OK) return rc;
+  if (floats) *floats = (int64_t)iterations * batch * p.tape_words;
+  return NRLDPC_OK;
+}
+
+int32_t nrldpc_train_forward_tape(const float* d_llr, int32_t batch, const ldpc_in_config_t* cfg, int32_t iterations,
+                                  const float* d_alpha, const float* d_beta, float clip, float* d_final, float* d_iter,
+                                  float* d_tape, void* stream) {
+  TrainTapeParams p;
+  const int rc = make_tape_params(cfg, iterations, batch, clip, &p);
+  if (rc != NRLDPC_OK) return rc;
+  if (batch == 0) return NRLDPC_OK;
+  if (!d_llr || !d_alpha || !d_beta || !d_final || !d_tape) return NRLDPC_ERR_ARG;
+  p.llr = d_llr;
+  p.alpha = d_alpha;
+  p.beta = d_beta;
+  p.final_llr = d_final;
+  p.iter_llr = d_iter;
+  p.tape = d_tape;
+  return launch_tape_kernel(&p, false, stream);
+}
+
+int32_t nrldpc_train_backward_tape(const float* d_llr, int32_t batch, const ldpc_in_config_t* cfg, int32_t iterations,
+                                   const float* d_alpha, const float* d_beta, float clip, int32_t detach,
+                                   const float* d_tape, const float* d_g_final, const float* d_g_iter, float* d_g_llr,
+                                   float* d_g_alpha, float* d_g_beta, void* stream) {
+  TrainTapeParams p;
+  const int rc = make_tape_params(cfg, iterations, batch, clip, &p);
+  if (rc != NRLDPC_OK) return rc;
+  if (batch == 0) return NRLDPC_OK;
+  if (!d_llr || !d_alpha || !d_beta || !d_tape || !d_g_llr || !d_g_alpha || !d_g_beta) return NRLDPC_ERR_ARG;
+  p.llr = d_llr;
+  p.alpha = d_alpha;
+  p.beta = d_beta;
+  p.detach = detach ? 1 : 0;
+  p.tape = const_cast<float*>(d_tape);
+  p.g_final = d_g_final;
+  p.g_iter = d_g_iter;
+  p.g_llr = d_g_llr;
+  p.g_alpha = d_g_alpha;
+  p.g_beta = d_g_beta;
+  return launch_tape_kernel(&p, true, stream);
 }
 
 }  // extern "C"

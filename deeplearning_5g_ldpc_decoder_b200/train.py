@@ -7,10 +7,10 @@ alpha sharing modes (single / checkpoint / degree, sigmoid-bounded to
 [alpha_min, alpha_max]), sigmoid-bounded beta per [iteration, row], optional
 LLR clipping and detached check-update inputs, and the same forward outputs.
 The decoder itself runs in two hand-written CUDA kernels wrapped in
-``MinSumUnrolled`` (a ``torch.autograd.Function``): the forward keeps one
-checkpoint of the decoder state per iteration and the backward recomputes each
-iteration from its checkpoint while back-propagating, instead of storing every
-intermediate tensor.
+``MinSumUnrolled`` (a ``torch.autograd.Function``): the float32 forward keeps a
+tape of every edge's extrinsic input, from which the backward back-propagates
+without recomputing anything; in float64 the forward keeps one checkpoint of the
+decoder state per iteration and the backward recomputes each iteration from it.
 
 ``export_int16_tables`` turns learned alpha / beta into the int16 tables of the
 fixed-point decoders (algo 2: per [iteration, row]; algo 3: per degree).
@@ -50,6 +50,16 @@ def checkpoint_sizes(cfg: capi.LdpcInConfig, T: int, batch: int, f64: bool) -> T
     return int(lq.value), int(msg.value)
 
 
+def tape_size(cfg: capi.LdpcInConfig, T: int, batch: int) -> int:
+    """Floats of the float32 training tape."""
+    lib = capi.load_library()
+    n = ctypes.c_int64(0)
+    rc = lib.nrldpc_train_tape_floats(ctypes.byref(cfg), T, batch, ctypes.byref(n))
+    if rc != 0:
+        raise ValueError(f"configuration not supported by the training kernels (float32): {rc}")
+    return int(n.value)
+
+
 class MinSumUnrolled(torch.autograd.Function):
     """(llr [batch, n], alpha [T, R], beta [T, R]) -> (final [batch, n], per-iteration [T, batch, n]).
 
@@ -69,20 +79,23 @@ class MinSumUnrolled(torch.autograd.Function):
         if beta_tab.shape != (T, R):
             raise ValueError("alpha and beta tables must both be [iterations, rows]")
         dev = llr.device
-        lq_elems, msg_words = checkpoint_sizes(cfg, T, batch, f64)
         final = torch.empty_like(llr)
         iters = torch.empty((T, batch, n), dtype=dt, device=dev) if want_iters else None
-        ck_lq = torch.empty(lq_elems, dtype=dt, device=dev)
-        ck_lr = torch.empty(max(msg_words, 2), dtype=torch.int32, device=dev)
         stream = ctypes.c_void_p(torch.cuda.current_stream(dev).cuda_stream)
-        fn = lib.nrldpc_train_forward_f64 if f64 else lib.nrldpc_train_forward
-        clip_arg = (ctypes.c_double if f64 else ctypes.c_float)(clip or INF_CLIP)
+        if f64:
+            lq_elems, msg_words = checkpoint_sizes(cfg, T, batch, True)
+            kept = (torch.empty(lq_elems, dtype=dt, device=dev),
+                    torch.empty(max(msg_words, 2), dtype=torch.int32, device=dev))
+            fn, clip_arg = lib.nrldpc_train_forward_f64, ctypes.c_double(clip or INF_CLIP)
+        else:
+            kept = (torch.empty(tape_size(cfg, T, batch), dtype=dt, device=dev),)
+            fn, clip_arg = lib.nrldpc_train_forward_tape, ctypes.c_float(clip or INF_CLIP)
         with torch.cuda.device(dev):
             rc = fn(_vp(llr), batch, ctypes.byref(cfg), T, _vp(alpha_tab), _vp(beta_tab), clip_arg, _vp(final),
-                    _vp(iters), _vp(ck_lq), _vp(ck_lr), stream)
+                    _vp(iters), *[_vp(k) for k in kept], stream)
         if rc != 0:
             raise RuntimeError(f"nrldpc_train_forward failed: {rc}")
-        ctx.save_for_backward(llr, alpha_tab, beta_tab, ck_lq, ck_lr)
+        ctx.save_for_backward(llr, alpha_tab, beta_tab, *kept)
         ctx.cfg = (cfg.bgn, cfg.A, cfg.crctype, cfg.E, cfg.rv, cfg.Qm, cfg.HARQ_on)
         ctx.clip = clip
         ctx.detach = detach
@@ -94,7 +107,7 @@ class MinSumUnrolled(torch.autograd.Function):
     @staticmethod
     def backward(ctx, g_final, g_iters):
         lib = capi.load_library()
-        llr, alpha_tab, beta_tab, ck_lq, ck_lr = ctx.saved_tensors
+        llr, alpha_tab, beta_tab, *kept = ctx.saved_tensors
         cfg = _cfg(ctx.cfg)
         f64 = llr.dtype == torch.float64
         T, R = alpha_tab.shape
@@ -107,11 +120,11 @@ class MinSumUnrolled(torch.autograd.Function):
         gi = (g_iters.contiguous().to(llr.dtype)
               if (g_iters is not None and g_iters.numel() == T * batch * n) else None)
         stream = ctypes.c_void_p(torch.cuda.current_stream(dev).cuda_stream)
-        fn = lib.nrldpc_train_backward_f64 if f64 else lib.nrldpc_train_backward
+        fn = lib.nrldpc_train_backward_f64 if f64 else lib.nrldpc_train_backward_tape
         clip_arg = (ctypes.c_double if f64 else ctypes.c_float)(ctx.clip or INF_CLIP)
         with torch.cuda.device(dev):
             rc = fn(_vp(llr), batch, ctypes.byref(cfg), T, _vp(alpha_tab), _vp(beta_tab), clip_arg, int(ctx.detach),
-                    _vp(ck_lq), _vp(ck_lr), _vp(gf), _vp(gi), _vp(g_llr), _vp(g_alpha), _vp(g_beta), stream)
+                    *[_vp(k) for k in kept], _vp(gf), _vp(gi), _vp(g_llr), _vp(g_alpha), _vp(g_beta), stream)
         if rc != 0:
             raise RuntimeError(f"nrldpc_train_backward failed: {rc}")
         return g_llr, g_alpha, g_beta, None, None, None, None
@@ -255,11 +268,11 @@ class NeuralLayeredMinSumDecoder(nn.Module):
 
     def memory_summary(self, batch_size: int, dtype_bytes: int = 4) -> dict:
         """Decoder state per batch in MB (reference convention: LQ + one message per
-        edge), plus what the training kernels keep: one checkpoint of LQ and of the
-        compressed messages (4 words per lifted row) per iteration."""
+        edge), plus what the float32 training kernels keep for the backward: the tape
+        of every edge's extrinsic input, per iteration."""
         lq = batch_size * self.n
         lr = batch_size * sum(self.row_degrees) * self.Zc
-        ck = self.num_iterations * batch_size * (self.n + 4 * self.num_rows * self.Zc)
+        ck = self.num_iterations * lr
         mb = 1024.0 * 1024.0
         return {"LQ_MB": lq * dtype_bytes / mb, "Lr_MB": lr * dtype_bytes / mb,
                 "total_message_MB": (lq + lr) * dtype_bytes / mb, "checkpoint_MB": ck * 4 / mb}

@@ -475,6 +475,22 @@ int32_t nrldpc_train_checkpoint_words(const ldpc_in_config_t *cfg, int32_t itera
                                       int32_t batch, int32_t f64, int64_t *lq_elems,
                                       int64_t *msg_words);
 
+/* The float32 pair again, with the same values and gradients, keeping the tape
+ * (the extrinsic input of every edge and iteration, *floats of them, from
+ * nrldpc_train_tape_floats) instead of the checkpoints: the backward recomputes
+ * nothing.  d_tape is written by the forward and read by the backward; its
+ * layout is the library's own.  Unlike the checkpoint form, the backward keeps
+ * nothing in d_g_llr between iterations, which may be d_g_final. */
+int32_t nrldpc_train_tape_floats(const ldpc_in_config_t *cfg, int32_t iterations, int32_t batch, int64_t *floats);
+int32_t nrldpc_train_forward_tape(const float *d_llr, int32_t batch, const ldpc_in_config_t *cfg,
+                                  int32_t iterations, const float *d_alpha, const float *d_beta, float clip,
+                                  float *d_final, float *d_iter, float *d_tape, void *stream);
+int32_t nrldpc_train_backward_tape(const float *d_llr, int32_t batch, const ldpc_in_config_t *cfg,
+                                   int32_t iterations, const float *d_alpha, const float *d_beta, float clip,
+                                   int32_t detach, const float *d_tape, const float *d_g_final,
+                                   const float *d_g_iter, float *d_g_llr, float *d_g_alpha, float *d_g_beta,
+                                   void *stream);
+
 /* Replace the per-(iteration, row) alpha/beta tables used by algo 2 for one
  * base graph (the reference compiles these in:
  * c_lib/BG1_trained_ldpc_weights.c:34,171, c_lib/BG2_trained_ldpc_weights.c).

@@ -269,3 +269,57 @@ def test_learned_tables_decode_bit_exact_vs_c(cuda, oracle):
         set_degree_alpha(None)
         oracle.set_trained(2, None)
         oracle.set_degree_alpha(None)
+
+
+def _checkpoint_form(cfg, x, a, b, clip, detach, gf, gi):
+    """Forward and gradients through the checkpoint entry points of the C ABI."""
+    import ctypes
+
+    from deeplearning_5g_ldpc_decoder_b200 import capi
+    from deeplearning_5g_ldpc_decoder_b200.train import checkpoint_sizes
+
+    lib, c = capi.load_library(), capi.make_in_config(*cfg)
+    T, batch = a.shape[0], x.shape[0]
+    lq, msg = checkpoint_sizes(c, T, batch, False)
+    ck = [torch.empty(lq, device="cuda"), torch.empty(msg, dtype=torch.int32, device="cuda")]
+    fin, its = torch.empty_like(x), torch.empty((T, *x.shape), device="cuda")
+    gx, ga, gb = torch.empty_like(x), torch.zeros_like(a), torch.zeros_like(b)
+    s, v = torch.cuda.current_stream().cuda_stream, [t.data_ptr() for t in (x, a, b, fin, its, *ck, gf, gi, gx, ga, gb)]
+    assert lib.nrldpc_train_forward(v[0], batch, ctypes.byref(c), T, v[1], v[2], clip or 0.0, v[3], v[4], v[5], v[6],
+                                    s) == 0
+    assert lib.nrldpc_train_backward(v[0], batch, ctypes.byref(c), T, v[1], v[2], clip or 0.0, int(detach), v[5], v[6],
+                                     v[7], v[8], v[9], v[10], v[11], s) == 0
+    return fin, its, gx, ga, gb
+
+
+@pytest.mark.parametrize("cfg,T,batch,clip,detach", [
+    ((2, 8, 1, 96, 0, 2, 0), 3, 1, None, False),          # a few rows per warp
+    ((2, 40, 1, 200, 0, 2, 0), 2, 5, 6.0, False),         # Zc 11: slices off the 16-byte grid
+    ((2, 40, 1, 200, 0, 2, 0), 60, 700, None, True),      # gradient sums that do not fit shared memory; several blocks per CTA
+    ((2, 488, 1, 1920, 0, 2, 0), 1, 2500, None, True),    # one iteration, more blocks than CTAs in flight
+    ((1, 600, 1, 1500, 0, 2, 0), 4, 33, 9.0, True),       # BG1, Zc 30
+    ((1, 2440, 1, 7392, 0, 2, 0), 3, 1900, None, False),  # BG1, Zc 112: a warp partly empty
+    ((1, 8424, 1, 25344, 0, 2, 0), 2, 3, 12.0, False),    # the largest block
+])
+def test_tape_form_matches_checkpoint_form(cuda, cfg, T, batch, clip, detach):
+    """The tape-keeping kernels against the checkpoint kernels on the same inputs: values equal bit for bit, gradients
+    to 1e-4 of the largest (the two sum a row's gradients in different orders)."""
+    from deeplearning_5g_ldpc_decoder_b200 import capi
+    from deeplearning_5g_ldpc_decoder_b200.train import MinSumUnrolled
+
+    p = capi.gen_ldpc_parameters(capi.make_in_config(*cfg))
+    n, R = p.N + 2 * p.Zc, capi.BG_ROWS[p.bgn]
+    g = torch.Generator(device="cuda").manual_seed(batch + T)
+    x = torch.randn((batch, n), device="cuda", generator=g) * 4 + 3
+    x[:, : 2 * p.Zc] = 0.0                                 # punctured columns start at exact zeros
+    a = torch.rand((T, R), device="cuda", generator=g) * 0.4 + 0.5
+    b = torch.rand((T, R), device="cuda", generator=g) * 0.1
+    gf = torch.randn((batch, n), device="cuda", generator=g)
+    gi = torch.randn((T, batch, n), device="cuda", generator=g) * 0.1
+    leaves = [t.clone().requires_grad_(True) for t in (x, a, b)]
+    fin, its = MinSumUnrolled.apply(*leaves, cfg, clip, detach, True)
+    torch.autograd.backward([fin, its], [gf, gi])
+    want = _checkpoint_form(cfg, x, a, b, clip, detach, gf, gi)
+    assert torch.equal(fin, want[0]) and torch.equal(its, want[1])
+    for got, ref in zip([t.grad for t in leaves], want[2:]):
+        assert (got - ref).abs().max().item() <= 1e-4 * ref.abs().max().item() + 1e-12
