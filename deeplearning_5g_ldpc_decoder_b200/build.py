@@ -35,6 +35,7 @@ SOURCES = [
     "nrldpc_mixed.cu",
     "nrldpc_mixed_api.cu",
     "nrldpc_noalloc.cu",
+    "nrldpc_split.cu",
     "nrldpc_tb.cu",
     "nrldpc_train.cu",
     "nrldpc_train_tape.cu",

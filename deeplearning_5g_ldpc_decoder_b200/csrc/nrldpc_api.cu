@@ -198,13 +198,24 @@ struct Plan {
   int grid, block, smem;
   int clip;   // check-node arithmetic variant of the fixed-point kernel (fixed_clip_mode)
   int algo;
+  bool split;        // the small-batch kernel: one code block per CTA, no scratch
+  SplitShape shape;
   size_t scratch_bytes;
 };
+
+// CTAs per SM of a kernel, asked from the driver once per key (kernel and launch shape).
+template <typename F>
+int cached_occupancy(DeviceState* st, uint64_t key, F ask) {
+  auto hit = st->occupancy.find(key);
+  if (hit == st->occupancy.end()) hit = st->occupancy.emplace(key, ask()).first;
+  return hit->second;
+}
 
 // Fill the launch parameters of one uniform batch.
 int make_plan(const CodeParams& cp, const ldpc_decoder_cfg_t& dc, int num_cw, DeviceState* st, Plan* plan) {
   DecodeParams& p = plan->p;
   memset(&p, 0, sizeof(p));
+  plan->split = false;
   const BaseGraph& g = base_graph(cp.bgn);
   p.Zc = cp.Zc;
   p.R = g.rows;
@@ -275,6 +286,25 @@ int make_plan(const CodeParams& cp, const ldpc_decoder_cfg_t& dc, int num_cw, De
   p.f_max = (float)dc.max_llr / 128.0f;
   p.f_min = (float)dc.min_llr / 128.0f;
   plan->clip = fixed_clip_mode(dc, p.w_inline, g.rows);
+  // The small-batch kernel while all blocks run at once.  Measured, 8 iterations,
+  // pair kernel / small-batch kernel in us: BG1 Zc 24, 1 to 148 blocks 230 / 108,
+  // 444 (three per SM, its last) 234 / 136, 888 in two rounds 236 / 265; BG2 Zc 64,
+  // 64 blocks 155 / 86, 444 155 / 132, 592 155 / 197; BG1 Zc 112, 148 blocks
+  // 246 / 148, 149 246 / 288; BG1 Zc 208, 148 blocks 308 / 273, 149 308 / 541.
+  if (fixed && num_cw <= 32 * st->num_sms) {
+    split_layout(g, p.lr_off);
+    if (split_shape(cp.Zc, g.cols, (int)(p.lr_off[g.rows] & 0xFFFFu), &plan->shape)) {
+      const uint64_t key = 6ull << 56 | (uint64_t)plan->clip << 48 | (uint64_t)plan->shape.table << 47 |
+                           (uint64_t)plan->shape.block << 32 | (uint64_t)(uint32_t)plan->shape.smem;
+      const int occ = cached_occupancy(st, key, [&] { return occupancy_split(plan->shape, plan->clip); });
+      if (num_cw <= occ * st->num_sms) {
+        plan->split = true;
+        plan->grid = p.num_items = num_cw;
+        plan->scratch_bytes = 0;
+        return 0;
+      }
+    }
+  }
 
   // Scratch layout per CTA, layer by layer.
   uint32_t off = 0;
@@ -297,20 +327,10 @@ int make_plan(const CodeParams& cp, const ldpc_decoder_cfg_t& dc, int num_cw, De
 
   const uint64_t key = ((uint64_t)(fixed ? 1 : algo == 4 ? 2 : 3) << 56) | ((uint64_t)(fixed ? plan->clip : 0) << 48) |
                        ((uint64_t)plan->block << 32) | (uint64_t)(uint32_t)plan->smem;
-  int occ;
-  auto hit = st->occupancy.find(key);
-  if (hit != st->occupancy.end()) {
-    occ = hit->second;
-  } else {
-    if (fixed) {
-      occ = occupancy_fixed(plan->block, plan->smem, plan->clip, true);
-    } else if (algo == 4) {
-      occ = occupancy_float_minsum(plan->block, plan->smem);
-    } else {
-      occ = occupancy_float_bp(plan->block, plan->smem);
-    }
-    st->occupancy[key] = occ;
-  }
+  int occ = cached_occupancy(st, key, [&] {
+    if (fixed) return occupancy_fixed(plan->block, plan->smem, plan->clip, true);
+    return algo == 4 ? occupancy_float_minsum(plan->block, plan->smem) : occupancy_float_bp(plan->block, plan->smem);
+  });
   if (occ < 1) occ = 1;
   plan->grid = std::min(p.num_items, occ * st->num_sms);
   if (plan->grid < 1) plan->grid = 1;
@@ -319,6 +339,7 @@ int make_plan(const CodeParams& cp, const ldpc_decoder_cfg_t& dc, int num_cw, De
 }
 
 int launch_plan(Plan* plan, void* stream) {
+  if (plan->split) return launch_split(plan->p, plan->shape, plan->clip, stream);
   switch (plan->algo) {
     case 1:
     case 2:
@@ -362,9 +383,9 @@ int32_t decode_batch_locked(const int16_t* d_llr, int64_t llr_stride, int32_t nu
   if (make_plan(cp, *dc, num_cw, st, &plan) != 0) return NRLDPC_ERR_CUDA;
   uint32_t* scratch = nullptr;
   cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
-  if (scratch_for(st, s, plan.scratch_bytes, &scratch) != 0) return NRLDPC_ERR_CUDA;
+  if (!plan.split && scratch_for(st, s, plan.scratch_bytes, &scratch) != 0) return NRLDPC_ERR_CUDA;
   DecodeParams& p = plan.p;
-  if (p.num_items > plan.grid) {
+  if (!plan.split && p.num_items > plan.grid) {
     // More than one wave: work comes from the stream's queue (zeroed once,
     // rewound by each launch's last CTA): fixed point refills half lanes from
     // it, the float kernels take work items from it.  Within one wave there is
@@ -712,13 +733,12 @@ int pick_tape_groups(DeviceState* st, TrainTapeParams* p, bool backward, int* bl
     const int blk = (G * p->Zc + 31) & ~31;
     const uint64_t key = (backward ? 5ull : 4ull) << 56 | (uint64_t)(p->R == NRLDPC_BG2_ROWS) << 48 | (uint64_t)blk << 32 |
                          (uint64_t)(uint32_t)bytes;
-    auto hit = st->occupancy.find(key);
-    if (hit == st->occupancy.end())
-      hit = st->occupancy.emplace(key, occupancy_train_tape(backward, p->R == NRLDPC_BG2_ROWS, blk, bytes)).first;
-    if (hit->second * G > best_cw) {
-      best_cw = hit->second * G;
+    const int occ =
+        cached_occupancy(st, key, [&] { return occupancy_train_tape(backward, p->R == NRLDPC_BG2_ROWS, blk, bytes); });
+    if (occ * G > best_cw) {
+      best_cw = occ * G;
       best_g = G;
-      best_occ = hit->second;
+      best_occ = occ;
     }
   }
   if (best_g == 0) return 0;
@@ -980,8 +1000,8 @@ int32_t nrldpc_bounds_check_status(uint32_t* out, int32_t reset) {
   if (!out) return NRLDPC_ERR_ARG;
   out[0] = out[1] = out[2] = out[3] = 0u;
   if (!kBoundsChecked) return 0;
-  // first record among the kernels' translation units (fixed-point, float, mixed)
-  int (*readers[3])(uint32_t*, bool) = {bounds_read_fixed, bounds_read_float, bounds_read_mixed};
+  // first record among the kernels' translation units (fixed-point, small-batch, float, mixed)
+  int (*readers[4])(uint32_t*, bool) = {bounds_read_fixed, bounds_read_split, bounds_read_float, bounds_read_mixed};
   for (auto rd : readers) {
     uint32_t r[4];
     if (rd(r, reset != 0) != 0) return NRLDPC_ERR_CUDA;

@@ -65,5 +65,6 @@ constexpr bool kBoundsChecked = false;
 int bounds_read_fixed(uint32_t* out, bool reset);
 int bounds_read_float(uint32_t* out, bool reset);
 int bounds_read_mixed(uint32_t* out, bool reset);
+int bounds_read_split(uint32_t* out, bool reset);
 
 }  // namespace nrldpc

@@ -59,6 +59,13 @@ __device__ __forceinline__ uint32_t scale_pair(uint32_t c, int32_t alpha0, int32
   return scale_half(lo, alpha0, beta0) | (scale_half(hi, alpha1, beta1) << 16);
 }
 
+// The same with beta = 0, alpha >= 0 and both halves in [0, 32767]: (2 alpha m +
+// 2^15) >> 16 is (alpha m + 2^14) >> 15, and the shift is a byte permute.
+__device__ __forceinline__ uint32_t scale_open(uint32_t m, int32_t alpha) {
+  const uint32_t a2 = 2u * (uint32_t)alpha;
+  return __byte_perm((m & 0xFFFFu) * a2 + 0x8000u, (m >> 16) * a2 + 0x8000u, 0x7632);
+}
+
 // clip_llr (c_lib/fixedpoint_ldpc_decoder.c:28-36) of the exact int32 sum, for
 // configurations with min_llr > max_llr where clamping is not a min/max pair.
 __device__ __forceinline__ uint32_t clip_half_degen(int32_t v, int32_t mx, int32_t mn) {

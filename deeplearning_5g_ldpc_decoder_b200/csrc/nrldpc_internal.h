@@ -277,6 +277,16 @@ int launch_channel(const uint8_t* rm, int64_t rm_stride, int32_t num_cw, int32_t
                    float sigma, float A, uint64_t seed, int16_t* llr, int64_t llr_stride, float* symbols,
                    void* stream);
 int launch_fixed(const DecodeParams& p, int grid, int block, int smem, int clip_mode, void* stream);
+// The small-batch fixed-point kernel (nrldpc_split.cu): one code block per CTA.
+// In its DecodeParams lr_off is what split_layout writes.
+struct SplitShape {
+  int words, slots, block, smem;   // words of beliefs, message slots, threads, dynamic shared memory
+  bool table;                      // the slots' addresses are kept in shared memory
+};
+void split_layout(const BaseGraph& g, uint32_t* lr_off);
+bool split_shape(int Zc, int cols, int slots, SplitShape* out);   // false: does not fit an SM
+int launch_split(const DecodeParams& p, const SplitShape& s, int clip_mode, void* stream);
+int occupancy_split(const SplitShape& s, int clip_mode);
 int launch_float_minsum(const DecodeParams& p, int grid, int block, int smem, void* stream);
 int launch_float_bp(const DecodeParams& p, int grid, int block, int smem, void* stream);
 
