@@ -12,8 +12,8 @@
 //
 // Mapping: one code block per group of Zc threads, up to G = floor(384 / Zc) groups
 // per CTA, FP32 beliefs in shared memory, persistent grid.  Min-sum messages
-// are stored compressed per lifted check row (two minima, flip bits, the
-// minimum's position: 16 bytes); BP messages are stored per edge.
+// are stored compressed per lifted check row (two minima, one word of flip bits
+// and the minimum's position: 12 bytes); BP messages are stored per edge.
 #include <cuda_runtime.h>
 #include <float.h>
 #include <math.h>
@@ -54,42 +54,56 @@ __device__ __forceinline__ void st_lq(const DecodeParams& p, float* lq, uint32_t
 }
 
 // ---------------------------------------------------------------- float min-sum
-// Stored message of a lifted check row (4 planes): new_min1, new_min2 (float
-// bits), bit j = message of edge j negated, bit j = edge j carries new_min2.
-template <int D>
-__device__ __forceinline__ void fms_row(const DecodeParams& p, float* __restrict__ lq, uint32_t zx, int e0,
-                                        bool first, uint32_t* __restrict__ lrp, int NT) {
-  float n1 = 0.f, n2 = 0.f;
-  uint32_t xf = 0u, xi = 0u;
-  if (!first) {
-    n1 = __uint_as_float(lrp[0]);
-    n2 = __uint_as_float(lrp[NT]);
-    xf = lrp[2 * NT];
-    xi = lrp[3 * NT];
-  }
+// The edge table again as byte offsets {column * Zc * 4, (V mod Zc) * 4}, staged
+// by the min-sum kernel: an address is then three instructions.
+__shared__ uint2 s_fedge4[kMaxNnz];
+
+// Stored message of a lifted check row (3 planes): new_min1, new_min2 (float
+// bits), and a word with edge j's sign flip in bit D - 1 - j and the position of
+// new_min2's edge from bit 20.  The kernel loads a row's words while the row
+// before it computes.
+struct FloatMsg {
+  float n1, n2;
+  uint32_t f;
+};
+
+// One row, operation for operation as the reference.  A belief of -0.0 counts as
+// positive there (`< 0`), so signs are taken from v + 0.0f, whose sign bit is set
+// exactly where v < 0; then parity, flip and the sign of a message are bit
+// operations on sign bits.  The ALU pipe bounds the kernel (76 % busy, 25 of 45
+// instructions per edge).  8 iterations of 4096 blocks BG1 Zc=384: 6.91 -> 6.29 ms,
+// 777 blocks BG1 Zc=208 957 -> 877 us, against bit tests and compares on values
+// and messages loaded where the row starts.  Address adds as multiply-adds on the
+// FMA pipe: 6.51 ms and 869 us, because of spills at Zc=384, and not used.
+// kRange: min_llr <= max_llr, so the clip is a min and a max.
+template <int D, bool kRange>
+__device__ __forceinline__ void fms_row(const DecodeParams& p, char* __restrict__ lq, uint32_t zx4, int e0,
+                                        const FloatMsg& old, uint32_t* __restrict__ lrp, int NT) {
   if (!NRLDPC_INBOUNDS(e0 + D - 1, kMaxNnz, kBoundsEdge)) return;   // debug build
+  const uint32_t zc4 = 4u * (uint32_t)p.Zc;
+  [[maybe_unused]] const uint32_t limit = 4u * (uint32_t)p.lq_len;   // bytes of beliefs (debug build)
+  const int ix = (int)(old.f >> 20);
   float rel[D];
   uint32_t addr[D];
   float m1 = FLT_MAX, m2 = FLT_MAX;
   int idx = 0;
-  bool neg = false;
+  uint32_t sg = 0u;
 #pragma unroll
   for (int j = 0; j < D; ++j) {
-    addr[j] = edge_addr(p, e0 + j, zx);
-    float r = ((xi >> j) & 1u) ? n2 : n1;
-    r = ((xf >> j) & 1u) ? -r : r;
-    const float v = __fsub_rn(ld_lq(p, lq, addr[j]), r);
+    const uint2 e = s_fedge4[e0 + j];
+    const uint32_t t = e.y + zx4;
+    addr[j] = min(t, t - zc4) + e.x;
+    const float q = NRLDPC_INBOUNDS(addr[j], limit, kBoundsLq) ? *reinterpret_cast<const float*>(lq + addr[j]) : 0.0f;
+    const uint32_t r = __float_as_uint(j == ix ? old.n2 : old.n1) ^ ((old.f << (32 - D + j)) & 0x80000000u);
+    const float v = __fsub_rn(q, __uint_as_float(r));
     rel[j] = v;
-    neg ^= (v < 0.0f);
+    sg ^= __float_as_uint(__fadd_rn(v, 0.0f));
     const float a = fabsf(v);
     // float_update_two_minima (:171-180): strict <, first index wins.
-    if (a < m1) {
-      m2 = m1;
-      m1 = a;
-      idx = j;
-    } else if (a < m2) {
-      m2 = a;
-    }
+    const bool lt = a < m1;
+    m2 = lt ? m1 : fminf(m2, a);
+    m1 = fminf(m1, a);
+    idx = lt ? j : idx;
   }
   const float c1 = clipf(m1, p.f_max, 0.0f);
   const float c2 = clipf(m2, p.f_max, 0.0f);
@@ -99,33 +113,33 @@ __device__ __forceinline__ void fms_row(const DecodeParams& p, float* __restrict
   o2 = o2 < 0.0f ? 0.0f : o2;
   const float s1 = __fmul_rn(p.f_alpha, o1);
   const float s2 = __fmul_rn(p.f_alpha, o2);
-  uint32_t XF = 0u;
+  uint32_t flips = 0u;
 #pragma unroll
   for (int j = 0; j < D; ++j) {
-    const float nv = (j == idx) ? s2 : s1;
-    const bool flip = (rel[j] < 0.0f) != neg;
-    const float msg = flip ? -nv : nv;      // edge_sign * new_val, edge_sign = +-1
-    XF |= (flip ? 1u : 0u) << j;
-    st_lq(p, lq, addr[j], clipf(__fadd_rn(rel[j], msg), p.f_max, p.f_min));
+    const uint32_t f = __float_as_uint(__fadd_rn(rel[j], 0.0f)) ^ sg;   // sign bit: the message is negated
+    flips = __funnelshift_l(f, flips, 1);
+    const uint32_t msg = __float_as_uint(j == idx ? s2 : s1) ^ (f & 0x80000000u);
+    const float v = __fadd_rn(rel[j], __uint_as_float(msg));
+    if (NRLDPC_INBOUNDS(addr[j], limit, kBoundsLq))
+      *reinterpret_cast<float*>(lq + addr[j]) = kRange ? fminf(fmaxf(v, p.f_min), p.f_max) : clipf(v, p.f_max, p.f_min);
   }
   lrp[0] = __float_as_uint(s1);
   lrp[NT] = __float_as_uint(s2);
-  lrp[2 * NT] = XF;
-  lrp[3 * NT] = 1u << idx;
+  lrp[2 * NT] = flips | (uint32_t)idx << 20;
 }
 
-__device__ __forceinline__ void fms_dispatch(int deg, const DecodeParams& p, float* lq, uint32_t zx, int e0,
-                                             bool first, uint32_t* lrp, int NT) {
+template <bool kRange>
+__device__ __forceinline__ void fms_dispatch(int deg, const DecodeParams& p, char* lq, uint32_t zx4, int e0, const FloatMsg& old, uint32_t* lrp, int NT) {
   switch (deg) {
-    case 3: fms_row<3>(p, lq, zx, e0, first, lrp, NT); break;
-    case 4: fms_row<4>(p, lq, zx, e0, first, lrp, NT); break;
-    case 5: fms_row<5>(p, lq, zx, e0, first, lrp, NT); break;
-    case 6: fms_row<6>(p, lq, zx, e0, first, lrp, NT); break;
-    case 7: fms_row<7>(p, lq, zx, e0, first, lrp, NT); break;
-    case 8: fms_row<8>(p, lq, zx, e0, first, lrp, NT); break;
-    case 9: fms_row<9>(p, lq, zx, e0, first, lrp, NT); break;
-    case 10: fms_row<10>(p, lq, zx, e0, first, lrp, NT); break;
-    default: fms_row<19>(p, lq, zx, e0, first, lrp, NT); break;
+    case 3: fms_row<3, kRange>(p, lq, zx4, e0, old, lrp, NT); break;
+    case 4: fms_row<4, kRange>(p, lq, zx4, e0, old, lrp, NT); break;
+    case 5: fms_row<5, kRange>(p, lq, zx4, e0, old, lrp, NT); break;
+    case 6: fms_row<6, kRange>(p, lq, zx4, e0, old, lrp, NT); break;
+    case 7: fms_row<7, kRange>(p, lq, zx4, e0, old, lrp, NT); break;
+    case 8: fms_row<8, kRange>(p, lq, zx4, e0, old, lrp, NT); break;
+    case 9: fms_row<9, kRange>(p, lq, zx4, e0, old, lrp, NT); break;
+    case 10: fms_row<10, kRange>(p, lq, zx4, e0, old, lrp, NT); break;
+    default: fms_row<19, kRange>(p, lq, zx4, e0, old, lrp, NT); break;
   }
 }
 
@@ -294,11 +308,19 @@ __device__ void emit_float_block(const DecodeParams& p, const float* lq, int zx,
   }
 }
 
-template <bool kBP>
+// Kernel variants: belief propagation, min-sum with min_llr <= max_llr, min-sum otherwise.
+enum { kFloatBp = 0, kFloatRange = 1, kFloatDegen = 2 };
+
+template <int kMode>
 __global__ void __launch_bounds__(kThreadsTarget, 2) float_kernel(const __grid_constant__ DecodeParams p) {
+  constexpr bool kBP = kMode == kFloatBp;
   extern __shared__ __align__(16) float s_lqf[];     // [G][lq_len]
   __shared__ uint32_t s_crc[kMaxGroups];
-  for (int e = threadIdx.x; e < kMaxNnz; e += blockDim.x) s_fedge[e] = p.edge[e];   // read after the first barrier
+  // read after the first barrier
+  for (int e = threadIdx.x; e < kMaxNnz; e += blockDim.x) {
+    if (kBP) s_fedge[e] = p.edge[e];
+    else s_fedge4[e] = p.edge_cs4[e];
+  }
   // BP: per row, the 16-byte-aligned part of the next row's message slice
   // (row 0 of the next iteration after the last row) as {byte offset from the
   // CTA's scratch, bytes}, for the bulk L2 prefetch in the row loop.
@@ -356,6 +378,7 @@ __global__ void __launch_bounds__(kThreadsTarget, 2) float_kernel(const __grid_c
     __syncthreads();
 
     int it = 0;
+    FloatMsg nxt{0.0f, 0.0f, 0u};   // row 0 of the first iteration: zero messages
     for (; it < p.max_it; ++it) {
       for (int row = 0; row < p.R; ++row) {
         if (active) {
@@ -377,7 +400,13 @@ __global__ void __launch_bounds__(kThreadsTarget, 2) float_kernel(const __grid_c
           if (kBP) {
             bp_dispatch(deg, p, lq, (uint32_t)zx, e0, it == 0, lrp, NT);
           } else {
-            fms_dispatch(deg, p, lq, (uint32_t)zx, e0, it == 0, lrp, NT);
+            const FloatMsg cur = nxt;
+            const bool wrap = row + 1 == p.R;
+            if (wrap || it > 0) {
+              const uint32_t* m = scratch + p.lr_off[wrap ? 0 : row + 1] + tid;
+              nxt = FloatMsg{__uint_as_float(m[0]), __uint_as_float(m[NT]), m[2 * NT]};
+            }
+            fms_dispatch<kMode == kFloatRange>(deg, p, reinterpret_cast<char*>(lq), 4u * (uint32_t)zx, e0, cur, lrp, NT);
           }
         }
         __syncthreads();
@@ -469,17 +498,20 @@ int occupancy_impl(K kernel, std::atomic<uint32_t>* attr_done, int block, int sm
 
 }  // namespace
 
-static std::atomic<uint32_t> g_attr_minsum{0}, g_attr_bp{0};   // raise_smem_limit_once, per kernel
+static std::atomic<uint32_t> g_attr[3];   // raise_smem_limit_once, per kernel
 
 int launch_float_minsum(const DecodeParams& p, int grid, int block, int smem, void* stream) {
-  return launch_impl(float_kernel<false>, &g_attr_minsum, p, grid, block, smem, stream);
+  return p.f_min <= p.f_max ? launch_impl(float_kernel<kFloatRange>, &g_attr[kFloatRange], p, grid, block, smem, stream)
+                            : launch_impl(float_kernel<kFloatDegen>, &g_attr[kFloatDegen], p, grid, block, smem, stream);
 }
 int launch_float_bp(const DecodeParams& p, int grid, int block, int smem, void* stream) {
-  return launch_impl(float_kernel<true>, &g_attr_bp, p, grid, block, smem, stream);
+  return launch_impl(float_kernel<kFloatBp>, &g_attr[kFloatBp], p, grid, block, smem, stream);
 }
 int bounds_read_float(uint32_t* out, bool reset) { return bounds_read_tu(out, reset); }
 
-int occupancy_float_minsum(int block, int smem) { return occupancy_impl(float_kernel<false>, &g_attr_minsum, block, smem); }
-int occupancy_float_bp(int block, int smem) { return occupancy_impl(float_kernel<true>, &g_attr_bp, block, smem); }
+int occupancy_float_minsum(int block, int smem) {
+  return occupancy_impl(float_kernel<kFloatRange>, &g_attr[kFloatRange], block, smem);
+}
+int occupancy_float_bp(int block, int smem) { return occupancy_impl(float_kernel<kFloatBp>, &g_attr[kFloatBp], block, smem); }
 
 }  // namespace nrldpc
