@@ -12,7 +12,7 @@
 #include <utility>
 #include <vector>
 
-#include <math.h>
+#include <cmath>
 
 #include "nrldpc_bounds.cuh"
 #include "nrldpc_internal.h"
@@ -692,7 +692,7 @@ int train_backward(const void* d_llr, int32_t batch, const ldpc_in_config_t* cfg
   return launch_train_backward(p, f64, grid, block, smem_b, stream) == 0 ? NRLDPC_OK : NRLDPC_ERR_CUDA;
 }
 
-constexpr int kTapeSmemCap = 227 * 1024 - 1024;   // opt-in shared memory per block, less the static reduction buffer
+constexpr int kTapeSmemCap = 227 * 1024 - 1024;   // opt-in shared memory per block, less the static row table
 constexpr int kTapeAccCap = 16 * 1024;            // of it for the backward's alpha / beta sums
 
 // Parameters of the tape-keeping training kernels for one configuration.
@@ -711,7 +711,7 @@ int make_tape_params(const ldpc_in_config_t* cfg, int32_t T, int32_t batch, floa
   p->clip = clip > 0.0f ? clip : INFINITY;
   p->tape_words = (int64_t)g.nnz * cp.Zc;
   for (int e = 0; e < g.nnz; ++e)
-    p->edge[e] = (uint32_t)g.col[e] * (uint32_t)cp.Zc | ((uint32_t)(g.vij[cp.iLS][e] % cp.Zc) << 16);
+    p->edge4[e] = make_uint2(4u * (uint32_t)g.col[e] * (uint32_t)cp.Zc, 4u * (uint32_t)(g.vij[cp.iLS][e] % cp.Zc));
   for (int r = 0; r <= g.rows; ++r) p->row_off[r] = g.row_off[r];
   return NRLDPC_OK;
 }
@@ -724,27 +724,29 @@ int make_tape_params(const ldpc_in_config_t* cfg, int32_t T, int32_t batch, floa
 int pick_tape_groups(DeviceState* st, TrainTapeParams* p, bool backward, int* block, int* smem) {
   p->acc = backward && 2 * p->T * p->R * 4 <= kTapeAccCap;
   const int acc = p->acc ? 2 * p->T * p->R * 4 : 0;
+  const bool clipped = std::isfinite(p->clip);
   const int spread = std::max(1, (p->batch + st->num_sms - 1) / std::max(1, st->num_sms));
   const int gmax = std::max(1, std::min(kThreadsTarget / p->Zc, spread));
   int best_g = 0, best_cw = 0, best_occ = 0;
   for (int G = 1; G <= gmax; ++G) {
-    const int bytes = G * p->n * 4 + acc;
-    if (bytes > kTapeSmemCap) break;
     const int blk = (G * p->Zc + 31) & ~31;
-    const uint64_t key = (backward ? 5ull : 4ull) << 56 | (uint64_t)(p->R == NRLDPC_BG2_ROWS) << 48 | (uint64_t)blk << 32 |
-                         (uint64_t)(uint32_t)bytes;
+    const int bytes = G * p->n * 4 + (backward ? acc + 2 * p->R * (blk / 32) * 4 : 0);
+    if (bytes > kTapeSmemCap) break;
+    const uint64_t key = (backward ? 5ull : 4ull) << 56 |
+                         (uint64_t)((p->R == NRLDPC_BG2_ROWS) | p->vec << 1 | (backward && clipped) << 2) << 48 |
+                         (uint64_t)blk << 32 | (uint64_t)(uint32_t)bytes;
     const int occ =
-        cached_occupancy(st, key, [&] { return occupancy_train_tape(backward, p->R == NRLDPC_BG2_ROWS, blk, bytes); });
+        cached_occupancy(st, key, [&] { return occupancy_train_tape(*p, backward, blk, bytes); });
     if (occ * G > best_cw) {
       best_cw = occ * G;
       best_g = G;
       best_occ = occ;
+      *block = blk;
+      *smem = bytes;
     }
   }
-  if (best_g == 0) return 0;
+  if (best_g == 0) return 0;   // does not fit
   p->G = best_g;
-  *block = (best_g * p->Zc + 31) & ~31;
-  *smem = best_g * p->n * 4 + acc;
   return best_occ;
 }
 
@@ -753,7 +755,8 @@ int launch_tape_kernel(TrainTapeParams* p, bool backward, void* stream) {
   std::lock_guard<std::mutex> lock(g_mu);
   DeviceState* st = nullptr;
   if (device_state(&st) != 0) return NRLDPC_ERR_CUDA;
-  int block, smem;
+  p->vec = p->Zc % 4 == 0 && reinterpret_cast<uintptr_t>(p->tape) % 16 == 0;   // (the carry is the library's own)
+  int block = 0, smem = 0;
   const int occ = pick_tape_groups(st, p, backward, &block, &smem);
   if (occ < 1) return NRLDPC_ERR_CUDA;
   const int items = (p->batch + p->G - 1) / p->G;

@@ -239,13 +239,14 @@ struct TrainParams {
 struct TrainTapeParams {
   int32_t Zc, R, n, G, nnz, T, batch, detach;
   int32_t acc;                // backward: the CTA sums its alpha / beta gradients in shared memory
+  int32_t vec;                // Zc a multiple of 4 and the tape 16-byte aligned: groups of four edges per access
   float clip;                 // +inf when LLRs are not clipped
   const float* llr;           // [batch][n] decoder-layout input LLRs
   const float* alpha;         // [T][R]
   const float* beta;          // [T][R]
   float* final_llr;           // [batch][n]
   float* iter_llr;            // [T][batch][n] or null
-  float* tape;                // [T][batch][nnz][Zc]: rel of every edge
+  float* tape;                // [T][batch][nnz Zc]: rel of every edge, a slice of degree * Zc per row
   int64_t tape_words;         // nnz Zc
   const float* g_final;       // [batch][n] or null
   const float* g_iter;        // [T][batch][n] or null
@@ -254,7 +255,7 @@ struct TrainTapeParams {
   float* g_beta;              // [T][R], accumulated
   float* carry;               // per CTA: G * nnz * Zc
   int64_t carry_per_cta;
-  uint32_t edge[kMaxNnz];     // base column * Zc in the low 16 bits, V mod Zc in the high
+  uint2 edge4[kMaxNnz];       // {base column * Zc * 4, (V mod Zc) * 4}
   uint16_t row_off[kMaxRows + 1];
 };
 
@@ -264,7 +265,7 @@ int launch_train_forward(const TrainParams& p, bool f64, int grid, int block, in
 int launch_train_backward(const TrainParams& p, bool f64, int grid, int block, int smem, void* stream);
 int occupancy_train(bool backward, bool f64, bool bg2, int block, int smem, bool alias = false);
 int launch_train_tape(const TrainTapeParams& p, bool backward, int grid, int block, int smem, void* stream);
-int occupancy_train_tape(bool backward, bool bg2, int block, int smem);
+int occupancy_train_tape(const TrainTapeParams& p, bool backward, int block, int smem);
 // Mixed-size kernel classes: 0 = 384 threads per CTA (all of them active at
 // most), 1 = 256 threads with at most 240 active, three CTAs per SM.  A graph
 // of a class holds G = floor(capacity / Zc) lane pairs per CTA.

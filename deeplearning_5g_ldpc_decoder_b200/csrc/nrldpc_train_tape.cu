@@ -24,8 +24,11 @@
 // One code block per CTA where its Zc threads fill their warps, so a row's
 // barrier holds two to twelve warps and a dozen blocks per SM hide each other's
 // latency.  Both kernels are then bound by instruction issue.
-//   BG2 Zc64, batch 4096, 10 iterations: forward 1422 -> 1207 us, backward 6133 -> 2837 us
+//   batch 4096, 10 iterations, us    forward        backward
+//   BG2 Zc64                      1422 -> 1012    6133 -> 1652
+//   BG1 Zc112                     3500 -> 2990   16300 -> 6010
 //   (before: a checkpoint per iteration, recomputed by the backward, six-block CTAs)
+// ALU pipe 67 % (forward) and 55 % (backward) busy, 1.1 TB/s and 3.0 TB/s of HBM.
 #include <cuda_runtime.h>
 #include <math.h>
 #include <stdint.h>
@@ -46,99 +49,181 @@ __device__ __forceinline__ void bulk_prefetch_l2(const void* lo, size_t bytes) {
   if (b > a) asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(a), "r"((uint32_t)(b - a)));
 }
 
-__device__ __forceinline__ uint32_t tape_addr(const TrainTapeParams& p, int e, uint32_t zx) {
-  const uint32_t ed = p.edge[e];
-  uint32_t t = zx + (ed >> 16);
-  t = min(t, t - (uint32_t)p.Zc);
-  return (ed & 0xFFFFu) + t;
+// Byte address of edge e's word for lifted row zx4 / 4 (edge: {column * Zc * 4, (V mod Zc) * 4}).
+__device__ __forceinline__ uint32_t tape_addr(const TrainTapeParams& p, int e, uint32_t zx4) {
+  const uint2 ed = p.edge4[e];
+  const uint32_t t = zx4 + ed.y;
+  return min(t, t - 4u * (uint32_t)p.Zc) + ed.x;
 }
 
-// Forward of one lifted check row: the old message comes from the row's slot of
-// this iteration (none in the first), rel goes there, and the new message to the
-// slot of the next iteration (none after the last).
-template <int D>
-__device__ __forceinline__ void tape_row_fwd(const TrainTapeParams& p, float* __restrict__ lq, uint32_t zx, int e0,
-                                              float alpha, float beta, bool first, float* slot, float* next) {
-  const int Zc = p.Zc;
-  const float clip = p.clip;
-  float n1 = 0, n2 = 0;
-  uint32_t fl = 0u;   // flips in bits 0..18, position of the minimum from bit 20
-  if (!first) {
-    n1 = slot[0];
-    n2 = slot[Zc];
-    fl = __float_as_uint(slot[2 * Zc]);
+// D floats of lifted row zx in a row's slice of D Zc floats.  kVec (Zc a multiple
+// of 4, 16-byte aligned buffers): groups of four edges as one float4 per row,
+// then what is left as a float2 and a float, so a row moves D floats in a
+// quarter to a half of the instructions; otherwise one plane of Zc floats per
+// edge.  Either way a thread's words are its own.
+template <int D, bool kVec>
+__device__ __forceinline__ void load_row(const float* slice, int zx, int Zc, float (&v)[D]) {
+  if constexpr (kVec) {
+#pragma unroll
+    for (int c = 0; c < D / 4; ++c) {
+      const float4 q = __ldcs(reinterpret_cast<const float4*>(slice + 4 * c * Zc) + zx);
+      v[4 * c] = q.x;
+      v[4 * c + 1] = q.y;
+      v[4 * c + 2] = q.z;
+      v[4 * c + 3] = q.w;
+    }
+    constexpr int b = D / 4 * 4;
+    const float* rest = slice + b * Zc;
+    if constexpr ((D & 2) != 0) {
+      const float2 q = __ldcs(reinterpret_cast<const float2*>(rest) + zx);
+      v[b] = q.x;
+      v[b + 1] = q.y;
+    }
+    if constexpr ((D & 1) != 0) v[D - 1] = __ldcs(rest + ((D & 2) ? 2 * Zc : 0) + zx);
+  } else {
+#pragma unroll
+    for (int j = 0; j < D; ++j) v[j] = __ldcs(slice + j * Zc + zx);
   }
-  const int ix = (int)(fl >> 20);
+}
+// kStream: written once and read much later (the tape); otherwise kept near (the carry).
+template <int D, bool kVec, bool kStream>
+__device__ __forceinline__ void store_row(float* slice, int zx, int Zc, const float (&v)[D]) {
+  const auto put = [](auto* a, auto x) {
+    if constexpr (kStream) __stcs(a, x);
+    else *a = x;
+  };
+  if constexpr (kVec) {
+#pragma unroll
+    for (int c = 0; c < D / 4; ++c)
+      put(reinterpret_cast<float4*>(slice + 4 * c * Zc) + zx, make_float4(v[4 * c], v[4 * c + 1], v[4 * c + 2], v[4 * c + 3]));
+    constexpr int b = D / 4 * 4;
+    float* rest = slice + b * Zc;
+    if constexpr ((D & 2) != 0) put(reinterpret_cast<float2*>(rest) + zx, make_float2(v[b], v[b + 1]));
+    if constexpr ((D & 1) != 0) put(rest + ((D & 2) ? 2 * Zc : 0) + zx, v[D - 1]);
+  } else {
+#pragma unroll
+    for (int j = 0; j < D; ++j) put(slice + j * Zc + zx, v[j]);
+  }
+}
+
+// A row's message in its tape slot of the next iteration, in words of the
+// thread's own: magnitudes of the edges that carry the first and the second
+// minimum, and a word with edge j's sign flip in bit D - 1 - j and the second
+// minimum's edge from bit 20.
+struct TapeMsg {
+  float n1, n2;
+  uint32_t f;
+};
+template <int D, bool kVec>
+__device__ __forceinline__ TapeMsg load_msg(const float* slice, int zx, int Zc) {
+  if constexpr (kVec && D >= 4) {
+    const float4 q = reinterpret_cast<const float4*>(slice)[zx];
+    return TapeMsg{q.x, q.y, __float_as_uint(q.z)};
+  } else if constexpr (kVec) {
+    const float2 q = reinterpret_cast<const float2*>(slice)[zx];
+    return TapeMsg{q.x, q.y, __float_as_uint(slice[2 * Zc + zx])};
+  } else {
+    return TapeMsg{slice[zx], slice[Zc + zx], __float_as_uint(slice[2 * Zc + zx])};
+  }
+}
+template <int D, bool kVec>
+__device__ __forceinline__ void store_msg(float* slice, int zx, int Zc, const TapeMsg& m) {
+  if constexpr (kVec && D >= 4) {
+    reinterpret_cast<float4*>(slice)[zx] = make_float4(m.n1, m.n2, __uint_as_float(m.f), 0.0f);
+  } else {
+    if constexpr (kVec) {
+      reinterpret_cast<float2*>(slice)[zx] = make_float2(m.n1, m.n2);
+    } else {
+      slice[zx] = m.n1;
+      slice[Zc + zx] = m.n2;
+    }
+    slice[2 * Zc + zx] = __uint_as_float(m.f);
+  }
+}
+
+// Sign of x as the model takes it, in bit 31: set where x < 0.  (Adding +0.0
+// turns -0.0 into +0.0, and the sum of a NaN has its sign bit clear.)
+__device__ __forceinline__ uint32_t sign_of(float x) { return __float_as_uint(__fadd_rn(x, 0.0f)); }
+
+// Forward of one lifted check row: rel goes to the row's slice of this iteration's
+// tape, from where the old message is taken first (zero in the first iteration),
+// and the new message to the slice of the next iteration (none after the last).
+template <int D, bool kVec>
+__device__ __forceinline__ void tape_row_fwd(const TrainTapeParams& p, char* __restrict__ lq, int zx, int e0, float alpha,
+                                             float beta, bool first, float* slice, float* next) {
+  const float clip = p.clip;
+  TapeMsg m{0.0f, 0.0f, 0u};
+  if (!first) m = load_msg<D, kVec>(slice, zx, p.Zc);
+  const int ix = (int)(m.f >> 20);
   float rel[D];
   uint32_t addr[D];
-  bool neg = false;
+  uint32_t sg = 0u;
   float m1 = INFINITY, m2 = INFINITY;
   int idx = 0;
 #pragma unroll
   for (int j = 0; j < D; ++j) {
-    addr[j] = tape_addr(p, e0 + j, zx);
-    float old = ix == j ? n2 : n1;
-    old = ((fl >> j) & 1u) ? -old : old;
-    const float r = __fsub_rn(lq[addr[j]], old);
+    addr[j] = tape_addr(p, e0 + j, 4u * (uint32_t)zx);
+    const uint32_t old = __float_as_uint(ix == j ? m.n2 : m.n1) ^ ((m.f << (32 - D + j)) & 0x80000000u);
+    const float r = __fsub_rn(*reinterpret_cast<const float*>(lq + addr[j]), __uint_as_float(old));
     rel[j] = r;
-    neg ^= (r < 0.0f);
+    sg ^= sign_of(r);
     const float a = fabsf(r);
-    const bool lt1 = a < m1;
-    m2 = lt1 ? m1 : (a < m2 ? a : m2);
-    m1 = lt1 ? a : m1;
-    idx = lt1 ? j : idx;
+    const bool lt = a < m1;   // a NaN is never below, and fminf passes it over
+    m2 = lt ? m1 : fminf(m2, a);
+    m1 = fminf(m1, a);
+    idx = lt ? j : idx;
   }
-#pragma unroll
-  for (int j = 0; j < D; ++j) __stcs(slot + (size_t)j * Zc, rel[j]);
+  store_row<D, kVec, true>(slice, zx, p.Zc, rel);
   const float s1 = __fmul_rn(alpha, fmaxf(__fsub_rn(m1, beta), 0.0f));
   const float s2 = __fmul_rn(alpha, fmaxf(__fsub_rn(m2, beta), 0.0f));
-  uint32_t flips = (uint32_t)idx << 20;
+  uint32_t flips = 0u;
 #pragma unroll
   for (int j = 0; j < D; ++j) {
-    const bool flip = (rel[j] < 0.0f) != neg;
-    const float mag = (j == idx) ? s2 : s1;
-    flips |= (flip ? 1u : 0u) << j;
-    float v = __fadd_rn(rel[j], flip ? -mag : mag);
-    v = fminf(fmaxf(v, -clip), clip);
-    lq[addr[j]] = v;
+    const uint32_t f = sign_of(rel[j]) ^ sg;
+    flips = __funnelshift_l(f, flips, 1);
+    const uint32_t msg = __float_as_uint((j == idx) ? s2 : s1) ^ (f & 0x80000000u);
+    const float v = __fadd_rn(rel[j], __uint_as_float(msg));
+    *reinterpret_cast<float*>(lq + addr[j]) = fminf(fmaxf(v, -clip), clip);
   }
-  if (next) {
-    next[0] = s1;
-    next[Zc] = s2;
-    next[2 * Zc] = __uint_as_float(flips);
-  }
+  if (next) store_msg<D, kVec>(next, zx, p.Zc, TapeMsg{s1, s2, flips | (uint32_t)idx << 20});
 }
 
-// Backward of one lifted check row (see the file comment).
-template <int D>
-__device__ __forceinline__ void tape_row_bwd(const TrainTapeParams& p, float* __restrict__ glq, uint32_t zx, int e0,
-                                              float alpha, float beta, const float* slot, float* carry, bool last, bool first,
-                                              float* ga, float* gb) {
-  const int Zc = p.Zc;
-  const float clip = p.clip;
-  // Rows of more than 10 edges keep only rel in registers: edge addresses are
-  // recomputed and the incoming gradient is read again in the last pass (no
-  // other edge of the row writes that word).
-  constexpr bool kLean = D > 10;
-  constexpr int kKeep = kLean ? 1 : D;
-  float rel[D];
-  float cv[kKeep], g_in[kKeep];
-  uint32_t addr[kKeep];
-#pragma unroll
-  for (int j = 0; j < D; ++j) rel[j] = __ldcs(slot + (size_t)j * Zc);
-  if constexpr (!kLean) {
-#pragma unroll
-    for (int j = 0; j < D; ++j) cv[j] = last ? 0.0f : carry[(size_t)j * Zc];
-  }
+// What a row's backward needs besides its loop over edges.
+struct BwdRow {
+  float s1, s2, r1, r2, k1, k2;
+};
+__device__ __forceinline__ BwdRow bwd_row(float m1, float m2, float alpha, float beta) {
+  BwdRow b;
+  const float o1 = __fsub_rn(m1, beta), o2 = __fsub_rn(m2, beta);
+  b.r1 = fmaxf(o1, 0.0f);
+  b.r2 = fmaxf(o2, 0.0f);
+  b.k1 = o1 >= 0.0f ? alpha : 0.0f;   // d mag / d u
+  b.k2 = o2 >= 0.0f ? alpha : 0.0f;
+  b.s1 = __fmul_rn(alpha, b.r1);
+  b.s2 = __fmul_rn(alpha, b.r2);
+  return b;
+}
+
+// Backward of one lifted check row with infinities or NaN among its inputs: the
+// loops of tape_row_bwd with every test of the model spelled out, over values
+// read again from memory.
+template <bool kVec>
+__device__ __noinline__ void tape_row_bwd_odd(const TrainTapeParams& p, char* glq, int zx, int e0, int D, float alpha,
+                                              float beta, const float* slice, float* carry, bool last, bool first, float* ga,
+                                              float* gb) {
+  const int Zc = p.Zc, quads = D / 4 * 4;
+  const auto at = [&](int j) {   // load_row's place of edge j
+    if (!kVec) return j * Zc + zx;
+    if (j < quads) return (j & ~3) * Zc + 4 * zx + (j & 3);
+    if ((D & 2) && j < quads + 2) return quads * Zc + 2 * zx + (j - quads);
+    return (D - 1) * Zc + zx;
+  };
   bool neg = false;
   float m1 = INFINITY, m2 = INFINITY;
-  // idx: first minimum; idx2: first minimum of the others (torch.min's choices),
-  // none (-1) where no other is below infinity
   int idx = -1, idx2 = -1;
-#pragma unroll
   for (int j = 0; j < D; ++j) {
-    neg ^= (rel[j] < 0.0f);
-    const float a = fabsf(rel[j]);
+    const float rel = slice[at(j)], a = fabsf(rel);
+    neg ^= rel < 0.0f;
     const bool lt1 = a < m1, lt2 = a < m2;
     idx2 = lt1 ? idx : (lt2 ? j : idx2);
     idx = lt1 ? j : idx;
@@ -146,81 +231,139 @@ __device__ __forceinline__ void tape_row_bwd(const TrainTapeParams& p, float* __
     m1 = lt1 ? a : m1;
   }
   idx = idx < 0 ? 0 : idx;
-  const float o1 = __fsub_rn(m1, beta), o2 = __fsub_rn(m2, beta);
-  const float r1 = fmaxf(o1, 0.0f), r2 = fmaxf(o2, 0.0f);
-  const float k1 = o1 >= 0.0f ? alpha : 0.0f;   // d mag / d u
-  const float k2 = o2 >= 0.0f ? alpha : 0.0f;
-  const float s1 = __fmul_rn(alpha, r1), s2 = __fmul_rn(alpha, r2);
-  // g_mag of the edges that carry the first minimum (summed), and of edge idx
-  float sum1 = 0, gm2 = 0;
-#pragma unroll
+  const BwdRow b = bwd_row(m1, m2, alpha, beta);
+  const auto incoming = [&](int j, float rel, bool flip) {
+    const float mag = j == idx ? b.s2 : b.s1;
+    const float v = __fadd_rn(rel, flip ? -mag : mag);
+    return v >= -p.clip && v <= p.clip ? *reinterpret_cast<const float*>(glq + tape_addr(p, e0 + j, 4u * (uint32_t)zx)) : 0.0f;
+  };
+  float sum1 = 0.0f, gm2 = 0.0f;
   for (int j = 0; j < D; ++j) {
-    const uint32_t a = tape_addr(p, e0 + j, zx);
-    const bool flip = (rel[j] < 0.0f) != neg;
-    const float mag = (j == idx) ? s2 : s1;
-    const float v = __fadd_rn(rel[j], flip ? -mag : mag);
-    const float gv = (v >= -clip && v <= clip) ? glq[a] : 0.0f;
-    if constexpr (!kLean) {
-      addr[j] = a;
-      g_in[j] = gv;
-    }
-    const float g_lrt = (kLean ? (last ? 0.0f : carry[(size_t)j * Zc]) : cv[kLean ? 0 : j]) + gv;
+    const float rel = slice[at(j)];
+    const bool flip = (rel < 0.0f) != neg;
+    const float g_lrt = (last ? 0.0f : carry[at(j)]) + incoming(j, rel, flip);
     const float g_mag = flip ? -g_lrt : g_lrt;
     if (j == idx) gm2 = g_mag;
     else sum1 += g_mag;
   }
-  *ga += sum1 * r1 + gm2 * r2;
-  const float g1 = sum1 * k1, g2 = gm2 * k2;   // gradients of the two minima
+  *ga += sum1 * b.r1 + gm2 * b.r2;
+  const float g1 = sum1 * b.k1, g2 = gm2 * b.k2;
   *gb -= g1 + g2;
-#pragma unroll
   for (int j = 0; j < D; ++j) {
-    uint32_t a;
-    float gv;
-    if constexpr (kLean) {
-      a = tape_addr(p, e0 + j, zx);
-      const bool flip = (rel[j] < 0.0f) != neg;
-      const float mag = (j == idx) ? s2 : s1;
-      const float v = __fadd_rn(rel[j], flip ? -mag : mag);
-      gv = (v >= -clip && v <= clip) ? glq[a] : 0.0f;
-    } else {
-      a = addr[j];
-      gv = g_in[j];
-    }
-    float g_rel = 0;
-    if (!p.detach) {
-      const float g_a = j == idx ? g1 : (j == idx2 ? g2 : 0.0f);
-      g_rel = gv + (rel[j] > 0.0f ? g_a : (rel[j] < 0.0f ? -g_a : 0.0f));
-    }
-    glq[a] = g_rel;
-    if (!first) carry[(size_t)j * Zc] = -g_rel;
+    const float rel = slice[at(j)];
+    const float gv = incoming(j, rel, (rel < 0.0f) != neg);
+    const float g_a = j == idx ? g1 : (j == idx2 ? g2 : 0.0f);
+    const float g_rel = p.detach ? 0.0f : gv + (rel > 0.0f ? g_a : (rel < 0.0f ? -g_a : 0.0f));
+    *reinterpret_cast<float*>(glq + tape_addr(p, e0 + j, 4u * (uint32_t)zx)) = g_rel;
+    if (!first) carry[at(j)] = -g_rel;
   }
 }
 
-#define NRLDPC_TAPE_DISPATCH(FN, deg, ...)   \
-  switch (deg) {                                 \
-    case 3: FN<3>(__VA_ARGS__); break;        \
-    case 4: FN<4>(__VA_ARGS__); break;        \
-    case 5: FN<5>(__VA_ARGS__); break;        \
-    case 6: FN<6>(__VA_ARGS__); break;        \
-    case 7: FN<7>(__VA_ARGS__); break;        \
-    case 8: FN<8>(__VA_ARGS__); break;        \
-    case 9: FN<9>(__VA_ARGS__); break;        \
-    case 10: FN<10>(__VA_ARGS__); break;      \
-    default: FN<(kMaxD > 10 ? 19 : 10)>(__VA_ARGS__); break;      \
+// Backward of one lifted check row (see the file comment).  kClip: LLRs are
+// clipped, so a sum outside the range passes no gradient.
+template <int D, bool kVec, bool kClip>
+__device__ __forceinline__ void tape_row_bwd(const TrainTapeParams& p, char* __restrict__ glq, int zx, int e0, float alpha,
+                                             float beta, const float* slice, float* carry, bool last, bool first, float* ga,
+                                             float* gb) {
+  const int Zc = p.Zc;
+  float rel[D];
+  load_row<D, kVec>(slice, zx, Zc, rel);
+  float cv[D];
+  if (last) {
+#pragma unroll
+    for (int j = 0; j < D; ++j) cv[j] = 0.0f;
+  } else {
+    load_row<D, kVec>(carry, zx, Zc, cv);
+  }
+  uint32_t sg = 0u;
+  float m1 = INFINITY, m2 = INFINITY, total = 0.0f;
+  // idx: first minimum; idx2: first minimum of the others (torch.min's choices)
+  int idx = 0, idx2 = 0;
+#pragma unroll
+  for (int j = 0; j < D; ++j) {
+    sg ^= sign_of(rel[j]);
+    const float a = fabsf(rel[j]);
+    total += a;
+    const bool lt1 = a < m1, lt2 = a < m2;
+    idx2 = lt1 ? idx : (lt2 ? j : idx2);
+    idx = lt1 ? j : idx;
+    m2 = lt1 ? m1 : fminf(m2, a);
+    m1 = fminf(m1, a);
+  }
+  const BwdRow b = bwd_row(m1, m2, alpha, beta);
+  if (!(total + fabsf(b.s1) + fabsf(b.s2) < INFINITY)) {   // an infinity or a NaN in the row
+    tape_row_bwd_odd<kVec>(p, glq, zx, e0, D, alpha, beta, slice, carry, last, first, ga, gb);
+    return;
+  }
+  // From here every |rel| is finite: a clip test can only fail by the range, and
+  // rel is zero at idx (idx2) exactly when m1 (m2) is.
+  float sum1 = 0.0f, gm2 = 0.0f;   // g_mag of the edges that carry the first minimum (summed), and of edge idx
+#pragma unroll
+  for (int j = 0; j < D; ++j) {
+    const uint32_t f = (sign_of(rel[j]) ^ sg) & 0x80000000u;   // the message is negated
+    float gv = *reinterpret_cast<const float*>(glq + tape_addr(p, e0 + j, 4u * (uint32_t)zx));
+    if constexpr (kClip) {
+      const float v = __fadd_rn(rel[j], __uint_as_float(__float_as_uint(j == idx ? b.s2 : b.s1) ^ f));
+      gv = fabsf(v) <= p.clip ? gv : 0.0f;
+    }
+    const float g_mag = __uint_as_float(__float_as_uint(cv[j] + gv) ^ f);
+    cv[j] = gv;
+    if (j == idx) gm2 = g_mag;
+    else sum1 += g_mag;
+  }
+  *ga += sum1 * b.r1 + gm2 * b.r2;
+  float g1 = sum1 * b.k1, g2 = gm2 * b.k2;   // gradients of the two minima
+  *gb -= g1 + g2;
+  g1 = m1 > 0.0f ? g1 : 0.0f;                // d|rel| / d rel is 0 at 0
+  g2 = m2 > 0.0f ? g2 : 0.0f;
+#pragma unroll
+  for (int j = 0; j < D; ++j) {
+    const float g_a = j == idx ? g1 : (j == idx2 ? g2 : 0.0f);
+    const float g_rel = p.detach ? 0.0f : cv[j] + __uint_as_float(__float_as_uint(g_a) ^ (__float_as_uint(rel[j]) & 0x80000000u));
+    *reinterpret_cast<float*>(glq + tape_addr(p, e0 + j, 4u * (uint32_t)zx)) = g_rel;
+    cv[j] = -g_rel;
+  }
+  if (!first) store_row<D, kVec, false>(carry, zx, Zc, cv);
+}
+
+#define NRLDPC_TAPE_DISPATCH(deg, CALL) \
+  switch (deg) {                        \
+    case 3: { CALL(3); break; }         \
+    case 4: { CALL(4); break; }         \
+    case 5: { CALL(5); break; }         \
+    case 6: { CALL(6); break; }         \
+    case 7: { CALL(7); break; }         \
+    case 8: { CALL(8); break; }         \
+    case 9: { CALL(9); break; }         \
+    case 10: { CALL(10); break; }       \
+    default: { CALL((kMaxD > 10 ? 19 : 10)); break; } \
   }
 
 // kMaxD: the largest row degree of the base graph (19 for BG1, 10 for BG2); a
-// BG2 instantiation carries no degree-19 code and needs fewer registers.
-template <int kMaxD>
-__global__ void __launch_bounds__(kThreadsTarget, 2)
-    tape_forward_kernel(const __grid_constant__ TrainTapeParams p) {
-  extern __shared__ __align__(16) unsigned char s_raw[];
-  float* s_lq = reinterpret_cast<float*>(s_raw);
-  const float* llr = p.llr;
-  const float* alpha_t = p.alpha;
-  const float* beta_t = p.beta;
-  float* final_llr = p.final_llr;
-  float* iter_llr = p.iter_llr;
+// BG2 instantiation carries no degree-19 code and needs fewer registers.  The
+// launch bound sets the registers: 72 for BG2, 14 CTAs of 64 threads on an SM
+// (backward at Zc=64 1774 us; 1930 with 80 registers and 12 CTAs, 2009 with 64;
+// before rows were staged), and 80 for BG1, whose degree-19 rows would spill
+// (Zc=112 6261 us; 6494 with 72).
+constexpr int launch_threads(int max_deg) { return max_deg <= 10 ? 448 : kThreadsTarget; }
+
+// A row of iteration t, staged in shared memory: one 16-byte load instead of
+// parameter and global loads and their address arithmetic in every row.
+struct __align__(16) RowDesc {
+  uint16_t e0, deg;
+  uint32_t off;   // floats before the row's slice
+  float alpha, beta;
+};
+__device__ __forceinline__ void stage_rows(const TrainTapeParams& p, RowDesc* s_rows, int t) {
+  for (int r = threadIdx.x; r < p.R; r += blockDim.x)
+    s_rows[r] = RowDesc{p.row_off[r], (uint16_t)(p.row_off[r + 1] - p.row_off[r]), (uint32_t)p.row_off[r] * (uint32_t)p.Zc,
+                        p.alpha[t * p.R + r], p.beta[t * p.R + r]};
+}
+
+template <int kMaxD, bool kVec>
+__global__ void __launch_bounds__(launch_threads(kMaxD), 2) tape_forward_kernel(const __grid_constant__ TrainTapeParams p) {
+  extern __shared__ __align__(16) float s_lq[];
+  __shared__ RowDesc s_rows[kMaxRows];
   const float clip = p.clip;
   const int tid = threadIdx.x;
   const int g = tid / p.Zc, zx = tid - g * p.Zc;
@@ -230,28 +373,32 @@ __global__ void __launch_bounds__(kThreadsTarget, 2)
     const int cw = item * p.G + g;
     const bool valid = active && cw < p.batch;
     if (valid)
-      for (int i = zx; i < p.n; i += p.Zc) lq[i] = fminf(fmaxf(llr[(size_t)cw * p.n + i], -clip), clip);
-    __syncthreads();
+      for (int i = zx; i < p.n; i += p.Zc) lq[i] = fminf(fmaxf(p.llr[(size_t)cw * p.n + i], -clip), clip);
     for (int t = 0; t < p.T; ++t) {
-      float* tape = p.tape + ((size_t)t * p.batch + (valid ? cw : 0)) * p.tape_words + zx;
+      stage_rows(p, s_rows, t);   // the last row's barrier lies between its reads and this
+      __syncthreads();
+      float* tape = p.tape + ((size_t)t * p.batch + (valid ? cw : 0)) * p.tape_words;
       float* tnext = tape + (size_t)p.batch * p.tape_words;
       for (int row = 0; row < p.R; ++row) {
         if (valid) {
-          const int e0 = p.row_off[row], deg = p.row_off[row + 1] - e0;
-          const float alpha = alpha_t[t * p.R + row], beta = beta_t[t * p.R + row];
-          float* slot = tape + (size_t)e0 * p.Zc;
-          float* next = t + 1 < p.T ? tnext + (size_t)e0 * p.Zc : nullptr;
-          NRLDPC_TAPE_DISPATCH(tape_row_fwd, deg, p, lq, (uint32_t)zx, e0, alpha, beta, t == 0, slot, next)
+          const RowDesc d = s_rows[row];
+          const int e0 = d.e0, deg = d.deg;
+          float* slice = tape + d.off;
+          float* next = t + 1 < p.T ? tnext + d.off : nullptr;
+#define NRLDPC_FWD(D) tape_row_fwd<D, kVec>(p, reinterpret_cast<char*>(lq), zx, e0, d.alpha, d.beta, t == 0, slice, next)
+          NRLDPC_TAPE_DISPATCH(deg, NRLDPC_FWD)
+#undef NRLDPC_FWD
         }
         __syncthreads();
       }
-      if (valid && iter_llr) {
-        for (int i = zx; i < p.n; i += p.Zc) iter_llr[((size_t)t * p.batch + cw) * p.n + i] = lq[i];
+      if (p.iter_llr) {
+        if (valid)
+          for (int i = zx; i < p.n; i += p.Zc) p.iter_llr[((size_t)t * p.batch + cw) * p.n + i] = lq[i];
+        __syncthreads();   // read before the next iteration's rows write
       }
-      if (iter_llr) __syncthreads();   // read before the next iteration's rows write
     }
     if (valid)
-      for (int i = zx; i < p.n; i += p.Zc) final_llr[(size_t)cw * p.n + i] = lq[i];
+      for (int i = zx; i < p.n; i += p.Zc) p.final_llr[(size_t)cw * p.n + i] = lq[i];
     __syncthreads();
   }
 }
@@ -265,85 +412,78 @@ __device__ __forceinline__ float warp_sum_pair(float a, float b) {
   return v;
 }
 
-template <int kMaxD>
-__global__ void __launch_bounds__(kThreadsTarget, 2)
-    tape_backward_kernel(const __grid_constant__ TrainTapeParams p) {
-  extern __shared__ __align__(16) unsigned char s_raw[];
-  __shared__ float s_red[2][2][kThreadsTarget / 32];   // [row parity][alpha, beta][warp]
-  float* s_glq = reinterpret_cast<float*>(s_raw);       // dLQ of each code block
-  // Sums of the CTA's alpha / beta gradients, [T][R][2], added to the outputs at
-  // the end; with very many iterations they do not fit and every row adds its own.
-  float* s_acc = s_glq + (size_t)p.G * p.n;
-  const float* llr = p.llr;
-  const float* alpha_t = p.alpha;
-  const float* beta_t = p.beta;
-  const float* g_final = p.g_final;
-  const float* g_iter = p.g_iter;
-  float* g_llr = p.g_llr;
-  float* g_alpha = p.g_alpha;
-  float* g_beta = p.g_beta;
-  const float clip = p.clip;
+template <int kMaxD, bool kVec, bool kClip>
+__global__ void __launch_bounds__(launch_threads(kMaxD), 2) tape_backward_kernel(const __grid_constant__ TrainTapeParams p) {
+  // dLQ of each code block; the iteration's alpha / beta gradients per row and
+  // warp, [R][2][warps]; the CTA's sums of them, [T][R][2], added to the outputs
+  // at the end (with very many iterations they do not fit, and every iteration
+  // adds its own).
+  extern __shared__ __align__(16) float s_glq[];
+  __shared__ RowDesc s_rows[kMaxRows];
   const int tid = threadIdx.x;
   const int warps = blockDim.x >> 5;
+  float* s_part = s_glq + (size_t)p.G * p.n;
+  float* s_acc = s_part + 2 * p.R * warps;
   const int g = tid / p.Zc, zx = tid - g * p.Zc;
   const bool active = g < p.G;
   float* glq = s_glq + (active ? g : 0) * p.n;
-  float* carry = p.carry + (size_t)blockIdx.x * p.carry_per_cta +
-                (size_t)(active ? g : 0) * (size_t)p.nnz * p.Zc + zx;
+  float* carry = p.carry + (size_t)blockIdx.x * p.carry_per_cta + (size_t)(active ? g : 0) * p.tape_words;
   if (p.acc)
-    for (int k = tid; k < 2 * p.T * p.R; k += blockDim.x) s_acc[k] = 0;
+    for (int k = tid; k < 2 * p.T * p.R; k += blockDim.x) s_acc[k] = 0.0f;
   for (int item = blockIdx.x; item * p.G < p.batch; item += gridDim.x) {
     const int cw = item * p.G + g;
     const bool valid = active && cw < p.batch;
     if (valid)
-      for (int i = zx; i < p.n; i += p.Zc) glq[i] = g_final ? g_final[(size_t)cw * p.n + i] : 0.0f;
+      for (int i = zx; i < p.n; i += p.Zc) glq[i] = p.g_final ? p.g_final[(size_t)cw * p.n + i] : 0.0f;
     for (int t = p.T - 1; t >= 0; --t) {
       // own indices i = zx + k Zc, like the loads above; rows need all of them
-      if (valid && g_iter)
-        for (int i = zx; i < p.n; i += p.Zc) glq[i] += g_iter[((size_t)t * p.batch + cw) * p.n + i];
-      __syncthreads();
-      const float* tape = p.tape + ((size_t)t * p.batch + (valid ? cw : 0)) * p.tape_words + zx;
+      if (valid && p.g_iter)
+        for (int i = zx; i < p.n; i += p.Zc) glq[i] += p.g_iter[((size_t)t * p.batch + cw) * p.n + i];
+      stage_rows(p, s_rows, t);
+      __syncthreads();   // also: the sums over s_part below have been read
+      const float* tape = p.tape + ((size_t)t * p.batch + (valid ? cw : 0)) * p.tape_words;
       for (int row = p.R - 1; row >= 0; --row) {
-        float ga = 0, gb = 0;
+        float ga = 0.0f, gb = 0.0f;
         if (valid) {
-          const int e0 = p.row_off[row], deg = p.row_off[row + 1] - e0;
+          const RowDesc d = s_rows[row];
+          const int e0 = d.e0, deg = d.deg;
           // the tape comes from HBM: a row's slice a few rows ahead of its use
           if (zx == 0 && row >= kTapeAhead) {
-            const int ep = p.row_off[row - kTapeAhead];
-            bulk_prefetch_l2(tape + (size_t)ep * p.Zc, (size_t)(p.row_off[row - kTapeAhead + 1] - ep) * (size_t)p.Zc * 4u);
+            const RowDesc a = s_rows[row - kTapeAhead];
+            bulk_prefetch_l2(tape + a.off, (size_t)a.deg * (size_t)p.Zc * 4u);
           }
-          const float alpha = alpha_t[t * p.R + row], beta = beta_t[t * p.R + row];
-          const float* slot = tape + (size_t)e0 * p.Zc;
-          NRLDPC_TAPE_DISPATCH(tape_row_bwd, deg, p, glq, (uint32_t)zx, e0, alpha, beta, slot,
-                                carry + (size_t)e0 * p.Zc, t == p.T - 1, t == 0, &ga, &gb)
+          const float* slice = tape + d.off;
+          float* cs = carry + d.off;
+#define NRLDPC_BWD(D) \
+  tape_row_bwd<D, kVec, kClip>(p, reinterpret_cast<char*>(glq), zx, e0, d.alpha, d.beta, slice, cs, t == p.T - 1, t == 0, &ga, &gb)
+          NRLDPC_TAPE_DISPATCH(deg, NRLDPC_BWD)
+#undef NRLDPC_BWD
         }
-        // Sum of the row's alpha / beta gradient over the CTA.  Double-buffered
-        // by row parity: the next row's writes never meet this row's reads,
-        // which end before the barrier after that row.
         const float v = warp_sum_pair(ga, gb);
-        if ((tid & 15) == 0) s_red[row & 1][(tid >> 4) & 1][tid >> 5] = v;
+        if ((tid & 15) == 0) s_part[(2 * row + ((tid >> 4) & 1)) * warps + (tid >> 5)] = v;
         __syncthreads();
-        if (tid < 2) {
-          float s = 0;
-          for (int w = 0; w < warps; ++w) s += s_red[row & 1][tid][w];
-          const int k = t * p.R + row;
-          if (p.acc) s_acc[2 * k + tid] += s;
-          else if (s != 0.0f) atomicAdd((tid ? g_beta : g_alpha) + k, s);
-        }
+      }
+      // the iteration's gradients, summed over the CTA's warps
+      for (int k = tid; k < 2 * p.R; k += blockDim.x) {
+        float s = 0.0f;
+        for (int w = 0; w < warps; ++w) s += s_part[k * warps + w];
+        if (p.acc) s_acc[2 * t * p.R + k] += s;
+        else if (s != 0.0f) atomicAdd(((k & 1) ? p.g_beta : p.g_alpha) + t * p.R + (k >> 1), s);
       }
     }
     if (valid)
       for (int i = zx; i < p.n; i += p.Zc) {
-        const float x = llr[(size_t)cw * p.n + i];
-        g_llr[(size_t)cw * p.n + i] = (x >= -clip && x <= clip) ? glq[i] : 0.0f;
+        const float x = p.llr[(size_t)cw * p.n + i];
+        p.g_llr[(size_t)cw * p.n + i] = (x >= -p.clip && x <= p.clip) ? glq[i] : 0.0f;
       }
     // the next item's first writes are to this thread's own words
   }
-  if (p.acc) {
-    __syncthreads();
-    for (int k = tid; k < 2 * p.T * p.R; k += blockDim.x)
-      if (s_acc[k] != 0.0f) atomicAdd(((k & 1) ? g_beta : g_alpha) + (k >> 1), s_acc[k]);
-  }
+  if (p.acc)   // every thread wrote, and now adds, the same entries
+    for (int k = tid; k < 2 * p.R; k += blockDim.x)
+      for (int t = 0; t < p.T; ++t) {
+        const float s = s_acc[2 * t * p.R + k];
+        if (s != 0.0f) atomicAdd(((k & 1) ? p.g_beta : p.g_alpha) + t * p.R + (k >> 1), s);
+      }
 }
 
 template <typename K>
@@ -365,21 +505,33 @@ int occupancy_tape_one(K kernel, int block, int smem) {
 
 }  // namespace
 
-int launch_train_tape(const TrainTapeParams& p, bool backward, int grid, int block, int smem, void* stream) {
-  const bool bg2 = p.R == NRLDPC_BG2_ROWS;
-  if (backward)
-    return bg2 ? launch_tape(tape_backward_kernel<10>, p, grid, block, smem, stream)
-               : launch_tape(tape_backward_kernel<19>, p, grid, block, smem, stream);
-  return bg2 ? launch_tape(tape_forward_kernel<10>, p, grid, block, smem, stream)
-             : launch_tape(tape_forward_kernel<19>, p, grid, block, smem, stream);
+namespace {
+
+// Calls op(kernel) with the instance of a launch.
+template <typename Op>
+int with_tape_kernel(bool backward, bool bg2, bool vec, bool clipped, Op op) {
+  if (!backward) {
+    if (bg2) return vec ? op(tape_forward_kernel<10, true>) : op(tape_forward_kernel<10, false>);
+    return vec ? op(tape_forward_kernel<19, true>) : op(tape_forward_kernel<19, false>);
+  }
+  if (bg2) {
+    if (vec) return clipped ? op(tape_backward_kernel<10, true, true>) : op(tape_backward_kernel<10, true, false>);
+    return clipped ? op(tape_backward_kernel<10, false, true>) : op(tape_backward_kernel<10, false, false>);
+  }
+  if (vec) return clipped ? op(tape_backward_kernel<19, true, true>) : op(tape_backward_kernel<19, true, false>);
+  return clipped ? op(tape_backward_kernel<19, false, true>) : op(tape_backward_kernel<19, false, false>);
 }
 
-int occupancy_train_tape(bool backward, bool bg2, int block, int smem) {
-  if (backward)
-    return bg2 ? occupancy_tape_one(tape_backward_kernel<10>, block, smem)
-               : occupancy_tape_one(tape_backward_kernel<19>, block, smem);
-  return bg2 ? occupancy_tape_one(tape_forward_kernel<10>, block, smem)
-             : occupancy_tape_one(tape_forward_kernel<19>, block, smem);
+}  // namespace
+
+int launch_train_tape(const TrainTapeParams& p, bool backward, int grid, int block, int smem, void* stream) {
+  return with_tape_kernel(backward, p.R == NRLDPC_BG2_ROWS, p.vec != 0, isfinite(p.clip),
+                          [&](auto k) { return launch_tape(k, p, grid, block, smem, stream); });
+}
+
+int occupancy_train_tape(const TrainTapeParams& p, bool backward, int block, int smem) {
+  return with_tape_kernel(backward, p.R == NRLDPC_BG2_ROWS, p.vec != 0, isfinite(p.clip),
+                          [&](auto k) { return occupancy_tape_one(k, block, smem); });
 }
 
 }  // namespace nrldpc
