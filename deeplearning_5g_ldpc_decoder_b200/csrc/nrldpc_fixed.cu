@@ -54,8 +54,10 @@ using namespace fixedrow;
 
 
 // Write the results of code block `cw` (half h of the pair in `lq`) using the
-// Zc threads of its group.
-__device__ void emit_block(const DecodeParams& p, const uint32_t* lq, int zx, int cw, int h, int status,
+// Zc threads of its group.  kPar: the parity columns of rows 4 and up hold rel, and
+// their beliefs need the rows' messages (`msg`: this thread's words in the scratch).
+template <bool kPar>
+__device__ void emit_block(const DecodeParams& p, const uint32_t* lq, const uint32_t* msg, int zx, int cw, int h, int status,
                            int iters) {
   const int shift = 16 * h;
   if (iters > 0 && p.bits) {
@@ -74,7 +76,13 @@ __device__ void emit_block(const DecodeParams& p, const uint32_t* lq, int zx, in
   }
   if (p.app) {
     int16_t* out = reinterpret_cast<int16_t*>(p.app) + (int64_t)cw * p.app_stride;
-    for (int i = zx; i < p.lq_len; i += p.Zc) out[i] = (int16_t)(lq[i] >> shift);
+    const int cols = kPar && iters > 0 ? p.lq_len - (p.R - kCoreRows) * p.Zc : p.lq_len;   // words that hold beliefs
+    for (int i = zx; i < cols; i += p.Zc) out[i] = (int16_t)(lq[i] >> shift);
+    if (kPar && iters > 0)
+      for (int r = kCoreRows; r < p.R; ++r) {
+        const int i = cols + (r - kCoreRows) * p.Zc + zx;
+        out[i] = parity_belief(lq[i], msg + p.lr_off[r], p.row_off[r + 1] - p.row_off[r], h);
+      }
   }
   if (zx == 0) {
     if (p.status) p.status[cw] = status;
@@ -266,7 +274,7 @@ __global__ void __launch_bounds__(kThreadsTarget, 2) fixed_pair_kernel(const __g
           } else {
             ab0 = ab1 = d.z;
           }
-          layer_dispatch<kClip, true, kG1>(row_deg(d.y), p, s_edges, reinterpret_cast<char*>(s_lq), zx4, zxm4, gb4,
+          layer_dispatch<kClip, true, kG1>(row_deg(d.y), row >= kCoreRows, p, s_edges, reinterpret_cast<char*>(s_lq), zx4, zxm4, gb4,
                                            lq_limit, row_e0(d.y), (int32_t)(int16_t)(ab0 & 0xFFFFu), ((int32_t)ab0) >> 16,
                                            (int32_t)(int16_t)(ab1 & 0xFFFFu), ((int32_t)ab1) >> 16, cur, fresh,
                                            scratch + d.x + tid);
@@ -285,7 +293,7 @@ __global__ void __launch_bounds__(kThreadsTarget, 2) fixed_pair_kernel(const __g
           const int ith = (int)(h ? itv >> 16 : itv & 0xFFFFu);
           const bool pass = run && s_crc[2 * g + h] == 0u;
           if (pass || ith >= p.max_it) {
-            emit_block(p, lq, zx, c, h, pass ? 0 : 1, ith);
+            emit_block<parity_words(kClip)>(p, lq, scratch + tid, zx, c, h, pass ? 0 : 1, ith);
             fin[h] = true;
           }
         }
@@ -368,7 +376,7 @@ __global__ void __launch_bounds__(kThreadsTarget, 2) fixed_pair_kernel(const __g
             const uint32_t ab = p.weights_T > 0 ? __ldg(p.weights + (min(it, p.weights_T - 1) * p.R + row)) : d.z;
             const int32_t alpha = (int32_t)(int16_t)(ab & 0xFFFFu);
             const int32_t beta = ((int32_t)ab) >> 16;
-            layer_dispatch<kClip, true, kG1>(row_deg(d.y), p, s_edges, reinterpret_cast<char*>(s_lq), zx4, zxm4, gb4,
+            layer_dispatch<kClip, true, kG1>(row_deg(d.y), row >= kCoreRows, p, s_edges, reinterpret_cast<char*>(s_lq), zx4, zxm4, gb4,
                                              lq_limit, row_e0(d.y), alpha, beta, alpha, beta, cur,
                                              it == 0 ? 0xFFFFFFFFu : 0u, scratch + d.x + tid);
           }
@@ -382,8 +390,8 @@ __global__ void __launch_bounds__(kThreadsTarget, 2) fixed_pair_kernel(const __g
         if (active) {
           pass0 = !done0 && s_crc[2 * g] == 0u;
           pass1 = !done1 && s_crc[2 * g + 1] == 0u;
-          if (pass0) emit_block(p, lq, zx, cw0, 0, 0, it + 1);
-          if (pass1) emit_block(p, lq, zx, cw1, 1, 0, it + 1);
+          if (pass0) emit_block<parity_words(kClip)>(p, lq, scratch + tid, zx, cw0, 0, 0, it + 1);
+          if (pass1) emit_block<parity_words(kClip)>(p, lq, scratch + tid, zx, cw1, 1, 0, it + 1);
           done0 = done0 || pass0;
           done1 = done1 || pass1;
         }
@@ -396,8 +404,8 @@ __global__ void __launch_bounds__(kThreadsTarget, 2) fixed_pair_kernel(const __g
         }
       }
       if (active) {
-        if (!done0) emit_block(p, lq, zx, cw0, 0, 1, it);
-        if (!done1) emit_block(p, lq, zx, cw1, 1, 1, it);
+        if (!done0) emit_block<parity_words(kClip)>(p, lq, scratch + tid, zx, cw0, 0, 1, it);
+        if (!done1) emit_block<parity_words(kClip)>(p, lq, scratch + tid, zx, cw1, 1, 1, it);
       }
       __syncthreads();   // LQ and s_crc are reused by the next work item
     }

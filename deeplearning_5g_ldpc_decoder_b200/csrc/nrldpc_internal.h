@@ -18,6 +18,7 @@ constexpr int kMaxDegree = NRLDPC_MAX_DEGREE;
 constexpr int kMaxZc = NRLDPC_MAX_ZC;
 constexpr int kMaxB = 8448;                  // BG1 K at Zc=384
 constexpr int kThreadsTarget = 384;          // lifted rows handled by one CTA
+constexpr int kCoreRows = 4;                 // rows before those with a parity column of their own
 constexpr int kMaxGroups = kThreadsTarget / 2;  // Zc=2 packs 192 groups
 
 // One base graph with its CSR view (reference layout, for gen_ldpc_parameters)
@@ -77,16 +78,25 @@ inline uint32_t qm_magic(int qm) {
 //  * kClipClamp: clip(rel + msg) is a clamp to [min_llr, max_llr];
 //  * kClipDegen: min_llr > max_llr, where the reference's clip is not a clamp
 //    (exact int32 arithmetic);
-//  * kClipOpenMax: max_llr = 32767 and, in every layer, alpha >= 0 and
-//    beta = 0 (algos 1 and 3): the minima need no clip, the offset step is the
+//  * kClipOpenMax: max_llr = 32767, min_llr <= -32767 and, in every layer, alpha >= 0
+//    and beta = 0 (algos 1 and 3): the minima need no clip, the offset step is the
 //    identity, the scaled minima lie in [0, 32766], and the clamp of the new
 //    beliefs is a max with min_llr.  This is the reference's default decoder
 //    row.
 // `ab` holds each layer's packed alpha | beta << 16 as the kernels read it.
 enum { kClipClamp = 0, kClipDegen = 1, kClipOpenMax = 2 };
+// Whether the parity columns of rows 4 and up hold the row's extrinsic input
+// instead of the belief (nrldpc_fixed_row.cuh).  Only with the open maximum: the
+// check that the clip keeps the sum is then one packed add.  In the clamp
+// variant the check and its branch made converging batches slower (1001 blocks of
+// BG1 Zc=384, algo 2: 1232 -> 1310 us), although 8192 got 2 % faster.
+#ifdef __CUDACC__
+__host__ __device__
+#endif
+constexpr bool parity_words(int clip) { return clip == kClipOpenMax; }
 inline int fixed_clip_mode(const ldpc_decoder_cfg_t& dc, const uint32_t* ab, int rows) {
   if (dc.min_llr > dc.max_llr) return kClipDegen;
-  if ((dc.algo != 1 && dc.algo != 3) || dc.max_llr != 32767) return kClipClamp;
+  if ((dc.algo != 1 && dc.algo != 3) || dc.max_llr != 32767 || dc.min_llr > -32767) return kClipClamp;
   for (int r = 0; r < rows; ++r)
     if ((ab[r] >> 15) != 0u) return kClipClamp;   // alpha < 0 (bit 15) or beta != 0 (bits 16-31)
   return kClipOpenMax;

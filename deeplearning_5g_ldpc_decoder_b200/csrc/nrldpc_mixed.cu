@@ -258,7 +258,7 @@ __global__ void __launch_bounds__(kThreads, kMinBlocks) fixed_mixed_kernel(const
           } else {
             ab0 = ab1 = d.z;
           }
-          layer_dispatch<kClip, true, false>(row_deg(d.y), p, s_g.edges, reinterpret_cast<char*>(s_lq), zx4, zxm4, gb4,
+          layer_dispatch<kClip, true, false>(row_deg(d.y), row >= kCoreRows, p, s_g.edges, reinterpret_cast<char*>(s_lq), zx4, zxm4, gb4,
                                            4u * (uint32_t)(G * lq_len), row_e0(d.y),
                                            (int32_t)(int16_t)(ab0 & 0xFFFFu), ((int32_t)ab0) >> 16,
                                            (int32_t)(int16_t)(ab1 & 0xFFFFu), ((int32_t)ab1) >> 16, cur, fresh,

@@ -105,3 +105,45 @@ def test_upper_clamp_at_32767_is_identity_on_int16():
     s = np.arange(-32768, 32768, dtype=np.int64)
     for min_llr in (-32768, -32767, -10000, 0):
         assert np.array_equal(np.minimum(np.maximum(s, min_llr), 32767), np.maximum(s, min_llr))
+
+
+def test_parity_word_keeps_the_belief():
+    """The parity-column form of the open-max row: the word holds rel; unless |rel| + min2 has its top bit set (unsigned
+    16 bits), clip(rel + msg) - msg is rel, and otherwise the word becomes clip(rel + msg) - msg.  Word + message is the
+    belief of the plain form in every case, over many iterations of one edge."""
+    rng = np.random.default_rng(5)
+    n = 20000
+    for mn in (-32767, -32768):
+        belief = rng.choice([-32768, -32767, -20000, -1, 0, 1, 12345, 32767], n)
+        belief = np.where(rng.random(n) < 0.5, belief, rng.integers(-32768, 32768, n)).astype(np.int64)
+        word, msg = belief.copy(), np.zeros(n, dtype=np.int64)
+        for _ in range(12):
+            rel = ((belief - msg + 32768) & 0xFFFF) - 32768            # int16 wrap of LQ - old message
+            assert np.array_equal(rel, word)
+            s2 = rng.integers(0, 32767, n)                              # scaled minima lie in [0, 32766]
+            msg = np.where(rng.random(n) < 0.5, s2, rng.integers(0, s2 + 1)) * rng.choice([-1, 1], n)
+            belief = np.clip(rel + msg, mn, 32767)
+            odd = ((np.abs(word) + s2) & 0x8000) != 0
+            assert np.array_equal(np.where(odd, rel, belief - msg), rel)
+            word = np.where(odd, ((belief - msg + 32768) & 0xFFFF) - 32768, word)
+            assert np.array_equal(((word + msg + 32768) & 0xFFFF) - 32768, belief)
+
+
+def test_open_scaling_is_a_byte_permute():
+    """(2 alpha m + 2^15) >> 16 equals (alpha m + 2^14) >> 15 in 32 unsigned bits for m, alpha in [0, 32767]."""
+    m = np.arange(32768, dtype=np.uint64)
+    for alpha in (0, 1, 22527, 22936, 26623, 32766, 32767):
+        wide = m * np.uint64(2 * alpha) + np.uint64(1 << 15)
+        assert wide.max() < 1 << 32
+        assert np.array_equal(wide >> np.uint64(16), (m * np.uint64(alpha) + np.uint64(1 << 14)) >> np.uint64(15))
+
+
+def test_extension_rows_end_in_their_own_unshifted_parity_column(oracle):
+    from oracle.oracle import in_config
+
+    for bgn, kb, A in ((1, 22, 8424), (2, 10, 3816), (1, 22, 488), (2, 10, 120)):
+        p, col, shift, off = oracle.graph(in_config(bgn, A, 1, 960, 0, 2, 0))
+        for r in range(4, p.rows):
+            e = int(off[r + 1]) - 1
+            assert int(col[e]) == kb + r and int(shift[e]) % p.Zc == 0
+            assert (np.asarray(col[: int(off[p.rows])]) == kb + r).sum() == 1
