@@ -21,10 +21,11 @@
 //    Qm interleaved streams as 32-bit windows of that buffer.
 //  * 32 symbols are interleaved at once: an 8 x 8 bit transpose per 8 symbols
 //    gives one byte per symbol, and Qm < 8 packs the bytes' top Qm bits.
-// The kernel is bound by instruction issue (about 2000 warp instructions for a
-// BG1 Zc=384 block, a third of them the CRC) and, for one block, by the latency
-// of its eight phases.  4096 blocks of BG1 Zc=384, E=25344, Qm=8: 783 us with
-// one byte per bit and a gather per output bit, 51 us in this form.
+// The kernel is bound by instruction issue (about 8000 warp instructions for a
+// BG1 Zc=384 block, 60 % of the issue slots; leaving out the CRC saves 15 % of the
+// time, the interleave 16 %, the extension rows 11 %) and, for one block, by the
+// latency of its eight phases.  4096 blocks of BG1 Zc=384, E=25344, Qm=8: 783 us with
+// one byte per bit and a gather per output bit, 47 us in this form.
 #include <cuda_runtime.h>
 #include <stdint.h>
 
@@ -101,8 +102,10 @@ __device__ __forceinline__ uint32_t pack_symbols(uint32_t t) {
 
 // Rate-matched bytes of one block from its compacted circular buffer: 32 symbols
 // (Qm words) per thread and step.
+// stream[b]: buffer position of bit 0 of stream b.
 template <int Qm>
-__device__ __forceinline__ void rate_match(const EncodeParams& p, const uint32_t* comp, uint8_t* out, bool vec) {
+__device__ __forceinline__ void rate_match(const EncodeParams& p, const uint32_t* comp, const uint32_t* stream, uint8_t* out,
+                                           bool vec) {
   const int nbytes = (p.E + 7) >> 3;
   for (int s0 = 32 * threadIdx.x; s0 < p.symbols; s0 += 32 * blockDim.x) {
     const int left = p.symbols - s0;
@@ -111,9 +114,12 @@ __device__ __forceinline__ void rate_match(const EncodeParams& p, const uint32_t
     for (int b = 0; b < 8; ++b) {
       v[b] = 0u;
       if (b < Qm) {
-        // stream b starts at de-interleaved bit b (E / Qm); E may exceed Nv (repetition)
-        const uint32_t k = (uint32_t)(p.c0 + b * p.symbols + s0);
-        v[b] = window32(comp, (uint32_t)p.Nv, k % (uint32_t)p.Nv);
+        uint32_t c = stream[b] + (uint32_t)s0;
+        if (c >= (uint32_t)p.Nv) {
+          c -= (uint32_t)p.Nv;
+          if (c >= (uint32_t)p.Nv) c %= (uint32_t)p.Nv;   // E beyond the buffer: repetition
+        }
+        v[b] = window32(comp, (uint32_t)p.Nv, c);
         if (left < 32) v[b] &= (1u << left) - 1u;
         v[b] = __brev(v[b]);   // symbol s0 on top
       }
@@ -172,15 +178,16 @@ __device__ __forceinline__ void rate_match(const EncodeParams& p, const uint32_t
   }
 }
 
-__global__ void __launch_bounds__(kEncThreads) encode_kernel(const __grid_constant__ EncodeParams p) {
+__global__ void __launch_bounds__(kEncThreads, 12) encode_kernel(const __grid_constant__ EncodeParams p) {
   __shared__ uint32_t s_lin[(kMaxB + 31) / 32 + 3];            // K systematic bits: payload, CRC, filler zeros
-  __shared__ uint32_t s_col[kEncCols * kEncDoubled];           // doubled columns, W2 words each
-  __shared__ uint32_t s_comp[(66 * kMaxZc + 31) / 32 + 3];     // compacted circular buffer
+  __shared__ uint32_t s_col[kEncCols * kEncDoubled + 2];       // doubled columns, W2 words each (and two read past the last)
+  __shared__ uint32_t s_comp[(66 * kMaxZc + 31) / 32 + 4];     // compacted circular buffer
   __shared__ uint32_t s_par[4][kEncZcWords + 2];               // core parities, Zc bits each
   __shared__ uint32_t s_L[4][kEncZcWords + 2];                 // syndromes, then [0]: their sum
   __shared__ uint32_t s_sum[kEncZcWords + 2];
   __shared__ uint32_t s_edge[kMaxNnz];                         // word offset in s_col | bit shift << 16
   __shared__ uint16_t s_off[kMaxRows + 1];
+  __shared__ uint32_t s_stream[8];
   __shared__ uint32_t s_crc;
   const int tid = threadIdx.x, nt = blockDim.x;
   const uint32_t Zc = (uint32_t)p.Zc;
@@ -189,11 +196,15 @@ __global__ void __launch_bounds__(kEncThreads) encode_kernel(const __grid_consta
   const uint32_t last = (Zc & 31u) ? (1u << (Zc & 31u)) - 1u : 0xFFFFFFFFu;   // valid bits of a column's last word
   const int info_bits = p.B - 2 * p.Zc;                        // systematic bits of the circular buffer
   const int info_words = (info_bits + 31) >> 5;
-  const int comp_words = ((info_bits + p.R * p.Zc + 31) >> 5) + 2;
+  const int comp_words = ((info_bits + p.R * p.Zc + 31) >> 5) + 3;
   const int lin_words = ((p.K + 31) >> 5) + 2;
-  const uint32_t mul_w2 = 65536u / (uint32_t)W2 + 1u, mul_w = 65536u / (uint32_t)W + 1u;   // exact for the small indices below
+  const uint32_t mul_w2 = 65536u / (uint32_t)W2 + 1u, mul_w = 65536u / (uint32_t)W + 1u;
+  const uint32_t mul_w1 = 65536u / (uint32_t)((W + 1) >> 1) + 1u;   // exact for the small indices below
   for (int e = tid; e < p.num_edges; e += nt) s_edge[e] = p.edge[e];
   for (int r = tid; r <= p.R; r += nt) s_off[r] = p.row_off[r];
+  // stream b of the interleave starts at de-interleaved bit b (E / Qm)
+  if (tid < p.Qm) s_stream[tid] = (uint32_t)(p.c0 + tid * p.symbols) % (uint32_t)p.Nv;
+  const bool whole = (p.Zc & 31) == 0;   // columns are whole words: no shifts where they are only copied
 
   for (int cw = blockIdx.x; cw < p.num_cw; cw += gridDim.x) {
     const uint8_t* info = p.info + (int64_t)cw * p.info_stride;
@@ -232,6 +243,13 @@ __global__ void __launch_bounds__(kEncThreads) encode_kernel(const __grid_consta
     // Doubled systematic columns, and the systematic part of the circular buffer.
     for (int k = tid; k < p.Kb * W2; k += nt) {
       const uint32_t c = ((uint32_t)k * mul_w2) >> 16;
+      if (whole) {
+        int w = k - (int)c * W2;
+        w -= w >= W ? W : 0;
+        w -= w >= W ? W : 0;   // the word after the second copy
+        s_col[k] = s_lin[(int)c * W + w];
+        continue;
+      }
       uint32_t start = 32u * ((uint32_t)k - c * (uint32_t)W2);
       while (start >= Zc) start -= Zc;
       s_col[k] = cyclic32(s_lin, c * Zc, Zc, start);
@@ -295,33 +313,46 @@ __global__ void __launch_bounds__(kEncThreads) encode_kernel(const __grid_consta
       s_col[p.Kb * W2 + k] = cyclic32(s_par[c], 0u, Zc, start);
     }
     __syncthreads();
-    // Every row's parity word: rows 0..3 are solved, an extension row is the XOR
-    // over its systematic + core columns.
-    for (int k = tid; k < p.R * W; k += nt) {
-      const int r = (int)(((uint32_t)k * mul_w) >> 16), w = k - r * W;
-      uint32_t s = 0u;
+    // Every row's parity words: rows 0..3 are solved, an extension row is the XOR
+    // over its systematic + core columns.  Two words per thread share an edge's
+    // record and the word between them.
+    const int W1 = (W + 1) >> 1;
+    for (int k = tid; k < p.R * W1; k += nt) {
+      const int r = (int)(((uint32_t)k * mul_w1) >> 16), w = 2 * (k - r * W1);
+      uint32_t s0 = 0u, s1 = 0u;
       if (r < 4) {
-        s = s_par[r][w];
+        s0 = s_par[r][w];
+        s1 = s_par[r][w + 1];
       } else {
-        for (int e = s_off[r]; e < s_off[r + 1]; ++e) {
+        const int e1 = s_off[r + 1];
+#pragma unroll 2
+        for (int e = s_off[r]; e < e1; ++e) {
           const uint32_t ed = s_edge[e];
           const uint32_t* a = s_col + (ed & 0xFFFFu) + w;
-          s ^= __funnelshift_r(a[0], a[1], ed >> 16);
+          const uint32_t mid = a[1];
+          s0 ^= __funnelshift_r(a[0], mid, ed >> 16);
+          s1 ^= __funnelshift_r(mid, a[2], ed >> 16);   // (unused past the last word)
         }
-        if (w == W - 1) s &= last;
+        if (w == W - 1) s0 &= last;
+        if (w + 1 == W - 1) s1 &= last;
       }
-      const uint32_t pos = (uint32_t)(info_bits + r * p.Zc + 32 * w);
-      atomicOr(&s_comp[pos >> 5], s << (pos & 31u));
-      if (pos & 31u) atomicOr(&s_comp[(pos >> 5) + 1], s >> (32u - (pos & 31u)));
+      if (w + 1 >= W) s1 = 0u;
+      const uint32_t pos = (uint32_t)(info_bits + r * p.Zc + 32 * w), sh = pos & 31u;
+      uint32_t* d = s_comp + (pos >> 5);
+      atomicOr(d, s0 << sh);
+      const uint32_t carry = __funnelshift_l(s0, s1, sh);   // s1 << sh | s0 >> (32 - sh)
+      if (carry) atomicOr(d + 1, carry);
+      const uint32_t top = sh ? s1 >> (32u - sh) : 0u;
+      if (top) atomicOr(d + 2, top);
     }
     __syncthreads();
     uint8_t* out = p.rm + (int64_t)cw * p.rm_stride;
     switch (p.Qm) {
-      case 1: rate_match<1>(p, s_comp, out, p.rm_vec != 0); break;
-      case 2: rate_match<2>(p, s_comp, out, p.rm_vec != 0); break;
-      case 4: rate_match<4>(p, s_comp, out, p.rm_vec != 0); break;
-      case 6: rate_match<6>(p, s_comp, out, p.rm_vec != 0); break;
-      default: rate_match<8>(p, s_comp, out, p.rm_vec != 0); break;
+      case 1: rate_match<1>(p, s_comp, s_stream, out, p.rm_vec != 0); break;
+      case 2: rate_match<2>(p, s_comp, s_stream, out, p.rm_vec != 0); break;
+      case 4: rate_match<4>(p, s_comp, s_stream, out, p.rm_vec != 0); break;
+      case 6: rate_match<6>(p, s_comp, s_stream, out, p.rm_vec != 0); break;
+      default: rate_match<8>(p, s_comp, s_stream, out, p.rm_vec != 0); break;
     }
     __syncthreads();   // the shared arrays are reused by the next block
   }
