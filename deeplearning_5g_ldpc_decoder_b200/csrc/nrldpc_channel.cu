@@ -56,14 +56,12 @@ __constant__ Seg kQam256[4][15] = {
 };
 __constant__ int kQam256N[4] = {15, 14, 12, 8};
 
-// x / nv, correctly rounded.  kFast: from r = RN(1 / nv), two remainder steps
+// x / nv, correctly rounded, from r = RN(1 / nv) by two remainder steps
 // (Markstein's theorem: with a correctly rounded reciprocal and a quotient
 // within an ulp, q + r (x - q nv) in fused operations rounds correctly).  The
 // host asks for it only where neither the reciprocal nor a remainder can leave
 // the normal range.
-template <bool kFast>
 __device__ __forceinline__ float div_nv(float x, float nv, float r) {
-  if constexpr (!kFast) return __fdiv_rn(x, nv);
   float q = __fmul_rn(x, r);
   q = __fmaf_rn(__fmaf_rn(-q, nv, x), r, q);
   return __fmaf_rn(__fmaf_rn(-q, nv, x), r, q);
@@ -84,19 +82,48 @@ __device__ __forceinline__ uint64_t splitmix(uint64_t z) {
 }
 
 // PAM cell of r for 2^m levels spaced 2A: the number of boundaries
-// (2 c - 2^m) A, c = 1 .. 2^m - 1, that r is not below.  The estimate from a
-// multiply is off by one at most and is settled by the boundaries themselves.
+// (2 c - 2^m) A, c = 1 .. 2^m - 1, that r is not below.  The cell is the floor of
+// r / 2A + 2^(m-1), held a quarter away from the ends of the range (a NaN gives
+// cell 0); that estimate is within 1e-5 of the exact quotient, so only
+// one within 1e-4 of an integer needs the boundaries themselves.
 template <int m>
 __device__ __forceinline__ int pam_cell(float r, float A, float inv_2a) {
   constexpr int n = 1 << m;
-  int c = (int)floorf(__fmaf_rn(r, inv_2a, (float)(n / 2)));
-  c = min(max(c, 0), n - 1);
-  if (c > 0 && r < __fmul_rn((float)(2 * c - n), A)) {
-    --c;
-  } else if (c < n - 1 && !(r < __fmul_rn((float)(2 * c + 2 - n), A))) {
-    ++c;
+  const float x = fminf(fmaxf(__fmaf_rn(r, inv_2a, (float)(n / 2)), 0.25f), (float)n - 0.25f);
+  const float t = __fadd_rz(x, 8388608.0f);   // 2^23 + floor(x): the floor in the low mantissa bits
+  int c = (int)(__float_as_uint(t) & (uint32_t)(n - 1));
+  const float d = x - (t - 8388608.0f);
+  if (fabsf(d - 0.5f) > 0.4999f) {
+    if (c > 0 && r < __fmul_rn((float)(2 * c - n), A)) {
+      --c;
+    } else if (c < n - 1 && !(r < __fmul_rn((float)(2 * c + 2 - n), A))) {
+      ++c;
+    }
   }
   return c;
+}
+
+// Two quantised LLRs in one word, from scaled = 128 LLR (finite): the integer part
+// of |scaled| + 0.5, at most 10000, taken from the mantissa after a truncating
+// add of 2^23, and the signs applied to both halves at once.
+__device__ __forceinline__ uint32_t quantize_pair(float s0, float s1) {
+  const float n0 = __fadd_rz(fminf(__fadd_rn(fabsf(s0), 0.5f), 10000.5f), 8388608.0f);
+  const float n1 = __fadd_rz(fminf(__fadd_rn(fabsf(s1), 0.5f), 10000.5f), 8388608.0f);
+  const uint32_t n = __byte_perm(__float_as_uint(n0), __float_as_uint(n1), 0x5410);
+  uint32_t neg;   // all ones in the half of a negative value
+  asm("prmt.b32 %0, %1, %2, 0xFFBB;" : "=r"(neg) : "r"(__float_as_uint(s0)), "r"(__float_as_uint(s1)));
+  return __vadd2(n ^ neg, neg & 0x00010001u);
+}
+
+// 128 x / nv.  Scaling by a power of two commutes with the rounding of the
+// division, so the fast form divides 128 x.
+template <bool kFast>
+__device__ __forceinline__ uint32_t llr_pair(float x0, float x1, float nv, float rnv) {
+  if constexpr (kFast) {
+    return quantize_pair(div_nv(x0, nv, rnv), div_nv(x1, nv, rnv));
+  } else {
+    return (uint32_t)(uint16_t)quantize(__fdiv_rn(x0, nv)) | (uint32_t)(uint16_t)quantize(__fdiv_rn(x1, nv)) << 16;
+  }
 }
 
 constexpr int kChannelThreads = 256;
@@ -104,22 +131,26 @@ constexpr int kGroup = 4;   // symbols per thread and step
 
 // One thread takes four consecutive symbols: their 4 Qm bits start on a nibble,
 // and their 4 Qm LLRs are one run of 8 Qm bytes, stored 16 bytes at a time
-// where rows are aligned (kVec).  Every pair's max-log line is looked up by
-// the PAM cell of the coordinate (one cell per coordinate serves all Qm / 2
-// pairs) in a shared table of 8-byte entries, at most 16 per pair, which no
-// lane pattern makes conflict; the division by the noise power, the same for
-// every LLR, is a multiplication and two remainder steps.  Bound by
-// instruction issue: the counter generator's four 64-bit products, logf, sqrtf
-// and sincospif per symbol, then about 15 instructions per LLR.
+// where rows are aligned (`vec`).  The symbol's point and every pair's max-log line
+// come from shared tables, the line by the PAM cell of the coordinate (one cell
+// per coordinate serves all Qm / 2 pairs); the line's 8-byte entries, at most 16
+// per pair, conflict for no lane pattern.  The division by the noise power, the
+// same for every LLR, is a multiplication and two remainder steps, and nothing is
+// converted on the slow conversion pipe.  Bound by instruction issue: the counter
+// generator's four 64-bit products, logf, sqrtf and sincospif per symbol take half
+// of it, then 13 instructions per LLR.
 // 2048 x 25344 LLRs, 64QAM: 286 us with one symbol per thread, a search of the
-// segments in constant memory and 2-byte stores, 107 us in this form.
+// segments in constant memory and 2-byte stores; 107 us with the tables for the
+// lines alone; 84 us in this form.
 template <int Qm, bool kFast>
 __global__ void __launch_bounds__(kChannelThreads) channel_kernel(const uint8_t* __restrict__ rm, int64_t rm_stride, int32_t num_cw, int32_t E,
                                float nv, float sigma, float A, uint64_t seed,
                                int16_t* __restrict__ llr, int64_t llr_stride, float* __restrict__ symbols, bool vec) {
   constexpr int m = Qm > 2 ? Qm / 2 : 1, kCells = 1 << m;
-  // per pair and cell: s c1 A and c2 A of the line (c1 A) (s r + c2 A); c1 A > 0
+  constexpr float kScale = kFast ? 128.0f : 1.0f;   // the fast form divides 128 x (llr_pair)
+  // per pair and cell: s c1 A (scaled) and c2 A of the line (c1 A) (s r + c2 A); c1 A > 0
   __shared__ float2 s_line[m][kCells];
+  __shared__ float2 s_point[1 << Qm];   // constellation
   if constexpr (Qm > 2) {
     for (int k = threadIdx.x; k < m * kCells; k += blockDim.x) {
       const int p = k / kCells, c = k - p * kCells;
@@ -127,10 +158,11 @@ __global__ void __launch_bounds__(kChannelThreads) channel_kernel(const uint8_t*
       const int n = Qm == 4 ? kQam16N[p & 1] : Qm == 6 ? kQam64N[p % 3] : kQam256N[p & 3];
       int j = 0;
       while (j < n - 1 && seg[j].thr <= (float)(2 * c - kCells)) ++j;   // segments the cell lies above
-      s_line[p][c] = make_float2(copysignf(__fmul_rn(seg[j].c1, A), seg[j].s), __fmul_rn(seg[j].c2, A));
+      s_line[p][c] = make_float2(copysignf(__fmul_rn(__fmul_rn(seg[j].c1, A), kScale), seg[j].s), __fmul_rn(seg[j].c2, A));
     }
-    __syncthreads();
   }
+  for (int k = threadIdx.x; k < (1 << Qm); k += blockDim.x) s_point[k] = map_symbol<Qm>((uint32_t)k, A);
+  __syncthreads();
   const float rnv = kFast ? __frcp_rn(nv) : 0.0f;
   const float inv_2a = 0.5f / A;
   const uint32_t nsym = (uint32_t)(E / Qm);
@@ -155,25 +187,7 @@ __global__ void __launch_bounds__(kChannelThreads) channel_kernel(const uint8_t*
     uint32_t q[2 * Qm];   // 4 Qm int16 LLRs
 #pragma unroll
     for (int i = 0; i < kGroup; ++i) {
-      const auto sign = [&](int j) { return (int32_t)(word << (i * Qm + j)) < 0 ? -1.0f : 1.0f; };   // 1 - 2 b_j
-      float re, im;
-      if constexpr (Qm == 1) {
-        re = im = __fmul_rn(sign(0), A);
-      } else if constexpr (Qm == 2) {
-        re = __fmul_rn(sign(0), A);
-        im = __fmul_rn(sign(1), A);
-      } else if constexpr (Qm == 4) {
-        re = __fmul_rn(__fmul_rn(sign(0), __fsub_rn(2.0f, sign(2))), A);
-        im = __fmul_rn(__fmul_rn(sign(1), __fsub_rn(2.0f, sign(3))), A);
-      } else if constexpr (Qm == 6) {
-        re = __fmul_rn(__fmul_rn(sign(0), __fsub_rn(4.0f, __fmul_rn(sign(2), __fsub_rn(2.0f, sign(4))))), A);
-        im = __fmul_rn(__fmul_rn(sign(1), __fsub_rn(4.0f, __fmul_rn(sign(3), __fsub_rn(2.0f, sign(5))))), A);
-      } else {
-        re = __fmul_rn(__fmul_rn(sign(0), __fsub_rn(8.0f, __fmul_rn(sign(2), __fsub_rn(4.0f,
-                       __fmul_rn(sign(4), __fsub_rn(2.0f, sign(6))))))), A);
-        im = __fmul_rn(__fmul_rn(sign(1), __fsub_rn(8.0f, __fmul_rn(sign(3), __fsub_rn(4.0f,
-                       __fmul_rn(sign(5), __fsub_rn(2.0f, sign(7))))))), A);
-      }
+      const float2 point = s_point[(word >> (32 - (i + 1) * Qm)) & ((1u << Qm) - 1u)];
       // Box-Muller from a counter-based generator.
       const uint64_t z = splitmix(seed ^ splitmix(((uint64_t)cw << 32) ^ (uint64_t)(s0 + i)));
       const float u1 = ((float)(z >> 40) + 1.0f) * (1.0f / 16777218.0f);
@@ -181,33 +195,30 @@ __global__ void __launch_bounds__(kChannelThreads) channel_kernel(const uint8_t*
       const float rad = sqrtf(-2.0f * logf(u1));
       float sn, cs;
       sincospif(2.0f * u2, &sn, &cs);
-      re = __fadd_rn(re, __fmul_rn(sigma, __fmul_rn(rad, cs)));
-      im = __fadd_rn(im, __fmul_rn(sigma, __fmul_rn(rad, sn)));
+      const float re = __fadd_rn(point.x, __fmul_rn(sigma, __fmul_rn(rad, cs)));
+      const float im = __fadd_rn(point.y, __fmul_rn(sigma, __fmul_rn(rad, sn)));
       if (symbols && (uint32_t)i < left) {
         float* o = symbols + 2 * ((int64_t)cw * nsym + s0 + i);
         o[0] = re;
         o[1] = im;
       }
-      const auto put = [&](int j, int16_t v) {   // LLR j of symbol i
-        const int k = i * Qm + j;
-        if (k & 1) q[k >> 1] |= (uint32_t)(uint16_t)v << 16;
-        else q[k >> 1] = (uint32_t)(uint16_t)v;
-      };
       if constexpr (Qm == 1) {
-        put(0, quantize(div_nv<kFast>(__fmul_rn(__fmul_rn(4.0f, __fadd_rn(re, im)), A), nv, rnv)));
+        const float x = __fmul_rn(__fmul_rn(__fmul_rn(4.0f, __fadd_rn(re, im)), A), kScale);
+        const uint32_t v = llr_pair<kFast>(x, x, nv, rnv);
+        q[i >> 1] = i & 1 ? (q[i >> 1] & 0xFFFFu) | (v & 0xFFFF0000u) : v;
       } else if constexpr (Qm == 2) {
-        put(0, quantize(div_nv<kFast>(__fmul_rn(__fmul_rn(4.0f, re), A), nv, rnv)));
-        put(1, quantize(div_nv<kFast>(__fmul_rn(__fmul_rn(4.0f, im), A), nv, rnv)));
+        q[i] = llr_pair<kFast>(__fmul_rn(__fmul_rn(__fmul_rn(4.0f, re), A), kScale),
+                               __fmul_rn(__fmul_rn(__fmul_rn(4.0f, im), A), kScale), nv, rnv);
       } else {
         const int cr = pam_cell<m>(re, A, inv_2a), ci = pam_cell<m>(im, A, inv_2a);
+        // (c1 A) (s r + c2 A): the sign of the table's first entry is s
+        const auto line = [](float2 l, float r) {
+          const float sr = __uint_as_float(__float_as_uint(r) ^ (__float_as_uint(l.x) & 0x80000000u));
+          return __fmul_rn(fabsf(l.x), __fadd_rn(sr, l.y));
+        };
 #pragma unroll
-        for (int p = 0; p < m; ++p) {
-          const float2 lr = s_line[p][cr], li = s_line[p][ci];
-          const float xr = __fmul_rn(fabsf(lr.x), __fadd_rn(__fmul_rn(copysignf(1.0f, lr.x), re), lr.y));
-          const float xi = __fmul_rn(fabsf(li.x), __fadd_rn(__fmul_rn(copysignf(1.0f, li.x), im), li.y));
-          put(2 * p, quantize(div_nv<kFast>(xr, nv, rnv)));
-          put(2 * p + 1, quantize(div_nv<kFast>(xi, nv, rnv)));
-        }
+        for (int p = 0; p < m; ++p)
+          q[i * m + p] = llr_pair<kFast>(line(s_line[p][cr], re), line(s_line[p][ci], im), nv, rnv);
       }
     }
     int16_t* out = llr + (int64_t)cw * llr_stride + (int64_t)s0 * Qm;
