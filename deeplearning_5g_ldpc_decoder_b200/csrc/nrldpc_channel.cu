@@ -126,6 +126,32 @@ __device__ __forceinline__ uint32_t llr_pair(float x0, float x1, float nv, float
   }
 }
 
+// Constellation point of the Qm bits in the low bits of w, first bit on top, by
+// the reference's float expressions.
+template <int Qm>
+__device__ __forceinline__ float2 map_symbol(uint32_t w, float A) {
+  const auto sign = [&](int j) { return (w >> (Qm - 1 - j)) & 1u ? -1.0f : 1.0f; };   // 1 - 2 b_j
+  float re, im;
+  if constexpr (Qm == 1) {
+    re = im = __fmul_rn(sign(0), A);
+  } else if constexpr (Qm == 2) {
+    re = __fmul_rn(sign(0), A);
+    im = __fmul_rn(sign(1), A);
+  } else if constexpr (Qm == 4) {
+    re = __fmul_rn(__fmul_rn(sign(0), __fsub_rn(2.0f, sign(2))), A);
+    im = __fmul_rn(__fmul_rn(sign(1), __fsub_rn(2.0f, sign(3))), A);
+  } else if constexpr (Qm == 6) {
+    re = __fmul_rn(__fmul_rn(sign(0), __fsub_rn(4.0f, __fmul_rn(sign(2), __fsub_rn(2.0f, sign(4))))), A);
+    im = __fmul_rn(__fmul_rn(sign(1), __fsub_rn(4.0f, __fmul_rn(sign(3), __fsub_rn(2.0f, sign(5))))), A);
+  } else {
+    re = __fmul_rn(__fmul_rn(sign(0), __fsub_rn(8.0f, __fmul_rn(sign(2), __fsub_rn(4.0f,
+                   __fmul_rn(sign(4), __fsub_rn(2.0f, sign(6))))))), A);
+    im = __fmul_rn(__fmul_rn(sign(1), __fsub_rn(8.0f, __fmul_rn(sign(3), __fsub_rn(4.0f,
+                   __fmul_rn(sign(5), __fsub_rn(2.0f, sign(7))))))), A);
+  }
+  return make_float2(re, im);
+}
+
 constexpr int kChannelThreads = 256;
 constexpr int kGroup = 4;   // symbols per thread and step
 
