@@ -53,18 +53,45 @@ struct SegParams {
   int16_t key_by_rank[kKeys];     // keys in descending work per block; -1 past the end
 };
 
+// Inclusive scan of one value per thread over the CTA (32 warps); s_warp: 32 words.
+__device__ __forceinline__ int block_scan(int v, int* s_warp) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const int u = __shfl_up_sync(0xFFFFFFFFu, v, o);
+    if (lane >= o) v += u;
+  }
+  if (lane == 31) s_warp[warp] = v;
+  __syncthreads();
+  if (warp == 0) {
+    int w = s_warp[lane];
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int u = __shfl_up_sync(0xFFFFFFFFu, w, o);
+      if (lane >= o) w += u;
+    }
+    s_warp[lane] = w;
+  }
+  __syncthreads();
+  return v + (warp > 0 ? s_warp[warp - 1] : 0);
+}
+
+// One CTA: the whole batch's code-block list needs one scan.  Bound by latency, so
+// no step is serial over blocks or graphs: a thread per transport block counts,
+// a thread per code block (found by a binary search of the scan) writes its
+// descriptor, a thread per graph its queue.  32 transport blocks, 155 code blocks:
+// 25.7 us with a thread per transport block writing all its code blocks and one
+// thread walking the graphs, 8.5 us in this form.
 __global__ void __launch_bounds__(kSegThreads) tb_segment_kernel(const nrldpc_tb_t* __restrict__ tbs, int n,
                                                                  const __grid_constant__ SegParams sp) {
-  __shared__ int s_scan[kSegThreads];
-  __shared__ int s_count[kKeys], s_cursor[kKeys], s_item_base[kKeys], s_cb_base[kKeys], s_items[kKeys];
-  __shared__ int s_total, s_num_items, s_err;
+  __shared__ int s_warp[32];
+  __shared__ int s_count[kKeys], s_cursor[kKeys], s_cb_base[kKeys], s_item_end[kKeys], s_rank_key[kKeys];
   const int tid = threadIdx.x;
   if (tid < kKeys) {
     s_count[tid] = 0;
     s_cursor[tid] = 0;
-    s_items[tid] = 0;
+    s_rank_key[tid] = sp.key_by_rank[tid];
   }
-  if (tid == 0) s_err = 0;
   // 1. code blocks per transport block, contiguous chunk of blocks per thread
   const int per = (n + kSegThreads - 1) / kSegThreads;
   const int t0 = min(n, tid * per), t1 = min(n, t0 + per);
@@ -74,19 +101,12 @@ __global__ void __launch_bounds__(kSegThreads) tb_segment_kernel(const nrldpc_tb
     int e = tb_segment(tbs[t].A, tbs[t].G, tbs[t].Qm, tbs[t].bgn, tbs[t].tbs_lbrm, &s);
     if (!e && tbs[t].rv > 3) e = kTbBadArg;
     sp.tb_err[t] = e;
+    sp.tb_first[t] = local;   // within the thread's chunk, for now
     if (!e) local += s.C;
   }
-  s_scan[tid] = local;
-  __syncthreads();
-  for (int off = 1; off < kSegThreads; off <<= 1) {   // inclusive Hillis-Steele scan
-    const int v = tid >= off ? s_scan[tid - off] : 0;
-    __syncthreads();
-    s_scan[tid] += v;
-    __syncthreads();
-  }
-  if (tid == kSegThreads - 1) s_total = s_scan[tid];
-  __syncthreads();
-  const int total = s_total;
+  const int end = block_scan(local, s_warp);
+  const int total = s_warp[31];
+  for (int t = t0; t < t1; ++t) sp.tb_first[t] += end - local;
   if (total > sp.max_cbs) {   // over capacity: nothing decodes, every block reports -4
     if (tid == 0) {
       sp.num_items[0] = 0;
@@ -95,58 +115,57 @@ __global__ void __launch_bounds__(kSegThreads) tb_segment_kernel(const nrldpc_tb
     }
     return;
   }
-  // 2. code-block descriptors
-  int cb = s_scan[tid] - local;
-  for (int t = t0; t < t1; ++t) {
-    sp.tb_first[t] = cb;
-    if (sp.tb_err[t]) continue;
+  __syncthreads();   // tb_first and tb_err of all blocks, s_warp read
+  // 2. code-block descriptors: the block of code block cb is the last one that
+  // starts at or before it and has code blocks (invalid ones have none and share
+  // their start with the next)
+  for (int cb = tid; cb < total; cb += kSegThreads) {
+    int lo = 0, hi = n - 1;
+    while (lo < hi) {
+      const int mid = (lo + hi + 1) >> 1;
+      if (sp.tb_first[mid] <= cb) lo = mid;
+      else hi = mid - 1;
+    }
+    while (sp.tb_err[lo]) --lo;
+    const nrldpc_tb_t tb = tbs[lo];
+    const int r = cb - sp.tb_first[lo];
     TbSeg s;
-    tb_segment(tbs[t].A, tbs[t].G, tbs[t].Qm, tbs[t].bgn, tbs[t].tbs_lbrm, &s);
+    tb_segment(tb.A, tb.G, tb.Qm, tb.bgn, tb.tbs_lbrm, &s);
     const int key = tb_graph_key(s.bgn, s.Zc, s.iLS);
-    for (int r = 0; r < s.C; ++r, ++cb) {
-      const int E = tb_cb_E(s, r);
-      const CbDerived d = tb_cb_derive(s, E, tbs[t].rv, tbs[t].Qm);
-      MixedCw c;
-      c.B = d.B;
-      c.E = E;
-      c.Qm = tbs[t].Qm;
-      c.symbols = d.symbols;
-      c.c0 = d.c0;
-      c.Nv = d.Nv;
-      c.F = d.F;
-      c.crctype = s.crc_cb;
-      c.llr_off = tbs[t].llr_offset + tb_cb_llr_start(s, r);
-      c.bits_off = (int64_t)cb * kCbBitsStride;
-      c.ncb = d.Ncb;
-      c.harq_mode = tbs[t].flags & (NRLDPC_TB_HARQ_COMBINE | NRLDPC_TB_HARQ_STORE);
-      c.harq_off = tbs[t].harq_offset + (int64_t)r * (d.N + 2 * s.Zc);
-      sp.cws[cb] = c;
-      sp.cb_key[cb] = key;
-      atomicAdd(&s_count[key], 1);
-    }
+    const int E = tb_cb_E(s, r);
+    const CbDerived d = tb_cb_derive(s, E, tb.rv, tb.Qm);
+    MixedCw c;
+    c.B = d.B;
+    c.E = E;
+    c.Qm = tb.Qm;
+    c.symbols = d.symbols;
+    c.c0 = d.c0;
+    c.Nv = d.Nv;
+    c.F = d.F;
+    c.crctype = s.crc_cb;
+    c.llr_off = tb.llr_offset + tb_cb_llr_start(s, r);
+    c.bits_off = (int64_t)cb * kCbBitsStride;
+    c.ncb = d.Ncb;
+    c.harq_mode = tb.flags & (NRLDPC_TB_HARQ_COMBINE | NRLDPC_TB_HARQ_STORE);
+    c.harq_off = tb.harq_offset + (int64_t)r * (d.N + 2 * s.Zc);
+    sp.cws[cb] = c;
+    sp.cb_key[cb] = key;
+    atomicAdd(&s_count[key], 1);
   }
   __syncthreads();
-  // 3. block queues and work items per (BG, Zc), largest lifting sizes first
-  if (tid == 0) {
-    int ib = 0, cbb = 0;
-    for (int rank = 0; rank < kKeys; ++rank) {
-      const int k = sp.key_by_rank[rank];
-      if (k < 0) break;
-      const int cnt = s_count[k];
-      if (!cnt) continue;
-      const int pairs = (cnt + 1) / 2, Gk = sp.key_G[k];
-      const int items = (pairs + Gk - 1) / Gk;
-      s_item_base[k] = ib;
-      s_cb_base[k] = cbb;
-      s_items[k] = items;
-      ib += items;
-      cbb += cnt;
-    }
-    s_num_items = ib;
-    if (ib > sp.max_items) s_err = 1;
-  }
+  // 3. block queues and work items per (BG, Zc), largest lifting sizes first: two
+  // scans over the graphs in rank order (thread = rank)
+  const int key = tid < kKeys ? s_rank_key[tid] : -1;
+  const int cnt = key >= 0 ? s_count[key] : 0;
+  const int items = cnt ? ((cnt + 1) / 2 + sp.key_G[key] - 1) / sp.key_G[key] : 0;
+  const int cb_end = block_scan(cnt, s_warp);
+  if (key >= 0) s_cb_base[key] = cb_end - cnt;
+  __syncthreads();   // s_warp is reused
+  const int item_end = block_scan(items, s_warp);
+  const int num_items = s_warp[31];
+  if (tid < kKeys) s_item_end[tid] = item_end;
   __syncthreads();
-  if (s_err) {
+  if (num_items > sp.max_items) {
     if (tid == 0) {
       sp.num_items[0] = 0;
       sp.num_items[1] = 1;
@@ -166,49 +185,35 @@ __global__ void __launch_bounds__(kSegThreads) tb_segment_kernel(const nrldpc_tb
     const int pos = atomicAdd(&s_cursor[k], 1);
     sp.cb_list[s_cb_base[k] + pos] = c;
   }
-  // 5. item records: a claim on graph k's queue
-  for (int i = tid; i < s_num_items; i += kSegThreads) {
-    int k = -1;
-    for (int rank = 0; rank < kKeys; ++rank) {
-      const int kk = sp.key_by_rank[rank];
-      if (kk < 0) break;
-      if (s_items[kk] && i >= s_item_base[kk] && i < s_item_base[kk] + s_items[kk]) {
-        k = kk;
-        break;
-      }
+  // 5. item records: a claim on the queue of the first graph whose items end past i
+  for (int i = tid; i < num_items; i += kSegThreads) {
+    int lo = 0, hi = kKeys - 1;
+    while (lo < hi) {
+      const int mid = (lo + hi) >> 1;
+      if (s_item_end[mid] > i) hi = mid;
+      else lo = mid + 1;
     }
     MixedItem m;
-    m.graph = k;
+    m.graph = s_rank_key[lo];
     m.pad0 = m.pad1 = m.pad2 = 0;
     sp.items[i] = m;
   }
   if (tid == 0) {
-    sp.num_items[0] = s_num_items;
+    sp.num_items[0] = num_items;
     sp.num_items[1] = 0;
     *sp.counter = 0;
   }
 }
 
-// r(x) * b(x) mod g(x) for 24-bit remainders (g given without its x^24 term).
-__device__ __forceinline__ uint32_t crc24_mulmod(uint32_t a, uint32_t b, uint32_t poly) {
-  uint32_t r = 0;
-  for (int i = 23; i >= 0; --i) {
-    r <<= 1;
-    if (r & 0x1000000u) r ^= 0x1000000u | poly;
-    if ((b >> i) & 1u) r ^= a;
-  }
-  return r;
-}
-
-// x^k mod g(x).
-__device__ __forceinline__ uint32_t crc24_xpow(uint64_t k, uint32_t poly) {
-  uint32_t result = 1u, base = 2u;
-  while (k) {
-    if (k & 1u) result = crc24_mulmod(result, base, poly);
-    base = crc24_mulmod(base, base, poly);
-    k >>= 1;
-  }
-  return result;
+// a(x) b(x) mod g(x) for 24-bit remainders, by a whole warp: lane i adds b_i x^i a,
+// the warp XORs the 48-bit product together, and lane j reduces its bit 24 + j with
+// t = T[j] = x^(24+j) mod g(x) (lanes 24 and up: 0).
+__device__ __forceinline__ uint32_t crc24_mulmod(uint32_t a, uint32_t b, uint32_t t) {
+  const int lane = threadIdx.x & 31;
+  const uint64_t term = lane < 24 && ((b >> lane) & 1u) ? (uint64_t)a << lane : 0ull;
+  const uint32_t lo = __reduce_xor_sync(0xFFFFFFFFu, (uint32_t)term & 0xFFFFFFu);
+  const uint32_t hi = __reduce_xor_sync(0xFFFFFFFFu, (uint32_t)(term >> 24));
+  return lo ^ __reduce_xor_sync(0xFFFFFFFFu, (hi >> lane) & 1u ? t : 0u);
 }
 
 struct FinishParams {
@@ -224,13 +229,23 @@ struct FinishParams {
   int32_t* iters;
 };
 
-__global__ void __launch_bounds__(512) tb_finish_kernel(const nrldpc_tb_t* __restrict__ tbs, int n,
-                                                        const __grid_constant__ FinishParams fp) {
+// A transport block's CTA: verdict, payload bytes, and for several code blocks the
+// transport-block CRC, sum over code blocks of their remainder times x^(bits
+// after the block).  Remainders: a warp per half code block, four positions per
+// lane and step with 16-byte table loads.  The
+// shift is a power of X = x^(bits per block), by squaring, a warp per code block.
+// Bound by latency.  32 transport blocks of up to 24 code blocks: 77 us with a bit
+// per lane and step, and the powers of x multiplied bit by bit by one lane; 17.3 us
+// in this form.
+constexpr int kFinishThreads = 512;
+constexpr int kFinishBlocks = 256;   // code blocks whose remainders are held at once
+__global__ void __launch_bounds__(kFinishThreads) tb_finish_kernel(const nrldpc_tb_t* __restrict__ tbs, int n,
+                                                                   const __grid_constant__ FinishParams fp) {
   const int tb = blockIdx.x;
   if (tb >= n) return;
   const int tid = threadIdx.x;
   __shared__ int s_fail, s_iters;
-  __shared__ uint32_t s_rem;
+  __shared__ uint32_t s_rem, s_part[kFinishBlocks];
   if (*fp.batch_err) {
     if (tid == 0) {
       fp.status[tb] = NRLDPC_ERR_ARG;
@@ -254,33 +269,66 @@ __global__ void __launch_bounds__(512) tb_finish_kernel(const nrldpc_tb_t* __res
     s_rem = 0u;
   }
   __syncthreads();
-  for (int r = tid; r < s.C; r += blockDim.x) {
+  for (int r = tid; r < s.C; r += kFinishThreads) {
     if (fp.cb_status[first + r] != 0) atomicOr(&s_fail, 1);
     atomicMax(&s_iters, fp.cb_iters[first + r]);
   }
+  const int lane = tid & 31, warp = tid >> 5;
+  constexpr int kWarps = kFinishThreads / 32;
   // payload bytes: code block r carries bytes [r*chunk, (r+1)*chunk) of the
-  // transport block (its information part; C == 1: the whole payload)
+  // transport block (its information part; C == 1: the whole payload), a warp per
+  // code block, four bytes per lane and step
   const int pay_bytes = tbs[tb].A / 8;
   const int chunk = s.C == 1 ? pay_bytes : s.A_cb / 8;
   uint8_t* out = fp.out + tbs[tb].out_offset;
-  for (int i = tid; i < pay_bytes; i += blockDim.x) {
-    const int r = i / chunk;
-    out[i] = fp.cb_bits[(int64_t)(first + r) * kCbBitsStride + (i - r * chunk)];
+  for (int r = warp; r < s.C; r += kWarps) {
+    const uint32_t* src = reinterpret_cast<const uint32_t*>(fp.cb_bits + (int64_t)(first + r) * kCbBitsStride);
+    uint8_t* dst = out + (int64_t)r * chunk;
+    const int len = min(chunk, pay_bytes - r * chunk);   // the last block's CRC bits are not payload
+    const bool aligned = (reinterpret_cast<uintptr_t>(dst) & 3u) == 0;
+    for (int i = 4 * lane; i < len; i += 128) {
+      const uint32_t w = src[i >> 2];
+      if (aligned && i + 4 <= len) {
+        *reinterpret_cast<uint32_t*>(dst + i) = w;
+      } else {
+        for (int b = 0; b < 4; ++b)
+          if (i + b < len) dst[i + b] = (uint8_t)(w >> (8 * b));
+      }
+    }
   }
   if (s.C > 1) {
     // transport-block CRC24A over A + 24 bits spread over the code blocks
-    const int lane = tid & 31, warp = tid >> 5, nwarps = blockDim.x >> 5;
-    const int nbits = s.A_cb;
-    for (int r = warp; r < s.C; r += nwarps) {
-      const uint8_t* bits = fp.cb_bits + (int64_t)(first + r) * kCbBitsStride;
-      uint32_t rem = 0u;
-      for (int i = lane; i < nbits; i += 32)
-        if ((bits[i >> 3] >> (7 - (i & 7))) & 1u) rem ^= __ldg(fp.crc24a_tab + (nbits - 1 - i));
-      rem = __reduce_xor_sync(0xFFFFFFFFu, rem);
-      if (lane == 0) {
-        const uint64_t after = (uint64_t)s.B - (uint64_t)(r + 1) * nbits;
-        atomicXor(&s_rem, crc24_mulmod(rem, crc24_xpow(after, 0x864CFBu), 0x864CFBu));
+    const int nbits = s.A_cb;                       // a multiple of 8
+    const uint32_t t = lane < 24 ? __ldg(fp.crc24a_tab + lane) : 0u;
+    const uint32_t X = __ldg(fp.crc24a_tab + (nbits - 24));   // x^nbits
+    for (int r0 = 0; r0 < s.C; r0 += kFinishBlocks) {
+      const int nb = min(kFinishBlocks, s.C - r0);
+      for (int r = tid; r < nb; r += kFinishThreads) s_part[r] = 0u;
+      __syncthreads();
+      // a warp takes half of a code block's runs at a time, four runs' loads in flight
+      for (int k = warp; k < 2 * nb; k += kWarps) {
+        const int r = k >> 1;
+        const uint8_t* bits = fp.cb_bits + (int64_t)(first + r0 + r) * kCbBitsStride;
+        uint32_t rem = 0u;
+#pragma unroll 4
+        for (int i0 = 128 * (k & 1) + 4 * lane; i0 < nbits; i0 += 256) {
+          const uint32_t v = (uint32_t)__ldg(bits + (i0 >> 3)) >> ((i0 & 4) ? 0 : 4);
+          const uint4 tv = __ldg(reinterpret_cast<const uint4*>(fp.crc24a_tab + (nbits - 4 - i0)));
+          rem ^= ((v & 8u) ? tv.w : 0u) ^ ((v & 4u) ? tv.z : 0u) ^ ((v & 2u) ? tv.y : 0u) ^ ((v & 1u) ? tv.x : 0u);
+        }
+        rem = __reduce_xor_sync(0xFFFFFFFFu, rem);
+        if (lane == 0 && rem) atomicXor(&s_part[r], rem);
       }
+      __syncthreads();
+      for (int r = warp; r < nb; r += kWarps) {
+        uint32_t v = s_part[r], base = X;   // v X^(C-1-r)
+        for (int k = s.C - 1 - (r0 + r); k; k >>= 1) {
+          if (k & 1) v = crc24_mulmod(v, base, t);
+          if (k > 1) base = crc24_mulmod(base, base, t);
+        }
+        if (lane == 0 && v) atomicXor(&s_rem, v);
+      }
+      __syncthreads();
     }
   }
   __syncthreads();
@@ -445,7 +493,7 @@ int engine_decode(TbEngine* e, int lane, const nrldpc_tb_t* d_tbs, int n, const 
   fp.out = d_out;
   fp.status = d_status;
   fp.iters = d_iters;
-  tb_finish_kernel<<<n, 512, 0, s>>>(d_tbs, n, fp);
+  tb_finish_kernel<<<n, kFinishThreads, 0, s>>>(d_tbs, n, fp);
   count_launch();
   return cudaGetLastError() == cudaSuccess ? NRLDPC_OK : NRLDPC_ERR_CUDA;
 }
