@@ -73,12 +73,24 @@ __device__ __forceinline__ uint32_t clip_half_degen(int32_t v, int32_t mx, int32
   return (uint32_t)r & 0xFFFFu;
 }
 
-// |x| of each int16 half as an unsigned 16-bit value: max(x, -x) with the
-// native packed subtract and signed max.  |-32768| comes out as 32768; in the
-// unsigned minimum search below (which starts at 32767) that value never
-// becomes a minimum, exactly like the reference's saturated 32767
+// |x| of each int16 half as an unsigned 16-bit value.  |-32768| comes out as
+// 32768; in the unsigned minimum search below (which starts at 32767) that
+// value never becomes a minimum, exactly like the reference's saturated 32767
 // (c_lib/fixedpoint_ldpc_decoder.c:48-66), so no saturation step is needed.
-__device__ __forceinline__ uint32_t abs_u16x2(uint32_t x) { return __vmaxs2(x, __vsub2(0u, x)); }
+// Two forms: max(~x + 1, x) with the fused add-and-maximum (two instructions of
+// the integer pipe), and max(x, 0 - x) (two of that pipe, one of the FMA pipe).
+// The fused one wins in rows of up to ten edges, whose rate is the issue
+// slots'; in the 19-edge rows, unrolled over more registers than there are, it
+// costs a few more spills than the slot is worth.  Ten iterations, kernel time,
+// with max(x, 0 - x) everywhere / fused everywhere / fused up to ten edges:
+// 8192 blocks BG1 Zc384 8.32 / 8.40 / 8.13 ms with the open maximum and 9.67 /
+// 9.43 / 9.47 ms without it; 65536 blocks BG2 Zc64 7.53 / 7.29 / 7.31 ms; 8192
+// blocks BG2 Zc384 5.59 / 5.50 / 5.43 ms; 777 blocks BG1 Zc208 634 / 618 / 617 us.
+template <bool kFused = true>
+__device__ __forceinline__ uint32_t abs_u16x2(uint32_t x) {
+  if constexpr (kFused) return __viaddmax_s16x2(~x, 0x00010001u, x);
+  else return __vmaxs2(x, __vsub2(0u, x));
+}
 
 // m ? -v : v per half (two's complement, wrapping like the reference's int16
 // store of sign * new_val): (v ^ m) - m.
@@ -216,7 +228,7 @@ __device__ __forceinline__ void row_update(const P& p, const uint2* __restrict__
     const uint32_t x = __vadd2(__vadd2(q, bsel(mi, n2, n1) ^ nmf), nmf & 0x00010001u);
     rel[j] = x;
     sg ^= x;
-    const uint32_t a = abs_u16x2(x);
+    const uint32_t a = abs_u16x2<(D <= 10)>(x);
     bool ph, pl;
     const uint32_t nm1 = __vibmin_u16x2(a, m1, &ph, &pl);   // per half: a <= m1
     m2 = __vmaxu2(m1, __vminu2(m2, a));

@@ -138,6 +138,28 @@ def test_open_scaling_is_a_byte_permute():
         assert np.array_equal(wide >> np.uint64(16), (m * np.uint64(alpha) + np.uint64(1 << 14)) >> np.uint64(15))
 
 
+def test_fused_magnitude_equals_the_pair_form():
+    """max(~x + 1, x) and max(x, 0 - x) per half, the sum wrapping, for every int16."""
+    x = np.arange(-32768, 32768, dtype=np.int64)
+    fused = np.maximum(wrap16((u16(x) ^ M16) + 1), x)
+    assert np.array_equal(fused, np.maximum(x, wrap16(-x)))
+    assert np.array_equal(u16(fused), np.abs(x))
+
+
+@pytest.mark.parametrize("flip", [False, True])
+def test_sum_with_the_sign_on_the_other_operand(flip):
+    """With w = rel ^ mf and 0 <= v (an open maximum's scaled minimum), (w + v) ^ mf is
+    rel + (flip ? -v : v) modulo 2^16, and u & ~w is its exact overflow flag."""
+    mf = M16 if flip else 0
+    rel = np.arange(-32768, 32768, dtype=np.int64)
+    for v in [0, 1, 2, 32766, 32767] + list(np.random.default_rng(5).integers(0, 32768, 40)):
+        v = int(v)
+        w = u16(rel) ^ mf
+        u = (w + v) & M16
+        assert np.array_equal(wrap16(u ^ mf), wrap16(rel - v if flip else rel + v))
+        assert np.array_equal(((u & ~w) & 0x8000) != 0, _true_overflow(rel, -v if flip else v))
+
+
 def test_extension_rows_end_in_their_own_unshifted_parity_column(oracle):
     from oracle.oracle import in_config
 
