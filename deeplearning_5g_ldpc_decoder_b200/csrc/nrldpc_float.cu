@@ -32,32 +32,12 @@ __device__ __forceinline__ float clipf(float v, float mx, float mn) {
   return v > mx ? mx : (v < mn ? mn : v);
 }
 
-// The code's edge table, staged into shared memory at kernel start: the rows
-// read it twice per edge, and a shared load is cheaper than a dynamically
-// indexed parameter read (BP: 39.0 -> 37.4 ms for 8192 BG1 Zc=384 blocks).
-__shared__ uint32_t s_fedge[kMaxNnz];
-
-__device__ __forceinline__ uint32_t edge_addr(const DecodeParams& p, int e, uint32_t zx) {
-  const uint32_t ed = s_fedge[e];
-  uint32_t t = zx + (ed >> 16);
-  t = min(t, t - (uint32_t)p.Zc);
-  return (ed & 0xFFFFu) + t;
-}
-
-// Belief word a of the code block's LQ (debug build: a < lq_len, else the load
-// reads 0 and the store is dropped).
-__device__ __forceinline__ float ld_lq(const DecodeParams& p, const float* lq, uint32_t a) {
-  return NRLDPC_INBOUNDS(a, p.lq_len, kBoundsLq) ? lq[a] : 0.0f;
-}
-__device__ __forceinline__ void st_lq(const DecodeParams& p, float* lq, uint32_t a, float v) {
-  if (NRLDPC_INBOUNDS(a, p.lq_len, kBoundsLq)) lq[a] = v;
-}
-
-// ---------------------------------------------------------------- float min-sum
-// The edge table again as byte offsets {column * Zc * 4, (V mod Zc) * 4}, staged
-// by the min-sum kernel: an address is then three instructions.
+// The code's edge table as byte offsets {column * Zc * 4, (V mod Zc) * 4}, staged
+// into shared memory at kernel start: a shared load is cheaper than a dynamically
+// indexed parameter read, and an address is three instructions more.
 __shared__ uint2 s_fedge4[kMaxNnz];
 
+// ---------------------------------------------------------------- float min-sum
 // Stored message of a lifted check row (3 planes): new_min1, new_min2 (float
 // bits), and a word with edge j's sign flip in bit D - 1 - j and the position of
 // new_min2's edge from bit 20.  The kernel loads a row's words while the row
@@ -151,42 +131,70 @@ __device__ __forceinline__ void bulk_prefetch_l2(const void* a, uint32_t bytes) 
 }
 
 __device__ __forceinline__ float bp_message(float prod) {
-  // bp_message_from_product (:54-62)
-  if (prod >= 1.0f) return 2.0f * kBpAtanhClip;
-  if (prod <= -1.0f) return -2.0f * kBpAtanhClip;
-  return __fmul_rn(2.0f, atanhf(prod));
+  // bp_message_from_product (:54-62): +-2 * 19.07 for a product of +-1.  A product
+  // of tanh values is never beyond +-1, atanhf(+-1) is +-inf and atanhf of the next
+  // float 8.7, so the two compares are a clamp.
+  const float m = __fmul_rn(2.0f, atanhf(prod));
+  return fminf(fmaxf(m, -2.0f * kBpAtanhClip), 2.0f * kBpAtanhClip);
 }
 
-// Registers are what limits this kernel's occupancy, so the row keeps only
-// tanh values and suffix products live: rel = LQ - old message is parked in
-// LQ's own shared-memory word until the update (a row's edges are distinct
-// words that no other thread touches during the layer), edge addresses are
-// recomputed from the constant-cache table, and the prefix product runs as a
-// scalar.  The arithmetic and its order are unchanged.
+// One row.  The messages of all edges are loaded before anything else, and no
+// branch stands between the edges, so the loads (L2, or memory) overlap.  Rows of
+// up to ten edges keep rel = LQ - old message and the edges' addresses in
+// registers; a 19-edge row has no room for them, parks rel in LQ's own word (a
+// row's edges are distinct words that no other thread touches during the layer)
+// and computes the addresses twice.  The products keep the reference's order.
+// Issue slots bound it (73 % busy; 83 instructions per edge, most of them in
+// tanhf and atanhf).  10 iterations of 1024 blocks BG1 Zc=384: 3.78 -> 2.31 ms
+// against loads one edge at a time behind a branch on a zero input (107
+// instructions per edge, 61 % busy, waiting on the loads).
 template <int D>
-__device__ __forceinline__ void bp_row(const DecodeParams& p, float* __restrict__ lq, uint32_t zx, int e0,
-                                       bool first, uint32_t* __restrict__ lrp, int NT) {
+__device__ __forceinline__ void bp_row(const DecodeParams& p, char* __restrict__ lq, uint32_t zx4, int e0, bool first,
+                                       float* __restrict__ lrp, int NT) {
   if (!NRLDPC_INBOUNDS(e0 + D - 1, kMaxNnz, kBoundsEdge)) return;   // debug build
+  constexpr bool kKeep = D <= 10;
+  const uint32_t zc4 = 4u * (uint32_t)p.Zc;
+  [[maybe_unused]] const uint32_t limit = 4u * (uint32_t)p.lq_len;   // bytes of beliefs (debug build)
+  const auto address = [&](int j) {
+    const uint2 e = s_fedge4[e0 + j];
+    const uint32_t t = e.y + zx4;
+    return min(t, t - zc4) + e.x;
+  };
+  const auto load = [&](uint32_t a) { return NRLDPC_INBOUNDS(a, limit, kBoundsLq) ? *reinterpret_cast<const float*>(lq + a) : 0.0f; };
+  const auto store = [&](uint32_t a, float v) {
+    if (NRLDPC_INBOUNDS(a, limit, kBoundsLq)) *reinterpret_cast<float*>(lq + a) = v;
+  };
   float th[D];
-  int nz = 0, zidx = -1;
-  float nzprod = 1.0f;
-  // compute_tanh_values (:65-82): tanh(rel/2), zero count, product of non-zeros.
+  [[maybe_unused]] float rel[kKeep ? D : 1];
+  [[maybe_unused]] uint32_t addr[kKeep ? D : 1];
+#pragma unroll
+  for (int j = 0; j < D; ++j) th[j] = first ? 0.0f : lrp[j * NT];
+  // compute_tanh_values (:65-82): tanh(rel/2); a zero input (tanh is +-0 then)
+  // sends the row to the form below.
+  bool zero = false;
 #pragma unroll
   for (int j = 0; j < D; ++j) {
-    const uint32_t a = edge_addr(p, e0 + j, zx);
-    const float old = first ? 0.0f : __uint_as_float(lrp[j * NT]);
-    const float v = __fsub_rn(ld_lq(p, lq, a), old);
-    st_lq(p, lq, a, v);
-    if (v == 0.0f) {
-      ++nz;
-      zidx = j;
-      th[j] = 0.0f;
+    const uint32_t a = address(j);
+    const float v = __fsub_rn(load(a), th[j]);
+    if constexpr (kKeep) {
+      addr[j] = a;
+      rel[j] = v;
     } else {
-      th[j] = tanhf(__fmul_rn(v, 0.5f));
-      nzprod = __fmul_rn(nzprod, th[j]);
+      store(a, v);
     }
+    zero |= v == 0.0f;
+    th[j] = tanhf(__fmul_rn(v, 0.5f));
   }
-  if (nz == 0) {
+  const auto update = [&](int j, float m) {   // no clipping in BP (:148-150)
+    lrp[j * NT] = m;
+    if constexpr (kKeep) {
+      store(addr[j], __fadd_rn(rel[j], m));
+    } else {
+      const uint32_t a = address(j);
+      store(a, __fadd_rn(load(a), m));
+    }
+  };
+  if (!zero) {
     // prefix/suffix products (:85-96, :135-145), same multiplication order:
     // sf[j] = th[D-1] * ... * th[j+1] accumulated right to left (sf[D-1] = 1),
     // the prefix th[0] * ... * th[j-1] left to right.
@@ -199,36 +207,43 @@ __device__ __forceinline__ void bp_row(const DecodeParams& p, float* __restrict_
     for (int j = 0; j < D; ++j) {
       const float m = bp_message(__fmul_rn(pre, sf[j]));
       pre = __fmul_rn(pre, th[j]);
-      const uint32_t a = edge_addr(p, e0 + j, zx);
-      lrp[j * NT] = __float_as_uint(m);
-      st_lq(p, lq, a, __fadd_rn(ld_lq(p, lq, a), m));   // no clipping in BP (:148-150)
+      update(j, m);
     }
   } else {
     // one zero input: only its edge gets a message (the product of the
-    // others); two or more: every message is zero
-    const float mz = nz == 1 ? bp_message(nzprod) : 0.0f;
+    // others, left to right); two or more: every message is zero
+    int nz = 0, zidx = -1;
+    float nzprod = 1.0f;
 #pragma unroll
     for (int j = 0; j < D; ++j) {
-      const float m = j == zidx && nz == 1 ? mz : 0.0f;
-      const uint32_t a = edge_addr(p, e0 + j, zx);
-      lrp[j * NT] = __float_as_uint(m);
-      st_lq(p, lq, a, __fadd_rn(ld_lq(p, lq, a), m));
+      float v;
+      if constexpr (kKeep) v = rel[j];
+      else v = load(address(j));
+      if (v == 0.0f) {
+        ++nz;
+        zidx = j;
+      } else {
+        nzprod = __fmul_rn(nzprod, th[j]);
+      }
     }
+    const float mz = nz == 1 ? bp_message(nzprod) : 0.0f;
+#pragma unroll
+    for (int j = 0; j < D; ++j) update(j, j == zidx ? mz : 0.0f);
   }
 }
 
-__device__ __forceinline__ void bp_dispatch(int deg, const DecodeParams& p, float* lq, uint32_t zx, int e0,
-                                            bool first, uint32_t* lrp, int NT) {
+__device__ __forceinline__ void bp_dispatch(int deg, const DecodeParams& p, char* lq, uint32_t zx4, int e0, bool first,
+                                            float* lrp, int NT) {
   switch (deg) {
-    case 3: bp_row<3>(p, lq, zx, e0, first, lrp, NT); break;
-    case 4: bp_row<4>(p, lq, zx, e0, first, lrp, NT); break;
-    case 5: bp_row<5>(p, lq, zx, e0, first, lrp, NT); break;
-    case 6: bp_row<6>(p, lq, zx, e0, first, lrp, NT); break;
-    case 7: bp_row<7>(p, lq, zx, e0, first, lrp, NT); break;
-    case 8: bp_row<8>(p, lq, zx, e0, first, lrp, NT); break;
-    case 9: bp_row<9>(p, lq, zx, e0, first, lrp, NT); break;
-    case 10: bp_row<10>(p, lq, zx, e0, first, lrp, NT); break;
-    default: bp_row<19>(p, lq, zx, e0, first, lrp, NT); break;
+    case 3: bp_row<3>(p, lq, zx4, e0, first, lrp, NT); break;
+    case 4: bp_row<4>(p, lq, zx4, e0, first, lrp, NT); break;
+    case 5: bp_row<5>(p, lq, zx4, e0, first, lrp, NT); break;
+    case 6: bp_row<6>(p, lq, zx4, e0, first, lrp, NT); break;
+    case 7: bp_row<7>(p, lq, zx4, e0, first, lrp, NT); break;
+    case 8: bp_row<8>(p, lq, zx4, e0, first, lrp, NT); break;
+    case 9: bp_row<9>(p, lq, zx4, e0, first, lrp, NT); break;
+    case 10: bp_row<10>(p, lq, zx4, e0, first, lrp, NT); break;
+    default: bp_row<19>(p, lq, zx4, e0, first, lrp, NT); break;
   }
 }
 
@@ -317,10 +332,7 @@ __global__ void __launch_bounds__(kThreadsTarget, 2) float_kernel(const __grid_c
   extern __shared__ __align__(16) float s_lqf[];     // [G][lq_len]
   __shared__ uint32_t s_crc[kMaxGroups];
   // read after the first barrier
-  for (int e = threadIdx.x; e < kMaxNnz; e += blockDim.x) {
-    if (kBP) s_fedge[e] = p.edge[e];
-    else s_fedge4[e] = p.edge_cs4[e];
-  }
+  for (int e = threadIdx.x; e < kMaxNnz; e += blockDim.x) s_fedge4[e] = p.edge_cs4[e];
   // BP: per row, the 16-byte-aligned part of the next row's message slice
   // (row 0 of the next iteration after the last row) as {byte offset from the
   // CTA's scratch, bytes}, for the bulk L2 prefetch in the row loop.
@@ -398,7 +410,7 @@ __global__ void __launch_bounds__(kThreadsTarget, 2) float_kernel(const __grid_c
             }
           }
           if (kBP) {
-            bp_dispatch(deg, p, lq, (uint32_t)zx, e0, it == 0, lrp, NT);
+            bp_dispatch(deg, p, reinterpret_cast<char*>(lq), 4u * (uint32_t)zx, e0, it == 0, reinterpret_cast<float*>(lrp), NT);
           } else {
             const FloatMsg cur = nxt;
             const bool wrap = row + 1 == p.R;
