@@ -315,7 +315,7 @@ int make_plan(const CodeParams& cp, const ldpc_decoder_cfg_t& dc, int num_cw, De
     if (algo == 0) {
       planes = deg;
     } else if (fixed) {
-      planes = fixed_row_planes(deg);
+      planes = fixed_row_planes(r, deg, true);
     } else {
       planes = 3;
     }

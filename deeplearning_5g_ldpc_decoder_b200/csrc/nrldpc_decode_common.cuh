@@ -162,15 +162,27 @@ __device__ __forceinline__ int div_bp(int k, uint32_t magic) { return (int)__umu
 // Per-layer descriptor staged in shared memory at kernel start, one 16-byte
 // load per layer instead of several dynamically indexed parameter reads:
 // x = the layer's word offset in the CTA's message scratch,
-// y = first edge | degree << 16 | (five message planes) << 24,
+// y = row_word: first edge | degree << 16 | message words << 24 | direct << 31,
 // z = the layer's packed alpha | beta << 16 (unused with per-iteration weights).
-__device__ __forceinline__ uint4 row_descriptor(const DecodeParams& p, int r) {
-  const uint32_t e0 = p.row_off[r], deg = (uint32_t)p.row_off[r + 1] - e0;
-  const uint32_t five = p.lr_off[r + 1] - p.lr_off[r] > 4u * kThreadsTarget ? 1u : 0u;
-  return make_uint4(p.lr_off[r], e0 | (deg << 16) | (five << 24), p.w_inline[r], 0u);
+//
+// A row is direct (row_update_direct) when its scratch has a plane per message, up
+// to the limit of its arithmetic variant.  `beliefs`: the batch returns beliefs, so
+// rows with a parity column of their own are compressed, because that column's
+// message is read back from the compressed words (parity_belief).
+__device__ __forceinline__ uint32_t row_word(uint32_t e0, uint32_t deg, uint32_t planes, int clip, bool par, bool beliefs) {
+  const uint32_t n = par ? deg - 1u : deg;
+  const bool direct = n <= planes && n <= (uint32_t)(clip == kClipOpenMax ? kDirectOpen : kDirectClip) && !(par && beliefs);
+  return e0 | deg << 16 | (direct ? n : deg > 16u ? 5u : 4u) << 24 | (direct ? 1u << 31 : 0u);
+}
+__device__ __forceinline__ uint4 row_descriptor(const DecodeParams& p, int r, int clip) {
+  return make_uint4(p.lr_off[r],
+                    row_word(p.row_off[r], (uint32_t)p.row_off[r + 1] - p.row_off[r], (p.lr_off[r + 1] - p.lr_off[r]) / kThreadsTarget,
+                             clip, parity_words(clip) && r >= kCoreRows, p.app != nullptr),
+                    p.w_inline[r], 0u);
 }
 __device__ __forceinline__ int row_e0(uint32_t y) { return (int)(y & 0xFFFFu); }
 __device__ __forceinline__ int row_deg(uint32_t y) { return (int)((y >> 16) & 0xFFu); }
-__device__ __forceinline__ bool row_five(uint32_t y) { return (y >> 24) != 0u; }
+__device__ __forceinline__ int row_words(uint32_t y) { return (int)(y >> 24 & 0x7Fu); }
+__device__ __forceinline__ bool row_direct(uint32_t y) { return (y >> 31) != 0u; }
 
 }  // namespace nrldpc

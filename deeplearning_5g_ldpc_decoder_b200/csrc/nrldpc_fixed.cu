@@ -18,10 +18,10 @@
 //  * The beliefs LQ of all G pairs live in shared memory for the whole decode.
 //    Circulant shifts are resolved as shared-memory word addresses
 //    col*Zc + (V_ij mod Zc + zx) mod Zc.
-//  * Check-to-variable messages are kept compressed per lifted check row and
-//    pair (two scaled minima, the position of the minimum, one sign bit per
-//    edge: 16 or 20 bytes for both code blocks instead of 4*degree) in a
-//    per-CTA global scratch that stays resident in L2.
+//  * Check-to-variable messages live in a per-CTA global scratch that stays
+//    resident in L2: one word per edge for both code blocks of a pair in rows of
+//    up to ten messages, and compressed (two scaled minima, the position of the
+//    minimum, one sign bit per edge: 16 or 20 bytes) in longer rows.
 //  * The grid is persistent.  With a block cursor (DecodeParams::cursor: the
 //    queue head and a count of finished CTAs, both zero at launch and rewound
 //    by the last CTA to finish) every int16 half lane takes code blocks from one
@@ -32,9 +32,9 @@
 //    cursor (launches of one wave or less, and the no-allocation entry point)
 //    each CTA loops over fixed work items of G pairs until every block of the
 //    item has finished.
-//  * Each row's compressed message words are loaded while the row before it
+//  * Each row's first message words are loaded while the row before it
 //    computes (load_row_msg), hiding their L2 latency.
-//  * Per-layer descriptors (scratch offset, first edge, degree, plane count,
+//  * Per-layer descriptors (scratch offset, first edge, degree, message form,
 //    alpha|beta) are staged in shared memory at kernel start: one 16-byte
 //    shared load per layer replaces six dynamically indexed parameter reads.
 //  * CRC early termination runs every iteration inside the kernel: each hard
@@ -212,12 +212,13 @@ __device__ __forceinline__ void take_blocks(const DecodeParams& p, bool q0, bool
 // shared-memory base are compile-time zeros and free registers in the layer loop.
 template <int kClip, bool kRefill, bool kG1>
 __global__ void __launch_bounds__(kThreadsTarget, 2) fixed_pair_kernel(const __grid_constant__ DecodeParams p) {
+  constexpr int kAhead = ahead_words(kG1);
   extern __shared__ __align__(16) uint32_t s_lq[];        // [G][lq_len] int16x2
   __shared__ uint32_t s_crc[2 * kMaxGroups];
   __shared__ uint2 s_edges[kMaxNnz];   // per-edge (col*Zc*4, (V mod Zc)*4), read with warp-uniform indices
   __shared__ uint4 s_rows[kMaxRows];   // per-layer descriptors (row_descriptor)
   for (int e = threadIdx.x; e < kMaxNnz; e += blockDim.x) s_edges[e] = p.edge_cs4[e];
-  for (int r = threadIdx.x; r < p.R; r += blockDim.x) s_rows[r] = row_descriptor(p, r);
+  for (int r = threadIdx.x; r < p.R; r += blockDim.x) s_rows[r] = row_descriptor(p, r, kClip);
 
   const int tid = threadIdx.x;
   const int g = kG1 ? 0 : tid / p.Zc;
@@ -258,15 +259,15 @@ __global__ void __launch_bounds__(kThreadsTarget, 2) fixed_pair_kernel(const __g
     uint32_t itv = 0u;   // iterations of half 0 in bits 0-15, half 1 in bits 16-31
     uint32_t fresh = 0xFFFFFFFFu;   // both halves start their first iteration
     const bool run = p.max_it > 0;   // max_iterations == 0: rate recovery only, status 1
-    RowMsg nxt{};
+    RowMsg<kAhead> nxt{};
     while (!idle) {
       for (int row = 0; run && row < p.R; ++row) {
         if (active) {
-          const RowMsg cur = nxt;
+          const RowMsg<kAhead> cur = nxt;
           const uint4 d = s_rows[row];
           const int rn = row + 1 < p.R ? row + 1 : 0;
           const uint2 dn = *reinterpret_cast<const uint2*>(&s_rows[rn]);
-          nxt = load_row_msg(scratch + dn.x + tid, row_five(dn.y));
+          nxt = load_row_msg<kAhead>(scratch + dn.x + tid, row_words(dn.y));
           uint32_t ab0, ab1;
           if (p.weights_T > 0) {
             ab0 = __ldg(p.weights + (min((int)(itv & 0xFFFFu), p.weights_T - 1) * p.R + row));
@@ -274,7 +275,7 @@ __global__ void __launch_bounds__(kThreadsTarget, 2) fixed_pair_kernel(const __g
           } else {
             ab0 = ab1 = d.z;
           }
-          layer_dispatch<kClip, true, kG1>(row_deg(d.y), row >= kCoreRows, p, s_edges, reinterpret_cast<char*>(s_lq), zx4, zxm4, gb4,
+          layer_dispatch<kClip, true, kG1>(row_deg(d.y), row >= kCoreRows, row_direct(d.y), p, s_edges, reinterpret_cast<char*>(s_lq), zx4, zxm4, gb4,
                                            lq_limit, row_e0(d.y), (int32_t)(int16_t)(ab0 & 0xFFFFu), ((int32_t)ab0) >> 16,
                                            (int32_t)(int16_t)(ab1 & 0xFFFFu), ((int32_t)ab1) >> 16, cur, fresh,
                                            scratch + d.x + tid);
@@ -364,19 +365,19 @@ __global__ void __launch_bounds__(kThreadsTarget, 2) fixed_pair_kernel(const __g
       __syncthreads();
 
       int it = 0;
-      RowMsg nxt{};
+      RowMsg<kAhead> nxt{};
       for (; it < p.max_it; ++it) {
         for (int row = 0; row < p.R; ++row) {
           if (active) {
-            const RowMsg cur = nxt;
+            const RowMsg<kAhead> cur = nxt;
             const uint4 d = s_rows[row];
             const int rn = row + 1 < p.R ? row + 1 : 0;
             const uint2 dn = *reinterpret_cast<const uint2*>(&s_rows[rn]);
-            nxt = load_row_msg(scratch + dn.x + tid, row_five(dn.y));
+            nxt = load_row_msg<kAhead>(scratch + dn.x + tid, row_words(dn.y));
             const uint32_t ab = p.weights_T > 0 ? __ldg(p.weights + (min(it, p.weights_T - 1) * p.R + row)) : d.z;
             const int32_t alpha = (int32_t)(int16_t)(ab & 0xFFFFu);
             const int32_t beta = ((int32_t)ab) >> 16;
-            layer_dispatch<kClip, true, kG1>(row_deg(d.y), row >= kCoreRows, p, s_edges, reinterpret_cast<char*>(s_lq), zx4, zxm4, gb4,
+            layer_dispatch<kClip, true, kG1>(row_deg(d.y), row >= kCoreRows, row_direct(d.y), p, s_edges, reinterpret_cast<char*>(s_lq), zx4, zxm4, gb4,
                                              lq_limit, row_e0(d.y), alpha, beta, alpha, beta, cur,
                                              it == 0 ? 0xFFFFFFFFu : 0u, scratch + d.x + tid);
           }

@@ -99,7 +99,7 @@ __device__ __forceinline__ uint32_t cond_neg16x2(uint32_t v, uint32_t m) { retur
 // One layer step of one lifted check row, for both code blocks of a pair.
 //
 // Compressed old message of the row (planes of the CTA scratch, kThreadsTarget
-// words apart), with J = min(D, 16):
+// words apart), with J = min(D, 16); row_update_direct has the other form:
 //   w0 = new_min1 pair, w1 = new_min2 pair,
 //   w2 = sign flip of edge j < 16 at bit 15-(J-1-j) (block 0) and 31-(J-1-j)
 //        (block 1),
@@ -127,38 +127,42 @@ __device__ __forceinline__ uint32_t cond_neg16x2(uint32_t v, uint32_t m) { retur
 // Instruction budget: packed add/sub run on the FMA pipe, packed min/max,
 // PRMT and LOP3 on the ALU pipe (the bottleneck); the emulated saturating
 // packed ops are kept off the common path.
-// The compressed old message words of one lifted row (w0..w4 below), loaded
-// by the kernels one row ahead so that their L2 latency overlaps the row
-// before.
+// The first words of a lifted row's old message (w0..w4 above, or the messages of
+// row_update_direct), loaded by the kernels one row ahead so that their L2 latency
+// overlaps the row before; the row loads the rest itself.  Four words always (a
+// row has at least four planes), and with one lane pair per CTA a fifth where the
+// row has it.  With groups there is no register for it: 65536 blocks of BG2 Zc=64
+// take 6.49 ms with four words and 7.40 ms with five; with one pair, 8192 of BG1
+// Zc=384, it is 8.03 and 7.38 ms (six: 7.78 ms).
+template <int kAhead>
 struct RowMsg {
-  uint32_t n1, n2, xf, xi, y;
+  uint32_t w[kAhead];
 };
-__device__ __forceinline__ RowMsg load_row_msg(const uint32_t* lrp, bool five) {
+__host__ __device__ constexpr int ahead_words(bool g1) { return g1 ? 5 : 4; }
+template <int kAhead>
+__device__ __forceinline__ RowMsg<kAhead> load_row_msg(const uint32_t* lrp, int words) {
   constexpr int S = kThreadsTarget;
-  RowMsg m;
-  m.n1 = lrp[0];
-  m.n2 = lrp[S];
-  m.xf = lrp[2 * S];
-  m.xi = lrp[3 * S];
-  m.y = five ? lrp[4 * S] : 0u;
+  RowMsg<kAhead> m;
+#pragma unroll
+  for (int k = 0; k < kAhead; ++k) m.w[k] = k < 4 || k < words ? lrp[k * S] : 0u;
   return m;
 }
 
 template <int D, bool kPar, int kClip, bool kSmemEdges, bool kG1, typename P>
 __device__ __forceinline__ void row_update(const P& p, const uint2* __restrict__ sedges, char* __restrict__ lqs, uint32_t zx4,
                                            uint32_t zxm4, uint32_t gb4, uint32_t lq_limit, int e0, int32_t alpha, int32_t beta,
-                                           int32_t alpha1, int32_t beta1, const RowMsg& old, uint32_t fresh,
+                                           int32_t alpha1, int32_t beta1, const RowMsg<ahead_words(kG1)>& old, uint32_t fresh,
                                            uint32_t* __restrict__ lrp) {
   constexpr int J = D < 16 ? D : 16;
   constexpr int S = kThreadsTarget;    // plane stride (words)
   constexpr int N = kPar ? D - 1 : D;  // edges with a belief to write
   uint32_t n1 = 0u, n2 = 0u, xf = 0u, xi = 0u, y = 0u;
   if (fresh != 0xFFFFFFFFu) {
-    n1 = old.n1;
-    n2 = old.n2;
-    xf = old.xf;
-    xi = old.xi;
-    if (D > 16) y = old.y;
+    n1 = old.w[0];
+    n2 = old.w[1];
+    xf = old.w[2];
+    xi = old.w[3];
+    if (D > 16) y = ahead_words(kG1) > 4 ? old.w[ahead_words(kG1) - 1] : lrp[4 * S];
     if (fresh) {
       const uint32_t keep = ~fresh;
       n1 &= keep;
@@ -345,6 +349,122 @@ __device__ __forceinline__ void row_update(const P& p, const uint2* __restrict__
   if (D > 16) lrp[4 * S] = Y;
 }
 
+// The same step for a row that keeps its messages as they are: plane j holds edge
+// j's negated message of both blocks, so x = LQ + plane, and the row neither
+// unpacks flips and positions nor packs new ones, about 12 of an edge's 45
+// instructions.  The edge that carries the second minimum is found by |rel| ==
+// min1 afterwards (at a tie both minima are equal, so marking several edges
+// changes no message).  It costs message traffic: N words a row instead of four,
+// which the rows here have to gain by.  Rows of up to four messages cost nothing
+// more; the limits (kDirectOpen, kDirectClip) are where the batch of 8192 blocks
+// BG1 Zc=384, whose messages then take 99 of L2's 126 MB, stops gaining: with
+// limits 4, 7, 8, 9 and the open maximum 7.75, 7.48, 7.37, 7.31 ms.  19-edge rows
+// would take L2's rest.  8 iterations, compressed -> direct, open maximum / clamp:
+// 8192 of BG1 Zc=384 8.13 -> 7.31 / 9.47 -> 8.9 ms, 65536 of BG2 Zc=64 7.31 ->
+// 6.38 / 8.67 -> 7.66 ms, 16384 of BG1 Zc=112 5.62 -> 5.27 / 6.41 -> 6.17 ms,
+// 8192 of BG2 Zc=384 5.43 -> 4.61 / 6.43 -> 5.65 ms.
+template <int D, bool kPar, int kClip, bool kSmemEdges, bool kG1, typename P>
+__device__ __forceinline__ void row_update_direct(const P& p, const uint2* __restrict__ sedges, char* __restrict__ lqs,
+                                                  uint32_t zx4, uint32_t zxm4, uint32_t gb4, uint32_t lq_limit, int e0,
+                                                  int32_t alpha, int32_t beta, int32_t alpha1, int32_t beta1,
+                                                  const RowMsg<ahead_words(kG1)>& old, uint32_t fresh, uint32_t* __restrict__ lrp) {
+  constexpr int S = kThreadsTarget;    // plane stride (words)
+  constexpr int N = kPar ? D - 1 : D;  // edges with a message
+  if (!NRLDPC_INBOUNDS(e0 + D - 1, kMaxNnz, kBoundsEdge)) return;   // debug build
+  uint32_t nr[N];
+#pragma unroll
+  for (int j = 0; j < N; ++j) nr[j] = j < ahead_words(kG1) ? old.w[j < ahead_words(kG1) ? j : 0] : lrp[j * S];
+  if (fresh) {
+#pragma unroll
+    for (int j = 0; j < N; ++j) nr[j] &= ~fresh;
+  }
+  const auto table = [&](int j) {
+    if constexpr (kSmemEdges) return sedges[e0 + j];
+    else return p.edge_cs4[e0 + j];
+  };
+  const auto load = [&](uint32_t a) {
+    return NRLDPC_INBOUNDS(a, lq_limit, kBoundsLq) ? *reinterpret_cast<const uint32_t*>(lqs + a) : 0u;
+  };
+  const auto store = [&](uint32_t a, uint32_t v) {
+    if (NRLDPC_INBOUNDS(a, lq_limit, kBoundsLq)) *reinterpret_cast<uint32_t*>(lqs + a) = v;
+  };
+  uint32_t rel[D], addr[D], mag[D];
+  uint32_t sg = 0u, m1 = 0x7FFF7FFFu, m2 = 0x7FFF7FFFu;
+  if constexpr (kPar) {
+    const uint32_t cx = table(N).x;
+    addr[N] = kG1 ? zx4 + cx : zx4 + cx + gb4;
+    rel[N] = load(addr[N]);
+    sg = rel[N];
+    mag[N] = abs_u16x2(rel[N]);
+    m1 = __vminu2(m1, mag[N]);
+  }
+#pragma unroll
+  for (int j = 0; j < N; ++j) {
+    const uint2 cs = table(j);
+    if constexpr (kClip == kClipOpenMax) {   // (see row_update)
+      const uint32_t a4 = add_fma(p, cs.y, zx4);
+      const uint32_t t = __viaddmin_u32(a4, zxm4 - zx4, a4);
+      addr[j] = kG1 ? add_fma(p, t, cs.x) : add_fma(p, t, cs.x) + gb4;
+    } else {
+      addr[j] = min(zx4 + cs.y, zxm4 + cs.y) + cs.x + gb4;
+    }
+    const uint32_t x = __vadd2(load(addr[j]), nr[j]);
+    rel[j] = x;
+    sg ^= x;
+    mag[j] = abs_u16x2(x);
+    m2 = __vmaxu2(m1, __vminu2(m2, mag[j]));
+    m1 = __vminu2(m1, mag[j]);
+  }
+  const uint32_t maxp = ((uint32_t)(uint16_t)p.max_llr) * 0x10001u;
+  const uint32_t minp = ((uint32_t)(uint16_t)p.min_llr) * 0x10001u;
+  uint32_t s1, s2;
+  if constexpr (kClip == kClipOpenMax) {
+    s1 = scale_open(m1, alpha);
+    s2 = scale_open(m2, alpha);
+  } else {
+    s1 = scale_pair(__vmins2(m1, maxp), alpha, beta, alpha1, beta1);
+    s2 = scale_pair(__vmins2(m2, maxp), alpha, beta, alpha1, beta1);
+  }
+  // The magnitude of edge j's message: new_min2 where |rel| is the minimum (at a
+  // tie both minima are equal), else new_min1.
+  const auto magnitude = [&](int j) { return bsel(__vminu2(mag[j] ^ m1, 0x00010001u) * 0xFFFFu, s1, s2); };
+  uint32_t ovf = 0u;
+#pragma unroll
+  for (int j = 0; j < N; ++j) {
+    const uint32_t mf = sign_mask(sg ^ rel[j]), nmf = ~mf;
+    const uint32_t v = magnitude(j);
+    lrp[j * S] = __vadd2(v ^ nmf, nmf & 0x00010001u);   // mf ? v : -v
+    uint32_t nq;
+    if constexpr (kClip == kClipOpenMax) {
+      // v >= 0: rel + message with the message's sign put on the other operand
+      const uint32_t w = rel[j] ^ mf, u = __vadd2(w, v);
+      ovf |= u & ~w;
+      nq = __vmaxs2(u ^ mf, minp);
+    } else {
+      const uint32_t lr = __vadd2(v ^ mf, mf & 0x00010001u);
+      if constexpr (kClip == kClipClamp) {
+        const uint32_t sum = __vadd2(rel[j], lr);
+        ovf |= (sum ^ rel[j]) & ~(rel[j] ^ lr);
+        nq = __vmins2(__vmaxs2(sum, minp), maxp);
+      } else {
+        const int32_t lo = (int32_t)(int16_t)(rel[j] & 0xFFFFu) + (int32_t)(int16_t)(lr & 0xFFFFu);
+        const int32_t hi = (((int32_t)rel[j]) >> 16) + (((int32_t)lr) >> 16);
+        nq = clip_half_degen(lo, p.max_llr, p.min_llr) | (clip_half_degen(hi, p.max_llr, p.min_llr) << 16);
+      }
+    }
+    store(addr[j], nq);
+  }
+  if constexpr (kPar) ovf |= __vadd2(mag[N], s2);
+  if (kClip != kClipDegen && (ovf & 0x80008000u) != 0u) {   // rare (see row_update)
+#pragma unroll
+    for (int j = 0; j < D; ++j) {
+      const uint32_t lr = cond_neg16x2(magnitude(j), sign_mask(sg ^ rel[j]));
+      const uint32_t q = __vmins2(__vmaxs2(__vaddss2(rel[j], lr), minp), maxp);
+      store(addr[j], j < N ? q : __vsub2(q, lr));
+    }
+  }
+}
+
 // Belief (half h) of a parity column that belongs to row `deg` alone, from the
 // column's word and the row's message words (kPar above; edge deg - 1 of the row).
 __device__ __forceinline__ int16_t parity_belief(uint32_t word, const uint32_t* lrp, int deg, int h) {
@@ -356,43 +476,61 @@ __device__ __forceinline__ int16_t parity_belief(uint32_t word, const uint32_t* 
   return (int16_t)((int16_t)(word >> shift) + (flip ? -v : v));
 }
 
-// `par`: a row with a parity column of its own (row 4 and up).
+// `par`: a row with a parity column of its own (row 4 and up).  `direct`: the row
+// keeps its messages uncompressed (row_word in nrldpc_decode_common.cuh decides).
 template <int kClip, bool kSmemEdges, bool kG1, typename P>
-__device__ __forceinline__ void layer_dispatch(int deg, bool par, const P& p, const uint2* sedges, char* lqs, uint32_t zx4, uint32_t zxm4,
+__device__ __forceinline__ void layer_dispatch(int deg, bool par, bool direct, const P& p, const uint2* sedges, char* lqs, uint32_t zx4, uint32_t zxm4,
                                                uint32_t gb4, uint32_t lq_limit, int e0, int32_t alpha, int32_t beta,
-                                               int32_t alpha1, int32_t beta1, const RowMsg& old, uint32_t fresh,
+                                               int32_t alpha1, int32_t beta1, const RowMsg<ahead_words(kG1)>& old, uint32_t fresh,
                                                uint32_t* lrp) {
 #define NRLDPC_ROW(D, PAR) \
   row_update<D, PAR, kClip, kSmemEdges, kG1>(p, sedges, lqs, zx4, zxm4, gb4, lq_limit, e0, alpha, beta, alpha1, beta1, old, fresh, lrp); break;
+#define NRLDPC_SHORT(D, PAR) \
+  row_update_direct<D, PAR, kClip, kSmemEdges, kG1>(p, sedges, lqs, zx4, zxm4, gb4, lq_limit, e0, alpha, beta, alpha1, beta1, old, fresh, lrp); break;
   if constexpr (parity_words(kClip)) {
-    switch (par ? deg : deg + 32) {
-      case 3: NRLDPC_ROW(3, true)
-      case 4: NRLDPC_ROW(4, true)
-      case 5: NRLDPC_ROW(5, true)
-      case 6: NRLDPC_ROW(6, true)
-      case 7: NRLDPC_ROW(7, true)
-      case 8: NRLDPC_ROW(8, true)
-      case 9: NRLDPC_ROW(9, true)
-      case 10: NRLDPC_ROW(10, true)
+    switch (deg + (par ? 0 : 32) + (direct ? 0 : 64)) {
+      case 3: NRLDPC_SHORT(3, true)
+      case 4: NRLDPC_SHORT(4, true)
+      case 5: NRLDPC_SHORT(5, true)
+      case 6: NRLDPC_SHORT(6, true)
+      case 7: NRLDPC_SHORT(7, true)
+      case 8: NRLDPC_SHORT(8, true)
+      case 9: NRLDPC_SHORT(9, true)
+      case 10: NRLDPC_SHORT(10, true)
+      case 64 + 3: NRLDPC_ROW(3, true)
+      case 64 + 4: NRLDPC_ROW(4, true)
+      case 64 + 5: NRLDPC_ROW(5, true)
+      case 64 + 6: NRLDPC_ROW(6, true)
+      case 64 + 7: NRLDPC_ROW(7, true)
+      case 64 + 8: NRLDPC_ROW(8, true)
+      case 64 + 9: NRLDPC_ROW(9, true)
+      case 64 + 10: NRLDPC_ROW(10, true)
       // core rows: BG2 has 8 and 10 edges, BG1 19
-      case 32 + 8: NRLDPC_ROW(8, false)
-      case 32 + 10: NRLDPC_ROW(10, false)
+      case 32 + 8: NRLDPC_SHORT(8, false)
+      case 32 + 10: NRLDPC_SHORT(10, false)
+      case 96 + 8: NRLDPC_ROW(8, false)
+      case 96 + 10: NRLDPC_ROW(10, false)
       default: NRLDPC_ROW(19, false)
     }
   } else {
-    switch (deg) {
-      case 3: NRLDPC_ROW(3, false)
-      case 4: NRLDPC_ROW(4, false)
-      case 5: NRLDPC_ROW(5, false)
-      case 6: NRLDPC_ROW(6, false)
-      case 7: NRLDPC_ROW(7, false)
-      case 8: NRLDPC_ROW(8, false)
-      case 9: NRLDPC_ROW(9, false)
-      case 10: NRLDPC_ROW(10, false)
+    switch (deg + (direct ? 0 : 64)) {
+      case 7: NRLDPC_SHORT(7, false)
+      case 8: NRLDPC_SHORT(8, false)
+      case 3: NRLDPC_SHORT(3, false)
+      case 4: NRLDPC_SHORT(4, false)
+      case 5: NRLDPC_SHORT(5, false)
+      case 6: NRLDPC_SHORT(6, false)
+      case 64 + 5: NRLDPC_ROW(5, false)
+      case 64 + 6: NRLDPC_ROW(6, false)
+      case 64 + 7: NRLDPC_ROW(7, false)
+      case 64 + 8: NRLDPC_ROW(8, false)
+      case 64 + 9: NRLDPC_ROW(9, false)
+      case 64 + 10: NRLDPC_ROW(10, false)
       default: NRLDPC_ROW(19, false)
     }
   }
 #undef NRLDPC_ROW
+#undef NRLDPC_SHORT
 }
 
 }  // namespace fixedrow

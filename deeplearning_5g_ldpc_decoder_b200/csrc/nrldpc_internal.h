@@ -56,10 +56,20 @@ uint32_t crc_remainder(const uint8_t* data, int len, int crctype);
 // message whose only set bit sits d positions before its end.
 void crc_position_table(int crctype, uint32_t* out /* kMaxB */);
 
-// Scratch planes (kThreadsTarget words each) of one lifted check row of degree
-// d in the fixed-point kernels: the two minima, the flip bits and the min2
-// bits, plus a fifth word for degree-19 rows (layout in nrldpc_fixed_row.cuh).
-inline int fixed_row_planes(int d) { return d > 16 ? 5 : 4; }
+// Scratch planes (kThreadsTarget words each) of lifted check row r, degree d, in the
+// fixed-point kernels (layout in nrldpc_fixed_row.cuh).  At least the compressed
+// message: the two minima, the flip bits and the min2 bits, plus a fifth word for
+// degree-19 rows.  `direct`: also room for one word per message in the rows that
+// may keep their messages as they are, 258 planes in all for BG1 instead of 188
+// and 203 for BG2 instead of 168.  (The no-allocation entry point's static scratch
+// bounds its CTAs in flight, so it stays with the smaller layout.)
+constexpr int kDirectOpen = 10, kDirectClip = 8;   // messages of such a row at most, with the open maximum and without
+inline int fixed_row_planes(int r, int d, bool direct) {
+  const int compressed = d > 16 ? 5 : 4;
+  const int open = r < kCoreRows ? d : d - 1;   // messages with the open maximum, and without it d
+  const int n = open <= kDirectOpen ? (d <= kDirectClip ? d : open) : 0;
+  return direct && n > compressed ? n : compressed;
+}
 // Scratch words per CTA of the mixed-size kernel: the larger of the two base
 // graphs' layouts (all rows' planes x kThreadsTarget).
 uint32_t mixed_scratch_words_per_cta();

@@ -173,6 +173,7 @@ __device__ __forceinline__ void mixed_crc_flush(uint32_t* s_crc, int gg, uint32_
 
 template <int kClip, int kThreads, int kCap, int kMinBlocks>
 __global__ void __launch_bounds__(kThreads, kMinBlocks) fixed_mixed_kernel(const __grid_constant__ MixedParams p) {
+  constexpr int kAhead = ahead_words(false);
   constexpr int kGroups = kCap / 2;       // G = floor(kCap / Zc) <= kCap / 2 (Zc >= 2)
   extern __shared__ __align__(16) uint32_t s_lq[];
   __shared__ uint32_t s_crc[2 * kGroups];
@@ -214,8 +215,10 @@ __global__ void __launch_bounds__(kThreads, kMinBlocks) fixed_mixed_kernel(const
     const int bi = s_g.bgn == 1 ? 0 : 1;
     for (int r = tid; r < s_g.R; r += blockDim.x) {
       const uint32_t e0 = s_g.row_off[r], dg = (uint32_t)s_g.row_off[r + 1] - e0;
-      const uint32_t five = s_g.lr_off[r + 1] - s_g.lr_off[r] > 4u * kThreadsTarget ? 1u : 0u;
-      s_rows[r] = make_uint4(s_g.lr_off[r], e0 | (dg << 16) | (five << 24), p.w_inline[bi][r], 0u);
+      s_rows[r] = make_uint4(s_g.lr_off[r],
+                             row_word(e0, dg, (s_g.lr_off[r + 1] - s_g.lr_off[r]) / kThreadsTarget, kClip,
+                                      parity_words(kClip) && r >= kCoreRows, false),
+                             p.w_inline[bi][r], 0u);
     }
     if (tid < 2 * G) s_cw[tid] = take_block(p, key);
     __syncthreads();
@@ -241,16 +244,16 @@ __global__ void __launch_bounds__(kThreads, kMinBlocks) fixed_mixed_kernel(const
     const uint32_t zx4 = 4u * (uint32_t)zx;
     const uint32_t zxm4 = zx4 - 4u * (uint32_t)Zc;
     const uint32_t gb4 = 4u * (uint32_t)((active ? g : 0) * lq_len);
-    RowMsg nxt{};
+    RowMsg<kAhead> nxt{};
     for (;;) {
       const bool run = p.max_it > 0;   // max_iterations == 0: rate recovery only, status 1
       for (int row = 0; run && row < s_g.R; ++row) {
         if (busy) {
-          const RowMsg cur = nxt;
+          const RowMsg<kAhead> cur = nxt;
           const uint4 d = s_rows[row];
           const int rn = row + 1 < s_g.R ? row + 1 : 0;
           const uint2 dn = *reinterpret_cast<const uint2*>(&s_rows[rn]);
-          nxt = load_row_msg(scratch + dn.x + tid, row_five(dn.y));
+          nxt = load_row_msg<kAhead>(scratch + dn.x + tid, row_words(dn.y));
           uint32_t ab0, ab1;
           if (p.weights_T[bi] > 0) {
             ab0 = __ldg(p.weights[bi] + (min((int)(itv & 0xFFFFu), p.weights_T[bi] - 1) * s_g.R + row));
@@ -258,7 +261,7 @@ __global__ void __launch_bounds__(kThreads, kMinBlocks) fixed_mixed_kernel(const
           } else {
             ab0 = ab1 = d.z;
           }
-          layer_dispatch<kClip, true, false>(row_deg(d.y), row >= kCoreRows, p, s_g.edges, reinterpret_cast<char*>(s_lq), zx4, zxm4, gb4,
+          layer_dispatch<kClip, true, false>(row_deg(d.y), row >= kCoreRows, row_direct(d.y), p, s_g.edges, reinterpret_cast<char*>(s_lq), zx4, zxm4, gb4,
                                            4u * (uint32_t)(G * lq_len), row_e0(d.y),
                                            (int32_t)(int16_t)(ab0 & 0xFFFFu), ((int32_t)ab0) >> 16,
                                            (int32_t)(int16_t)(ab1 & 0xFFFFu), ((int32_t)ab1) >> 16, cur, fresh,

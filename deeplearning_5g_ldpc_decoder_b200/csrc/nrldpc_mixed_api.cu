@@ -76,7 +76,7 @@ uint32_t mixed_scratch_words_per_cta() {
   for (int bgn = 1; bgn <= 2; ++bgn) {
     const BaseGraph& g = base_graph(bgn);
     uint32_t planes = 0;
-    for (int r = 0; r < g.rows; ++r) planes += (uint32_t)fixed_row_planes(g.degree[r]);
+    for (int r = 0; r < g.rows; ++r) planes += (uint32_t)fixed_row_planes(r, g.degree[r], true);
     best = std::max(best, planes * (uint32_t)kThreadsTarget);
   }
   return best;
@@ -98,7 +98,7 @@ MixedGraph make_graph(int bgn, int Zc, int iLS, int cap) {
   uint32_t off = 0;
   for (int r = 0; r < g.rows; ++r) {
     m.lr_off[r] = off;
-    off += (uint32_t)fixed_row_planes(g.degree[r]) * kThreadsTarget;
+    off += (uint32_t)fixed_row_planes(r, g.degree[r], true) * kThreadsTarget;
     m.row_off[r] = g.row_off[r];
   }
   m.lr_off[g.rows] = off;

@@ -178,7 +178,7 @@ extern "C" int32_t nrldpc_decode_batch_noalloc(const int16_t* d_llr, int64_t llr
   uint32_t off = 0;
   for (int r = 0; r < g.rows; ++r) {
     p.lr_off[r] = off;
-    off += (uint32_t)fixed_row_planes(g.degree[r]) * (uint32_t)kThreadsTarget;
+    off += (uint32_t)fixed_row_planes(r, g.degree[r], false) * (uint32_t)kThreadsTarget;
   }
   p.lr_off[g.rows] = off;
   p.scratch_words = off;

@@ -384,7 +384,7 @@ MixedGraph tb_make_graph(int bgn, int Zc, int iLS) {
   uint32_t off = 0;
   for (int r = 0; r < g.rows; ++r) {
     m.lr_off[r] = off;
-    off += (uint32_t)fixed_row_planes(g.degree[r]) * kThreadsTarget;
+    off += (uint32_t)fixed_row_planes(r, g.degree[r], true) * kThreadsTarget;
     m.row_off[r] = g.row_off[r];
   }
   m.lr_off[g.rows] = off;
