@@ -286,15 +286,26 @@ int make_plan(const CodeParams& cp, const ldpc_decoder_cfg_t& dc, int num_cw, De
   p.f_max = (float)dc.max_llr / 128.0f;
   p.f_min = (float)dc.min_llr / 128.0f;
   plan->clip = fixed_clip_mode(dc, p.w_inline, g.rows);
-  // The small-batch kernel while all blocks run at once.  Measured, 8 iterations,
-  // pair kernel / small-batch kernel in us: BG1 Zc 24, 1 to 148 blocks 230 / 108,
-  // 444 (three per SM, its last) 234 / 136, 888 in two rounds 236 / 265; BG2 Zc 64,
-  // 64 blocks 155 / 86, 444 155 / 132, 592 155 / 197; BG1 Zc 112, 148 blocks
-  // 246 / 148, 149 246 / 288; BG1 Zc 208, 148 blocks 308 / 273, 149 308 / 541.
+  // The small-batch kernel while all blocks run at once, with eight lanes per row
+  // pair while an SM then holds few threads (its rows have a shorter chain, but
+  // issue more in all), else with four; eight again where only they fit.  Measured,
+  // 8 iterations, us for the pair kernel / four lanes / eight lanes: BG1 Zc 24, 64
+  // blocks 230 / 103 / 85, 444 (three per SM, 576 threads) 234 / 132 / 123, 592
+  // 230 / does not fit / 149; BG1 Zc 40, 296 blocks (640 threads) - / 134 / 126;
+  // BG1 Zc 48, 296 blocks (768) - / 134 / 142; BG1 Zc 80, 64 blocks (640) - / 134 /
+  // 126; BG1 Zc 112, 64 blocks 246 / 146 / 155, 149 in two rounds 246 / 288; BG2 Zc
+  // 22, 64 blocks (192) - / 77 / 73; BG2 Zc 40 (320) - / 83 / 83; BG2 Zc 64, 64
+  // blocks (512) 155 / 83 / 91, 592 in two rounds 155 / 197; BG1 Zc 208, 148 blocks
+  // 308 / 273, 149 308 / 541.
   if (fixed && num_cw <= 32 * st->num_sms) {
-    split_layout(g, p.lr_off);
-    if (split_shape(cp.Zc, g.cols, (int)(p.lr_off[g.rows] & 0xFFFFu), &plan->shape)) {
-      const uint64_t key = 6ull << 56 | (uint64_t)plan->clip << 48 | (uint64_t)plan->shape.table << 47 |
+    const int per_sm = (num_cw + st->num_sms - 1) / st->num_sms;
+    const int few = cp.bgn == 1 ? 640 : 320;
+    for (int k = 0; k < 3; ++k) {
+      const int lanes = k == 1 ? 4 : 8;
+      split_layout(g, lanes, p.lr_off);
+      if (!split_shape(cp.Zc, g.cols, lanes, (int)(p.lr_off[g.rows] & 0xFFFFu), &plan->shape)) continue;
+      if (k == 0 && plan->shape.block * per_sm > few) continue;
+      const uint64_t key = (lanes == 8 ? 7ull : 6ull) << 56 | (uint64_t)plan->clip << 48 | (uint64_t)plan->shape.table << 47 |
                            (uint64_t)plan->shape.block << 32 | (uint64_t)(uint32_t)plan->shape.smem;
       const int occ = cached_occupancy(st, key, [&] { return occupancy_split(plan->shape, plan->clip); });
       if (num_cw <= occ * st->num_sms) {

@@ -301,11 +301,12 @@ int launch_fixed(const DecodeParams& p, int grid, int block, int smem, int clip_
 // The small-batch fixed-point kernel (nrldpc_split.cu): one code block per CTA.
 // In its DecodeParams lr_off is what split_layout writes.
 struct SplitShape {
+  int lanes;                       // lanes per row pair: 4 or 8
   int words, slots, block, smem;   // words of beliefs, message slots, threads, dynamic shared memory
   bool table;                      // the slots' addresses are kept in shared memory
 };
-void split_layout(const BaseGraph& g, uint32_t* lr_off);
-bool split_shape(int Zc, int cols, int slots, SplitShape* out);   // false: does not fit an SM
+void split_layout(const BaseGraph& g, int lanes, uint32_t* lr_off);
+bool split_shape(int Zc, int cols, int lanes, int slots, SplitShape* out);   // false: does not fit an SM
 int launch_split(const DecodeParams& p, const SplitShape& s, int clip_mode, void* stream);
 int occupancy_split(const SplitShape& s, int clip_mode);
 int launch_float_minsum(const DecodeParams& p, int grid, int block, int smem, void* stream);

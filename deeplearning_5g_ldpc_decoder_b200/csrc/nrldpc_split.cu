@@ -1,6 +1,6 @@
 // nrldpc_split.cu — fixed-point layered min-sum decoder (algos 1, 2, 3) for
 // batches too small to fill the GPU: one code block per CTA, each lifted check
-// row split over four lanes.
+// row split over four or eight lanes.
 //
 // Bit-exact with c_lib/fixedpoint_ldpc_decoder.c:103-222 like the pair kernel
 // (nrldpc_fixed.cu), from which it differs in where the parallelism comes from:
@@ -9,8 +9,8 @@
 //    rows are zx and zx + H.  Both rows of an edge lie in the one word
 //    (zx + V) mod H, in this order or the other: a byte permute on load and
 //    store.  (An odd Zc, 3 to 15, keeps one belief per word: H = Zc, no permute.)
-//  * Four lanes share a row pair's edges: lane l takes edges l, l + 4, ...
-//    Minima and sign parity meet in two shuffle steps.  The edge that carries
+//  * Four or eight lanes (kLanes) share a row pair's edges: lane l takes edges l,
+//    l + kLanes, ...  Minima and sign parity meet in two or three shuffle steps.  The edge that carries
 //    the second minimum is found by |rel| == min1 afterwards; at a tie both
 //    minima are equal, so marking several edges changes no message.
 //  * Two consecutive layers without a common base column touch disjoint beliefs
@@ -25,13 +25,16 @@
 //    and old messages are loaded while the row before it still computes, so
 //    only the beliefs' load follows the layer barrier.
 //
-// A step is one dependent chain of about 140 instructions in each of a few
-// warps, 600 to 700 cycles (a thread that walks a whole row takes over 1000
+// A step is one dependent chain of about 140 instructions (four lanes) in each of
+// a few warps, 600 to 700 cycles (a thread that walks a whole row takes over 1000
 // cycles a layer), so what bounds the kernel is that chain, not a throughput.
 // One iteration of BG1 Zc=24: 25.8 us in the pair kernel, 11.2 us here; BG2
 // Zc=64 17.2 and 8.9 us; BG1 Zc=112 27.6 and 15.8 us.  With one group per step
 // 18.2, 10.7 and 17.8 us; with the pair kernel's compressed messages (16 or 32
-// flag bits per lane) and one group 21, 14 and 23 us.
+// flag bits per lane) and one group 21, 14 and 23 us.  With eight lanes a thread
+// has one edge of a row of up to eight: 8 iterations of Zc=24 take 104 us with four
+// and 85 us with eight, Zc=2 98 and 77 us; the shuffle step and the warps more cost
+// more than that gives from Zc=112 (BG1) or 48 (BG2) on.
 #include <cuda_runtime.h>
 #include <stdint.h>
 
@@ -44,11 +47,9 @@ namespace {
 
 using namespace fixedrow;
 
-constexpr int kLanes = 4;          // lanes per row pair
-constexpr int kAhead = 3;          // slots per lane loaded a row ahead (degree <= 12)
-constexpr int kMostSlots = (kMaxDegree + kLanes - 1) / kLanes;
+constexpr int kAhead = 3;          // slots per lane loaded a row ahead (degree <= 12 with four lanes, all with eight)
 constexpr int kGroupsPerStep = 2;
-constexpr int kSplitThreads = 1024;   // two groups of 4 H threads, Zc <= 256 (what fits shared memory ends below that)
+constexpr int kSplitThreads = 1024;   // two groups of kLanes H threads: Zc <= 256 or 128 (what fits shared memory may end below that)
 
 // Permute selectors: the word as it is, and with its halves swapped.
 constexpr uint32_t kStraight = 0x3210u, kSwapBit = 0x2222u;
@@ -88,7 +89,7 @@ struct Slots {
 
 // One layer for one thread: K = ceil(degree / 4) slots.  Threads that own no rows
 // (`active` false) only take part in the shuffles; `tail`: the last slot has an edge.
-template <int K, int kClip, typename AtSlot>
+template <int K, int kLanes, int kClip, typename AtSlot>
 __device__ __forceinline__ void split_row(const DecodeParams& p, const Geometry& g, char* __restrict__ lq, const Slots& in,
                                           AtSlot at_slot, uint32_t* __restrict__ msg, int stride, bool active, bool tail, int32_t alpha,
                                           int32_t beta) {
@@ -215,13 +216,14 @@ __device__ __forceinline__ void split_recover(const DecodeParams& p, const Geome
 // kTable: the slots' words come from a table in shared memory (beside the
 // messages: one 8-byte load per slot) instead of being computed from the edge
 // records.
-template <int kClip, bool kTable>
+template <int kClip, bool kTable, int kLanes>
 __global__ void __launch_bounds__(kSplitThreads, 1) split_kernel(const __grid_constant__ DecodeParams p) {
   // beliefs [cols][H], four words (the neutral one first), slots [slots][threads of a group]
   extern __shared__ __align__(16) uint32_t s_lq[];
   __shared__ uint4 s_edges[kMaxNnz];
   __shared__ uint4 s_steps[kMaxRows * kGroupsPerStep];
   __shared__ uint32_t s_crc;
+  constexpr int kMostSlots = (kMaxDegree + kLanes - 1) / kLanes;
   const int tid = threadIdx.x, nt = blockDim.x;
   const int cw = blockIdx.x;
   const int T = nt / kGroupsPerStep;                 // threads of a group, whole warps
@@ -262,8 +264,8 @@ __global__ void __launch_bounds__(kSplitThreads, 1) split_kernel(const __grid_co
   __syncthreads();
 
   const int lane = tid & (kLanes - 1);
-  const bool active = (t >> 2) < g.H;
-  const uint32_t zx4 = active ? 4u * (uint32_t)(t >> 2) : 0u;
+  const bool active = (t / kLanes) < g.H;
+  const uint32_t zx4 = active ? 4u * (uint32_t)(t / kLanes) : 0u;
   const uint32_t neutral = ((uint32_t)(4 * words) << 16) | kStraight;
   char* lq = reinterpret_cast<char*>(s_lq);
   // slot k of the row d
@@ -312,15 +314,15 @@ __global__ void __launch_bounds__(kSplitThreads, 1) split_kernel(const __grid_co
         const int32_t alpha = (int32_t)(int16_t)(ab & 0xFFFFu), beta = ((int32_t)ab) >> 16;
         uint32_t* msg = mine + d.y + (kTable ? 1 : 0);
         const auto at_slot = [&](int k) { return kTable ? msg[k * stride - 1] : compute_slot(d, k); };
-        const int left = deg - lane;   // slot k has an edge while 4 k < left
-        if (deg <= 4) {
-          split_row<1, kClip>(p, g, lq, cur, at_slot, msg, stride, active, active && left > 0, alpha, beta);
-        } else if (deg <= 8) {
-          split_row<2, kClip>(p, g, lq, cur, at_slot, msg, stride, active, active && left > kLanes, alpha, beta);
-        } else if (deg <= 12) {
-          split_row<3, kClip>(p, g, lq, cur, at_slot, msg, stride, active, active && left > 2 * kLanes, alpha, beta);
+        const int left = deg - lane;   // slot k has an edge while kLanes k < left
+        if (deg <= kLanes) {
+          split_row<1, kLanes, kClip>(p, g, lq, cur, at_slot, msg, stride, active, active && left > 0, alpha, beta);
+        } else if (deg <= 2 * kLanes) {
+          split_row<2, kLanes, kClip>(p, g, lq, cur, at_slot, msg, stride, active, active && left > kLanes, alpha, beta);
+        } else if (deg <= 3 * kLanes) {
+          split_row<3, kLanes, kClip>(p, g, lq, cur, at_slot, msg, stride, active, active && left > 2 * kLanes, alpha, beta);
         } else {
-          split_row<kMostSlots, kClip>(p, g, lq, cur, at_slot, msg, stride, active, active && left > (kMostSlots - 1) * kLanes,
+          split_row<kMostSlots, kLanes, kClip>(p, g, lq, cur, at_slot, msg, stride, active, active && left > (kMostSlots - 1) * kLanes,
                                        alpha, beta);
         }
       }
@@ -378,24 +380,31 @@ __global__ void __launch_bounds__(kSplitThreads, 1) split_kernel(const __grid_co
 // Opt-in shared memory per CTA less the static arrays.
 constexpr int kSplitSmemMax = 227 * 1024 - 16 * (kMaxNnz + kGroupsPerStep * kMaxRows) - 128;
 
-template <int kClip, bool kTable>
+template <int kClip, bool kTable, int kLanes>
 int split_op(const DecodeParams* p, int block, int smem, cudaStream_t s, int* occ) {
   static std::atomic<uint32_t> attr_done{0};
-  const int err = raise_smem_limit_once(split_kernel<kClip, kTable>, &attr_done, kSplitSmemMax);
+  const int err = raise_smem_limit_once(split_kernel<kClip, kTable, kLanes>, &attr_done, kSplitSmemMax);
   if (err != 0) return err;
-  if (occ) return (int)cudaOccupancyMaxActiveBlocksPerMultiprocessor(occ, split_kernel<kClip, kTable>, block, smem);
-  split_kernel<kClip, kTable><<<p->num_cw, block, smem, s>>>(*p);
+  if (occ) return (int)cudaOccupancyMaxActiveBlocksPerMultiprocessor(occ, split_kernel<kClip, kTable, kLanes>, block, smem);
+  split_kernel<kClip, kTable, kLanes><<<p->num_cw, block, smem, s>>>(*p);
   count_launch();
   return (int)cudaGetLastError();
 }
 
-template <bool kTable>
-int split_dispatch(const DecodeParams* p, int block, int smem, int clip_mode, cudaStream_t s, int* occ) {
+template <bool kTable, int kLanes>
+int split_clip(const DecodeParams* p, int block, int smem, int clip_mode, cudaStream_t s, int* occ) {
   switch (clip_mode) {
-    case kClipDegen: return split_op<kClipDegen, kTable>(p, block, smem, s, occ);
-    case kClipOpenMax: return split_op<kClipOpenMax, kTable>(p, block, smem, s, occ);
-    default: return split_op<kClipClamp, kTable>(p, block, smem, s, occ);
+    case kClipDegen: return split_op<kClipDegen, kTable, kLanes>(p, block, smem, s, occ);
+    case kClipOpenMax: return split_op<kClipOpenMax, kTable, kLanes>(p, block, smem, s, occ);
+    default: return split_op<kClipClamp, kTable, kLanes>(p, block, smem, s, occ);
   }
+}
+
+// Eight lanes always have their table: they are for lifting sizes where it fits.
+int split_dispatch(const DecodeParams* p, const SplitShape& sh, int clip_mode, cudaStream_t s, int* occ) {
+  if (sh.lanes == 8) return split_clip<true, 8>(p, sh.block, sh.smem, clip_mode, s, occ);
+  return sh.table ? split_clip<true, 4>(p, sh.block, sh.smem, clip_mode, s, occ)
+                  : split_clip<false, 4>(p, sh.block, sh.smem, clip_mode, s, occ);
 }
 
 int split_smem(const SplitShape& s) { return 4 * (s.words + 4 + (s.table ? 2 : 1) * s.slots * s.block / kGroupsPerStep); }
@@ -407,7 +416,7 @@ int bounds_read_split(uint32_t* out, bool reset) { return bounds_read_tu(out, re
 // lr_off of a base graph for split_kernel: each row's first slot, step and group
 // (a row joins the step of the row before it when that one is alone there and
 // they share no column), and in lr_off[rows] the numbers of slots and steps.
-void split_layout(const BaseGraph& g, uint32_t* lr_off) {
+void split_layout(const BaseGraph& g, int lanes, uint32_t* lr_off) {
   uint32_t slot = 0;
   int step = -1, group = kGroupsPerStep;
   for (int r = 0; r < g.rows; ++r) {
@@ -418,20 +427,21 @@ void split_layout(const BaseGraph& g, uint32_t* lr_off) {
     group = joins ? group + 1 : 0;
     step += joins ? 0 : 1;
     lr_off[r] = slot | (uint32_t)step << 16 | (uint32_t)group << 24;
-    slot += (uint32_t)((g.degree[r] + kLanes - 1) / kLanes);
+    slot += (uint32_t)((g.degree[r] + lanes - 1) / lanes);
   }
   lr_off[g.rows] = slot | (uint32_t)(step + 1) << 16;
 }
 
-bool split_shape(int Zc, int cols, int slots, SplitShape* out) {
+bool split_shape(int Zc, int cols, int lanes, int slots, SplitShape* out) {
   SplitShape s;
   const int H = (Zc & 1) ? Zc : Zc / 2;
+  s.lanes = lanes;
   s.words = (cols * H + 3) & ~3;
   s.slots = slots;
-  s.block = kGroupsPerStep * ((kLanes * H + 31) & ~31);
+  s.block = kGroupsPerStep * ((lanes * H + 31) & ~31);
   s.table = true;
   s.smem = split_smem(s);
-  if (s.smem > kSplitSmemMax) {
+  if (s.smem > kSplitSmemMax && lanes == 4) {
     s.table = false;
     s.smem = split_smem(s);
   }
@@ -440,14 +450,11 @@ bool split_shape(int Zc, int cols, int slots, SplitShape* out) {
 }
 
 int launch_split(const DecodeParams& p, const SplitShape& s, int clip_mode, void* stream) {
-  cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
-  return s.table ? split_dispatch<true>(&p, s.block, s.smem, clip_mode, st, nullptr)
-                 : split_dispatch<false>(&p, s.block, s.smem, clip_mode, st, nullptr);
+  return split_dispatch(&p, s, clip_mode, reinterpret_cast<cudaStream_t>(stream), nullptr);
 }
 int occupancy_split(const SplitShape& s, int clip_mode) {
   int n = 0;
-  if (s.table) split_dispatch<true>(nullptr, s.block, s.smem, clip_mode, nullptr, &n);
-  else split_dispatch<false>(nullptr, s.block, s.smem, clip_mode, nullptr, &n);
+  split_dispatch(nullptr, s, clip_mode, nullptr, &n);
   return n;
 }
 

@@ -81,3 +81,19 @@ def test_small_batches_equal_the_pair_kernel(oracle, cuda, lib, row, bgn, A, E, 
         es, eb, ei, lq = oracle.decode(np.ascontiguousarray(host[i, :E]), in_config(*cfg), dec_cfg(r))
         assert int(got.status[i]) == es and int(got.iterations[i]) == ei
         assert np.array_equal(got.app[i].cpu().numpy(), lq)
+
+
+@pytest.mark.parametrize("row", [0, 2, 3, 5])
+@pytest.mark.parametrize("bgn,A,E,Qm,per_sm,extra", [
+    (1, 488, 1536, 2, 3, 0),          # Zc 24: eight lanes, the last batch of three blocks per SM
+    (1, 488, 1536, 2, 4, 0),          # four per SM: only eight lanes fit
+    (1, 840, 2400, 4, 2, 0),          # Zc 40: 640 threads on an SM
+    (1, 1736, 5000, 4, 0, 5),         # Zc 80: the last size with eight lanes
+    (1, 1744, 5000, 4, 1, 1),         # Zc 88 and above, two rounds of one block: pair kernel or four lanes
+    (2, 120, 400, 2, 2, 0),           # Zc 24 of BG2: 384 threads, four lanes
+    (2, 104, 400, 2, 1, 0),           # eight lanes
+    (2, 24, 100, 2, 10, 0),           # four lanes do not fit
+])
+def test_lane_counts_equal_the_pair_kernel(oracle, cuda, lib, row, bgn, A, E, Qm, per_sm, extra):
+    n = per_sm * torch.cuda.get_device_properties(0).multi_processor_count + extra
+    test_small_batches_equal_the_pair_kernel(oracle, cuda, lib, row, bgn, A, E, 0, Qm, n, 0)
