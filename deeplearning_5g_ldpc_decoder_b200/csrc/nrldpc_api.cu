@@ -328,7 +328,7 @@ int make_plan(const CodeParams& cp, const ldpc_decoder_cfg_t& dc, int num_cw, De
     } else if (fixed) {
       planes = fixed_row_planes(r, deg, true);
     } else {
-      planes = 3;
+      planes = float_row_planes(deg);
     }
     // The fixed-point kernel addresses its planes with a compile-time stride.
     off += (uint32_t)planes * (uint32_t)(fixed ? kThreadsTarget : p.nact);

@@ -13,7 +13,8 @@
 // Mapping: one code block per group of Zc threads, up to G = floor(384 / Zc) groups
 // per CTA, FP32 beliefs in shared memory, persistent grid.  Min-sum messages
 // are stored compressed per lifted check row (two minima, one word of flip bits
-// and the minimum's position: 12 bytes); BP messages are stored per edge.
+// and the minimum's position: 12 bytes) in rows of more than five edges; messages
+// of shorter rows and of BP are stored per edge.
 #include <cuda_runtime.h>
 #include <float.h>
 #include <math.h>
@@ -38,13 +39,14 @@ __device__ __forceinline__ float clipf(float v, float mx, float mn) {
 __shared__ uint2 s_fedge4[kMaxNnz];
 
 // ---------------------------------------------------------------- float min-sum
-// Stored message of a lifted check row (3 planes): new_min1, new_min2 (float
-// bits), and a word with edge j's sign flip in bit D - 1 - j and the position of
-// new_min2's edge from bit 20.  The kernel loads a row's words while the row
-// before it computes.
+// Stored message of a lifted check row: in rows of up to five edges (kFloatDirect)
+// the messages themselves, one plane each, otherwise three planes: new_min1,
+// new_min2 (float bits), and a word with edge j's sign flip in bit D - 1 - j and the
+// position of new_min2's edge from bit 20.  The kernel loads a row's first words
+// while the row before it computes.
+constexpr int kFloatAhead = 3;   // words loaded a row ahead
 struct FloatMsg {
-  float n1, n2;
-  uint32_t f;
+  uint32_t w[kFloatAhead];
 };
 
 // One row, operation for operation as the reference.  A belief of -0.0 counts as
@@ -52,7 +54,8 @@ struct FloatMsg {
 // exactly where v < 0; then parity, flip and the sign of a message are bit
 // operations on sign bits.  The ALU pipe bounds the kernel (76 % busy, 25 of 45
 // instructions per edge).  8 iterations of 4096 blocks BG1 Zc=384: 6.91 -> 6.29 ms,
-// 777 blocks BG1 Zc=208 957 -> 877 us, against bit tests and compares on values
+// 777 blocks BG1 Zc=208 957 -> 877 us (and 6.12 ms and 835 us with short rows in
+// the form below and the second minimum by a min and a max), against bit tests and compares on values
 // and messages loaded where the row starts.  Address adds as multiply-adds on the
 // FMA pipe: 6.51 ms and 869 us, because of spills at Zc=384, and not used.
 // kRange: min_llr <= max_llr, so the clip is a min and a max.
@@ -62,7 +65,8 @@ __device__ __forceinline__ void fms_row(const DecodeParams& p, char* __restrict_
   if (!NRLDPC_INBOUNDS(e0 + D - 1, kMaxNnz, kBoundsEdge)) return;   // debug build
   const uint32_t zc4 = 4u * (uint32_t)p.Zc;
   [[maybe_unused]] const uint32_t limit = 4u * (uint32_t)p.lq_len;   // bytes of beliefs (debug build)
-  const int ix = (int)(old.f >> 20);
+  const float n1 = __uint_as_float(old.w[0]), n2 = __uint_as_float(old.w[1]);
+  const int ix = (int)(old.w[2] >> 20);
   float rel[D];
   uint32_t addr[D];
   float m1 = FLT_MAX, m2 = FLT_MAX;
@@ -74,14 +78,14 @@ __device__ __forceinline__ void fms_row(const DecodeParams& p, char* __restrict_
     const uint32_t t = e.y + zx4;
     addr[j] = min(t, t - zc4) + e.x;
     const float q = NRLDPC_INBOUNDS(addr[j], limit, kBoundsLq) ? *reinterpret_cast<const float*>(lq + addr[j]) : 0.0f;
-    const uint32_t r = __float_as_uint(j == ix ? old.n2 : old.n1) ^ ((old.f << (32 - D + j)) & 0x80000000u);
+    const uint32_t r = __float_as_uint(j == ix ? n2 : n1) ^ ((old.w[2] << (32 - D + j)) & 0x80000000u);
     const float v = __fsub_rn(q, __uint_as_float(r));
     rel[j] = v;
     sg ^= __float_as_uint(__fadd_rn(v, 0.0f));
     const float a = fabsf(v);
     // float_update_two_minima (:171-180): strict <, first index wins.
     const bool lt = a < m1;
-    m2 = lt ? m1 : fminf(m2, a);
+    m2 = fminf(m2, fmaxf(m1, a));
     m1 = fminf(m1, a);
     idx = lt ? j : idx;
   }
@@ -108,19 +112,74 @@ __device__ __forceinline__ void fms_row(const DecodeParams& p, char* __restrict_
   lrp[2 * NT] = flips | (uint32_t)idx << 20;
 }
 
-template <bool kRange>
-__device__ __forceinline__ void fms_dispatch(int deg, const DecodeParams& p, char* lq, uint32_t zx4, int e0, const FloatMsg& old, uint32_t* lrp, int NT) {
-  switch (deg) {
-    case 3: fms_row<3, kRange>(p, lq, zx4, e0, old, lrp, NT); break;
-    case 4: fms_row<4, kRange>(p, lq, zx4, e0, old, lrp, NT); break;
-    case 5: fms_row<5, kRange>(p, lq, zx4, e0, old, lrp, NT); break;
-    case 6: fms_row<6, kRange>(p, lq, zx4, e0, old, lrp, NT); break;
-    case 7: fms_row<7, kRange>(p, lq, zx4, e0, old, lrp, NT); break;
-    case 8: fms_row<8, kRange>(p, lq, zx4, e0, old, lrp, NT); break;
-    case 9: fms_row<9, kRange>(p, lq, zx4, e0, old, lrp, NT); break;
-    case 10: fms_row<10, kRange>(p, lq, zx4, e0, old, lrp, NT); break;
-    default: fms_row<19, kRange>(p, lq, zx4, e0, old, lrp, NT); break;
+// The same for a short row that keeps its messages as they are: neither flips nor
+// positions to unpack and pack, about 7 of an edge's 45 instructions, for up to two
+// more words a row.  The edge that carries new_min2 is found by |rel| == min1 (at a
+// tie both minima are equal).  Rows of up to 3 / 5 / 7 / 10 edges in this form, 8
+// iterations: 4096 blocks BG1 Zc=384 6.24 / 6.12 / 6.49 / 7.19 ms (the messages
+// outgrow L2), 777 blocks BG1 Zc=208 868 / 835 / 835 / 865 us, 4096 blocks BG2
+// Zc=64 815 / 765 / 789 / 809 us; none 6.32 ms, 876 and 836 us.
+template <int D, bool kRange>
+__device__ __forceinline__ void fms_row_direct(const DecodeParams& p, char* __restrict__ lq, uint32_t zx4, int e0, bool first,
+                                               const FloatMsg& old, float* __restrict__ lrp, int NT) {
+  if (!NRLDPC_INBOUNDS(e0 + D - 1, kMaxNnz, kBoundsEdge)) return;   // debug build
+  const uint32_t zc4 = 4u * (uint32_t)p.Zc;
+  [[maybe_unused]] const uint32_t limit = 4u * (uint32_t)p.lq_len;   // bytes of beliefs (debug build)
+  float rel[D];
+  uint32_t addr[D];
+#pragma unroll
+  for (int j = 0; j < D; ++j)
+    rel[j] = j < kFloatAhead ? __uint_as_float(old.w[j < kFloatAhead ? j : 0]) : first ? 0.0f : lrp[j * NT];
+  float m1 = FLT_MAX, m2 = FLT_MAX;
+  uint32_t sg = 0u;
+#pragma unroll
+  for (int j = 0; j < D; ++j) {
+    const uint2 e = s_fedge4[e0 + j];
+    const uint32_t t = e.y + zx4;
+    addr[j] = min(t, t - zc4) + e.x;
+    const float q = NRLDPC_INBOUNDS(addr[j], limit, kBoundsLq) ? *reinterpret_cast<const float*>(lq + addr[j]) : 0.0f;
+    const float v = __fsub_rn(q, rel[j]);
+    rel[j] = v;
+    sg ^= __float_as_uint(__fadd_rn(v, 0.0f));
+    const float a = fabsf(v);
+    m2 = fminf(m2, fmaxf(m1, a));
+    m1 = fminf(m1, a);
   }
+  float o1 = __fsub_rn(clipf(m1, p.f_max, 0.0f), p.f_beta);
+  float o2 = __fsub_rn(clipf(m2, p.f_max, 0.0f), p.f_beta);
+  o1 = o1 < 0.0f ? 0.0f : o1;
+  o2 = o2 < 0.0f ? 0.0f : o2;
+  const float s1 = __fmul_rn(p.f_alpha, o1);
+  const float s2 = __fmul_rn(p.f_alpha, o2);
+#pragma unroll
+  for (int j = 0; j < D; ++j) {
+    const uint32_t f = __float_as_uint(__fadd_rn(rel[j], 0.0f)) ^ sg;   // sign bit: the message is negated
+    const float msg = __uint_as_float(__float_as_uint(fabsf(rel[j]) == m1 ? s2 : s1) ^ (f & 0x80000000u));
+    lrp[j * NT] = msg;
+    const float v = __fadd_rn(rel[j], msg);
+    if (NRLDPC_INBOUNDS(addr[j], limit, kBoundsLq))
+      *reinterpret_cast<float*>(lq + addr[j]) = kRange ? fminf(fmaxf(v, p.f_min), p.f_max) : clipf(v, p.f_max, p.f_min);
+  }
+}
+
+template <bool kRange>
+__device__ __forceinline__ void fms_dispatch(int deg, const DecodeParams& p, char* lq, uint32_t zx4, int e0, bool first, const FloatMsg& old, uint32_t* lrp, int NT) {
+#define NRLDPC_FROW(D) \
+  if constexpr (D <= kFloatDirect) fms_row_direct<D, kRange>(p, lq, zx4, e0, first, old, reinterpret_cast<float*>(lrp), NT); \
+  else fms_row<D, kRange>(p, lq, zx4, e0, old, lrp, NT); \
+  break;
+  switch (deg) {
+    case 3: NRLDPC_FROW(3)
+    case 4: NRLDPC_FROW(4)
+    case 5: NRLDPC_FROW(5)
+    case 6: NRLDPC_FROW(6)
+    case 7: NRLDPC_FROW(7)
+    case 8: NRLDPC_FROW(8)
+    case 9: NRLDPC_FROW(9)
+    case 10: NRLDPC_FROW(10)
+    default: NRLDPC_FROW(19)
+  }
+#undef NRLDPC_FROW
 }
 
 // --------------------------------------------------------------------- BP
@@ -390,7 +449,7 @@ __global__ void __launch_bounds__(kThreadsTarget, 2) float_kernel(const __grid_c
     __syncthreads();
 
     int it = 0;
-    FloatMsg nxt{0.0f, 0.0f, 0u};   // row 0 of the first iteration: zero messages
+    FloatMsg nxt{};   // row 0 of the first iteration: zero messages
     for (; it < p.max_it; ++it) {
       for (int row = 0; row < p.R; ++row) {
         if (active) {
@@ -416,9 +475,10 @@ __global__ void __launch_bounds__(kThreadsTarget, 2) float_kernel(const __grid_c
             const bool wrap = row + 1 == p.R;
             if (wrap || it > 0) {
               const uint32_t* m = scratch + p.lr_off[wrap ? 0 : row + 1] + tid;
-              nxt = FloatMsg{__uint_as_float(m[0]), __uint_as_float(m[NT]), m[2 * NT]};
+#pragma unroll
+              for (int k = 0; k < kFloatAhead; ++k) nxt.w[k] = m[k * NT];
             }
-            fms_dispatch<kMode == kFloatRange>(deg, p, reinterpret_cast<char*>(lq), 4u * (uint32_t)zx, e0, cur, lrp, NT);
+            fms_dispatch<kMode == kFloatRange>(deg, p, reinterpret_cast<char*>(lq), 4u * (uint32_t)zx, e0, it == 0, cur, lrp, NT);
           }
         }
         __syncthreads();

@@ -70,6 +70,9 @@ inline int fixed_row_planes(int r, int d, bool direct) {
   const int n = open <= kDirectOpen ? (d <= kDirectClip ? d : open) : 0;
   return direct && n > compressed ? n : compressed;
 }
+// Scratch planes of a float min-sum row of degree d (layout in nrldpc_float.cu).
+constexpr int kFloatDirect = 5;
+inline int float_row_planes(int d) { return d <= kFloatDirect ? d : 3; }
 // Scratch words per CTA of the mixed-size kernel: the larger of the two base
 // graphs' layouts (all rows' planes x kThreadsTarget).
 uint32_t mixed_scratch_words_per_cta();
