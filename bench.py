@@ -1105,7 +1105,7 @@ def run_train(args):
         for _ in range(3):
             step(True)
         n = model.n
-        ck_bytes = T * batch * (4 * n + 16 * model.num_rows * model.Zc)
+        ck_bytes = 4 * T * batch * sum(model.row_degrees) * model.Zc   # the tape of every edge's input
         legs[name] = {"ms_per_step": round(ms, 3), "codewords_per_s": round(batch / (ms * 1e-3), 1),
                       "forward_ms": round(fwd_ms / 3, 3), "backward_ms": round(bwd_ms / 3, 3),
                       "checkpoint_bytes": int(ck_bytes), "own_kernel_launches_per_step": int(launches),
