@@ -95,14 +95,7 @@ MixedGraph make_graph(int bgn, int Zc, int iLS, int cap) {
   m.G = std::max(1, cap / Zc);
   m.K = (bgn == 1 ? 22 : 10) * Zc;
   m.N = (bgn == 1 ? 66 : 50) * Zc;
-  uint32_t off = 0;
-  for (int r = 0; r < g.rows; ++r) {
-    m.lr_off[r] = off;
-    off += (uint32_t)fixed_row_planes(r, g.degree[r], true) * kThreadsTarget;
-    m.row_off[r] = g.row_off[r];
-  }
-  m.lr_off[g.rows] = off;
-  m.row_off[g.rows] = g.row_off[g.rows];
+  for (int r = 0; r <= g.rows; ++r) m.row_off[r] = g.row_off[r];   // lr_off: mixed_row_layout
   for (int e = 0; e < g.nnz; ++e)
     m.edges[e] = make_uint2(4u * (uint32_t)g.col[e] * (uint32_t)Zc, 4u * (uint32_t)(g.vij[iLS][e] % Zc));
   return m;
@@ -362,6 +355,7 @@ int32_t nrldpc_mixed_plan_create(const nrldpc_block_t* blocks, int32_t num_block
   // open-max arithmetic only when both base graphs' layers qualify
   pl->clip = fixed_clip_mode(*dc, p.w_inline[0], base_graph(1).rows);
   if (pl->clip == kClipOpenMax) pl->clip = fixed_clip_mode(*dc, p.w_inline[1], base_graph(2).rows);
+  for (MixedGraph& m : pl->graphs) mixed_row_layout(base_graph(m.bgn), pl->clip, m.lr_off);
   // per-graph block queues: members of each graph in pairing order
   std::vector<int32_t> queue;
   std::vector<int32_t> base(pl->graphs.size()), count(pl->graphs.size());

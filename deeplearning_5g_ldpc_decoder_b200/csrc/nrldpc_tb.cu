@@ -381,14 +381,7 @@ MixedGraph tb_make_graph(int bgn, int Zc, int iLS) {
   m.G = std::max(1, kThreadsTarget / Zc);
   m.K = (bgn == 1 ? 22 : 10) * Zc;
   m.N = (bgn == 1 ? 66 : 50) * Zc;
-  uint32_t off = 0;
-  for (int r = 0; r < g.rows; ++r) {
-    m.lr_off[r] = off;
-    off += (uint32_t)fixed_row_planes(r, g.degree[r], true) * kThreadsTarget;
-    m.row_off[r] = g.row_off[r];
-  }
-  m.lr_off[g.rows] = off;
-  m.row_off[g.rows] = g.row_off[g.rows];
+  for (int r = 0; r <= g.rows; ++r) m.row_off[r] = g.row_off[r];   // lr_off: mixed_row_layout
   for (int e = 0; e < g.nnz; ++e)
     m.edges[e] = make_uint2(4u * (uint32_t)g.col[e] * (uint32_t)Zc, 4u * (uint32_t)(g.vij[iLS][e] % Zc));
   return m;
@@ -611,8 +604,6 @@ int32_t nrldpc_tb_engine_create(int32_t max_tbs, int32_t max_cbs, const ldpc_dec
   if (occ < 1) occ = 1;
   e->grid = std::max(1, std::min(2, occ) * e->num_sms);
   bool ok = cudaMalloc(&e->d_graphs, kKeys * sizeof(MixedGraph)) == cudaSuccess &&
-            cudaMemcpy(e->d_graphs, graphs.data(), kKeys * sizeof(MixedGraph), cudaMemcpyHostToDevice) ==
-                cudaSuccess &&
             device_crc_table(&e->d_crc_tab) == NRLDPC_OK;
   if (!ok) {
     engine_free(e);
@@ -646,6 +637,12 @@ int32_t nrldpc_tb_engine_create(int32_t max_tbs, int32_t max_cbs, const ldpc_dec
   // open-max arithmetic only when both base graphs' layers qualify
   e->clip = fixed_clip_mode(*dc, p.w_inline[0], base_graph(1).rows);
   if (e->clip == kClipOpenMax) e->clip = fixed_clip_mode(*dc, p.w_inline[1], base_graph(2).rows);
+  for (MixedGraph& m : graphs)
+    if (m.bgn) mixed_row_layout(base_graph(m.bgn), e->clip, m.lr_off);
+  if (cudaMemcpy(e->d_graphs, graphs.data(), kKeys * sizeof(MixedGraph), cudaMemcpyHostToDevice) != cudaSuccess) {
+    engine_free(e);
+    return NRLDPC_ERR_CUDA;
+  }
   if (engine_lanes(e, 1) != NRLDPC_OK) {
     engine_free(e);
     return NRLDPC_ERR_CUDA;
