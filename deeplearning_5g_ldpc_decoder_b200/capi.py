@@ -93,6 +93,16 @@ class ServeStats(ctypes.Structure):
                 ("mean_batch_tbs", ctypes.c_double), ("expired", ctypes.c_int64)]
 
 
+class DecodeRoute(ctypes.Structure):
+    """nrldpc_route_t: the kernel of a uniform batch."""
+
+    _fields_ = [("kernel", ctypes.c_int32), ("arithmetic", ctypes.c_int32), ("lanes", ctypes.c_int32),
+                ("groups", ctypes.c_int32)]
+
+
+ROUTE_PAIR, ROUTE_SMALL_BATCH, ROUTE_FLOAT = 0, 1, 2
+ARITH_CLAMP, ARITH_DEGENERATE, ARITH_OPEN_PARITY, ARITH_OPEN = 0, 1, 2, 3
+
 NRLDPC_TB_DROPPED = -5
 NRLDPC_TB_EXPIRED = -6
 NRLDPC_TB_HARQ_COMBINE = 1
@@ -150,6 +160,7 @@ EXPORTED_SYMBOLS = (
     "nrldpc_tb_engine_views",
     "nrldpc_serve_run",
     "nrldpc_kernel_launch_count",
+    "nrldpc_decode_route",
     "nrldpc_version",
     "nrldpc_bounds_check_status",
 )
@@ -252,6 +263,9 @@ def _declare(lib: ctypes.CDLL) -> None:
     lib.nrldpc_set_trained_weights.restype = i32
     lib.nrldpc_set_degree_alpha.argtypes = [vp]
     lib.nrldpc_set_degree_alpha.restype = i32
+    lib.nrldpc_decode_route.argtypes = [ctypes.POINTER(LdpcInConfig), ctypes.POINTER(DecoderConfig), i32, i32,
+                                        ctypes.POINTER(DecodeRoute)]
+    lib.nrldpc_decode_route.restype = i32
     lib.nrldpc_kernel_launch_count.argtypes = []
     lib.nrldpc_kernel_launch_count.restype = i64
     lib.nrldpc_version.argtypes = []
@@ -266,6 +280,17 @@ def gen_ldpc_parameters(cfg: LdpcInConfig, lib=None) -> LdpcConfig:
     if lib.gen_ldpc_parameters(ctypes.byref(out), ctypes.byref(cfg)) != 0:
         raise ValueError("invalid LDPC configuration")
     return out
+
+
+def decode_route(inconfig, decoder_config, num_cw: int, beliefs: bool = False, lib=None) -> DecodeRoute:
+    """The kernel that a batch of num_cw blocks runs on (nothing is launched)."""
+    r = DecodeRoute()
+    rc = (lib or load_library()).nrldpc_decode_route(ctypes.byref(make_in_config(*inconfig)),
+                                                     ctypes.byref(make_decoder_config(decoder_config)), num_cw,
+                                                     int(beliefs), ctypes.byref(r))
+    if rc != NRLDPC_OK:
+        raise RuntimeError(f"nrldpc_decode_route failed: {rc}")
+    return r
 
 
 def kernel_launch_count(lib=None) -> int:

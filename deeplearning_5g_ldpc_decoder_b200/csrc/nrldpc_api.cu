@@ -211,8 +211,8 @@ int cached_occupancy(DeviceState* st, uint64_t key, F ask) {
   return hit->second;
 }
 
-// Fill the launch parameters of one uniform batch.
-int make_plan(const CodeParams& cp, const ldpc_decoder_cfg_t& dc, int num_cw, DeviceState* st, Plan* plan) {
+// Fill the launch parameters of one uniform batch (`beliefs`: the call returns them).
+int make_plan(const CodeParams& cp, const ldpc_decoder_cfg_t& dc, int num_cw, bool beliefs, DeviceState* st, Plan* plan) {
   DecodeParams& p = plan->p;
   memset(&p, 0, sizeof(p));
   plan->split = false;
@@ -285,7 +285,7 @@ int make_plan(const CodeParams& cp, const ldpc_decoder_cfg_t& dc, int num_cw, De
   p.f_beta = (float)dc.beta / 128.0f;
   p.f_max = (float)dc.max_llr / 128.0f;
   p.f_min = (float)dc.min_llr / 128.0f;
-  plan->clip = fixed_clip_mode(dc, p.w_inline, g.rows);
+  plan->clip = fixed_clip_mode(dc, p.w_inline, g.rows, beliefs);
   // The small-batch kernel while all blocks run at once, with eight lanes per row
   // pair while an SM then holds few threads (its rows have a shorter chain, but
   // issue more in all), else with four; eight again where only they fit.  Measured,
@@ -391,7 +391,7 @@ int32_t decode_batch_locked(const int16_t* d_llr, int64_t llr_stride, int32_t nu
   DeviceState* st = nullptr;
   if (device_state(&st) != 0) return NRLDPC_ERR_CUDA;
   Plan plan;
-  if (make_plan(cp, *dc, num_cw, st, &plan) != 0) return NRLDPC_ERR_CUDA;
+  if (make_plan(cp, *dc, num_cw, d_app != nullptr, st, &plan) != 0) return NRLDPC_ERR_CUDA;
   uint32_t* scratch = nullptr;
   cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
   if (!plan.split && scratch_for(st, s, plan.scratch_bytes, &scratch) != 0) return NRLDPC_ERR_CUDA;
@@ -907,7 +907,7 @@ int32_t nrldpc_decode_batch_host(const int16_t* h_llr, int64_t llr_stride, int32
   // run side by side and every chunk's CTAs start on the SMs that earlier
   // chunks' finishers leave free (no tail per chunk).
   Plan probe;
-  if (make_plan(cp, *decoder_cfg, num_cw, st, &probe) != 0) return NRLDPC_ERR_CUDA;
+  if (make_plan(cp, *decoder_cfg, num_cw, false, st, &probe) != 0) return NRLDPC_ERR_CUDA;
   const bool fixed = decoder_cfg->algo >= 1 && decoder_cfg->algo <= 3;
   const int64_t wave_cw = (int64_t)(fixed ? 2 : 1) * probe.p.G * probe.grid;
   std::vector<int64_t> cuts{0};   // chunk k covers blocks [cuts[k], cuts[k+1])
@@ -1005,6 +1005,25 @@ int32_t nrldpc_set_degree_alpha(const int16_t* degree_alpha_values) {
 }
 
 int64_t nrldpc_kernel_launch_count(void) { return g_launches.load(); }
+
+int32_t nrldpc_decode_route(const ldpc_in_config_t* inconfig, const ldpc_decoder_cfg_t* decoder_cfg, int32_t num_cw,
+                            int32_t beliefs, nrldpc_route_t* route) {
+  CodeParams cp;
+  if (!inconfig || !decoder_cfg || !route || num_cw < 1) return NRLDPC_ERR_ARG;
+  if (derive_params(*inconfig, &cp, true) != 0) return NRLDPC_ERR_CONFIG;
+  if (decoder_cfg->algo > 4) return NRLDPC_ERR_ALGO;
+  std::lock_guard<std::mutex> lock(g_mu);
+  DeviceState* st = nullptr;
+  if (device_state(&st) != 0) return NRLDPC_ERR_CUDA;
+  Plan plan;
+  if (make_plan(cp, *decoder_cfg, num_cw, beliefs != 0, st, &plan) != 0) return NRLDPC_ERR_CUDA;
+  const bool fixed = plan.algo >= 1 && plan.algo <= 3;
+  route->kernel = !fixed ? NRLDPC_ROUTE_FLOAT : plan.split ? NRLDPC_ROUTE_SMALL_BATCH : NRLDPC_ROUTE_PAIR;
+  route->arithmetic = fixed ? plan.clip : 0;
+  route->lanes = plan.split ? plan.shape.lanes : 1;
+  route->groups = plan.split ? 1 : plan.p.G;
+  return NRLDPC_OK;
+}
 
 const char* nrldpc_version(void) {
   return kBoundsChecked ? "nrldpc-b200 0.1.0 (sm_100a, bounds-checked debug build)" : "nrldpc-b200 0.1.0 (sm_100a)";

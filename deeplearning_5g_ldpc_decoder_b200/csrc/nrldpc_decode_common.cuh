@@ -166,18 +166,16 @@ __device__ __forceinline__ int div_bp(int k, uint32_t magic) { return (int)__umu
 // z = the layer's packed alpha | beta << 16 (unused with per-iteration weights).
 //
 // A row is direct (row_update_direct) when its scratch has a plane per message, up
-// to the limit of its arithmetic variant.  `beliefs`: the batch returns beliefs, so
-// rows with a parity column of their own are compressed, because that column's
-// message is read back from the compressed words (parity_belief).
-__device__ __forceinline__ uint32_t row_word(uint32_t e0, uint32_t deg, uint32_t planes, int clip, bool par, bool beliefs) {
+// to the limit of its arithmetic variant.
+__device__ __forceinline__ uint32_t row_word(uint32_t e0, uint32_t deg, uint32_t planes, int clip, bool par) {
   const uint32_t n = par ? deg - 1u : deg;
-  const bool direct = n <= planes && n <= (uint32_t)(clip == kClipOpenMax ? kDirectOpen : kDirectClip) && !(par && beliefs);
+  const bool direct = n <= planes && n <= (uint32_t)(open_max(clip) ? kDirectOpen : kDirectClip);
   return e0 | deg << 16 | (direct ? n : deg > 16u ? 5u : 4u) << 24 | (direct ? 1u << 31 : 0u);
 }
 __device__ __forceinline__ uint4 row_descriptor(const DecodeParams& p, int r, int clip) {
   return make_uint4(p.lr_off[r],
                     row_word(p.row_off[r], (uint32_t)p.row_off[r + 1] - p.row_off[r], (p.lr_off[r + 1] - p.lr_off[r]) / kThreadsTarget,
-                             clip, parity_words(clip) && r >= kCoreRows, p.app != nullptr),
+                             clip, parity_words(clip) && r >= kCoreRows),
                     p.w_inline[r], 0u);
 }
 __device__ __forceinline__ int row_e0(uint32_t y) { return (int)(y & 0xFFFFu); }

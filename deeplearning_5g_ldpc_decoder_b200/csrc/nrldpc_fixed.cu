@@ -54,10 +54,8 @@ using namespace fixedrow;
 
 
 // Write the results of code block `cw` (half h of the pair in `lq`) using the
-// Zc threads of its group.  kPar: the parity columns of rows 4 and up hold rel, and
-// their beliefs need the rows' messages (`msg`: this thread's words in the scratch).
-template <bool kPar>
-__device__ void emit_block(const DecodeParams& p, const uint32_t* lq, const uint32_t* msg, int zx, int cw, int h, int status,
+// Zc threads of its group.
+__device__ void emit_block(const DecodeParams& p, const uint32_t* lq, int zx, int cw, int h, int status,
                            int iters) {
   const int shift = 16 * h;
   if (iters > 0 && p.bits) {
@@ -76,13 +74,7 @@ __device__ void emit_block(const DecodeParams& p, const uint32_t* lq, const uint
   }
   if (p.app) {
     int16_t* out = reinterpret_cast<int16_t*>(p.app) + (int64_t)cw * p.app_stride;
-    const int cols = kPar && iters > 0 ? p.lq_len - (p.R - kCoreRows) * p.Zc : p.lq_len;   // words that hold beliefs
-    for (int i = zx; i < cols; i += p.Zc) out[i] = (int16_t)(lq[i] >> shift);
-    if (kPar && iters > 0)
-      for (int r = kCoreRows; r < p.R; ++r) {
-        const int i = cols + (r - kCoreRows) * p.Zc + zx;
-        out[i] = parity_belief(lq[i], msg + p.lr_off[r], p.row_off[r + 1] - p.row_off[r], h);
-      }
+    for (int i = zx; i < p.lq_len; i += p.Zc) out[i] = (int16_t)(lq[i] >> shift);
   }
   if (zx == 0) {
     if (p.status) p.status[cw] = status;
@@ -294,7 +286,7 @@ __global__ void __launch_bounds__(kThreadsTarget, 2) fixed_pair_kernel(const __g
           const int ith = (int)(h ? itv >> 16 : itv & 0xFFFFu);
           const bool pass = run && s_crc[2 * g + h] == 0u;
           if (pass || ith >= p.max_it) {
-            emit_block<parity_words(kClip)>(p, lq, scratch + tid, zx, c, h, pass ? 0 : 1, ith);
+            emit_block(p, lq, zx, c, h, pass ? 0 : 1, ith);
             fin[h] = true;
           }
         }
@@ -391,8 +383,8 @@ __global__ void __launch_bounds__(kThreadsTarget, 2) fixed_pair_kernel(const __g
         if (active) {
           pass0 = !done0 && s_crc[2 * g] == 0u;
           pass1 = !done1 && s_crc[2 * g + 1] == 0u;
-          if (pass0) emit_block<parity_words(kClip)>(p, lq, scratch + tid, zx, cw0, 0, 0, it + 1);
-          if (pass1) emit_block<parity_words(kClip)>(p, lq, scratch + tid, zx, cw1, 1, 0, it + 1);
+          if (pass0) emit_block(p, lq, zx, cw0, 0, 0, it + 1);
+          if (pass1) emit_block(p, lq, zx, cw1, 1, 0, it + 1);
           done0 = done0 || pass0;
           done1 = done1 || pass1;
         }
@@ -405,8 +397,8 @@ __global__ void __launch_bounds__(kThreadsTarget, 2) fixed_pair_kernel(const __g
         }
       }
       if (active) {
-        if (!done0) emit_block<parity_words(kClip)>(p, lq, scratch + tid, zx, cw0, 0, 1, it);
-        if (!done1) emit_block<parity_words(kClip)>(p, lq, scratch + tid, zx, cw1, 1, 1, it);
+        if (!done0) emit_block(p, lq, zx, cw0, 0, 1, it);
+        if (!done1) emit_block(p, lq, zx, cw1, 1, 1, it);
       }
       __syncthreads();   // LQ and s_crc are reused by the next work item
     }
@@ -449,6 +441,7 @@ int launch_fixed(const DecodeParams& p, int grid, int block, int smem, int clip_
   switch (clip_mode) {
     case kClipDegen: err = launch_fixed_c<kClipDegen>(p, grid, block, smem, s); break;
     case kClipOpenMax: err = launch_fixed_c<kClipOpenMax>(p, grid, block, smem, s); break;
+    case kClipOpen: err = launch_fixed_c<kClipOpen>(p, grid, block, smem, s); break;
     default: err = launch_fixed_c<kClipClamp>(p, grid, block, smem, s); break;
   }
   if (err != (int)cudaSuccess) return err;
@@ -463,6 +456,7 @@ int occupancy_fixed(int block, int smem, int clip_mode, bool refill) {
     case kClipDegen: return refill ? occupancy_fixed_t<kClipDegen, true>(block, smem) : occupancy_fixed_t<kClipDegen, false>(block, smem);
     case kClipOpenMax:
       return refill ? occupancy_fixed_t<kClipOpenMax, true>(block, smem) : occupancy_fixed_t<kClipOpenMax, false>(block, smem);
+    case kClipOpen: return refill ? occupancy_fixed_t<kClipOpen, true>(block, smem) : occupancy_fixed_t<kClipOpen, false>(block, smem);
     default: return refill ? occupancy_fixed_t<kClipClamp, true>(block, smem) : occupancy_fixed_t<kClipClamp, false>(block, smem);
   }
 }

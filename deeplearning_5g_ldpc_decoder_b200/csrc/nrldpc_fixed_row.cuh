@@ -119,8 +119,7 @@ __device__ __forceinline__ uint32_t cond_neg16x2(uint32_t v, uint32_t m) { retur
 // message there nor writes a belief, about 20 of an edge's 54 instructions on 42
 // of BG1's 316 edges and 38 of BG2's 197.  Where |rel| + min2 could leave
 // [min_llr, max_llr], the word becomes clip(rel + message) - message, which keeps
-// the belief equal to the word plus the latest message at all times
-// (parity_belief).  8 iterations of 8192 blocks of BG1 Zc=384: 8.75 -> 8.32 ms,
+// the belief equal to the word plus the latest message at all times.  8 iterations of 8192 blocks of BG1 Zc=384: 8.75 -> 8.32 ms,
 // 65536 of BG2 Zc=64 8.15 -> 7.53 ms, 16384 of BG1 Zc=112 6.12 -> 5.74 ms (the
 // column's input taken after the row's other edges: 8.29, 8.01, 5.91 ms).
 //
@@ -205,7 +204,7 @@ __device__ __forceinline__ void row_update(const P& p, const uint2* __restrict__
     } else {
       cs = p.edge_cs4[e0 + j];
     }
-    if constexpr (kClip == kClipOpenMax) {
+    if constexpr (open_max(kClip)) {
       // the adds as multiply-adds on the FMA pipe (measured: 10.02 -> 9.30 ms
       // for 8192 BG1 Zc=384 blocks together with the open-max arithmetic; on
       // the clamp path, whose extra registers spill, it measured 1 % slower)
@@ -248,7 +247,7 @@ __device__ __forceinline__ void row_update(const P& p, const uint2* __restrict__
   const uint32_t maxp = ((uint32_t)(uint16_t)p.max_llr) * 0x10001u;
   const uint32_t minp = ((uint32_t)(uint16_t)p.min_llr) * 0x10001u;
   uint32_t s1, s2;
-  if constexpr (kClip == kClipOpenMax) {
+  if constexpr (open_max(kClip)) {
     // Both minima lie in [0, 32767] = [0, max_llr], beta = 0 and both halves
     // have the same alpha >= 0.
     s1 = scale_open(m1, alpha);
@@ -285,7 +284,7 @@ __device__ __forceinline__ void row_update(const P& p, const uint2* __restrict__
       // agree in sign.
       const uint32_t t = bsel(mi, s2, s1) ^ mf;
       uint32_t sum;
-      if constexpr (kClip == kClipOpenMax) {
+      if constexpr (open_max(kClip)) {
         // Here alpha >= 0, so the scaled minima lie in [0, 32766] and lr has
         // mf's sign, except lr = 0 when v = 0 (the sum is rel then, and no
         // overflow is flagged either way).  Testing mf instead of lr keeps
@@ -303,7 +302,7 @@ __device__ __forceinline__ void row_update(const P& p, const uint2* __restrict__
         ovf |= (sum ^ rel[j]) & ~(rel[j] ^ lr);
       }
       // with max_llr = 32767 the upper clamp of an int16 is the identity
-      nq = kClip == kClipOpenMax ? __vmaxs2(sum, minp) : __vmins2(__vmaxs2(sum, minp), maxp);
+      nq = open_max(kClip) ? __vmaxs2(sum, minp) : __vmins2(__vmaxs2(sum, minp), maxp);
     } else {
       const uint32_t lr = cond_neg16x2(bsel(mi, s2, s1), mf);
       const int32_t lo = (int32_t)(int16_t)(rel[j] & 0xFFFFu) + (int32_t)(int16_t)(lr & 0xFFFFu);
@@ -401,7 +400,7 @@ __device__ __forceinline__ void row_update_direct(const P& p, const uint2* __res
 #pragma unroll
   for (int j = 0; j < N; ++j) {
     const uint2 cs = table(j);
-    if constexpr (kClip == kClipOpenMax) {   // (see row_update)
+    if constexpr (open_max(kClip)) {   // (see row_update)
       const uint32_t a4 = add_fma(p, cs.y, zx4);
       const uint32_t t = __viaddmin_u32(a4, zxm4 - zx4, a4);
       addr[j] = kG1 ? add_fma(p, t, cs.x) : add_fma(p, t, cs.x) + gb4;
@@ -418,7 +417,7 @@ __device__ __forceinline__ void row_update_direct(const P& p, const uint2* __res
   const uint32_t maxp = ((uint32_t)(uint16_t)p.max_llr) * 0x10001u;
   const uint32_t minp = ((uint32_t)(uint16_t)p.min_llr) * 0x10001u;
   uint32_t s1, s2;
-  if constexpr (kClip == kClipOpenMax) {
+  if constexpr (open_max(kClip)) {
     s1 = scale_open(m1, alpha);
     s2 = scale_open(m2, alpha);
   } else {
@@ -435,7 +434,7 @@ __device__ __forceinline__ void row_update_direct(const P& p, const uint2* __res
     const uint32_t v = magnitude(j);
     lrp[j * S] = __vadd2(v ^ nmf, nmf & 0x00010001u);   // mf ? v : -v
     uint32_t nq;
-    if constexpr (kClip == kClipOpenMax) {
+    if constexpr (open_max(kClip)) {
       // v >= 0: rel + message with the message's sign put on the other operand
       const uint32_t w = rel[j] ^ mf, u = __vadd2(w, v);
       ovf |= u & ~w;
@@ -463,17 +462,6 @@ __device__ __forceinline__ void row_update_direct(const P& p, const uint2* __res
       store(addr[j], j < N ? q : __vsub2(q, lr));
     }
   }
-}
-
-// Belief (half h) of a parity column that belongs to row `deg` alone, from the
-// column's word and the row's message words (kPar above; edge deg - 1 of the row).
-__device__ __forceinline__ int16_t parity_belief(uint32_t word, const uint32_t* lrp, int deg, int h) {
-  constexpr int S = kThreadsTarget;
-  const int shift = 16 * h;
-  const bool second = ((lrp[3 * S] >> (shift + deg - 1)) & 1u) != 0u;
-  const int16_t v = (int16_t)((second ? lrp[S] : lrp[0]) >> shift);
-  const bool flip = ((lrp[2 * S] >> (shift + 15)) & 1u) != 0u;   // the last edge's flip is on top
-  return (int16_t)((int16_t)(word >> shift) + (flip ? -v : v));
 }
 
 // `par`: a row with a parity column of its own (row 4 and up).  `direct`: the row
@@ -510,6 +498,23 @@ __device__ __forceinline__ void layer_dispatch(int deg, bool par, bool direct, c
       case 32 + 10: NRLDPC_SHORT(10, false)
       case 96 + 8: NRLDPC_ROW(8, false)
       case 96 + 10: NRLDPC_ROW(10, false)
+      default: NRLDPC_ROW(19, false)
+    }
+  } else if constexpr (open_max(kClip)) {
+    switch (deg + (direct ? 0 : 64)) {
+      case 3: NRLDPC_SHORT(3, false)
+      case 4: NRLDPC_SHORT(4, false)
+      case 5: NRLDPC_SHORT(5, false)
+      case 6: NRLDPC_SHORT(6, false)
+      case 7: NRLDPC_SHORT(7, false)
+      case 8: NRLDPC_SHORT(8, false)
+      case 10: NRLDPC_SHORT(10, false)
+      case 64 + 5: NRLDPC_ROW(5, false)
+      case 64 + 6: NRLDPC_ROW(6, false)
+      case 64 + 7: NRLDPC_ROW(7, false)
+      case 64 + 8: NRLDPC_ROW(8, false)
+      case 64 + 9: NRLDPC_ROW(9, false)
+      case 64 + 10: NRLDPC_ROW(10, false)
       default: NRLDPC_ROW(19, false)
     }
   } else {

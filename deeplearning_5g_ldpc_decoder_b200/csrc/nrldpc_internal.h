@@ -91,28 +91,36 @@ inline uint32_t qm_magic(int qm) {
 //  * kClipClamp: clip(rel + msg) is a clamp to [min_llr, max_llr];
 //  * kClipDegen: min_llr > max_llr, where the reference's clip is not a clamp
 //    (exact int32 arithmetic);
-//  * kClipOpenMax: max_llr = 32767, min_llr <= -32767 and, in every layer, alpha >= 0
-//    and beta = 0 (algos 1 and 3): the minima need no clip, the offset step is the
+//  * kClipOpen, kClipOpenMax: max_llr = 32767 and, in every layer, alpha >= 0 and
+//    beta = 0 (algos 1 and 3): the minima need no clip, the offset step is the
 //    identity, the scaled minima lie in [0, 32766], and the clamp of the new
-//    beliefs is a max with min_llr.  This is the reference's default decoder
-//    row.
+//    beliefs is a max with min_llr.  kClipOpenMax, the reference's default decoder
+//    row, also keeps parity words (below); kClipOpen is for the calls that cannot.
 // `ab` holds each layer's packed alpha | beta << 16 as the kernels read it.
-enum { kClipClamp = 0, kClipDegen = 1, kClipOpenMax = 2 };
-// Whether the parity columns of rows 4 and up hold the row's extrinsic input
-// instead of the belief (nrldpc_fixed_row.cuh).  Only with the open maximum: the
-// check that the clip keeps the sum is then one packed add.  In the clamp
-// variant the check and its branch made converging batches slower (1001 blocks of
-// BG1 Zc=384, algo 2: 1232 -> 1310 us), although 8192 got 2 % faster.
+enum { kClipClamp = 0, kClipDegen = 1, kClipOpenMax = 2, kClipOpen = 3 };
 #ifdef __CUDACC__
-__host__ __device__
+#define NRLDPC_HD __host__ __device__
+#else
+#define NRLDPC_HD
 #endif
-constexpr bool parity_words(int clip) { return clip == kClipOpenMax; }
-inline int fixed_clip_mode(const ldpc_decoder_cfg_t& dc, const uint32_t* ab, int rows) {
+NRLDPC_HD constexpr bool open_max(int clip) { return clip == kClipOpenMax || clip == kClipOpen; }
+// Whether the parity columns of rows 4 and up hold the row's extrinsic input
+// instead of the belief (nrldpc_fixed_row.cuh).  Only with the open maximum and a
+// range of at least +-32767, where the check that the clip keeps the sum is one
+// packed add, and not when the batch returns beliefs, which would have to be put
+// together from the rows' messages: done block by block as blocks finish, that
+// took longer than the words save (1136 blocks BG1 Zc=384: 1648 us, and 1332
+// without them before rows were uncompressed).  In the clamp variant the check and
+// its branch made converging batches slower (1001 blocks of BG1 Zc=384, algo 2:
+// 1232 -> 1310 us), although 8192 got 2 % faster.
+NRLDPC_HD constexpr bool parity_words(int clip) { return clip == kClipOpenMax; }
+// `beliefs`: the call returns beliefs.
+inline int fixed_clip_mode(const ldpc_decoder_cfg_t& dc, const uint32_t* ab, int rows, bool beliefs) {
   if (dc.min_llr > dc.max_llr) return kClipDegen;
-  if ((dc.algo != 1 && dc.algo != 3) || dc.max_llr != 32767 || dc.min_llr > -32767) return kClipClamp;
+  if ((dc.algo != 1 && dc.algo != 3) || dc.max_llr != 32767) return kClipClamp;
   for (int r = 0; r < rows; ++r)
     if ((ab[r] >> 15) != 0u) return kClipClamp;   // alpha < 0 (bit 15) or beta != 0 (bits 16-31)
-  return kClipOpenMax;
+  return dc.min_llr > -32767 || beliefs ? kClipOpen : kClipOpenMax;
 }
 
 // Scratch offsets of a mixed-size graph's rows, in words.  Rows of more than four
@@ -124,7 +132,7 @@ inline void mixed_row_layout(const BaseGraph& g, int clip, uint32_t* lr_off) {
   uint32_t off = 0;
   for (int r = 0; r < g.rows; ++r) {
     lr_off[r] = off;
-    off += (uint32_t)fixed_row_planes(r, g.degree[r], clip == kClipOpenMax) * kThreadsTarget;
+    off += (uint32_t)fixed_row_planes(r, g.degree[r], open_max(clip)) * kThreadsTarget;
   }
   lr_off[g.rows] = off;
 }

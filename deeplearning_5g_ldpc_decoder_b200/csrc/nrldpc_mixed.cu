@@ -217,7 +217,7 @@ __global__ void __launch_bounds__(kThreads, kMinBlocks) fixed_mixed_kernel(const
       const uint32_t e0 = s_g.row_off[r], dg = (uint32_t)s_g.row_off[r + 1] - e0;
       s_rows[r] = make_uint4(s_g.lr_off[r],
                              row_word(e0, dg, (s_g.lr_off[r + 1] - s_g.lr_off[r]) / kThreadsTarget, kClip,
-                                      parity_words(kClip) && r >= kCoreRows, false),
+                                      parity_words(kClip) && r >= kCoreRows),
                              p.w_inline[bi][r], 0u);
     }
     if (tid < 2 * G) s_cw[tid] = take_block(p, key);
@@ -405,6 +405,7 @@ int mixed_dispatch_c(int op, int clip_mode, const MixedParams* p, int grid, cuda
   switch (clip_mode) {
     case kClipDegen: return mixed_op<kClipDegen, C>(op, p, grid, s, occ);
     case kClipOpenMax: return mixed_op<kClipOpenMax, C>(op, p, grid, s, occ);
+    case kClipOpen: return mixed_op<kClipOpen, C>(op, p, grid, s, occ);
     default: return mixed_op<kClipClamp, C>(op, p, grid, s, occ);
   }
 }

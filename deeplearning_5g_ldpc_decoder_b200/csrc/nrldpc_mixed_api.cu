@@ -353,8 +353,8 @@ int32_t nrldpc_mixed_plan_create(const nrldpc_block_t* blocks, int32_t num_block
     }
   }
   // open-max arithmetic only when both base graphs' layers qualify
-  pl->clip = fixed_clip_mode(*dc, p.w_inline[0], base_graph(1).rows);
-  if (pl->clip == kClipOpenMax) pl->clip = fixed_clip_mode(*dc, p.w_inline[1], base_graph(2).rows);
+  pl->clip = fixed_clip_mode(*dc, p.w_inline[0], base_graph(1).rows, false);
+  if (open_max(pl->clip)) pl->clip = fixed_clip_mode(*dc, p.w_inline[1], base_graph(2).rows, false);
   for (MixedGraph& m : pl->graphs) mixed_row_layout(base_graph(m.bgn), pl->clip, m.lr_off);
   // per-graph block queues: members of each graph in pairing order
   std::vector<int32_t> queue;

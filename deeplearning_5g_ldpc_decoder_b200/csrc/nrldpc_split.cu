@@ -395,6 +395,7 @@ template <bool kTable, int kLanes>
 int split_clip(const DecodeParams* p, int block, int smem, int clip_mode, cudaStream_t s, int* occ) {
   switch (clip_mode) {
     case kClipDegen: return split_op<kClipDegen, kTable, kLanes>(p, block, smem, s, occ);
+    case kClipOpen:   // this kernel keeps no parity words
     case kClipOpenMax: return split_op<kClipOpenMax, kTable, kLanes>(p, block, smem, s, occ);
     default: return split_op<kClipClamp, kTable, kLanes>(p, block, smem, s, occ);
   }

@@ -635,8 +635,8 @@ int32_t nrldpc_tb_engine_create(int32_t max_tbs, int32_t max_cbs, const ldpc_dec
     }
   }
   // open-max arithmetic only when both base graphs' layers qualify
-  e->clip = fixed_clip_mode(*dc, p.w_inline[0], base_graph(1).rows);
-  if (e->clip == kClipOpenMax) e->clip = fixed_clip_mode(*dc, p.w_inline[1], base_graph(2).rows);
+  e->clip = fixed_clip_mode(*dc, p.w_inline[0], base_graph(1).rows, false);
+  if (open_max(e->clip)) e->clip = fixed_clip_mode(*dc, p.w_inline[1], base_graph(2).rows, false);
   for (MixedGraph& m : graphs)
     if (m.bgn) mixed_row_layout(base_graph(m.bgn), e->clip, m.lr_off);
   if (cudaMemcpy(e->d_graphs, graphs.data(), kKeys * sizeof(MixedGraph), cudaMemcpyHostToDevice) != cudaSuccess) {

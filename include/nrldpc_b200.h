@@ -510,6 +510,24 @@ int32_t nrldpc_set_degree_alpha(const int16_t *degree_alpha);
 /* Number of CUDA kernels this library has launched in this process. */
 int64_t nrldpc_kernel_launch_count(void);
 
+/* Which kernel nrldpc_decode_batch takes for a batch of num_cw blocks on the
+ * current device, for tests and diagnosis (nothing is launched).  `beliefs`:
+ * the call returns beliefs. */
+enum { NRLDPC_ROUTE_PAIR = 0, NRLDPC_ROUTE_SMALL_BATCH = 1, NRLDPC_ROUTE_FLOAT = 2 };
+enum {                              /* check-node arithmetic of algos 1 to 3 */
+    NRLDPC_ARITH_CLAMP = 0,         /* any range */
+    NRLDPC_ARITH_DEGENERATE = 1,    /* min_llr > max_llr */
+    NRLDPC_ARITH_OPEN_PARITY = 2,   /* max_llr 32767, alpha >= 0, beta 0, with parity words */
+    NRLDPC_ARITH_OPEN = 3           /* the same without them */
+};
+typedef struct {
+    int32_t kernel, arithmetic;
+    int32_t lanes;                  /* small-batch kernel: lanes per row pair */
+    int32_t groups;                 /* lane pairs (code blocks, float) per CTA */
+} nrldpc_route_t;
+int32_t nrldpc_decode_route(const ldpc_in_config_t *inconfig, const ldpc_decoder_cfg_t *decoder_cfg,
+                            int32_t num_cw, int32_t beliefs, nrldpc_route_t *route);
+
 /* Library version string. */
 const char *nrldpc_version(void);
 
