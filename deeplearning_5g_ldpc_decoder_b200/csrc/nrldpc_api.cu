@@ -302,14 +302,15 @@ int make_plan(const CodeParams& cp, const ldpc_decoder_cfg_t& dc, int num_cw, bo
     const int few = cp.bgn == 1 ? 640 : 320;
     for (int k = 0; k < 3; ++k) {
       const int lanes = k == 1 ? 4 : 8;
-      split_layout(g, lanes, p.lr_off);
-      if (!split_shape(cp.Zc, g.cols, lanes, (int)(p.lr_off[g.rows] & 0xFFFFu), &plan->shape)) continue;
+      const uint32_t* layout = split_layout(cp.bgn, lanes);
+      if (!split_shape(cp.Zc, g.cols, lanes, (int)(layout[g.rows] & 0xFFFFu), &plan->shape)) continue;
       if (k == 0 && plan->shape.block * per_sm > few) continue;
       const uint64_t key = (lanes == 8 ? 7ull : 6ull) << 56 | (uint64_t)plan->clip << 48 | (uint64_t)plan->shape.table << 47 |
                            (uint64_t)plan->shape.block << 32 | (uint64_t)(uint32_t)plan->shape.smem;
       const int occ = cached_occupancy(st, key, [&] { return occupancy_split(plan->shape, plan->clip); });
       if (num_cw <= occ * st->num_sms) {
         plan->split = true;
+        memcpy(p.lr_off, layout, sizeof(uint32_t) * (size_t)(g.rows + 1));
         plan->grid = p.num_items = num_cw;
         plan->scratch_bytes = 0;
         return 0;

@@ -330,7 +330,7 @@ struct SplitShape {
   int words, slots, block, smem;   // words of beliefs, message slots, threads, dynamic shared memory
   bool table;                      // the slots' addresses are kept in shared memory
 };
-void split_layout(const BaseGraph& g, int lanes, uint32_t* lr_off);
+const uint32_t* split_layout(int bgn, int lanes);   // [rows + 1]
 bool split_shape(int Zc, int cols, int lanes, int slots, SplitShape* out);   // false: does not fit an SM
 int launch_split(const DecodeParams& p, const SplitShape& s, int clip_mode, void* stream);
 int occupancy_split(const SplitShape& s, int clip_mode);

