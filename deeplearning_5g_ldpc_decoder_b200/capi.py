@@ -97,7 +97,7 @@ class DecodeRoute(ctypes.Structure):
     """nrldpc_route_t: the kernel of a uniform batch."""
 
     _fields_ = [("kernel", ctypes.c_int32), ("arithmetic", ctypes.c_int32), ("lanes", ctypes.c_int32),
-                ("groups", ctypes.c_int32)]
+                ("groups", ctypes.c_int32), ("wide", ctypes.c_int32)]
 
 
 ROUTE_PAIR, ROUTE_SMALL_BATCH, ROUTE_FLOAT = 0, 1, 2

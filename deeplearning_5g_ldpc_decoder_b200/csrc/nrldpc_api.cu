@@ -198,6 +198,7 @@ struct Plan {
   int grid, block, smem;
   int clip;   // check-node arithmetic variant of the fixed-point kernel (fixed_clip_mode)
   int algo;
+  bool wide;         // fixed_pair_kernel: rows of more than four messages uncompressed too (direct_row)
   bool split;        // the small-batch kernel: one code block per CTA, no scratch
   SplitShape shape;
   size_t scratch_bytes;
@@ -286,6 +287,15 @@ int make_plan(const CodeParams& cp, const ldpc_decoder_cfg_t& dc, int num_cw, bo
   p.f_max = (float)dc.max_llr / 128.0f;
   p.f_min = (float)dc.min_llr / 128.0f;
   plan->clip = fixed_clip_mode(dc, p.w_inline, g.rows, beliefs);
+  // Rows of more than four messages uncompressed (the wide kernels), but not in a CTA
+  // of several groups and fewer than five warps: it loads only four words of a row
+  // ahead, and so few warps do not hide the load of the others.  Measured, 8
+  // iterations, us compressed / wide, default row: BG1 Zc 4, 2000 blocks (28 threads)
+  // 244 / 264; Zc 24, 1136 (96) 211 / 220; Zc 40, 444 (80) 223 / 228, 1136 (160) 260 /
+  // 254; Zc 72, 1136 (288) 334 / 314; BG2 Zc 20, 2000 (140) 203 / 209; Zc 64, 592 (128)
+  // 144 / 151, 1136 (256) 181 / 181; one group per CTA, which loads five words ahead:
+  // Zc 72, 200 blocks 237 / 210, Zc 384, 100 blocks 353 / 321.
+  plan->wide = p.G == 1 || p.nact >= 160;
   // The small-batch kernel while all blocks run at once, with eight lanes per row
   // pair while an SM then holds few threads (its rows have a shorter chain, but
   // issue more in all), else with four; eight again where only they fit.  Measured,
@@ -318,24 +328,19 @@ int make_plan(const CodeParams& cp, const ldpc_decoder_cfg_t& dc, int num_cw, bo
     }
   }
 
-  // Scratch layout per CTA, layer by layer.
-  uint32_t off = 0;
-  for (int r = 0; r < g.rows; ++r) {
-    p.lr_off[r] = off;
-    const int deg = g.degree[r];
-    int planes;
-    if (algo == 0) {
-      planes = deg;
-    } else if (fixed) {
-      planes = fixed_row_planes(r, deg, true);
-    } else {
-      planes = float_row_planes(deg);
+  // Scratch layout per CTA, layer by layer.  (The fixed-point kernel addresses its
+  // planes with a compile-time stride.)
+  if (fixed) {
+    fixed_row_layout(g, plan->clip, plan->wide, p.lr_off);
+  } else {
+    uint32_t off = 0;
+    for (int r = 0; r < g.rows; ++r) {
+      p.lr_off[r] = off;
+      off += (uint32_t)(algo == 0 ? g.degree[r] : float_row_planes(g.degree[r])) * (uint32_t)p.nact;
     }
-    // The fixed-point kernel addresses its planes with a compile-time stride.
-    off += (uint32_t)planes * (uint32_t)(fixed ? kThreadsTarget : p.nact);
+    p.lr_off[g.rows] = off;
   }
-  p.lr_off[g.rows] = off;
-  p.scratch_words = off;
+  p.scratch_words = p.lr_off[g.rows];
 
   const uint64_t key = ((uint64_t)(fixed ? 1 : algo == 4 ? 2 : 3) << 56) | ((uint64_t)(fixed ? plan->clip : 0) << 48) |
                        ((uint64_t)plan->block << 32) | (uint64_t)(uint32_t)plan->smem;
@@ -356,7 +361,7 @@ int launch_plan(Plan* plan, void* stream) {
     case 1:
     case 2:
     case 3:
-      return launch_fixed(plan->p, plan->grid, plan->block, plan->smem, plan->clip, stream);
+      return launch_fixed(plan->p, plan->grid, plan->block, plan->smem, plan->clip, plan->wide, stream);
     case 4:
       return launch_float_minsum(plan->p, plan->grid, plan->block, plan->smem, stream);
     default:
@@ -1023,6 +1028,7 @@ int32_t nrldpc_decode_route(const ldpc_in_config_t* inconfig, const ldpc_decoder
   route->arithmetic = fixed ? plan.clip : 0;
   route->lanes = plan.split ? plan.shape.lanes : 1;
   route->groups = plan.split ? 1 : plan.p.G;
+  route->wide = fixed && !plan.split && plan.wide ? 1 : 0;
   return NRLDPC_OK;
 }
 

@@ -162,25 +162,22 @@ __device__ __forceinline__ int div_bp(int k, uint32_t magic) { return (int)__umu
 // Per-layer descriptor staged in shared memory at kernel start, one 16-byte
 // load per layer instead of several dynamically indexed parameter reads:
 // x = the layer's word offset in the CTA's message scratch,
-// y = row_word: first edge | degree << 16 | message words << 24 | direct << 31,
+// y = row_word: first edge | case << 16 | message words << 24,
 // z = the layer's packed alpha | beta << 16 (unused with per-iteration weights).
-//
-// A row is direct (row_update_direct) when its scratch has a plane per message, up
-// to the limit of its arithmetic variant.
-__device__ __forceinline__ uint32_t row_word(uint32_t e0, uint32_t deg, uint32_t planes, int clip, bool par) {
-  const uint32_t n = par ? deg - 1u : deg;
-  const bool direct = n <= planes && n <= (uint32_t)(open_max(clip) ? kDirectOpen : kDirectClip);
-  return e0 | deg << 16 | (direct ? n : deg > 16u ? 5u : 4u) << 24 | (direct ? 1u << 31 : 0u);
+// The case numbers of layer_dispatch are dense, for a jump table: the degree, but
+// with parity words BG2's core rows of 8 and 10 edges are cases 11 and 12.
+constexpr int kCaseCore8 = 11, kCaseCore10 = 12, kCase19 = 13;
+__device__ __forceinline__ uint32_t row_word(uint32_t e0, uint32_t deg, bool core, int clip, bool wide) {
+  const uint32_t kase = deg > 10u ? kCase19 : parity_words(clip) && core ? (deg == 8u ? kCaseCore8 : kCaseCore10) : deg;
+  const uint32_t words = direct_row((int)deg, core, clip, wide) ? (uint32_t)row_messages((int)deg, core, clip) : deg > 16u ? 5u : 4u;
+  return e0 | kase << 16 | words << 24;
 }
-__device__ __forceinline__ uint4 row_descriptor(const DecodeParams& p, int r, int clip) {
-  return make_uint4(p.lr_off[r],
-                    row_word(p.row_off[r], (uint32_t)p.row_off[r + 1] - p.row_off[r], (p.lr_off[r + 1] - p.lr_off[r]) / kThreadsTarget,
-                             clip, parity_words(clip) && r >= kCoreRows),
+__device__ __forceinline__ uint4 row_descriptor(const DecodeParams& p, int r, int clip, bool wide) {
+  return make_uint4(p.lr_off[r], row_word(p.row_off[r], (uint32_t)p.row_off[r + 1] - p.row_off[r], r < kCoreRows, clip, wide),
                     p.w_inline[r], 0u);
 }
 __device__ __forceinline__ int row_e0(uint32_t y) { return (int)(y & 0xFFFFu); }
-__device__ __forceinline__ int row_deg(uint32_t y) { return (int)((y >> 16) & 0xFFu); }
-__device__ __forceinline__ int row_words(uint32_t y) { return (int)(y >> 24 & 0x7Fu); }
-__device__ __forceinline__ bool row_direct(uint32_t y) { return (y >> 31) != 0u; }
+__device__ __forceinline__ int row_case(uint32_t y) { return (int)((y >> 16) & 0xFFu); }
+__device__ __forceinline__ int row_words(uint32_t y) { return (int)(y >> 24); }
 
 }  // namespace nrldpc

@@ -202,15 +202,15 @@ __device__ __forceinline__ void take_blocks(const DecodeParams& p, bool q0, bool
 // kG1: one lane pair per CTA (G = 1: Zc >= 193, or a batch small enough to
 // give every pair its own CTA), so the group index and its
 // shared-memory base are compile-time zeros and free registers in the layer loop.
-template <int kClip, bool kRefill, bool kG1>
+template <int kClip, bool kWide, bool kRefill, bool kG1>
 __global__ void __launch_bounds__(kThreadsTarget, 2) fixed_pair_kernel(const __grid_constant__ DecodeParams p) {
   constexpr int kAhead = ahead_words(kG1);
   extern __shared__ __align__(16) uint32_t s_lq[];        // [G][lq_len] int16x2
   __shared__ uint32_t s_crc[2 * kMaxGroups];
   __shared__ uint2 s_edges[kMaxNnz];   // per-edge (col*Zc*4, (V mod Zc)*4), read with warp-uniform indices
-  __shared__ uint4 s_rows[kMaxRows];   // per-layer descriptors (row_descriptor)
+  __shared__ uint4 s_rows[kMaxRows + 1];   // per-layer descriptors (row_descriptor), the first again after the last
   for (int e = threadIdx.x; e < kMaxNnz; e += blockDim.x) s_edges[e] = p.edge_cs4[e];
-  for (int r = threadIdx.x; r < p.R; r += blockDim.x) s_rows[r] = row_descriptor(p, r, kClip);
+  for (int r = threadIdx.x; r <= p.R; r += blockDim.x) s_rows[r] = row_descriptor(p, r < p.R ? r : 0, kClip, kWide);
 
   const int tid = threadIdx.x;
   const int g = kG1 ? 0 : tid / p.Zc;
@@ -248,7 +248,16 @@ __global__ void __launch_bounds__(kThreadsTarget, 2) fixed_pair_kernel(const __g
       if (tid < 2 * kMaxGroups) s_crc[tid] = 0u;
       idle = __syncthreads_and(!active || (c0 < 0 && c1 < 0));
     }
-    uint32_t itv = 0u;   // iterations of half 0 in bits 0-15, half 1 in bits 16-31
+    // Iterations of half 0 in bits 0-15, half 1 in bits 16-31.  The rows need them for
+    // per-iteration tables only; with the open maximum they wait in shared memory,
+    // because the register is one that the row loop would spill (8192 blocks BG1
+    // Zc=384: 7.46 -> 7.07 ms; algo 2 with 1001 blocks 1.15 -> 1.21 ms, not used there).
+    constexpr bool kStoreIt = open_max(kClip);
+    __shared__ uint32_t s_it[kStoreIt ? kMaxGroups : 1];
+    uint32_t itv = 0u;
+    if constexpr (kStoreIt) {
+      if (active && zx == 0) s_it[g] = 0u;
+    }
     uint32_t fresh = 0xFFFFFFFFu;   // both halves start their first iteration
     const bool run = p.max_it > 0;   // max_iterations == 0: rate recovery only, status 1
     RowMsg<kAhead> nxt{};
@@ -257,17 +266,16 @@ __global__ void __launch_bounds__(kThreadsTarget, 2) fixed_pair_kernel(const __g
         if (active) {
           const RowMsg<kAhead> cur = nxt;
           const uint4 d = s_rows[row];
-          const int rn = row + 1 < p.R ? row + 1 : 0;
-          const uint2 dn = *reinterpret_cast<const uint2*>(&s_rows[rn]);
+          const uint2 dn = *reinterpret_cast<const uint2*>(&s_rows[row + 1]);
           nxt = load_row_msg<kAhead>(scratch + dn.x + tid, row_words(dn.y));
           uint32_t ab0, ab1;
-          if (p.weights_T > 0) {
+          if (!kStoreIt && p.weights_T > 0) {
             ab0 = __ldg(p.weights + (min((int)(itv & 0xFFFFu), p.weights_T - 1) * p.R + row));
             ab1 = __ldg(p.weights + (min((int)(itv >> 16), p.weights_T - 1) * p.R + row));
           } else {
             ab0 = ab1 = d.z;
           }
-          layer_dispatch<kClip, true, kG1>(row_deg(d.y), row >= kCoreRows, row_direct(d.y), p, s_edges, reinterpret_cast<char*>(s_lq), zx4, zxm4, gb4,
+          layer_dispatch<kClip, kWide, true, kG1>(row_case(d.y), p, s_edges, reinterpret_cast<char*>(s_lq), zx4, zxm4, gb4,
                                            lq_limit, row_e0(d.y), (int32_t)(int16_t)(ab0 & 0xFFFFu), ((int32_t)ab0) >> 16,
                                            (int32_t)(int16_t)(ab1 & 0xFFFFu), ((int32_t)ab1) >> 16, cur, fresh,
                                            scratch + d.x + tid);
@@ -278,6 +286,7 @@ __global__ void __launch_bounds__(kThreadsTarget, 2) fixed_pair_kernel(const __g
       if (run) crc_pass(p, s_lq, s_crc);
       __syncthreads();
       bool fin[2] = {false, false};
+      if constexpr (kStoreIt) itv = active ? s_it[g] : 0u;
       if (active) {
         for (int h = 0; h < 2; ++h) {
           const int c = s_cw[2 * g + h];
@@ -294,7 +303,12 @@ __global__ void __launch_bounds__(kThreadsTarget, 2) fixed_pair_kernel(const __g
       // s_crc read and the finished blocks emitted before anything is reused
       const bool any = __syncthreads_or(fin[0] || fin[1]);
       if (tid < 2 * kMaxGroups) s_crc[tid] = 0u;
-      if (!any) continue;
+      if (!any) {
+        if constexpr (kStoreIt) {   // read again after the rows' barriers
+          if (active && zx == 0) s_it[g] = itv;
+        }
+        continue;
+      }
       int nc0 = -1, nc1 = -1;
       take_blocks(p, fin[0] && zx == 0, fin[1] && zx == 0, &nc0, &nc1);
       if (zx == 0) {
@@ -310,6 +324,9 @@ __global__ void __launch_bounds__(kThreadsTarget, 2) fixed_pair_kernel(const __g
           if ((h ? c1 : c0) >= 0) fresh |= h ? 0xFFFF0000u : 0x0000FFFFu;
         }
         if (!p.rr_scatter) recover_halves(p, lq, zx, c0, c1, fin[0], fin[1]);
+      }
+      if constexpr (kStoreIt) {
+        if (active && zx == 0) s_it[g] = itv;
       }
       // `any` is uniform here, so every thread of the CTA reaches the barriers inside
       if (p.rr_scatter) recover_scatter(p, lq, zx, active, c0, c1, fin[0], fin[1]);
@@ -363,13 +380,12 @@ __global__ void __launch_bounds__(kThreadsTarget, 2) fixed_pair_kernel(const __g
           if (active) {
             const RowMsg<kAhead> cur = nxt;
             const uint4 d = s_rows[row];
-            const int rn = row + 1 < p.R ? row + 1 : 0;
-            const uint2 dn = *reinterpret_cast<const uint2*>(&s_rows[rn]);
+            const uint2 dn = *reinterpret_cast<const uint2*>(&s_rows[row + 1]);
             nxt = load_row_msg<kAhead>(scratch + dn.x + tid, row_words(dn.y));
             const uint32_t ab = p.weights_T > 0 ? __ldg(p.weights + (min(it, p.weights_T - 1) * p.R + row)) : d.z;
             const int32_t alpha = (int32_t)(int16_t)(ab & 0xFFFFu);
             const int32_t beta = ((int32_t)ab) >> 16;
-            layer_dispatch<kClip, true, kG1>(row_deg(d.y), row >= kCoreRows, row_direct(d.y), p, s_edges, reinterpret_cast<char*>(s_lq), zx4, zxm4, gb4,
+            layer_dispatch<kClip, kWide, true, kG1>(row_case(d.y), p, s_edges, reinterpret_cast<char*>(s_lq), zx4, zxm4, gb4,
                                              lq_limit, row_e0(d.y), alpha, beta, alpha, beta, cur,
                                              it == 0 ? 0xFFFFFFFFu : 0u, scratch + d.x + tid);
           }
@@ -405,45 +421,53 @@ __global__ void __launch_bounds__(kThreadsTarget, 2) fixed_pair_kernel(const __g
   }
 }
 
-template <int kClip, bool kRefill, bool kG1>
+template <int kClip, bool kWide, bool kRefill, bool kG1>
 int launch_fixed_t(const DecodeParams& p, int grid, int block, int smem, cudaStream_t s) {
   static std::atomic<uint32_t> attr_done{0};
-  const int err = raise_smem_limit_once(fixed_pair_kernel<kClip, kRefill, kG1>, &attr_done);
+  const int err = raise_smem_limit_once(fixed_pair_kernel<kClip, kWide, kRefill, kG1>, &attr_done);
   if (err != 0) return err;
-  fixed_pair_kernel<kClip, kRefill, kG1><<<grid, block, smem, s>>>(p);
+  fixed_pair_kernel<kClip, kWide, kRefill, kG1><<<grid, block, smem, s>>>(p);
   return (int)cudaSuccess;
 }
 
-template <int kClip>
+template <int kClip, bool kWide>
 int launch_fixed_c(const DecodeParams& p, int grid, int block, int smem, cudaStream_t s) {
   const bool refill = p.cursor != nullptr;
   if (p.G == 1)   // one-pair specialisation
-    return refill ? launch_fixed_t<kClip, true, true>(p, grid, block, smem, s)
-                  : launch_fixed_t<kClip, false, true>(p, grid, block, smem, s);
-  return refill ? launch_fixed_t<kClip, true, false>(p, grid, block, smem, s)
-                : launch_fixed_t<kClip, false, false>(p, grid, block, smem, s);
+    return refill ? launch_fixed_t<kClip, kWide, true, true>(p, grid, block, smem, s)
+                  : launch_fixed_t<kClip, kWide, false, true>(p, grid, block, smem, s);
+  return refill ? launch_fixed_t<kClip, kWide, true, false>(p, grid, block, smem, s)
+                : launch_fixed_t<kClip, kWide, false, false>(p, grid, block, smem, s);
 }
 
+// The same for every row form (all kernels are bound to two CTAs of 384 threads per SM).
 template <int kClip, bool kRefill>
 int occupancy_fixed_t(int block, int smem) {
   int n = 0;
   static std::atomic<uint32_t> attr_done{0};
-  if (raise_smem_limit_once(fixed_pair_kernel<kClip, kRefill, false>, &attr_done) != 0) return 0;
-  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, fixed_pair_kernel<kClip, kRefill, false>, block, smem);
+  if (raise_smem_limit_once(fixed_pair_kernel<kClip, true, kRefill, false>, &attr_done) != 0) return 0;
+  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, fixed_pair_kernel<kClip, true, kRefill, false>, block, smem);
   return n;
+}
+
+// Calls op(constant) with the arithmetic variant as a compile-time constant.
+template <typename Op>
+int with_clip(int clip_mode, Op op) {
+  switch (clip_mode) {
+    case kClipDegen: return op(std::integral_constant<int, kClipDegen>{});
+    case kClipOpenMax: return op(std::integral_constant<int, kClipOpenMax>{});
+    case kClipOpen: return op(std::integral_constant<int, kClipOpen>{});
+    default: return op(std::integral_constant<int, kClipClamp>{});
+  }
 }
 
 }  // namespace
 
-int launch_fixed(const DecodeParams& p, int grid, int block, int smem, int clip_mode, void* stream) {
+int launch_fixed(const DecodeParams& p, int grid, int block, int smem, int clip_mode, bool wide, void* stream) {
   cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
-  int err;
-  switch (clip_mode) {
-    case kClipDegen: err = launch_fixed_c<kClipDegen>(p, grid, block, smem, s); break;
-    case kClipOpenMax: err = launch_fixed_c<kClipOpenMax>(p, grid, block, smem, s); break;
-    case kClipOpen: err = launch_fixed_c<kClipOpen>(p, grid, block, smem, s); break;
-    default: err = launch_fixed_c<kClipClamp>(p, grid, block, smem, s); break;
-  }
+  const int err = with_clip(clip_mode, [&](auto c) {
+    return wide ? launch_fixed_c<c.value, true>(p, grid, block, smem, s) : launch_fixed_c<c.value, false>(p, grid, block, smem, s);
+  });
   if (err != (int)cudaSuccess) return err;
   count_launch();
   return (int)cudaGetLastError();
@@ -452,13 +476,9 @@ int launch_fixed(const DecodeParams& p, int grid, int block, int smem, int clip_
 int bounds_read_fixed(uint32_t* out, bool reset) { return bounds_read_tu(out, reset); }
 
 int occupancy_fixed(int block, int smem, int clip_mode, bool refill) {
-  switch (clip_mode) {
-    case kClipDegen: return refill ? occupancy_fixed_t<kClipDegen, true>(block, smem) : occupancy_fixed_t<kClipDegen, false>(block, smem);
-    case kClipOpenMax:
-      return refill ? occupancy_fixed_t<kClipOpenMax, true>(block, smem) : occupancy_fixed_t<kClipOpenMax, false>(block, smem);
-    case kClipOpen: return refill ? occupancy_fixed_t<kClipOpen, true>(block, smem) : occupancy_fixed_t<kClipOpen, false>(block, smem);
-    default: return refill ? occupancy_fixed_t<kClipClamp, true>(block, smem) : occupancy_fixed_t<kClipClamp, false>(block, smem);
-  }
+  return with_clip(clip_mode, [&](auto c) {
+    return refill ? occupancy_fixed_t<c.value, true>(block, smem) : occupancy_fixed_t<c.value, false>(block, smem);
+  });
 }
 
 }  // namespace nrldpc

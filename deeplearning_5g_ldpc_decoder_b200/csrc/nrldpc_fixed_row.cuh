@@ -130,9 +130,9 @@ __device__ __forceinline__ uint32_t cond_neg16x2(uint32_t v, uint32_t m) { retur
 // row_update_direct), loaded by the kernels one row ahead so that their L2 latency
 // overlaps the row before; the row loads the rest itself.  Four words always (a
 // row has at least four planes), and with one lane pair per CTA a fifth where the
-// row has it.  With groups there is no register for it: 65536 blocks of BG2 Zc=64
-// take 6.49 ms with four words and 7.40 ms with five; with one pair, 8192 of BG1
-// Zc=384, it is 8.03 and 7.38 ms (six: 7.78 ms).
+// row has it: 8192 blocks of BG1 Zc=384 take 7.66 ms with four words, 6.96 ms with
+// five and 6.98 ms with six.  With groups a fifth gives nothing: 65536 of BG2 Zc=64
+// 6.18 and 6.07 ms with the open maximum, 7.26 and 7.38 ms without it.
 template <int kAhead>
 struct RowMsg {
   uint32_t w[kAhead];
@@ -355,13 +355,13 @@ __device__ __forceinline__ void row_update(const P& p, const uint2* __restrict__
 // min1 afterwards (at a tie both minima are equal, so marking several edges
 // changes no message).  It costs message traffic: N words a row instead of four,
 // which the rows here have to gain by.  Rows of up to four messages cost nothing
-// more; the limits (kDirectOpen, kDirectClip) are where the batch of 8192 blocks
+// more; the limits for longer ones (direct_row) are where the batch of 8192 blocks
 // BG1 Zc=384, whose messages then take 99 of L2's 126 MB, stops gaining: with
 // limits 4, 7, 8, 9 and the open maximum 7.75, 7.48, 7.37, 7.31 ms.  19-edge rows
-// would take L2's rest.  8 iterations, compressed -> direct, open maximum / clamp:
-// 8192 of BG1 Zc=384 8.13 -> 7.31 / 9.47 -> 8.9 ms, 65536 of BG2 Zc=64 7.31 ->
-// 6.38 / 8.67 -> 7.66 ms, 16384 of BG1 Zc=112 5.62 -> 5.27 / 6.41 -> 6.17 ms,
-// 8192 of BG2 Zc=384 5.43 -> 4.61 / 6.43 -> 5.65 ms.
+// would take L2's rest.  8 iterations, rows of more than four messages compressed ->
+// direct, open maximum / clamp: 8192 of BG1 Zc=384 7.33 -> 6.96 / 9.20 -> 8.66 ms,
+// 65536 of BG2 Zc=64 6.23 -> 6.18 / 7.69 -> 7.26 ms, 16384 of BG1 Zc=112 5.24 ->
+// 5.17 / 6.21 -> 5.82 ms, 8192 of BG2 Zc=384 4.56 -> 4.24 / 5.78 -> 5.41 ms.
 template <int D, bool kPar, int kClip, bool kSmemEdges, bool kG1, typename P>
 __device__ __forceinline__ void row_update_direct(const P& p, const uint2* __restrict__ sedges, char* __restrict__ lqs,
                                                   uint32_t zx4, uint32_t zxm4, uint32_t gb4, uint32_t lq_limit, int e0,
@@ -464,78 +464,37 @@ __device__ __forceinline__ void row_update_direct(const P& p, const uint2* __res
   }
 }
 
-// `par`: a row with a parity column of its own (row 4 and up).  `direct`: the row
-// keeps its messages uncompressed (row_word in nrldpc_decode_common.cuh decides).
-template <int kClip, bool kSmemEdges, bool kG1, typename P>
-__device__ __forceinline__ void layer_dispatch(int deg, bool par, bool direct, const P& p, const uint2* sedges, char* lqs, uint32_t zx4, uint32_t zxm4,
+// One row in the form that the kernel has for it (direct_row); kase: row_word.
+template <int kClip, bool kWide, bool kSmemEdges, bool kG1, typename P>
+__device__ __forceinline__ void layer_dispatch(int kase, const P& p, const uint2* sedges, char* lqs, uint32_t zx4, uint32_t zxm4,
                                                uint32_t gb4, uint32_t lq_limit, int e0, int32_t alpha, int32_t beta,
                                                int32_t alpha1, int32_t beta1, const RowMsg<ahead_words(kG1)>& old, uint32_t fresh,
                                                uint32_t* lrp) {
-#define NRLDPC_ROW(D, PAR) \
-  row_update<D, PAR, kClip, kSmemEdges, kG1>(p, sedges, lqs, zx4, zxm4, gb4, lq_limit, e0, alpha, beta, alpha1, beta1, old, fresh, lrp); break;
-#define NRLDPC_SHORT(D, PAR) \
-  row_update_direct<D, PAR, kClip, kSmemEdges, kG1>(p, sedges, lqs, zx4, zxm4, gb4, lq_limit, e0, alpha, beta, alpha1, beta1, old, fresh, lrp); break;
-  if constexpr (parity_words(kClip)) {
-    switch (deg + (par ? 0 : 32) + (direct ? 0 : 64)) {
-      case 3: NRLDPC_SHORT(3, true)
-      case 4: NRLDPC_SHORT(4, true)
-      case 5: NRLDPC_SHORT(5, true)
-      case 6: NRLDPC_SHORT(6, true)
-      case 7: NRLDPC_SHORT(7, true)
-      case 8: NRLDPC_SHORT(8, true)
-      case 9: NRLDPC_SHORT(9, true)
-      case 10: NRLDPC_SHORT(10, true)
-      case 64 + 3: NRLDPC_ROW(3, true)
-      case 64 + 4: NRLDPC_ROW(4, true)
-      case 64 + 5: NRLDPC_ROW(5, true)
-      case 64 + 6: NRLDPC_ROW(6, true)
-      case 64 + 7: NRLDPC_ROW(7, true)
-      case 64 + 8: NRLDPC_ROW(8, true)
-      case 64 + 9: NRLDPC_ROW(9, true)
-      case 64 + 10: NRLDPC_ROW(10, true)
-      // core rows: BG2 has 8 and 10 edges, BG1 19
-      case 32 + 8: NRLDPC_SHORT(8, false)
-      case 32 + 10: NRLDPC_SHORT(10, false)
-      case 96 + 8: NRLDPC_ROW(8, false)
-      case 96 + 10: NRLDPC_ROW(10, false)
-      default: NRLDPC_ROW(19, false)
-    }
-  } else if constexpr (open_max(kClip)) {
-    switch (deg + (direct ? 0 : 64)) {
-      case 3: NRLDPC_SHORT(3, false)
-      case 4: NRLDPC_SHORT(4, false)
-      case 5: NRLDPC_SHORT(5, false)
-      case 6: NRLDPC_SHORT(6, false)
-      case 7: NRLDPC_SHORT(7, false)
-      case 8: NRLDPC_SHORT(8, false)
-      case 10: NRLDPC_SHORT(10, false)
-      case 64 + 5: NRLDPC_ROW(5, false)
-      case 64 + 6: NRLDPC_ROW(6, false)
-      case 64 + 7: NRLDPC_ROW(7, false)
-      case 64 + 8: NRLDPC_ROW(8, false)
-      case 64 + 9: NRLDPC_ROW(9, false)
-      case 64 + 10: NRLDPC_ROW(10, false)
-      default: NRLDPC_ROW(19, false)
-    }
-  } else {
-    switch (deg + (direct ? 0 : 64)) {
-      case 7: NRLDPC_SHORT(7, false)
-      case 8: NRLDPC_SHORT(8, false)
-      case 3: NRLDPC_SHORT(3, false)
-      case 4: NRLDPC_SHORT(4, false)
-      case 5: NRLDPC_SHORT(5, false)
-      case 6: NRLDPC_SHORT(6, false)
-      case 64 + 5: NRLDPC_ROW(5, false)
-      case 64 + 6: NRLDPC_ROW(6, false)
-      case 64 + 7: NRLDPC_ROW(7, false)
-      case 64 + 8: NRLDPC_ROW(8, false)
-      case 64 + 9: NRLDPC_ROW(9, false)
-      case 64 + 10: NRLDPC_ROW(10, false)
-      default: NRLDPC_ROW(19, false)
-    }
+  // (without parity words core rows are like the others, and cases 11 and 12 unused)
+#define NRLDPC_ROW(D, CORE)                                                                                                  \
+  if constexpr (direct_row(D, CORE, kClip, kWide))                                                                           \
+    row_update_direct<D, parity_words(kClip) && !(CORE), kClip, kSmemEdges, kG1>(p, sedges, lqs, zx4, zxm4, gb4, lq_limit, e0, alpha, \
+                                                                                 beta, alpha1, beta1, old, fresh, lrp);      \
+  else                                                                                                                       \
+    row_update<D, parity_words(kClip) && !(CORE), kClip, kSmemEdges, kG1>(p, sedges, lqs, zx4, zxm4, gb4, lq_limit, e0, alpha, beta, \
+                                                                          alpha1, beta1, old, fresh, lrp);                   \
+  break;
+  switch (kase) {
+    case 3: NRLDPC_ROW(3, false)
+    case 4: NRLDPC_ROW(4, false)
+    case 5: NRLDPC_ROW(5, false)
+    case 6: NRLDPC_ROW(6, false)
+    case 7: NRLDPC_ROW(7, false)
+    case 8: NRLDPC_ROW(8, false)
+    case 9: NRLDPC_ROW(9, false)
+    case 10: NRLDPC_ROW(10, false)
+    case kCaseCore8:
+      if constexpr (parity_words(kClip)) { NRLDPC_ROW(8, true) }
+    case kCaseCore10:
+      if constexpr (parity_words(kClip)) { NRLDPC_ROW(10, true) }
+    default: NRLDPC_ROW(19, true)
   }
 #undef NRLDPC_ROW
-#undef NRLDPC_SHORT
 }
 
 }  // namespace fixedrow

@@ -56,26 +56,12 @@ uint32_t crc_remainder(const uint8_t* data, int len, int crctype);
 // message whose only set bit sits d positions before its end.
 void crc_position_table(int crctype, uint32_t* out /* kMaxB */);
 
-// Scratch planes (kThreadsTarget words each) of lifted check row r, degree d, in the
-// fixed-point kernels (layout in nrldpc_fixed_row.cuh).  At least the compressed
-// message: the two minima, the flip bits and the min2 bits, plus a fifth word for
-// degree-19 rows.  `direct`: also room for one word per message in the rows that
-// may keep their messages as they are, 258 planes in all for BG1 instead of 188
-// and 203 for BG2 instead of 168.  (The no-allocation entry point's static scratch
-// bounds its CTAs in flight, so it stays with the smaller layout.)
-constexpr int kDirectOpen = 10, kDirectClip = 8;   // messages of such a row at most, with the open maximum and without
-inline int fixed_row_planes(int r, int d, bool direct) {
-  const int compressed = d > 16 ? 5 : 4;
-  const int open = r < kCoreRows ? d : d - 1;   // messages with the open maximum, and without it d
-  const int n = open <= kDirectOpen ? (d <= kDirectClip ? d : open) : 0;
-  return direct && n > compressed ? n : compressed;
-}
 // Scratch planes of a float min-sum row of degree d (layout in nrldpc_float.cu).
 constexpr int kFloatDirect = 5;
 inline int float_row_planes(int d) { return d <= kFloatDirect ? d : 3; }
 // Scratch words per CTA of the mixed-size kernel: the larger of the two base
 // graphs' layouts (all rows' planes x kThreadsTarget).
-uint32_t mixed_scratch_words_per_cta();
+uint32_t mixed_scratch_words_per_cta(int clip);
 
 // ceil(2^32 / Qm), the constant that turns e / Qm into one high multiply in the
 // kernels' scatter-form rate recovery (div_qm); 0 for Qm = 1, whose quotient is
@@ -114,6 +100,26 @@ NRLDPC_HD constexpr bool open_max(int clip) { return clip == kClipOpenMax || cli
 // its branch made converging batches slower (1001 blocks of BG1 Zc=384, algo 2:
 // 1232 -> 1310 us), although 8192 got 2 % faster.
 NRLDPC_HD constexpr bool parity_words(int clip) { return clip == kClipOpenMax; }
+
+// Messages that check row r of degree d keeps for the next iteration, and whether it
+// keeps them as they are (direct, row_update_direct) or compressed (row_update).
+// Every kernel keeps rows of up to four messages direct, which takes no more words;
+// `wide` kernels longer rows too, up to the limits below: 258 words per lifted row
+// of columns in all for BG1 instead of 188, and 203 for BG2 instead of 168.  A
+// kernel has the code of one form per degree only: with both in one kernel (184 KB
+// of code against 138) 1136 blocks of BG1 Zc=24 took 243 us instead of 211, and
+// small mixed batches 3 to 5 % longer.
+NRLDPC_HD constexpr int row_messages(int d, bool core, int clip) { return parity_words(clip) && !core ? d - 1 : d; }
+NRLDPC_HD constexpr bool direct_row(int d, bool core, int clip, bool wide) {
+  return row_messages(d, core, clip) <= (!wide ? 4 : parity_words(clip) ? 10 : 8);
+}
+// Scratch planes (kThreadsTarget words each) of the row in the fixed-point kernels:
+// one per direct message, or the compressed message's two minima, flip bits and min2
+// bits, plus a fifth word for degree-19 rows; four at least, which are always loaded.
+NRLDPC_HD constexpr int fixed_row_planes(int d, bool core, int clip, bool wide) {
+  const int n = row_messages(d, core, clip);
+  return !direct_row(d, core, clip, wide) ? (d > 16 ? 5 : 4) : n > 4 ? n : 4;
+}
 // `beliefs`: the call returns beliefs.
 inline int fixed_clip_mode(const ldpc_decoder_cfg_t& dc, const uint32_t* ab, int rows, bool beliefs) {
   if (dc.min_llr > dc.max_llr) return kClipDegen;
@@ -123,19 +129,21 @@ inline int fixed_clip_mode(const ldpc_decoder_cfg_t& dc, const uint32_t* ab, int
   return dc.min_llr > -32767 || beliefs ? kClipOpen : kClipOpenMax;
 }
 
-// Scratch offsets of a mixed-size graph's rows, in words.  Rows of more than four
-// messages are uncompressed with the open maximum only: without it the row's extra
-// instructions leave too few registers to load their fifth to eighth message ahead,
-// and in a small batch nothing hides that load (78 blocks of up to 8424 bits, learned
-// table: 357 us compressed, 409 us not).
-inline void mixed_row_layout(const BaseGraph& g, int clip, uint32_t* lr_off) {
+// Scratch offsets of a graph's rows in the fixed-point kernels, in words; the last
+// entry is the total.
+inline void fixed_row_layout(const BaseGraph& g, int clip, bool wide, uint32_t* lr_off) {
   uint32_t off = 0;
   for (int r = 0; r < g.rows; ++r) {
     lr_off[r] = off;
-    off += (uint32_t)fixed_row_planes(r, g.degree[r], open_max(clip)) * kThreadsTarget;
+    off += (uint32_t)fixed_row_planes(g.degree[r], r < kCoreRows, clip, wide) * kThreadsTarget;
   }
   lr_off[g.rows] = off;
 }
+// Mixed-size kernels are wide with parity words only: without them the row's extra
+// instructions leave too few registers to load its fifth to eighth message ahead,
+// and in a small batch nothing hides that load (78 blocks of up to 8424 bits, learned
+// table: 357 us compressed, 409 us not).
+NRLDPC_HD constexpr bool mixed_wide(int clip) { return parity_words(clip); }
 
 // Alpha/beta per (iteration, row): alpha in the low 16 bits, beta in the high.
 inline uint32_t pack_ab(int16_t alpha, int16_t beta) {
@@ -322,7 +330,7 @@ int occupancy_mixed(int clip_mode, int cls = 0);
 int launch_channel(const uint8_t* rm, int64_t rm_stride, int32_t num_cw, int32_t E, int32_t Qm, float nv,
                    float sigma, float A, uint64_t seed, int16_t* llr, int64_t llr_stride, float* symbols,
                    void* stream);
-int launch_fixed(const DecodeParams& p, int grid, int block, int smem, int clip_mode, void* stream);
+int launch_fixed(const DecodeParams& p, int grid, int block, int smem, int clip_mode, bool wide, void* stream);
 // The small-batch fixed-point kernel (nrldpc_split.cu): one code block per CTA.
 // In its DecodeParams lr_off is what split_layout writes.
 struct SplitShape {

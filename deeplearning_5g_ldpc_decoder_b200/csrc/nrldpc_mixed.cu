@@ -215,10 +215,7 @@ __global__ void __launch_bounds__(kThreads, kMinBlocks) fixed_mixed_kernel(const
     const int bi = s_g.bgn == 1 ? 0 : 1;
     for (int r = tid; r < s_g.R; r += blockDim.x) {
       const uint32_t e0 = s_g.row_off[r], dg = (uint32_t)s_g.row_off[r + 1] - e0;
-      s_rows[r] = make_uint4(s_g.lr_off[r],
-                             row_word(e0, dg, (s_g.lr_off[r + 1] - s_g.lr_off[r]) / kThreadsTarget, kClip,
-                                      parity_words(kClip) && r >= kCoreRows),
-                             p.w_inline[bi][r], 0u);
+      s_rows[r] = make_uint4(s_g.lr_off[r], row_word(e0, dg, r < kCoreRows, kClip, mixed_wide(kClip)), p.w_inline[bi][r], 0u);
     }
     if (tid < 2 * G) s_cw[tid] = take_block(p, key);
     __syncthreads();
@@ -261,7 +258,7 @@ __global__ void __launch_bounds__(kThreads, kMinBlocks) fixed_mixed_kernel(const
           } else {
             ab0 = ab1 = d.z;
           }
-          layer_dispatch<kClip, true, false>(row_deg(d.y), row >= kCoreRows, row_direct(d.y), p, s_g.edges, reinterpret_cast<char*>(s_lq), zx4, zxm4, gb4,
+          layer_dispatch<kClip, mixed_wide(kClip), true, false>(row_case(d.y), p, s_g.edges, reinterpret_cast<char*>(s_lq), zx4, zxm4, gb4,
                                            4u * (uint32_t)(G * lq_len), row_e0(d.y),
                                            (int32_t)(int16_t)(ab0 & 0xFFFFu), ((int32_t)ab0) >> 16,
                                            (int32_t)(int16_t)(ab1 & 0xFFFFu), ((int32_t)ab1) >> 16, cur, fresh,

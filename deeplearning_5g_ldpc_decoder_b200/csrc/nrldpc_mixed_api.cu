@@ -71,13 +71,13 @@ void free_plan(MixedPlanImpl* pl) {
 
 }  // namespace
 
-uint32_t mixed_scratch_words_per_cta() {
+uint32_t mixed_scratch_words_per_cta(int clip) {
   uint32_t best = 0;
   for (int bgn = 1; bgn <= 2; ++bgn) {
     const BaseGraph& g = base_graph(bgn);
-    uint32_t planes = 0;
-    for (int r = 0; r < g.rows; ++r) planes += (uint32_t)fixed_row_planes(r, g.degree[r], true);
-    best = std::max(best, planes * (uint32_t)kThreadsTarget);
+    uint32_t off[kMaxRows + 1];
+    fixed_row_layout(g, clip, mixed_wide(clip), off);
+    best = std::max(best, off[g.rows]);
   }
   return best;
 }
@@ -95,7 +95,7 @@ MixedGraph make_graph(int bgn, int Zc, int iLS, int cap) {
   m.G = std::max(1, cap / Zc);
   m.K = (bgn == 1 ? 22 : 10) * Zc;
   m.N = (bgn == 1 ? 66 : 50) * Zc;
-  for (int r = 0; r <= g.rows; ++r) m.row_off[r] = g.row_off[r];   // lr_off: mixed_row_layout
+  for (int r = 0; r <= g.rows; ++r) m.row_off[r] = g.row_off[r];   // lr_off: fixed_row_layout
   for (int e = 0; e < g.nnz; ++e)
     m.edges[e] = make_uint2(4u * (uint32_t)g.col[e] * (uint32_t)Zc, 4u * (uint32_t)(g.vij[iLS][e] % Zc));
   return m;
@@ -190,7 +190,7 @@ int configure(MixedPlanImpl* pl, int ctas_per_sm, int order, int cls_mode) {
   if (pl->grid_c[1] > pl->scratch1_ctas) {
     cudaFree(pl->d_scratch1);
     pl->d_scratch1 = nullptr;
-    if (cudaMalloc(&pl->d_scratch1, (size_t)pl->grid_c[1] * mixed_scratch_words_per_cta() * sizeof(uint32_t)) !=
+    if (cudaMalloc(&pl->d_scratch1, (size_t)pl->grid_c[1] * pl->params.scratch_words * sizeof(uint32_t)) !=
         cudaSuccess)
       return NRLDPC_ERR_CUDA;
     pl->scratch1_ctas = pl->grid_c[1];
@@ -198,7 +198,7 @@ int configure(MixedPlanImpl* pl, int ctas_per_sm, int order, int cls_mode) {
   if (pl->grid > pl->scratch_ctas) {
     cudaFree(pl->d_scratch);
     pl->d_scratch = nullptr;
-    if (cudaMalloc(&pl->d_scratch, (size_t)pl->grid * mixed_scratch_words_per_cta() * sizeof(uint32_t)) != cudaSuccess)
+    if (cudaMalloc(&pl->d_scratch, (size_t)pl->grid * pl->params.scratch_words * sizeof(uint32_t)) != cudaSuccess)
       return NRLDPC_ERR_CUDA;
     pl->scratch_ctas = pl->grid;
   }
@@ -339,7 +339,6 @@ int32_t nrldpc_mixed_plan_create(const nrldpc_block_t* blocks, int32_t num_block
   p.max_llr = dc->max_llr;
   p.one = 1u;
   p.min_llr = dc->min_llr;
-  p.scratch_words = mixed_scratch_words_per_cta();
   for (int b = 0; b < 2; ++b) {
     const BaseGraph& g = base_graph(b + 1);
     for (int r = 0; r < g.rows; ++r) {
@@ -355,7 +354,8 @@ int32_t nrldpc_mixed_plan_create(const nrldpc_block_t* blocks, int32_t num_block
   // open-max arithmetic only when both base graphs' layers qualify
   pl->clip = fixed_clip_mode(*dc, p.w_inline[0], base_graph(1).rows, false);
   if (open_max(pl->clip)) pl->clip = fixed_clip_mode(*dc, p.w_inline[1], base_graph(2).rows, false);
-  for (MixedGraph& m : pl->graphs) mixed_row_layout(base_graph(m.bgn), pl->clip, m.lr_off);
+  p.scratch_words = mixed_scratch_words_per_cta(pl->clip);
+  for (MixedGraph& m : pl->graphs) fixed_row_layout(base_graph(m.bgn), pl->clip, mixed_wide(pl->clip), m.lr_off);
   // per-graph block queues: members of each graph in pairing order
   std::vector<int32_t> queue;
   std::vector<int32_t> base(pl->graphs.size()), count(pl->graphs.size());

@@ -175,20 +175,16 @@ extern "C" int32_t nrldpc_decode_batch_noalloc(const int16_t* d_llr, int64_t llr
     p.weights = dst;
     p.weights_T = T;
   }
-  uint32_t off = 0;
-  for (int r = 0; r < g.rows; ++r) {
-    p.lr_off[r] = off;
-    off += (uint32_t)fixed_row_planes(r, g.degree[r], false) * (uint32_t)kThreadsTarget;
-  }
-  p.lr_off[g.rows] = off;
-  p.scratch_words = off;
-  const size_t per_cta = (size_t)off * sizeof(uint32_t);
+  const int clip = fixed_clip_mode(*dc, p.w_inline, g.rows, d_app != nullptr);
+  // The static scratch bounds the CTAs in flight: the kernels with the smaller layout.
+  fixed_row_layout(g, clip, false, p.lr_off);
+  p.scratch_words = p.lr_off[g.rows];
+  const size_t per_cta = (size_t)p.scratch_words * sizeof(uint32_t);
   if (per_cta > kNoAllocScratchBytes) {
     fprintf(stderr, "nrldpc_decode_batch_noalloc: %zu bytes of scratch per CTA exceed the %zu-byte static array\n",
             per_cta, kNoAllocScratchBytes);
     return NRLDPC_ERR_ARG;
   }
-  const int clip = fixed_clip_mode(*dc, p.w_inline, g.rows, d_app != nullptr);
   const int block = (p.nact + 31) & ~31;
   const int smem = p.G * cp.lq_len * 4;
   int occ = occupancy_fixed(block, smem, clip);
@@ -207,6 +203,6 @@ extern "C" int32_t nrldpc_decode_batch_noalloc(const int16_t* d_llr, int64_t llr
   p.harq = d_harq;
   p.harq_stride = harq_stride;
   p.scratch = nd->scratch;
-  if (launch_fixed(p, grid, block, smem, clip, stream) != 0) return NRLDPC_ERR_CUDA;
+  if (launch_fixed(p, grid, block, smem, clip, false, stream) != 0) return NRLDPC_ERR_CUDA;
   return NRLDPC_OK;
 }

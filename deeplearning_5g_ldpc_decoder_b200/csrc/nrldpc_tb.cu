@@ -381,7 +381,7 @@ MixedGraph tb_make_graph(int bgn, int Zc, int iLS) {
   m.G = std::max(1, kThreadsTarget / Zc);
   m.K = (bgn == 1 ? 22 : 10) * Zc;
   m.N = (bgn == 1 ? 66 : 50) * Zc;
-  for (int r = 0; r <= g.rows; ++r) m.row_off[r] = g.row_off[r];   // lr_off: mixed_row_layout
+  for (int r = 0; r <= g.rows; ++r) m.row_off[r] = g.row_off[r];   // lr_off: fixed_row_layout
   for (int e = 0; e < g.nnz; ++e)
     m.edges[e] = make_uint2(4u * (uint32_t)g.col[e] * (uint32_t)Zc, 4u * (uint32_t)(g.vij[iLS][e] % Zc));
   return m;
@@ -426,7 +426,7 @@ int engine_lanes(TbEngine* e, int n) {
         cudaMalloc(&l->d_cb_bits, (size_t)max_cbs * kCbBitsStride) == cudaSuccess &&
         cudaMalloc(&l->d_cb_status, (size_t)max_cbs * sizeof(int32_t)) == cudaSuccess &&
         cudaMalloc(&l->d_cb_iters, (size_t)max_cbs * sizeof(int32_t)) == cudaSuccess &&
-        cudaMalloc(&l->d_scratch, (size_t)e->grid * mixed_scratch_words_per_cta() * sizeof(uint32_t)) == cudaSuccess &&
+        cudaMalloc(&l->d_scratch, (size_t)e->grid * e->mp.scratch_words * sizeof(uint32_t)) == cudaSuccess &&
         cudaMemset(l->d_num_items, 0, 2 * sizeof(int32_t)) == cudaSuccess;
     if (!ok) {
       lane_free(l);
@@ -616,7 +616,6 @@ int32_t nrldpc_tb_engine_create(int32_t max_tbs, int32_t max_cbs, const ldpc_dec
   p.graphs = e->d_graphs;
   p.num_items = 0;
   p.crc_tab = e->d_crc_tab;
-  p.scratch_words = mixed_scratch_words_per_cta();
   p.max_it = dc->max_iterations;
   p.fill = dc->filling_bit_value;
   p.max_llr = dc->max_llr;
@@ -637,8 +636,9 @@ int32_t nrldpc_tb_engine_create(int32_t max_tbs, int32_t max_cbs, const ldpc_dec
   // open-max arithmetic only when both base graphs' layers qualify
   e->clip = fixed_clip_mode(*dc, p.w_inline[0], base_graph(1).rows, false);
   if (open_max(e->clip)) e->clip = fixed_clip_mode(*dc, p.w_inline[1], base_graph(2).rows, false);
+  p.scratch_words = mixed_scratch_words_per_cta(e->clip);
   for (MixedGraph& m : graphs)
-    if (m.bgn) mixed_row_layout(base_graph(m.bgn), e->clip, m.lr_off);
+    if (m.bgn) fixed_row_layout(base_graph(m.bgn), e->clip, mixed_wide(e->clip), m.lr_off);
   if (cudaMemcpy(e->d_graphs, graphs.data(), kKeys * sizeof(MixedGraph), cudaMemcpyHostToDevice) != cudaSuccess) {
     engine_free(e);
     return NRLDPC_ERR_CUDA;

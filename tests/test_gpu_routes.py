@@ -1,11 +1,16 @@
 """Which kernel a uniform batch runs on, and results that depend on it: the arithmetic variant of the fixed-point kernels
 follows the decoder row, the tables and whether the call returns beliefs, and every variant equals the oracle."""
 
+import ctypes
+import os
+
 import numpy as np
 import pytest
 import torch
 
 from deeplearning_5g_ldpc_decoder_b200 import capi, ldpc_decode, set_degree_alpha
+from deeplearning_5g_ldpc_decoder_b200.build import DEBUG_LIB_PATH, build_library
+from deeplearning_5g_ldpc_decoder_b200.decoder import DecodeResult
 from oracle.oracle import dec_cfg, in_config
 
 pytestmark = pytest.mark.gpu
@@ -89,3 +94,82 @@ def test_open_maximum_without_parity_words(oracle, cuda, row, bgn, A, E, rv, Qm)
     llr = repeated(host, n, cuda)
     check_against_oracle(oracle, cfg, row, host, ldpc_decode(llr, cfg, row))
     check_against_oracle(oracle, cfg, row, host, ldpc_decode(llr, cfg, row, return_app=True))
+
+
+def _sizes(bgn):
+    """One (A, crctype) per lifting size of the base graph that a payload reaches."""
+    seen = {}
+    for A in range(8, (8448 if bgn == 1 else 3840) - 24 + 1, 8):
+        for crc in (1, 0):
+            p = capi.gen_ldpc_parameters(capi.make_in_config(bgn, A, crc, 960, 0, 2, 0))
+            seen.setdefault(int(p.Zc), (A, crc))
+    return sorted(seen.items())
+
+
+def _raw_decode(lib, llr, cfg, row, app):
+    p = capi.gen_ldpc_parameters(capi.make_in_config(*cfg), lib)
+    n = llr.shape[0]
+    bits = torch.zeros((n, (p.B + 7) // 8), dtype=torch.uint8, device=llr.device)
+    st, it = (torch.full((n,), -9, dtype=torch.int32, device=llr.device) for _ in range(2))
+    bel = torch.zeros((n, p.N + 2 * p.Zc), dtype=torch.int16, device=llr.device) if app else None
+    rc = lib.nrldpc_decode_batch(llr.data_ptr(), llr.shape[1], n, ctypes.byref(capi.make_in_config(*cfg)),
+                                 ctypes.byref(capi.make_decoder_config(row)), bits.data_ptr(), bits.shape[1], st.data_ptr(),
+                                 it.data_ptr(), bel.data_ptr() if app else 0, bel.shape[1] if app else 0, 0, 0,
+                                 torch.cuda.current_stream().cuda_stream)
+    assert rc == 0
+    return bits, st, it, bel
+
+
+def _set_tables(libs, bgn, alpha=None, beta=None):
+    for lib in libs:
+        assert lib.nrldpc_set_trained_weights(bgn, alpha.ctypes.data if alpha is not None else None,
+                                              beta.ctypes.data if beta is not None else None,
+                                              alpha.shape[0] if alpha is not None else 0) == 0
+
+
+@pytest.mark.parametrize("bgn", [1, 2])
+def test_every_lifting_size_on_the_pair_kernel(oracle, cuda, lib, bgn):
+    """Both row forms of the pair kernel at every lifting size, with groups that end inside a warp and an odd block at
+    the end: equal to the oracle, and the same in the bounds-checked library without a violation."""
+    if not os.path.exists(DEBUG_LIB_PATH):
+        build_library(debug=True)
+    dbg = capi.load_library(DEBUG_LIB_PATH)
+    rec = (ctypes.c_uint32 * 4)()
+    assert dbg.nrldpc_bounds_check_status(rec, 1) == 1
+    rows = [[1, 5, 22936, 0, 1280, 32767, -32767], [2, 5, 0, 0, 1280, 20000, -20000], OPEN_LOW,
+            [1, 3, 22936, 0, 1280, -100, 100]]
+    rng = np.random.default_rng(bgn)
+    alpha, beta = (rng.integers(lo, hi, (3, capi.BG_ROWS[bgn])).astype(np.int16) for lo, hi in ((15000, 30000), (0, 30)))
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    sizes = _sizes(bgn)
+    assert len(sizes) >= (51 if bgn == 1 else 45)
+    _set_tables((lib, dbg), bgn, alpha, beta)
+    oracle.set_trained(bgn, alpha, beta)
+    try:
+        for k, (zc, (A, crc)) in enumerate(sizes):
+            B = A + (16 if crc == 0 else 24)
+            cfg = (bgn, A, crc, 2 * ((2 * B + 1) // 2), k % 4, 2, 0)
+            host = noisy_blocks(oracle, cfg, zc)
+            for row in (rows[0], rows[1 + k % 3]):
+                n = pair_batch(cfg, row)
+                many = max(n, (2 * sms * -(-160 // zc) + 1) | 1)   # enough groups per CTA for the wide form
+                for m in sorted({n, many}):
+                    route = capi.decode_route(cfg, row, m)
+                    assert route.kernel == capi.ROUTE_PAIR
+                    assert route.wide == int(route.groups == 1 or route.groups * zc >= 160)
+                    llr = repeated(host, m, cuda)
+                    plain = _raw_decode(lib, llr, cfg, row, False)
+                    full = _raw_decode(lib, llr, cfg, row, True)
+                    for a, b in zip(plain[:3], full[:3]):
+                        assert torch.equal(a, b), (cfg, row, m)
+                    check_against_oracle(oracle, cfg, row, host, DecodeResult(*full))
+                    if m == many and m != n and k % 3:
+                        continue
+                    for app, ref in ((False, plain), (True, full)):
+                        got = _raw_decode(dbg, llr, cfg, row, app)
+                        torch.cuda.synchronize()
+                        assert all(torch.equal(a, b) for a, b in zip(got[:3 + app], ref[:3 + app])), (cfg, row, m)
+                        assert dbg.nrldpc_bounds_check_status(rec, 1) == 1 and list(rec) == [0] * 4, (cfg, row, m, list(rec))
+    finally:
+        _set_tables((lib, dbg), bgn)
+        oracle.set_trained(bgn)
