@@ -129,6 +129,7 @@ __device__ __forceinline__ void split_row(const DecodeParams& p, const Geometry&
     s2 = scale_pair(__vmins2(m2, maxp), alpha, beta, alpha, beta);
   }
   uint32_t ovf = 0u;
+  const uint32_t m_active = active ? 0xFFFFFFFFu : 0u, m_tail = tail ? 0xFFFFFFFFu : 0u;
   uint32_t lr[K];
 #pragma unroll
   for (int k = 0; k < K; ++k) {
@@ -137,7 +138,7 @@ __device__ __forceinline__ void split_row(const DecodeParams& p, const Geometry&
     const uint32_t ne = __vminu2(mag[k] ^ m1, 0x00010001u) * 0xFFFFu;
     const uint32_t v = bsel(ne, s1, s2);
     lr[k] = __vadd2(v ^ mf, mf & 0x00010001u);      // mf ? -v : v
-    uint32_t nq;
+    uint32_t nq, over = 0u;
     if constexpr (kClip == kClipOpenMax) {
       // v >= 0 here (no offset, no negative alpha), so the sum is taken with the
       // message's sign put on the other operand: w = rel ^ mf, (w + v) ^ mf is
@@ -145,17 +146,21 @@ __device__ __forceinline__ void split_row(const DecodeParams& p, const Geometry&
       // is.  8 iterations, 64 blocks: BG1 Zc24 106 -> 103.6 us, BG2 Zc64 85 ->
       // 83.2 us.
       const uint32_t w = rel[k] ^ mf, u = __vadd2(w, v);
-      ovf |= u & ~w;
+      over = u & ~w;
       nq = __vmaxs2(u ^ mf, minp);
     } else if constexpr (kClip == kClipClamp) {
       const uint32_t sum = __vadd2(rel[k], lr[k]);
-      ovf |= (sum ^ rel[k]) & ~(rel[k] ^ lr[k]);
+      over = (sum ^ rel[k]) & ~(rel[k] ^ lr[k]);
       nq = __vmins2(__vmaxs2(sum, minp), maxp);
     } else {
       const int32_t lo = (int32_t)(int16_t)(rel[k] & 0xFFFFu) + (int32_t)(int16_t)(lr[k] & 0xFFFFu);
       const int32_t hi = (((int32_t)rel[k]) >> 16) + (((int32_t)lr[k]) >> 16);
       nq = clip_half_degen(lo, p.max_llr, p.min_llr) | (clip_half_degen(hi, p.max_llr, p.min_llr) << 16);
     }
+    // A slot without an edge stores nothing, and must not flag its sum either: the
+    // neutral word plus any message overflows, in every second row with an idle lane.
+    // 8 iterations, 64 blocks, flagged / not: BG1 Zc112 150 / 131 us, BG2 Zc64 87 / 80 us.
+    ovf |= over & (k < K - 1 ? m_active : m_tail);
     if ((k < K - 1 ? active : tail) && NRLDPC_INBOUNDS(at[k] >> 16, g.limit, kBoundsLq)) {
       *reinterpret_cast<uint32_t*>(lq + (at[k] >> 16)) = __byte_perm(nq, 0u, at[k]);
       msg[k * stride] = __vadd2(~lr[k], 0x00010001u);
