@@ -299,17 +299,16 @@ int make_plan(const CodeParams& cp, const ldpc_decoder_cfg_t& dc, int num_cw, bo
   // The small-batch kernel while all blocks run at once, with eight lanes per row
   // pair while an SM then holds few threads (its rows have a shorter chain, but
   // issue more in all), else with four; eight again where only they fit.  Measured,
-  // 8 iterations, us for the pair kernel / four lanes / eight lanes: BG1 Zc 24, 64
-  // blocks 230 / 103 / 85, 444 (three per SM, 576 threads) 234 / 132 / 123, 592
-  // 230 / does not fit / 149; BG1 Zc 40, 296 blocks (640 threads) - / 134 / 126;
-  // BG1 Zc 48, 296 blocks (768) - / 134 / 142; BG1 Zc 80, 64 blocks (640) - / 134 /
-  // 126; BG1 Zc 112, 64 blocks 246 / 146 / 155, 149 in two rounds 246 / 288; BG2 Zc
-  // 22, 64 blocks (192) - / 77 / 73; BG2 Zc 40 (320) - / 83 / 83; BG2 Zc 64, 64
-  // blocks (512) 155 / 83 / 91, 592 in two rounds 155 / 197; BG1 Zc 208, 148 blocks
-  // 308 / 273, 149 308 / 541.
+  // 8 iterations, us for the pair kernel / four lanes / eight lanes: BG1 Zc 2, 600
+  // blocks (five per SM, 320 threads) 206 / 121 / 101; Zc 11, 300 (576) 226 / 131 / 119;
+  // Zc 18, 300 (576) 208 / 115 / 119; Zc 24, 64 blocks 198 / 88 / 85, 296 (384) 205 /
+  // 102 / 98, 444 (576) 211 / 117 / 120, 592 211 / does not fit / 145; Zc 40, 64 (320)
+  // 198 / 96 / 99, 30 / 28 after one iteration; Zc 48, 296 (768) 205 / 117 / 139; Zc 80,
+  // 64 (640) 203 / 114 / 124; BG2 Zc 7, 64 (64) 139 / 85 / 81; Zc 28, 64 (224) 178 / 72 /
+  // 76; Zc 64, 64 (512) 133 / 78 / 94.
   if (fixed && num_cw <= 32 * st->num_sms) {
     const int per_sm = (num_cw + st->num_sms - 1) / st->num_sms;
-    const int few = cp.bgn == 1 ? 640 : 320;
+    const int few = cp.bgn == 2 ? 320 : (cp.Zc & 1) ? 640 : 384;   // (an odd Zc has one belief per word)
     for (int k = 0; k < 3; ++k) {
       const int lanes = k == 1 ? 4 : 8;
       const uint32_t* layout = split_layout(cp.bgn, lanes);

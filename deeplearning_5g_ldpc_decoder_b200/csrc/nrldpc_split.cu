@@ -28,13 +28,13 @@
 // A step is one dependent chain of about 140 instructions (four lanes) in each of
 // a few warps, 600 to 700 cycles (a thread that walks a whole row takes over 1000
 // cycles a layer), so what bounds the kernel is that chain, not a throughput.
-// One iteration of BG1 Zc=24: 25.8 us in the pair kernel, 11.2 us here; BG2
-// Zc=64 17.2 and 8.9 us; BG1 Zc=112 27.6 and 15.8 us.  With one group per step
-// 18.2, 10.7 and 17.8 us; with the pair kernel's compressed messages (16 or 32
-// flag bits per lane) and one group 21, 14 and 23 us.  With eight lanes a thread
-// has one edge of a row of up to eight: 8 iterations of Zc=24 take 104 us with four
-// and 85 us with eight, Zc=2 98 and 77 us; the shuffle step and the warps more cost
-// more than that gives from Zc=112 (BG1) or 48 (BG2) on.
+// 64 blocks, 8 iterations: BG1 Zc=24 198 us in the pair kernel, 85 us here; BG2 Zc=64
+// 133 and 78 us.  Per iteration, when it was written: 11.2 us for BG1 Zc=24, 8.9 for
+// BG2 Zc=64, 15.8 for BG1 Zc=112; with one group per step 18.2, 10.7 and 17.8 us; with
+// the pair kernel's compressed messages (16 or 32 flag bits per lane) and one group
+// 21, 14 and 23 us.  With eight lanes a thread has one edge of a row of up to eight;
+// the shuffle step and the warps more cost more than that gives where an SM holds
+// many threads (the rule in nrldpc_api.cu).
 #include <cuda_runtime.h>
 #include <stdint.h>
 
@@ -49,7 +49,13 @@ using namespace fixedrow;
 
 constexpr int kAhead = 3;          // slots per lane loaded a row ahead (degree <= 12 with four lanes, all with eight)
 constexpr int kGroupsPerStep = 2;
-constexpr int kSplitThreads = 1024;   // two groups of kLanes H threads: Zc <= 256 or 128 (what fits shared memory may end below that)
+// Two groups of kLanes H threads: Zc <= 208 or 104 (what fits shared memory may end
+// below that).  Larger ones lose to the pair kernel: one block, 8 iterations, four lanes
+// / pair kernel BG1 Zc 192 233 / 243 us, 208 260 / 256 us, 224 262 / 245 us, BG2 Zc 208
+// 147 / 184 us, 224 200 / 174 us, 256 208 / 176 us.  The launch bound also sets the
+// registers: 64 for 1024 threads, 72 for 832 (BG1 Zc 160 219 -> 204 us, BG2 Zc 64 with
+// an offset 94 -> 84 us).
+constexpr int kSplitThreads = 832;
 
 // Permute selectors: the word as it is, and with its halves swapped.
 constexpr uint32_t kStraight = 0x3210u, kSwapBit = 0x2222u;
@@ -87,7 +93,7 @@ struct Slots {
   uint32_t at[kAhead], nr[kAhead];
 };
 
-// One layer for one thread: K = ceil(degree / 4) slots.  Threads that own no rows
+// One layer for one thread: K = ceil(degree / kLanes) slots.  Threads that own no rows
 // (`active` false) only take part in the shuffles; `tail`: the last slot has an edge.
 template <int K, int kLanes, int kClip, typename AtSlot>
 __device__ __forceinline__ void split_row(const DecodeParams& p, const Geometry& g, char* __restrict__ lq, const Slots& in,
