@@ -198,7 +198,7 @@ struct Plan {
   int grid, block, smem;
   int clip;   // check-node arithmetic variant of the fixed-point kernel (fixed_clip_mode)
   int algo;
-  bool wide;         // fixed_pair_kernel: rows of more than four messages uncompressed too (direct_row)
+  bool wide;         // longer rows uncompressed too (direct_row, float_direct)
   bool split;        // the small-batch kernel: one code block per CTA, no scratch
   SplitShape shape;
   size_t scratch_bytes;
@@ -327,20 +327,6 @@ int make_plan(const CodeParams& cp, const ldpc_decoder_cfg_t& dc, int num_cw, bo
     }
   }
 
-  // Scratch layout per CTA, layer by layer.  (The fixed-point kernel addresses its
-  // planes with a compile-time stride.)
-  if (fixed) {
-    fixed_row_layout(g, plan->clip, plan->wide, p.lr_off);
-  } else {
-    uint32_t off = 0;
-    for (int r = 0; r < g.rows; ++r) {
-      p.lr_off[r] = off;
-      off += (uint32_t)(algo == 0 ? g.degree[r] : float_row_planes(g.degree[r])) * (uint32_t)p.nact;
-    }
-    p.lr_off[g.rows] = off;
-  }
-  p.scratch_words = p.lr_off[g.rows];
-
   const uint64_t key = ((uint64_t)(fixed ? 1 : algo == 4 ? 2 : 3) << 56) | ((uint64_t)(fixed ? plan->clip : 0) << 48) |
                        ((uint64_t)plan->block << 32) | (uint64_t)(uint32_t)plan->smem;
   int occ = cached_occupancy(st, key, [&] {
@@ -350,6 +336,29 @@ int make_plan(const CodeParams& cp, const ldpc_decoder_cfg_t& dc, int num_cw, bo
   if (occ < 1) occ = 1;
   plan->grid = std::min(p.num_items, occ * st->num_sms);
   if (plan->grid < 1) plan->grid = 1;
+  // Scratch layout per CTA, layer by layer.  (The fixed-point kernel addresses its
+  // planes with a compile-time stride.)  Float min-sum is wide for batches of more than
+  // a wave, where other CTAs hide the messages that a row loads itself, unless a second
+  // wave would be the last and nearly full: then a CTA that runs ahead of the other on
+  // its SM, as CTAs of the wide form do, takes a third item.  8 iterations, us with rows
+  // of up to three / five edges uncompressed: 16 blocks BG2 Zc 64 127 / 146, 444 of BG1
+  // Zc 384 (one wave) 684 / 682; 777 of BG1 Zc 208 (1.75 waves) 864 / 830, 1184 of BG1
+  // Zc 144 (2.7) 874 / 849, 4096 of BG1 Zc 384 6.29 / 6.30 ms; 9000 of BG1 Zc 24 (1.9)
+  // 959 / 1143, 592 of BG1 Zc 384 (2) 949 / 1131, 888 of BG2 Zc 256 (2) 619 / 717.
+  if (!fixed)
+    plan->wide = algo == 4 && p.num_items > plan->grid &&
+                 (8 * (int64_t)p.num_items <= 15 * (int64_t)plan->grid || p.num_items > 2 * plan->grid);
+  if (fixed) {
+    fixed_row_layout(g, plan->clip, plan->wide, p.lr_off);
+  } else {
+    uint32_t off = 0;
+    for (int r = 0; r < g.rows; ++r) {
+      p.lr_off[r] = off;
+      off += (uint32_t)(algo == 0 ? g.degree[r] : float_row_planes(g.degree[r], plan->wide)) * (uint32_t)p.nact;
+    }
+    p.lr_off[g.rows] = off;
+  }
+  p.scratch_words = p.lr_off[g.rows];
   plan->scratch_bytes = (size_t)plan->grid * (size_t)p.scratch_words * sizeof(uint32_t);
   return 0;
 }
@@ -362,7 +371,7 @@ int launch_plan(Plan* plan, void* stream) {
     case 3:
       return launch_fixed(plan->p, plan->grid, plan->block, plan->smem, plan->clip, plan->wide, stream);
     case 4:
-      return launch_float_minsum(plan->p, plan->grid, plan->block, plan->smem, stream);
+      return launch_float_minsum(plan->p, plan->grid, plan->block, plan->smem, plan->wide, stream);
     default:
       return launch_float_bp(plan->p, plan->grid, plan->block, plan->smem, stream);
   }
@@ -1027,7 +1036,7 @@ int32_t nrldpc_decode_route(const ldpc_in_config_t* inconfig, const ldpc_decoder
   route->arithmetic = fixed ? plan.clip : 0;
   route->lanes = plan.split ? plan.shape.lanes : 1;
   route->groups = plan.split ? 1 : plan.p.G;
-  route->wide = fixed && !plan.split && plan.wide ? 1 : 0;
+  route->wide = !plan.split && plan.wide ? 1 : 0;
   return NRLDPC_OK;
 }
 

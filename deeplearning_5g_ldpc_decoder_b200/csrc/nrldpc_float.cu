@@ -13,8 +13,8 @@
 // Mapping: one code block per group of Zc threads, up to G = floor(384 / Zc) groups
 // per CTA, FP32 beliefs in shared memory, persistent grid.  Min-sum messages
 // are stored compressed per lifted check row (two minima, one word of flip bits
-// and the minimum's position: 12 bytes) in rows of more than five edges; messages
-// of shorter rows and of BP are stored per edge.
+// and the minimum's position: 12 bytes) in rows of more than three or five edges
+// (float_direct); messages of shorter rows and of BP are stored per edge.
 #include <cuda_runtime.h>
 #include <float.h>
 #include <math.h>
@@ -39,7 +39,7 @@ __device__ __forceinline__ float clipf(float v, float mx, float mn) {
 __shared__ uint2 s_fedge4[kMaxNnz];
 
 // ---------------------------------------------------------------- float min-sum
-// Stored message of a lifted check row: in rows of up to five edges (kFloatDirect)
+// Stored message of a lifted check row: in short rows (float_direct)
 // the messages themselves, one plane each, otherwise three planes: new_min1,
 // new_min2 (float bits), and a word with edge j's sign flip in bit D - 1 - j and the
 // position of new_min2's edge from bit 20.  The kernel loads a row's first words
@@ -162,10 +162,10 @@ __device__ __forceinline__ void fms_row_direct(const DecodeParams& p, char* __re
   }
 }
 
-template <bool kRange>
+template <bool kRange, bool kWide>
 __device__ __forceinline__ void fms_dispatch(int deg, const DecodeParams& p, char* lq, uint32_t zx4, int e0, bool first, const FloatMsg& old, uint32_t* lrp, int NT) {
 #define NRLDPC_FROW(D) \
-  if constexpr (D <= kFloatDirect) fms_row_direct<D, kRange>(p, lq, zx4, e0, first, old, reinterpret_cast<float*>(lrp), NT); \
+  if constexpr (D <= float_direct(kWide)) fms_row_direct<D, kRange>(p, lq, zx4, e0, first, old, reinterpret_cast<float*>(lrp), NT); \
   else fms_row<D, kRange>(p, lq, zx4, e0, old, lrp, NT); \
   break;
   switch (deg) {
@@ -382,10 +382,11 @@ __device__ void emit_float_block(const DecodeParams& p, const float* lq, int zx,
   }
 }
 
-// Kernel variants: belief propagation, min-sum with min_llr <= max_llr, min-sum otherwise.
+// Kernel variants: belief propagation, min-sum with min_llr <= max_llr, min-sum otherwise;
+// min-sum with either set of uncompressed rows (float_direct).
 enum { kFloatBp = 0, kFloatRange = 1, kFloatDegen = 2 };
 
-template <int kMode>
+template <int kMode, bool kWide>
 __global__ void __launch_bounds__(kThreadsTarget, 2) float_kernel(const __grid_constant__ DecodeParams p) {
   constexpr bool kBP = kMode == kFloatBp;
   extern __shared__ __align__(16) float s_lqf[];     // [G][lq_len]
@@ -478,7 +479,7 @@ __global__ void __launch_bounds__(kThreadsTarget, 2) float_kernel(const __grid_c
 #pragma unroll
               for (int k = 0; k < kFloatAhead; ++k) nxt.w[k] = m[k * NT];
             }
-            fms_dispatch<kMode == kFloatRange>(deg, p, reinterpret_cast<char*>(lq), 4u * (uint32_t)zx, e0, it == 0, cur, lrp, NT);
+            fms_dispatch<kMode == kFloatRange, kWide>(deg, p, reinterpret_cast<char*>(lq), 4u * (uint32_t)zx, e0, it == 0, cur, lrp, NT);
           }
         }
         __syncthreads();
@@ -570,20 +571,36 @@ int occupancy_impl(K kernel, std::atomic<uint32_t>* attr_done, int block, int sm
 
 }  // namespace
 
-static std::atomic<uint32_t> g_attr[3];   // raise_smem_limit_once, per kernel
+namespace {
 
-int launch_float_minsum(const DecodeParams& p, int grid, int block, int smem, void* stream) {
-  return p.f_min <= p.f_max ? launch_impl(float_kernel<kFloatRange>, &g_attr[kFloatRange], p, grid, block, smem, stream)
-                            : launch_impl(float_kernel<kFloatDegen>, &g_attr[kFloatDegen], p, grid, block, smem, stream);
+template <int kMode, bool kWide>
+int launch_float(const DecodeParams& p, int grid, int block, int smem, void* stream) {
+  static std::atomic<uint32_t> attr_done{0};   // raise_smem_limit_once, per kernel
+  return launch_impl(float_kernel<kMode, kWide>, &attr_done, p, grid, block, smem, stream);
+}
+
+// The same for every min-sum kernel (all are bound to two CTAs of 384 threads per SM).
+template <int kMode>
+int occupancy_float(int block, int smem) {
+  static std::atomic<uint32_t> attr_done{0};
+  return occupancy_impl(float_kernel<kMode, false>, &attr_done, block, smem);
+}
+
+}  // namespace
+
+int launch_float_minsum(const DecodeParams& p, int grid, int block, int smem, bool wide, void* stream) {
+  if (p.f_min <= p.f_max)
+    return wide ? launch_float<kFloatRange, true>(p, grid, block, smem, stream)
+                : launch_float<kFloatRange, false>(p, grid, block, smem, stream);
+  return wide ? launch_float<kFloatDegen, true>(p, grid, block, smem, stream)
+              : launch_float<kFloatDegen, false>(p, grid, block, smem, stream);
 }
 int launch_float_bp(const DecodeParams& p, int grid, int block, int smem, void* stream) {
-  return launch_impl(float_kernel<kFloatBp>, &g_attr[kFloatBp], p, grid, block, smem, stream);
+  return launch_float<kFloatBp, false>(p, grid, block, smem, stream);
 }
 int bounds_read_float(uint32_t* out, bool reset) { return bounds_read_tu(out, reset); }
 
-int occupancy_float_minsum(int block, int smem) {
-  return occupancy_impl(float_kernel<kFloatRange>, &g_attr[kFloatRange], block, smem);
-}
-int occupancy_float_bp(int block, int smem) { return occupancy_impl(float_kernel<kFloatBp>, &g_attr[kFloatBp], block, smem); }
+int occupancy_float_minsum(int block, int smem) { return occupancy_float<kFloatRange>(block, smem); }
+int occupancy_float_bp(int block, int smem) { return occupancy_float<kFloatBp>(block, smem); }
 
 }  // namespace nrldpc

@@ -56,9 +56,18 @@ uint32_t crc_remainder(const uint8_t* data, int len, int crctype);
 // message whose only set bit sits d positions before its end.
 void crc_position_table(int crctype, uint32_t* out /* kMaxB */);
 
+#ifdef __CUDACC__
+#define NRLDPC_HD __host__ __device__
+#else
+#define NRLDPC_HD
+#endif
+
 // Scratch planes of a float min-sum row of degree d (layout in nrldpc_float.cu).
-constexpr int kFloatDirect = 5;
-inline int float_row_planes(int d) { return d <= kFloatDirect ? d : 3; }
+// Rows of up to this many edges keep their messages as they are.  The kernels load
+// three words of a row ahead, so rows of three edges always do; the wide kernels also
+// those of four and five, whose other words are loaded where the row starts.
+NRLDPC_HD constexpr int float_direct(bool wide) { return wide ? 5 : 3; }
+inline int float_row_planes(int d, bool wide) { return d <= float_direct(wide) ? d : 3; }
 // Scratch words per CTA of the mixed-size kernel: the larger of the two base
 // graphs' layouts (all rows' planes x kThreadsTarget).
 uint32_t mixed_scratch_words_per_cta(int clip);
@@ -84,11 +93,6 @@ inline uint32_t qm_magic(int qm) {
 //    row, also keeps parity words (below); kClipOpen is for the calls that cannot.
 // `ab` holds each layer's packed alpha | beta << 16 as the kernels read it.
 enum { kClipClamp = 0, kClipDegen = 1, kClipOpenMax = 2, kClipOpen = 3 };
-#ifdef __CUDACC__
-#define NRLDPC_HD __host__ __device__
-#else
-#define NRLDPC_HD
-#endif
 NRLDPC_HD constexpr bool open_max(int clip) { return clip == kClipOpenMax || clip == kClipOpen; }
 // Whether the parity columns of rows 4 and up hold the row's extrinsic input
 // instead of the belief (nrldpc_fixed_row.cuh).  Only with the open maximum and a
@@ -342,7 +346,7 @@ const uint32_t* split_layout(int bgn, int lanes);   // [rows + 1]
 bool split_shape(int Zc, int cols, int lanes, int slots, SplitShape* out);   // false: does not fit an SM
 int launch_split(const DecodeParams& p, const SplitShape& s, int clip_mode, void* stream);
 int occupancy_split(const SplitShape& s, int clip_mode);
-int launch_float_minsum(const DecodeParams& p, int grid, int block, int smem, void* stream);
+int launch_float_minsum(const DecodeParams& p, int grid, int block, int smem, bool wide, void* stream);
 int launch_float_bp(const DecodeParams& p, int grid, int block, int smem, void* stream);
 
 // Occupancy helpers (per kernel variant).

@@ -524,7 +524,7 @@ typedef struct {
     int32_t kernel, arithmetic;
     int32_t lanes;                  /* small-batch kernel: lanes per row pair */
     int32_t groups;                 /* lane pairs (code blocks, float) per CTA */
-    int32_t wide;                   /* pair kernel: rows of more than four messages uncompressed */
+    int32_t wide;                   /* pair and float kernels: longer rows keep uncompressed messages */
 } nrldpc_route_t;
 int32_t nrldpc_decode_route(const ldpc_in_config_t *inconfig, const ldpc_decoder_cfg_t *decoder_cfg,
                             int32_t num_cw, int32_t beliefs, nrldpc_route_t *route);

@@ -173,3 +173,24 @@ def test_every_lifting_size_on_the_pair_kernel(oracle, cuda, lib, bgn):
     finally:
         _set_tables((lib, dbg), bgn)
         oracle.set_trained(bgn)
+
+
+@pytest.mark.parametrize("row", [[4, 5, 22936, 0, 1280, 32767, -32767], [4, 3, 22936, 0, 1280, -100, 100]])
+@pytest.mark.parametrize("bgn,A,E,Qm", [(1, 8, 96, 2), (2, 488, 1920, 2), (1, 4352, 8754, 6)])
+def test_both_row_forms_of_float_min_sum(oracle, cuda, row, bgn, A, E, Qm):
+    """Rows of up to five edges uncompressed in batches of more than a wave, of up to three in smaller ones."""
+    cfg = (bgn, A, 1, E, 0, Qm, 0)
+    host = noisy_blocks(oracle, cfg, A)
+    n = 1
+    while not capi.decode_route(cfg, row, n).wide:
+        n += max(1, n // 2)
+    small = ldpc_decode(repeated(host, DISTINCT, cuda), cfg, row, return_app=True)
+    large = ldpc_decode(repeated(host, n, cuda), cfg, row, return_app=True)
+    assert not capi.decode_route(cfg, row, DISTINCT).wide
+    for i in range(DISTINCT):
+        es, eb, ei, lq = oracle.decode(np.ascontiguousarray(host[i]), in_config(*cfg), dec_cfg(row))
+        for got in (small, large):
+            same = slice(i, got.status.shape[0], DISTINCT)
+            assert (got.status[same] == es).all() and (got.iterations[same] == ei).all()
+            assert (got.app[same] == torch.from_numpy(lq).to(cuda)).all()
+            assert (got.hardbits[same] == torch.from_numpy(eb).to(cuda)).all()
