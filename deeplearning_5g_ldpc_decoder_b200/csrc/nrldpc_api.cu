@@ -758,7 +758,7 @@ int pick_tape_groups(DeviceState* st, TrainTapeParams* p, bool backward, int* bl
     const int bytes = G * p->n * 4 + (backward ? acc + 2 * p->R * (blk / 32) * 4 : 0);
     if (bytes > kTapeSmemCap) break;
     const uint64_t key = (backward ? 5ull : 4ull) << 56 |
-                         (uint64_t)((p->R == NRLDPC_BG2_ROWS) | p->vec << 1 | (backward && clipped) << 2) << 48 |
+                         (uint64_t)((p->R == NRLDPC_BG2_ROWS) | p->access << 1 | (backward && clipped) << 3) << 48 |
                          (uint64_t)blk << 32 | (uint64_t)(uint32_t)bytes;
     const int occ =
         cached_occupancy(st, key, [&] { return occupancy_train_tape(*p, backward, blk, bytes); });
@@ -780,7 +780,7 @@ int launch_tape_kernel(TrainTapeParams* p, bool backward, void* stream) {
   std::lock_guard<std::mutex> lock(g_mu);
   DeviceState* st = nullptr;
   if (device_state(&st) != 0) return NRLDPC_ERR_CUDA;
-  p->vec = p->Zc % 4 == 0 && reinterpret_cast<uintptr_t>(p->tape) % 16 == 0;   // (the carry is the library's own)
+  p->access = p->Zc % 4 != 0 ? kTapePlanes : reinterpret_cast<uintptr_t>(p->tape) % 16 != 0 ? kTapeGroupWords : kTapeGroups;
   int block = 0, smem = 0;
   const int occ = pick_tape_groups(st, p, backward, &block, &smem);
   if (occ < 1) return NRLDPC_ERR_CUDA;

@@ -293,10 +293,13 @@ struct TrainParams {
 };
 
 // ---- the float32 training kernels that keep a tape (nrldpc_train_tape.cu) ----
+// The order of a row's words in the tape depends on Zc alone: a plane per edge, or for a
+// multiple of 4 groups of four edges (word by word where the tape is not 16-byte aligned).
+enum TapeAccess { kTapePlanes = 0, kTapeGroupWords = 1, kTapeGroups = 2 };
 struct TrainTapeParams {
   int32_t Zc, R, n, G, nnz, T, batch, detach;
   int32_t acc;                // backward: the CTA sums its alpha / beta gradients in shared memory
-  int32_t vec;                // Zc a multiple of 4 and the tape 16-byte aligned: groups of four edges per access
+  int32_t access;             // how a row's words are accessed (TapeAccess)
   float clip;                 // +inf when LLRs are not clipped
   const float* llr;           // [batch][n] decoder-layout input LLRs
   const float* alpha;         // [T][R]

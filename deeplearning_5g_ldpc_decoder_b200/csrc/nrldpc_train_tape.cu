@@ -33,6 +33,8 @@
 #include <math.h>
 #include <stdint.h>
 
+#include <type_traits>
+
 #include "nrldpc_internal.h"
 
 namespace nrldpc {
@@ -56,14 +58,22 @@ __device__ __forceinline__ uint32_t tape_addr(const TrainTapeParams& p, int e, u
   return min(t, t - 4u * (uint32_t)p.Zc) + ed.x;
 }
 
-// D floats of lifted row zx in a row's slice of D Zc floats.  kVec (Zc a multiple
-// of 4, 16-byte aligned buffers): groups of four edges as one float4 per row,
-// then what is left as a float2 and a float, so a row moves D floats in a
-// quarter to a half of the instructions; otherwise one plane of Zc floats per
-// edge.  Either way a thread's words are its own.
-template <int D, bool kVec>
+// Word of edge j of lifted row zx in a row's slice of D Zc floats.  With Zc a
+// multiple of 4: groups of four edges as one float4 per row, then what is left as a
+// float2 and a float, so a row moves D floats in a quarter to a half of the
+// instructions; otherwise one plane of Zc floats per edge.  Either way a thread's
+// words are its own.
+template <int kAccess>
+__device__ __forceinline__ int tape_place(int D, int j, int zx, int Zc) {
+  const int quads = D / 4 * 4;
+  if (kAccess == kTapePlanes) return j * Zc + zx;
+  if (j < quads) return (j & ~3) * Zc + 4 * zx + (j & 3);
+  if ((D & 2) && j < quads + 2) return quads * Zc + 2 * zx + (j - quads);
+  return (D - 1) * Zc + zx;
+}
+template <int D, int kAccess>
 __device__ __forceinline__ void load_row(const float* slice, int zx, int Zc, float (&v)[D]) {
-  if constexpr (kVec) {
+  if constexpr (kAccess == kTapeGroups) {
 #pragma unroll
     for (int c = 0; c < D / 4; ++c) {
       const float4 q = __ldcs(reinterpret_cast<const float4*>(slice + 4 * c * Zc) + zx);
@@ -82,17 +92,17 @@ __device__ __forceinline__ void load_row(const float* slice, int zx, int Zc, flo
     if constexpr ((D & 1) != 0) v[D - 1] = __ldcs(rest + ((D & 2) ? 2 * Zc : 0) + zx);
   } else {
 #pragma unroll
-    for (int j = 0; j < D; ++j) v[j] = __ldcs(slice + j * Zc + zx);
+    for (int j = 0; j < D; ++j) v[j] = __ldcs(slice + tape_place<kAccess>(D, j, zx, Zc));
   }
 }
 // kStream: written once and read much later (the tape); otherwise kept near (the carry).
-template <int D, bool kVec, bool kStream>
+template <int D, int kAccess, bool kStream>
 __device__ __forceinline__ void store_row(float* slice, int zx, int Zc, const float (&v)[D]) {
   const auto put = [](auto* a, auto x) {
     if constexpr (kStream) __stcs(a, x);
     else *a = x;
   };
-  if constexpr (kVec) {
+  if constexpr (kAccess == kTapeGroups) {
 #pragma unroll
     for (int c = 0; c < D / 4; ++c)
       put(reinterpret_cast<float4*>(slice + 4 * c * Zc) + zx, make_float4(v[4 * c], v[4 * c + 1], v[4 * c + 2], v[4 * c + 3]));
@@ -102,7 +112,7 @@ __device__ __forceinline__ void store_row(float* slice, int zx, int Zc, const fl
     if constexpr ((D & 1) != 0) put(rest + ((D & 2) ? 2 * Zc : 0) + zx, v[D - 1]);
   } else {
 #pragma unroll
-    for (int j = 0; j < D; ++j) put(slice + j * Zc + zx, v[j]);
+    for (int j = 0; j < D; ++j) put(slice + tape_place<kAccess>(D, j, zx, Zc), v[j]);
   }
 }
 
@@ -114,30 +124,30 @@ struct TapeMsg {
   float n1, n2;
   uint32_t f;
 };
-template <int D, bool kVec>
+template <int D, int kAccess>
 __device__ __forceinline__ TapeMsg load_msg(const float* slice, int zx, int Zc) {
-  if constexpr (kVec && D >= 4) {
+  if constexpr (kAccess == kTapeGroups && D >= 4) {
     const float4 q = reinterpret_cast<const float4*>(slice)[zx];
     return TapeMsg{q.x, q.y, __float_as_uint(q.z)};
-  } else if constexpr (kVec) {
+  } else if constexpr (kAccess == kTapeGroups) {
     const float2 q = reinterpret_cast<const float2*>(slice)[zx];
     return TapeMsg{q.x, q.y, __float_as_uint(slice[2 * Zc + zx])};
   } else {
-    return TapeMsg{slice[zx], slice[Zc + zx], __float_as_uint(slice[2 * Zc + zx])};
+    const auto at = [&](int j) { return slice[tape_place<kAccess>(D, j, zx, Zc)]; };
+    return TapeMsg{at(0), at(1), __float_as_uint(at(2))};
   }
 }
-template <int D, bool kVec>
+template <int D, int kAccess>
 __device__ __forceinline__ void store_msg(float* slice, int zx, int Zc, const TapeMsg& m) {
-  if constexpr (kVec && D >= 4) {
+  if constexpr (kAccess == kTapeGroups && D >= 4) {
     reinterpret_cast<float4*>(slice)[zx] = make_float4(m.n1, m.n2, __uint_as_float(m.f), 0.0f);
-  } else {
-    if constexpr (kVec) {
-      reinterpret_cast<float2*>(slice)[zx] = make_float2(m.n1, m.n2);
-    } else {
-      slice[zx] = m.n1;
-      slice[Zc + zx] = m.n2;
-    }
+  } else if constexpr (kAccess == kTapeGroups) {
+    reinterpret_cast<float2*>(slice)[zx] = make_float2(m.n1, m.n2);
     slice[2 * Zc + zx] = __uint_as_float(m.f);
+  } else {
+    slice[tape_place<kAccess>(D, 0, zx, Zc)] = m.n1;
+    slice[tape_place<kAccess>(D, 1, zx, Zc)] = m.n2;
+    slice[tape_place<kAccess>(D, 2, zx, Zc)] = __uint_as_float(m.f);
   }
 }
 
@@ -148,12 +158,12 @@ __device__ __forceinline__ uint32_t sign_of(float x) { return __float_as_uint(__
 // Forward of one lifted check row: rel goes to the row's slice of this iteration's
 // tape, from where the old message is taken first (zero in the first iteration),
 // and the new message to the slice of the next iteration (none after the last).
-template <int D, bool kVec>
+template <int D, int kAccess>
 __device__ __forceinline__ void tape_row_fwd(const TrainTapeParams& p, char* __restrict__ lq, int zx, int e0, float alpha,
                                              float beta, bool first, float* slice, float* next) {
   const float clip = p.clip;
   TapeMsg m{0.0f, 0.0f, 0u};
-  if (!first) m = load_msg<D, kVec>(slice, zx, p.Zc);
+  if (!first) m = load_msg<D, kAccess>(slice, zx, p.Zc);
   const int ix = (int)(m.f >> 20);
   float rel[D];
   uint32_t addr[D];
@@ -173,7 +183,7 @@ __device__ __forceinline__ void tape_row_fwd(const TrainTapeParams& p, char* __r
     m1 = fminf(m1, a);
     idx = lt ? j : idx;
   }
-  store_row<D, kVec, true>(slice, zx, p.Zc, rel);
+  store_row<D, kAccess, true>(slice, zx, p.Zc, rel);
   const float s1 = __fmul_rn(alpha, fmaxf(__fsub_rn(m1, beta), 0.0f));
   const float s2 = __fmul_rn(alpha, fmaxf(__fsub_rn(m2, beta), 0.0f));
   uint32_t flips = 0u;
@@ -185,7 +195,7 @@ __device__ __forceinline__ void tape_row_fwd(const TrainTapeParams& p, char* __r
     const float v = __fadd_rn(rel[j], __uint_as_float(msg));
     *reinterpret_cast<float*>(lq + addr[j]) = fminf(fmaxf(v, -clip), clip);
   }
-  if (next) store_msg<D, kVec>(next, zx, p.Zc, TapeMsg{s1, s2, flips | (uint32_t)idx << 20});
+  if (next) store_msg<D, kAccess>(next, zx, p.Zc, TapeMsg{s1, s2, flips | (uint32_t)idx << 20});
 }
 
 // What a row's backward needs besides its loop over edges.
@@ -207,17 +217,11 @@ __device__ __forceinline__ BwdRow bwd_row(float m1, float m2, float alpha, float
 // Backward of one lifted check row with infinities or NaN among its inputs: the
 // loops of tape_row_bwd with every test of the model spelled out, over values
 // read again from memory.
-template <bool kVec>
+template <int kAccess>
 __device__ __noinline__ void tape_row_bwd_odd(const TrainTapeParams& p, char* glq, int zx, int e0, int D, float alpha,
                                               float beta, const float* slice, float* carry, bool last, bool first, float* ga,
                                               float* gb) {
-  const int Zc = p.Zc, quads = D / 4 * 4;
-  const auto at = [&](int j) {   // load_row's place of edge j
-    if (!kVec) return j * Zc + zx;
-    if (j < quads) return (j & ~3) * Zc + 4 * zx + (j & 3);
-    if ((D & 2) && j < quads + 2) return quads * Zc + 2 * zx + (j - quads);
-    return (D - 1) * Zc + zx;
-  };
+  const auto at = [&](int j) { return tape_place<kAccess>(D, j, zx, p.Zc); };
   bool neg = false;
   float m1 = INFINITY, m2 = INFINITY;
   int idx = -1, idx2 = -1;
@@ -261,19 +265,19 @@ __device__ __noinline__ void tape_row_bwd_odd(const TrainTapeParams& p, char* gl
 
 // Backward of one lifted check row (see the file comment).  kClip: LLRs are
 // clipped, so a sum outside the range passes no gradient.
-template <int D, bool kVec, bool kClip>
+template <int D, int kAccess, bool kClip>
 __device__ __forceinline__ void tape_row_bwd(const TrainTapeParams& p, char* __restrict__ glq, int zx, int e0, float alpha,
                                              float beta, const float* slice, float* carry, bool last, bool first, float* ga,
                                              float* gb) {
   const int Zc = p.Zc;
   float rel[D];
-  load_row<D, kVec>(slice, zx, Zc, rel);
+  load_row<D, kAccess>(slice, zx, Zc, rel);
   float cv[D];
   if (last) {
 #pragma unroll
     for (int j = 0; j < D; ++j) cv[j] = 0.0f;
   } else {
-    load_row<D, kVec>(carry, zx, Zc, cv);
+    load_row<D, kAccess>(carry, zx, Zc, cv);
   }
   uint32_t sg = 0u;
   float m1 = INFINITY, m2 = INFINITY, total = 0.0f;
@@ -292,7 +296,7 @@ __device__ __forceinline__ void tape_row_bwd(const TrainTapeParams& p, char* __r
   }
   const BwdRow b = bwd_row(m1, m2, alpha, beta);
   if (!(total + fabsf(b.s1) + fabsf(b.s2) < INFINITY)) {   // an infinity or a NaN in the row
-    tape_row_bwd_odd<kVec>(p, glq, zx, e0, D, alpha, beta, slice, carry, last, first, ga, gb);
+    tape_row_bwd_odd<kAccess>(p, glq, zx, e0, D, alpha, beta, slice, carry, last, first, ga, gb);
     return;
   }
   // From here every |rel| is finite: a clip test can only fail by the range, and
@@ -323,7 +327,7 @@ __device__ __forceinline__ void tape_row_bwd(const TrainTapeParams& p, char* __r
     *reinterpret_cast<float*>(glq + tape_addr(p, e0 + j, 4u * (uint32_t)zx)) = g_rel;
     cv[j] = -g_rel;
   }
-  if (!first) store_row<D, kVec, false>(carry, zx, Zc, cv);
+  if (!first) store_row<D, kAccess, false>(carry, zx, Zc, cv);
 }
 
 #define NRLDPC_TAPE_DISPATCH(deg, CALL) \
@@ -360,7 +364,7 @@ __device__ __forceinline__ void stage_rows(const TrainTapeParams& p, RowDesc* s_
                         p.alpha[t * p.R + r], p.beta[t * p.R + r]};
 }
 
-template <int kMaxD, bool kVec>
+template <int kMaxD, int kAccess>
 __global__ void __launch_bounds__(launch_threads(kMaxD), 2) tape_forward_kernel(const __grid_constant__ TrainTapeParams p) {
   extern __shared__ __align__(16) float s_lq[];
   __shared__ RowDesc s_rows[kMaxRows];
@@ -385,7 +389,7 @@ __global__ void __launch_bounds__(launch_threads(kMaxD), 2) tape_forward_kernel(
           const int e0 = d.e0, deg = d.deg;
           float* slice = tape + d.off;
           float* next = t + 1 < p.T ? tnext + d.off : nullptr;
-#define NRLDPC_FWD(D) tape_row_fwd<D, kVec>(p, reinterpret_cast<char*>(lq), zx, e0, d.alpha, d.beta, t == 0, slice, next)
+#define NRLDPC_FWD(D) tape_row_fwd<D, kAccess>(p, reinterpret_cast<char*>(lq), zx, e0, d.alpha, d.beta, t == 0, slice, next)
           NRLDPC_TAPE_DISPATCH(deg, NRLDPC_FWD)
 #undef NRLDPC_FWD
         }
@@ -412,7 +416,7 @@ __device__ __forceinline__ float warp_sum_pair(float a, float b) {
   return v;
 }
 
-template <int kMaxD, bool kVec, bool kClip>
+template <int kMaxD, int kAccess, bool kClip>
 __global__ void __launch_bounds__(launch_threads(kMaxD), 2) tape_backward_kernel(const __grid_constant__ TrainTapeParams p) {
   // dLQ of each code block; the iteration's alpha / beta gradients per row and
   // warp, [R][2][warps]; the CTA's sums of them, [T][R][2], added to the outputs
@@ -455,7 +459,7 @@ __global__ void __launch_bounds__(launch_threads(kMaxD), 2) tape_backward_kernel
           const float* slice = tape + d.off;
           float* cs = carry + d.off;
 #define NRLDPC_BWD(D) \
-  tape_row_bwd<D, kVec, kClip>(p, reinterpret_cast<char*>(glq), zx, e0, d.alpha, d.beta, slice, cs, t == p.T - 1, t == 0, &ga, &gb)
+  tape_row_bwd<D, kAccess, kClip>(p, reinterpret_cast<char*>(glq), zx, e0, d.alpha, d.beta, slice, cs, t == p.T - 1, t == 0, &ga, &gb)
           NRLDPC_TAPE_DISPATCH(deg, NRLDPC_BWD)
 #undef NRLDPC_BWD
         }
@@ -509,28 +513,31 @@ namespace {
 
 // Calls op(kernel) with the instance of a launch.
 template <typename Op>
-int with_tape_kernel(bool backward, bool bg2, bool vec, bool clipped, Op op) {
-  if (!backward) {
-    if (bg2) return vec ? op(tape_forward_kernel<10, true>) : op(tape_forward_kernel<10, false>);
-    return vec ? op(tape_forward_kernel<19, true>) : op(tape_forward_kernel<19, false>);
-  }
-  if (bg2) {
-    if (vec) return clipped ? op(tape_backward_kernel<10, true, true>) : op(tape_backward_kernel<10, true, false>);
-    return clipped ? op(tape_backward_kernel<10, false, true>) : op(tape_backward_kernel<10, false, false>);
-  }
-  if (vec) return clipped ? op(tape_backward_kernel<19, true, true>) : op(tape_backward_kernel<19, true, false>);
-  return clipped ? op(tape_backward_kernel<19, false, true>) : op(tape_backward_kernel<19, false, false>);
+int with_tape_kernel(bool backward, bool bg2, int access, bool clipped, Op op) {
+  const auto tape = [&](auto max_degree, auto mode) {
+    constexpr int d = decltype(max_degree)::value, m = decltype(mode)::value;
+    if (!backward) return op(tape_forward_kernel<d, m>);
+    return clipped ? op(tape_backward_kernel<d, m, true>) : op(tape_backward_kernel<d, m, false>);
+  };
+  const auto graph = [&](auto max_degree) {
+    switch (access) {
+      case kTapePlanes: return tape(max_degree, std::integral_constant<int, kTapePlanes>{});
+      case kTapeGroupWords: return tape(max_degree, std::integral_constant<int, kTapeGroupWords>{});
+      default: return tape(max_degree, std::integral_constant<int, kTapeGroups>{});
+    }
+  };
+  return bg2 ? graph(std::integral_constant<int, 10>{}) : graph(std::integral_constant<int, 19>{});
 }
 
 }  // namespace
 
 int launch_train_tape(const TrainTapeParams& p, bool backward, int grid, int block, int smem, void* stream) {
-  return with_tape_kernel(backward, p.R == NRLDPC_BG2_ROWS, p.vec != 0, isfinite(p.clip),
+  return with_tape_kernel(backward, p.R == NRLDPC_BG2_ROWS, p.access, isfinite(p.clip),
                           [&](auto k) { return launch_tape(k, p, grid, block, smem, stream); });
 }
 
 int occupancy_train_tape(const TrainTapeParams& p, bool backward, int block, int smem) {
-  return with_tape_kernel(backward, p.R == NRLDPC_BG2_ROWS, p.vec != 0, isfinite(p.clip),
+  return with_tape_kernel(backward, p.R == NRLDPC_BG2_ROWS, p.access, isfinite(p.clip),
                           [&](auto k) { return occupancy_tape_one(k, block, smem); });
 }
 

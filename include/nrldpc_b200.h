@@ -479,7 +479,8 @@ int32_t nrldpc_train_checkpoint_words(const ldpc_in_config_t *cfg, int32_t itera
  * (the extrinsic input of every edge and iteration, *floats of them, from
  * nrldpc_train_tape_floats) instead of the checkpoints: the backward recomputes
  * nothing.  d_tape is written by the forward and read by the backward; its
- * layout is the library's own.  Unlike the checkpoint form, the backward keeps
+ * layout is the library's own and does not depend on its address, so a copy of it
+ * serves as well (16-byte aligned tapes are faster).  Unlike the checkpoint form, the backward keeps
  * nothing in d_g_llr between iterations, which may be d_g_final. */
 int32_t nrldpc_train_tape_floats(const ldpc_in_config_t *cfg, int32_t iterations, int32_t batch, int64_t *floats);
 int32_t nrldpc_train_forward_tape(const float *d_llr, int32_t batch, const ldpc_in_config_t *cfg,
