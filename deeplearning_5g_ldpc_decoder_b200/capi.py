@@ -145,6 +145,8 @@ EXPORTED_SYMBOLS = (
     "nrldpc_train_tape_floats",
     "nrldpc_train_forward_tape",
     "nrldpc_train_backward_tape",
+    "nrldpc_train_message_floats",
+    "nrldpc_train_evaluate",
     "nrldpc_set_trained_weights",
     "nrldpc_set_degree_alpha",
     "nrldpc_mixed_plan_create",
@@ -238,6 +240,10 @@ def _declare(lib: ctypes.CDLL) -> None:
     lib.nrldpc_train_tape_floats.restype = i32
     lib.nrldpc_train_forward_tape.argtypes = [vp, i32, ctypes.POINTER(LdpcInConfig), i32, vp, vp, f32, vp, vp, vp, vp]
     lib.nrldpc_train_forward_tape.restype = i32
+    lib.nrldpc_train_message_floats.argtypes = [ctypes.POINTER(LdpcInConfig), i32, ctypes.POINTER(ctypes.c_int64)]
+    lib.nrldpc_train_message_floats.restype = i32
+    lib.nrldpc_train_evaluate.argtypes = [vp, i32, ctypes.POINTER(LdpcInConfig), i32, vp, vp, f32, vp, vp, vp, vp]
+    lib.nrldpc_train_evaluate.restype = i32
     lib.nrldpc_train_backward_tape.argtypes = [vp, i32, ctypes.POINTER(LdpcInConfig), i32, vp, vp, f32, i32, vp, vp,
                                                vp, vp, vp, vp, vp]
     lib.nrldpc_train_backward_tape.restype = i32

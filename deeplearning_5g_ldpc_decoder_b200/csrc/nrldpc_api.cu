@@ -746,7 +746,8 @@ int make_tape_params(const ldpc_in_config_t* cfg, int32_t T, int32_t batch, floa
 // the most code blocks on an SM (G > 1 pays where Zc leaves a warp partly
 // empty), and never more than spreading the batch over the SMs needs.  Sets
 // p->G, p->acc, *block and *smem; returns the CTAs per SM.
-int pick_tape_groups(DeviceState* st, TrainTapeParams* p, bool backward, int* block, int* smem) {
+int pick_tape_groups(DeviceState* st, TrainTapeParams* p, TapePass pass, int* block, int* smem) {
+  const bool backward = pass == kTapeBackward;
   p->acc = backward && 2 * p->T * p->R * 4 <= kTapeAccCap;
   const int acc = p->acc ? 2 * p->T * p->R * 4 : 0;
   const bool clipped = std::isfinite(p->clip);
@@ -758,10 +759,11 @@ int pick_tape_groups(DeviceState* st, TrainTapeParams* p, bool backward, int* bl
     const int bytes = G * p->n * 4 + (backward ? acc + 2 * p->R * (blk / 32) * 4 : 0);
     if (bytes > kTapeSmemCap) break;
     const uint64_t key = (backward ? 5ull : 4ull) << 56 |
-                         (uint64_t)((p->R == NRLDPC_BG2_ROWS) | p->access << 1 | (backward && clipped) << 3) << 48 |
+                         (uint64_t)((p->R == NRLDPC_BG2_ROWS) | p->access << 1 | (backward && clipped) << 3 |
+                                    (pass == kTapeEvaluate) << 4) << 48 |
                          (uint64_t)blk << 32 | (uint64_t)(uint32_t)bytes;
     const int occ =
-        cached_occupancy(st, key, [&] { return occupancy_train_tape(*p, backward, blk, bytes); });
+        cached_occupancy(st, key, [&] { return occupancy_train_tape(*p, pass, blk, bytes); });
     if (occ * G > best_cw) {
       best_cw = occ * G;
       best_g = G;
@@ -775,24 +777,24 @@ int pick_tape_groups(DeviceState* st, TrainTapeParams* p, bool backward, int* bl
   return best_occ;
 }
 
-// Shared end of the two tape entry points (the buffers are set in p).
-int launch_tape_kernel(TrainTapeParams* p, bool backward, void* stream) {
+// Shared end of the tape entry points (the buffers are set in p).
+int launch_tape_kernel(TrainTapeParams* p, TapePass pass, void* stream) {
   std::lock_guard<std::mutex> lock(g_mu);
   DeviceState* st = nullptr;
   if (device_state(&st) != 0) return NRLDPC_ERR_CUDA;
   p->access = p->Zc % 4 != 0 ? kTapePlanes : reinterpret_cast<uintptr_t>(p->tape) % 16 != 0 ? kTapeGroupWords : kTapeGroups;
   int block = 0, smem = 0;
-  const int occ = pick_tape_groups(st, p, backward, &block, &smem);
+  const int occ = pick_tape_groups(st, p, pass, &block, &smem);
   if (occ < 1) return NRLDPC_ERR_CUDA;
   const int items = (p->batch + p->G - 1) / p->G;
   const int grid = std::max(1, std::min(items, occ * st->num_sms));
-  if (backward) {
+  if (pass == kTapeBackward) {
     p->carry_per_cta = (int64_t)p->G * p->tape_words;
     Buffer& b = st->train_scratch[reinterpret_cast<cudaStream_t>(stream)];
     if (ensure(&b, sizeof(float) * (size_t)grid * (size_t)p->carry_per_cta)) return NRLDPC_ERR_CUDA;
     p->carry = static_cast<float*>(b.ptr);
   }
-  return launch_train_tape(*p, backward, grid, block, smem, stream) == 0 ? NRLDPC_OK : NRLDPC_ERR_CUDA;
+  return launch_train_tape(*p, pass, grid, block, smem, stream) == 0 ? NRLDPC_OK : NRLDPC_ERR_CUDA;
 }
 
 }  // namespace
@@ -1213,7 +1215,33 @@ int32_t nrldpc_train_forward_tape(const float* d_llr, int32_t batch, const ldpc_
   p.final_llr = d_final;
   p.iter_llr = d_iter;
   p.tape = d_tape;
-  return launch_tape_kernel(&p, false, stream);
+  return launch_tape_kernel(&p, kTapeForward, stream);
+}
+
+int32_t nrldpc_train_message_floats(const ldpc_in_config_t* cfg, int32_t batch, int64_t* floats) {
+  TrainTapeParams p;
+  const int rc = make_tape_params(cfg, 1, batch, 0.0f, &p);
+  if (rc != NRLDPC_OK) return rc;
+  if (floats) *floats = (int64_t)batch * p.R * kTapeMessageWords * p.Zc;
+  return NRLDPC_OK;
+}
+
+int32_t nrldpc_train_evaluate(const float* d_llr, int32_t batch, const ldpc_in_config_t* cfg, int32_t iterations,
+                              const float* d_alpha, const float* d_beta, float clip, float* d_final, float* d_iter,
+                              float* d_messages, void* stream) {
+  TrainTapeParams p;
+  const int rc = make_tape_params(cfg, iterations, batch, clip, &p);
+  if (rc != NRLDPC_OK) return rc;
+  if (batch == 0) return NRLDPC_OK;
+  if (!d_llr || !d_alpha || !d_beta || !d_final || !d_messages) return NRLDPC_ERR_ARG;
+  p.llr = d_llr;
+  p.alpha = d_alpha;
+  p.beta = d_beta;
+  p.final_llr = d_final;
+  p.iter_llr = d_iter;
+  p.tape = d_messages;
+  p.tape_words = (int64_t)p.R * kTapeMessageWords * p.Zc;
+  return launch_tape_kernel(&p, kTapeEvaluate, stream);
 }
 
 int32_t nrldpc_train_backward_tape(const float* d_llr, int32_t batch, const ldpc_in_config_t* cfg, int32_t iterations,
@@ -1235,7 +1263,7 @@ int32_t nrldpc_train_backward_tape(const float* d_llr, int32_t batch, const ldpc
   p.g_llr = d_g_llr;
   p.g_alpha = d_g_alpha;
   p.g_beta = d_g_beta;
-  return launch_tape_kernel(&p, true, stream);
+  return launch_tape_kernel(&p, kTapeBackward, stream);
 }
 
 }  // extern "C"

@@ -296,6 +296,8 @@ struct TrainParams {
 // The order of a row's words in the tape depends on Zc alone: a plane per edge, or for a
 // multiple of 4 groups of four edges (word by word where the tape is not 16-byte aligned).
 enum TapeAccess { kTapePlanes = 0, kTapeGroupWords = 1, kTapeGroups = 2 };
+enum TapePass { kTapeForward = 0, kTapeBackward = 1, kTapeEvaluate = 2 };
+constexpr int kTapeMessageWords = 4;   // evaluation: floats per lifted row for its message
 struct TrainTapeParams {
   int32_t Zc, R, n, G, nnz, T, batch, detach;
   int32_t acc;                // backward: the CTA sums its alpha / beta gradients in shared memory
@@ -307,7 +309,7 @@ struct TrainTapeParams {
   float* final_llr;           // [batch][n]
   float* iter_llr;            // [T][batch][n] or null
   float* tape;                // [T][batch][nnz Zc]: rel of every edge, a slice of degree * Zc per row
-  int64_t tape_words;         // nnz Zc
+  int64_t tape_words;         // floats per code block and iteration: nnz Zc (evaluation: R kTapeMessageWords Zc)
   const float* g_final;       // [batch][n] or null
   const float* g_iter;        // [T][batch][n] or null
   float* g_llr;               // [batch][n]
@@ -324,8 +326,8 @@ int launch_encode(const EncodeParams& p, int num_sms, void* stream);
 int launch_train_forward(const TrainParams& p, bool f64, int grid, int block, int smem, void* stream);
 int launch_train_backward(const TrainParams& p, bool f64, int grid, int block, int smem, void* stream);
 int occupancy_train(bool backward, bool f64, bool bg2, int block, int smem, bool alias = false);
-int launch_train_tape(const TrainTapeParams& p, bool backward, int grid, int block, int smem, void* stream);
-int occupancy_train_tape(const TrainTapeParams& p, bool backward, int block, int smem);
+int launch_train_tape(const TrainTapeParams& p, TapePass pass, int grid, int block, int smem, void* stream);
+int occupancy_train_tape(const TrainTapeParams& p, TapePass pass, int block, int smem);
 // Mixed-size kernel classes: 0 = 384 threads per CTA (all of them active at
 // most), 1 = 256 threads with at most 240 active, three CTAs per SM.  A graph
 // of a class holds G = floor(capacity / Zc) lane pairs per CTA.

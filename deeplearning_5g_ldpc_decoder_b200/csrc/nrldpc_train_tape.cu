@@ -158,7 +158,8 @@ __device__ __forceinline__ uint32_t sign_of(float x) { return __float_as_uint(__
 // Forward of one lifted check row: rel goes to the row's slice of this iteration's
 // tape, from where the old message is taken first (zero in the first iteration),
 // and the new message to the slice of the next iteration (none after the last).
-template <int D, int kAccess>
+// Without kKeep (evaluation) there is no tape, only the message's slice.
+template <int D, int kAccess, bool kKeep>
 __device__ __forceinline__ void tape_row_fwd(const TrainTapeParams& p, char* __restrict__ lq, int zx, int e0, float alpha,
                                              float beta, bool first, float* slice, float* next) {
   const float clip = p.clip;
@@ -183,7 +184,7 @@ __device__ __forceinline__ void tape_row_fwd(const TrainTapeParams& p, char* __r
     m1 = fminf(m1, a);
     idx = lt ? j : idx;
   }
-  store_row<D, kAccess, true>(slice, zx, p.Zc, rel);
+  if constexpr (kKeep) store_row<D, kAccess, true>(slice, zx, p.Zc, rel);
   const float s1 = __fmul_rn(alpha, fmaxf(__fsub_rn(m1, beta), 0.0f));
   const float s2 = __fmul_rn(alpha, fmaxf(__fsub_rn(m2, beta), 0.0f));
   uint32_t flips = 0u;
@@ -358,13 +359,17 @@ struct __align__(16) RowDesc {
   uint32_t off;   // floats before the row's slice
   float alpha, beta;
 };
+template <bool kKeep>
 __device__ __forceinline__ void stage_rows(const TrainTapeParams& p, RowDesc* s_rows, int t) {
   for (int r = threadIdx.x; r < p.R; r += blockDim.x)
-    s_rows[r] = RowDesc{p.row_off[r], (uint16_t)(p.row_off[r + 1] - p.row_off[r]), (uint32_t)p.row_off[r] * (uint32_t)p.Zc,
-                        p.alpha[t * p.R + r], p.beta[t * p.R + r]};
+    s_rows[r] = RowDesc{p.row_off[r], (uint16_t)(p.row_off[r + 1] - p.row_off[r]),
+                        (uint32_t)(kKeep ? p.row_off[r] : kTapeMessageWords * r) * (uint32_t)p.Zc, p.alpha[t * p.R + r],
+                        p.beta[t * p.R + r]};
 }
 
-template <int kMaxD, int kAccess>
+// kKeep: the tape is kept for a backward.  Otherwise (evaluation) the rows' messages
+// lie in slices of kTapeMessageWords Zc floats, the same ones in every iteration.
+template <int kMaxD, int kAccess, bool kKeep>
 __global__ void __launch_bounds__(launch_threads(kMaxD), 2) tape_forward_kernel(const __grid_constant__ TrainTapeParams p) {
   extern __shared__ __align__(16) float s_lq[];
   __shared__ RowDesc s_rows[kMaxRows];
@@ -379,17 +384,17 @@ __global__ void __launch_bounds__(launch_threads(kMaxD), 2) tape_forward_kernel(
     if (valid)
       for (int i = zx; i < p.n; i += p.Zc) lq[i] = fminf(fmaxf(p.llr[(size_t)cw * p.n + i], -clip), clip);
     for (int t = 0; t < p.T; ++t) {
-      stage_rows(p, s_rows, t);   // the last row's barrier lies between its reads and this
+      stage_rows<kKeep>(p, s_rows, t);   // the last row's barrier lies between its reads and this
       __syncthreads();
-      float* tape = p.tape + ((size_t)t * p.batch + (valid ? cw : 0)) * p.tape_words;
-      float* tnext = tape + (size_t)p.batch * p.tape_words;
+      float* tape = p.tape + ((kKeep ? (size_t)t * p.batch : 0) + (valid ? cw : 0)) * p.tape_words;
+      float* tnext = kKeep ? tape + (size_t)p.batch * p.tape_words : tape;
       for (int row = 0; row < p.R; ++row) {
         if (valid) {
           const RowDesc d = s_rows[row];
           const int e0 = d.e0, deg = d.deg;
           float* slice = tape + d.off;
           float* next = t + 1 < p.T ? tnext + d.off : nullptr;
-#define NRLDPC_FWD(D) tape_row_fwd<D, kAccess>(p, reinterpret_cast<char*>(lq), zx, e0, d.alpha, d.beta, t == 0, slice, next)
+#define NRLDPC_FWD(D) tape_row_fwd<D, kAccess, kKeep>(p, reinterpret_cast<char*>(lq), zx, e0, d.alpha, d.beta, t == 0, slice, next)
           NRLDPC_TAPE_DISPATCH(deg, NRLDPC_FWD)
 #undef NRLDPC_FWD
         }
@@ -443,7 +448,7 @@ __global__ void __launch_bounds__(launch_threads(kMaxD), 2) tape_backward_kernel
       // own indices i = zx + k Zc, like the loads above; rows need all of them
       if (valid && p.g_iter)
         for (int i = zx; i < p.n; i += p.Zc) glq[i] += p.g_iter[((size_t)t * p.batch + cw) * p.n + i];
-      stage_rows(p, s_rows, t);
+      stage_rows<true>(p, s_rows, t);
       __syncthreads();   // also: the sums over s_part below have been read
       const float* tape = p.tape + ((size_t)t * p.batch + (valid ? cw : 0)) * p.tape_words;
       for (int row = p.R - 1; row >= 0; --row) {
@@ -513,10 +518,11 @@ namespace {
 
 // Calls op(kernel) with the instance of a launch.
 template <typename Op>
-int with_tape_kernel(bool backward, bool bg2, int access, bool clipped, Op op) {
+int with_tape_kernel(TapePass pass, bool bg2, int access, bool clipped, Op op) {
   const auto tape = [&](auto max_degree, auto mode) {
     constexpr int d = decltype(max_degree)::value, m = decltype(mode)::value;
-    if (!backward) return op(tape_forward_kernel<d, m>);
+    if (pass == kTapeEvaluate) return op(tape_forward_kernel<d, m, false>);
+    if (pass == kTapeForward) return op(tape_forward_kernel<d, m, true>);
     return clipped ? op(tape_backward_kernel<d, m, true>) : op(tape_backward_kernel<d, m, false>);
   };
   const auto graph = [&](auto max_degree) {
@@ -531,13 +537,13 @@ int with_tape_kernel(bool backward, bool bg2, int access, bool clipped, Op op) {
 
 }  // namespace
 
-int launch_train_tape(const TrainTapeParams& p, bool backward, int grid, int block, int smem, void* stream) {
-  return with_tape_kernel(backward, p.R == NRLDPC_BG2_ROWS, p.access, isfinite(p.clip),
+int launch_train_tape(const TrainTapeParams& p, TapePass pass, int grid, int block, int smem, void* stream) {
+  return with_tape_kernel(pass, p.R == NRLDPC_BG2_ROWS, p.access, isfinite(p.clip),
                           [&](auto k) { return launch_tape(k, p, grid, block, smem, stream); });
 }
 
-int occupancy_train_tape(const TrainTapeParams& p, bool backward, int block, int smem) {
-  return with_tape_kernel(backward, p.R == NRLDPC_BG2_ROWS, p.access, isfinite(p.clip),
+int occupancy_train_tape(const TrainTapeParams& p, TapePass pass, int block, int smem) {
+  return with_tape_kernel(pass, p.R == NRLDPC_BG2_ROWS, p.access, isfinite(p.clip),
                           [&](auto k) { return occupancy_tape_one(k, block, smem); });
 }
 

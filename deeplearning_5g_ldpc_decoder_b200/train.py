@@ -9,7 +9,8 @@ LLR clipping and detached check-update inputs, and the same forward outputs.
 The decoder itself runs in two hand-written CUDA kernels wrapped in
 ``MinSumUnrolled`` (a ``torch.autograd.Function``): the float32 forward keeps a
 tape of every edge's extrinsic input, from which the backward back-propagates
-without recomputing anything; in float64 the forward keeps one checkpoint of the
+without recomputing anything (and without a backward to come only one iteration's
+messages); in float64 the forward keeps one checkpoint of the
 decoder state per iteration and the backward recomputes each iteration from it.
 
 ``export_int16_tables`` turns learned alpha / beta into the int16 tables of the
@@ -60,13 +61,30 @@ def tape_size(cfg: capi.LdpcInConfig, T: int, batch: int) -> int:
     return int(n.value)
 
 
+def message_size(cfg: capi.LdpcInConfig, batch: int) -> int:
+    """Floats of one iteration's messages, all that the float32 forward keeps without a backward."""
+    lib = capi.load_library()
+    n = ctypes.c_int64(0)
+    rc = lib.nrldpc_train_message_floats(ctypes.byref(cfg), batch, ctypes.byref(n))
+    if rc != 0:
+        raise ValueError(f"configuration not supported by the training kernels (float32): {rc}")
+    return int(n.value)
+
+
+def _checkpoints(cfg: capi.LdpcInConfig, T: int, batch: int, dt, dev) -> Tuple[torch.Tensor, torch.Tensor]:
+    lq, msg = checkpoint_sizes(cfg, T, batch, dt == torch.float64)
+    return torch.empty(lq, dtype=dt, device=dev), torch.empty(max(msg, 2), dtype=torch.int32, device=dev)
+
+
 class MinSumUnrolled(torch.autograd.Function):
     """(llr [batch, n], alpha [T, R], beta [T, R]) -> (final [batch, n], per-iteration [T, batch, n]).
 
-    Runs in the dtype of ``llr``: float32 (training) or float64 (gradient checks)."""
+    Runs in the dtype of ``llr``: float32 (training) or float64 (gradient checks).  ``keep``: a backward may follow;
+    without it the float32 forward keeps one iteration's messages instead of the tape.  Where the tape does not fit the
+    device and checkpoints are smaller (BG1: 252 words per lifted column and iteration instead of 316), it keeps those."""
 
     @staticmethod
-    def forward(ctx, llr, alpha_tab, beta_tab, config, clip, detach, want_iters):
+    def forward(ctx, llr, alpha_tab, beta_tab, config, clip, detach, want_iters, keep=True):
         lib = capi.load_library()
         cfg = _cfg(config)
         f64 = llr.dtype == torch.float64
@@ -82,20 +100,25 @@ class MinSumUnrolled(torch.autograd.Function):
         final = torch.empty_like(llr)
         iters = torch.empty((T, batch, n), dtype=dt, device=dev) if want_iters else None
         stream = ctypes.c_void_p(torch.cuda.current_stream(dev).cuda_stream)
+        clip_arg = (ctypes.c_double if f64 else ctypes.c_float)(clip or INF_CLIP)
         if f64:
-            lq_elems, msg_words = checkpoint_sizes(cfg, T, batch, True)
-            kept = (torch.empty(lq_elems, dtype=dt, device=dev),
-                    torch.empty(max(msg_words, 2), dtype=torch.int32, device=dev))
-            fn, clip_arg = lib.nrldpc_train_forward_f64, ctypes.c_double(clip or INF_CLIP)
+            kept, fn = _checkpoints(cfg, T, batch, dt, dev), lib.nrldpc_train_forward_f64
+        elif not keep:
+            kept, fn = (torch.empty(message_size(cfg, batch), dtype=dt, device=dev),), lib.nrldpc_train_evaluate
         else:
-            kept = (torch.empty(tape_size(cfg, T, batch), dtype=dt, device=dev),)
-            fn, clip_arg = lib.nrldpc_train_forward_tape, ctypes.c_float(clip or INF_CLIP)
+            try:
+                kept, fn = (torch.empty(tape_size(cfg, T, batch), dtype=dt, device=dev),), lib.nrldpc_train_forward_tape
+            except torch.cuda.OutOfMemoryError:
+                if sum(checkpoint_sizes(cfg, T, batch, False)) >= tape_size(cfg, T, batch):
+                    raise
+                kept, fn = _checkpoints(cfg, T, batch, dt, dev), lib.nrldpc_train_forward
         with torch.cuda.device(dev):
             rc = fn(_vp(llr), batch, ctypes.byref(cfg), T, _vp(alpha_tab), _vp(beta_tab), clip_arg, _vp(final),
                     _vp(iters), *[_vp(k) for k in kept], stream)
         if rc != 0:
             raise RuntimeError(f"nrldpc_train_forward failed: {rc}")
-        ctx.save_for_backward(llr, alpha_tab, beta_tab, *kept)
+        if keep or f64:
+            ctx.save_for_backward(llr, alpha_tab, beta_tab, *kept)
         ctx.cfg = (cfg.bgn, cfg.A, cfg.crctype, cfg.E, cfg.rv, cfg.Qm, cfg.HARQ_on)
         ctx.clip = clip
         ctx.detach = detach
@@ -120,14 +143,15 @@ class MinSumUnrolled(torch.autograd.Function):
         gi = (g_iters.contiguous().to(llr.dtype)
               if (g_iters is not None and g_iters.numel() == T * batch * n) else None)
         stream = ctypes.c_void_p(torch.cuda.current_stream(dev).cuda_stream)
-        fn = lib.nrldpc_train_backward_f64 if f64 else lib.nrldpc_train_backward_tape
+        fn = (lib.nrldpc_train_backward_f64 if f64 else
+              lib.nrldpc_train_backward_tape if len(kept) == 1 else lib.nrldpc_train_backward)
         clip_arg = (ctypes.c_double if f64 else ctypes.c_float)(ctx.clip or INF_CLIP)
         with torch.cuda.device(dev):
             rc = fn(_vp(llr), batch, ctypes.byref(cfg), T, _vp(alpha_tab), _vp(beta_tab), clip_arg, int(ctx.detach),
                     *[_vp(k) for k in kept], _vp(gf), _vp(gi), _vp(g_llr), _vp(g_alpha), _vp(g_beta), stream)
         if rc != 0:
             raise RuntimeError(f"nrldpc_train_backward failed: {rc}")
-        return g_llr, g_alpha, g_beta, None, None, None, None
+        return g_llr, g_alpha, g_beta, None, None, None, None, None
 
 
 def _inverse_bounded_sigmoid(values, lo: float, hi: float) -> torch.Tensor:
@@ -243,8 +267,10 @@ class NeuralLayeredMinSumDecoder(nn.Module):
             llr = llr.unsqueeze(0)
         if llr.dim() != 2 or llr.shape[1] != self.n:
             raise ValueError(f"llr must have shape [batch, {self.n}]")
-        final, iters = MinSumUnrolled.apply(llr, self.alpha_table(), self.beta(), self.in_config, self.clip_llr,
-                                            self.detach_check_update_inputs, bool(return_iteration_llrs))
+        alpha, beta = self.alpha_table(), self.beta()
+        keep = torch.is_grad_enabled() and any(t.requires_grad for t in (llr, alpha, beta))
+        final, iters = MinSumUnrolled.apply(llr, alpha, beta, self.in_config, self.clip_llr,
+                                            self.detach_check_update_inputs, bool(return_iteration_llrs), keep)
         bits = (final < 0).to(torch.int64)
         iteration_llrs = list(iters.unbind(0)) if return_iteration_llrs else None
         if single:

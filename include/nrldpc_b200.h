@@ -486,6 +486,12 @@ int32_t nrldpc_train_tape_floats(const ldpc_in_config_t *cfg, int32_t iterations
 int32_t nrldpc_train_forward_tape(const float *d_llr, int32_t batch, const ldpc_in_config_t *cfg,
                                   int32_t iterations, const float *d_alpha, const float *d_beta, float clip,
                                   float *d_final, float *d_iter, float *d_tape, void *stream);
+/* The same values without a backward: only one iteration's messages are kept, in
+ * d_messages (*floats of them, from nrldpc_train_message_floats). */
+int32_t nrldpc_train_message_floats(const ldpc_in_config_t *cfg, int32_t batch, int64_t *floats);
+int32_t nrldpc_train_evaluate(const float *d_llr, int32_t batch, const ldpc_in_config_t *cfg,
+                              int32_t iterations, const float *d_alpha, const float *d_beta, float clip,
+                              float *d_final, float *d_iter, float *d_messages, void *stream);
 int32_t nrldpc_train_backward_tape(const float *d_llr, int32_t batch, const ldpc_in_config_t *cfg,
                                    int32_t iterations, const float *d_alpha, const float *d_beta, float clip,
                                    int32_t detach, const float *d_tape, const float *d_g_final,

@@ -1,5 +1,6 @@
-"""The tape of the float32 training kernels: its layout does not depend on where it lies, and rows with infinities or
-sums beyond float32 have the checkpoint form's values and gradients."""
+"""The tape of the float32 training kernels: its layout does not depend on where it lies, rows with infinities or sums
+beyond float32 have the checkpoint form's values and gradients, evaluation keeps no tape, and a batch whose tape does not
+fit the device trains with checkpoints."""
 
 import ctypes
 
@@ -7,6 +8,7 @@ import pytest
 import torch
 
 from deeplearning_5g_ldpc_decoder_b200 import capi
+from deeplearning_5g_ldpc_decoder_b200.train import MinSumUnrolled, NeuralLayeredMinSumDecoder
 from test_gpu_train import _checkpoint_form
 
 pytestmark = pytest.mark.gpu
@@ -86,3 +88,55 @@ def test_infinite_and_huge_inputs(cuda, lib, cfg, clip, detach):
             assert (g[i][ok[i]] - w[i][ok[i]]).abs().max().item() <= 1e-4 * scale + 1e-12, i
     for k in (3, 4):
         assert torch.equal(got[k].isnan(), want[k].isnan()), k
+
+
+@pytest.mark.parametrize("cfg,T,batch,clip", [((2, 488, 1, 1920, 0, 2, 0), 6, 700, None), ((1, 600, 1, 1500, 0, 2, 0), 4, 33, 9.0),
+                                              ((2, 40, 1, 200, 0, 2, 0), 3, 5, None), ((1, 2440, 1, 7392, 0, 2, 0), 5, 400, 12.0)])
+def test_evaluation_keeps_no_tape(cuda, cfg, T, batch, clip):
+    """Under no_grad, and where nothing needs a gradient: the same values, in a fraction of the tape's memory."""
+    x = _inputs(cfg, T, batch, 3)[0]
+    model = NeuralLayeredMinSumDecoder(cfg, num_iterations=T, alpha_mode="checkpoint", init_beta=0.02, clip_llr=clip).cuda()
+    bits, final, its = model(x, return_llr=True, return_iteration_llrs=True)
+    floats = ctypes.c_int64(0)
+    assert capi.load_library().nrldpc_train_tape_floats(ctypes.byref(capi.make_in_config(*cfg)), T, batch,
+                                                        ctypes.byref(floats)) == 0
+    with torch.no_grad():
+        got = model(x, return_llr=True, return_iteration_llrs=True)
+    assert torch.equal(got[0], bits) and torch.equal(got[1], final.detach())
+    assert all(torch.equal(a, b.detach()) for a, b in zip(got[2], its))
+    model.requires_grad_(False)
+    del bits, its, got
+    torch.cuda.synchronize()
+    before = torch.cuda.memory_allocated()
+    torch.cuda.reset_peak_memory_stats()
+    last = model(x, return_llr=True)[1]
+    assert torch.equal(last, final.detach()) and last.grad_fn is None
+    outputs = 4 * x.nelement() * 4
+    assert torch.cuda.max_memory_allocated() - before < 4 * floats.value // 2 + outputs
+
+
+def test_checkpoints_where_the_tape_does_not_fit(cuda):
+    """A BG1 batch between the checkpoints' size and the tape's trains all the same, with the same values and gradients."""
+    cfg, T, batch = (1, 2440, 1, 7392, 0, 2, 0), 10, 400
+    x, a, b, gf, gi = _inputs(cfg, T, batch, 5)
+
+    def step():
+        leaves = [t.clone().requires_grad_(True) for t in (x, a, b)]
+        final, _ = MinSumUnrolled.apply(*leaves, cfg, None, False, False)
+        final.backward(gf)
+        return (final.detach(), *[t.grad for t in leaves])
+
+    want = step()
+    torch.cuda.empty_cache()
+    total = torch.cuda.get_device_properties(0).total_memory
+    tape = 4 * T * batch * 316 * 112                       # 566 MB; checkpoints take 452 MB
+    limit = torch.cuda.memory_reserved() + int(0.92 * tape)
+    torch.cuda.set_per_process_memory_fraction(limit / total)
+    try:
+        got = step()
+    finally:
+        torch.cuda.set_per_process_memory_fraction(1.0)
+        torch.cuda.empty_cache()
+    assert torch.equal(got[0], want[0])
+    for g, w in zip(got[1:], want[1:]):
+        assert (g - w).abs().max().item() <= 1e-4 * w.abs().max().item()
