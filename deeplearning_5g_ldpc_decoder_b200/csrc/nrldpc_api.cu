@@ -337,17 +337,20 @@ int make_plan(const CodeParams& cp, const ldpc_decoder_cfg_t& dc, int num_cw, bo
   plan->grid = std::min(p.num_items, occ * st->num_sms);
   if (plan->grid < 1) plan->grid = 1;
   // Scratch layout per CTA, layer by layer.  (The fixed-point kernel addresses its
-  // planes with a compile-time stride.)  Float min-sum is wide for batches of more than
-  // a wave, where other CTAs hide the messages that a row loads itself, unless a second
+  // planes with a compile-time stride.)  Float min-sum is wide where an SM holds 512
+  // threads or more, which hide the messages that a row loads itself, unless a second
   // wave would be the last and nearly full: then a CTA that runs ahead of the other on
   // its SM, as CTAs of the wide form do, takes a third item.  8 iterations, us with rows
-  // of up to three / five edges uncompressed: 16 blocks BG2 Zc 64 127 / 146, 444 of BG1
-  // Zc 384 (one wave) 684 / 682; 777 of BG1 Zc 208 (1.75 waves) 864 / 830, 1184 of BG1
-  // Zc 144 (2.7) 874 / 849, 4096 of BG1 Zc 384 6.29 / 6.30 ms; 9000 of BG1 Zc 24 (1.9)
-  // 959 / 1143, 592 of BG1 Zc 384 (2) 949 / 1131, 888 of BG2 Zc 256 (2) 619 / 717.
-  if (!fixed)
-    plan->wide = algo == 4 && p.num_items > plan->grid &&
+  // of up to three / five edges uncompressed: 16 blocks BG2 Zc 64 (64 threads) 127 / 146,
+  // 592 (256) 168 / 178, 1136 (768) 357 / 342; 296 of BG2 Zc 104 (208) 177 / 187; 200 of
+  // BG2 Zc 256 (512) 266 / 258; 296 of BG2 Zc 384 (768) 359 / 345; 777 of BG1 Zc 208
+  // (1.75 waves) 864 / 830; 9000 of BG1 Zc 24 (1.9) 959 / 1143, 592 of BG1 Zc 384 (2)
+  // 949 / 1131, 888 of BG2 Zc 256 (2) 619 / 717.
+  if (!fixed) {
+    const int per_sm = (plan->grid + st->num_sms - 1) / st->num_sms;
+    plan->wide = algo == 4 && per_sm * plan->block >= 512 &&
                  (8 * (int64_t)p.num_items <= 15 * (int64_t)plan->grid || p.num_items > 2 * plan->grid);
+  }
   if (fixed) {
     fixed_row_layout(g, plan->clip, plan->wide, p.lr_off);
   } else {

@@ -178,7 +178,7 @@ def test_every_lifting_size_on_the_pair_kernel(oracle, cuda, lib, bgn):
 @pytest.mark.parametrize("row", [[4, 5, 22936, 0, 1280, 32767, -32767], [4, 3, 22936, 0, 1280, -100, 100]])
 @pytest.mark.parametrize("bgn,A,E,Qm", [(1, 8, 96, 2), (2, 488, 1920, 2), (1, 4352, 8754, 6)])
 def test_both_row_forms_of_float_min_sum(oracle, cuda, row, bgn, A, E, Qm):
-    """Rows of up to five edges uncompressed in batches of more than a wave, of up to three in smaller ones."""
+    """Rows of up to five edges uncompressed where an SM holds many threads, of up to three in smaller batches."""
     cfg = (bgn, A, 1, E, 0, Qm, 0)
     host = noisy_blocks(oracle, cfg, A)
     n = 1
