@@ -517,8 +517,8 @@ def run_gpu(args, rank, world, local_rank):
                                             if traffic_cw else "no ncu capture of this decoder's launch"),
                          "algorithmic_bytes_per_launch": alg, "kernel_ms": round(mean_launch_ms, 4),
                          "note": ("the algorithmic bytes count every belief and message access as HBM traffic; "
-                                  "this decoder keeps beliefs in shared memory and messages in an L2-resident "
-                                  "compressed form, so it runs above that model, and what limits it is the "
+                                  "this decoder keeps beliefs in shared memory and messages mostly in L2, "
+                                  "so it runs above that model, and what limits it is the "
                                   "integer ALU pipe (profile constant alu_pipe_busy)") if args.algo == 1 else None,
                          "alu_pipe_busy": _profile_constant("alu_pipe_busy") if args.algo == 1 else None,
                          "io_bytes_per_launch": float((2 * E + (B_BITS + 7) // 8 + 4) * n_cw)},

@@ -22,7 +22,7 @@
 //  * 32 symbols are interleaved at once: an 8 x 8 bit transpose per 8 symbols
 //    gives one byte per symbol, and Qm < 8 packs the bytes' top Qm bits.
 // The kernel is bound by instruction issue (about 8000 warp instructions for a
-// BG1 Zc=384 block, 60 % of the issue slots; leaving out the CRC saves 15 % of the
+// BG1 Zc=384 block, 64 % of the issue slots; leaving out the CRC saves 15 % of the
 // time, the interleave 16 %, the extension rows 11 %) and, for one block, by the
 // latency of its eight phases.  4096 blocks of BG1 Zc=384, E=25344, Qm=8: 783 us with
 // one byte per bit and a gather per output bit, 47 us in this form.

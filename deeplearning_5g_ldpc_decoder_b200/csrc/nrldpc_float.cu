@@ -52,7 +52,7 @@ struct FloatMsg {
 // One row, operation for operation as the reference.  A belief of -0.0 counts as
 // positive there (`< 0`), so signs are taken from v + 0.0f, whose sign bit is set
 // exactly where v < 0; then parity, flip and the sign of a message are bit
-// operations on sign bits.  The ALU pipe bounds the kernel (76 % busy, 25 of 45
+// operations on sign bits.  The ALU pipe bounds the kernel (76 % busy, 21 of 40
 // instructions per edge).  8 iterations of 4096 blocks BG1 Zc=384: 6.91 -> 6.29 ms,
 // 777 blocks BG1 Zc=208 957 -> 877 us (and 6.12 ms and 835 us with short rows in
 // the form below and the second minimum by a min and a max), against bit tests and compares on values
@@ -203,7 +203,7 @@ __device__ __forceinline__ float bp_message(float prod) {
 // registers; a 19-edge row has no room for them, parks rel in LQ's own word (a
 // row's edges are distinct words that no other thread touches during the layer)
 // and computes the addresses twice.  The products keep the reference's order.
-// Issue slots bound it (73 % busy; 83 instructions per edge, most of them in
+// Issue slots bound it (80 % busy; 83 instructions per edge, most of them in
 // tanhf and atanhf).  10 iterations of 1024 blocks BG1 Zc=384: 3.78 -> 2.31 ms
 // against loads one edge at a time behind a branch on a zero input (107
 // instructions per edge, 61 % busy, waiting on the loads).

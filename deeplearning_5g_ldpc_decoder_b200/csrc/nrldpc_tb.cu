@@ -79,7 +79,7 @@ __device__ __forceinline__ int block_scan(int v, int* s_warp) {
 // One CTA: the whole batch's code-block list needs one scan.  Bound by latency, so
 // no step is serial over blocks or graphs: a thread per transport block counts,
 // a thread per code block (found by a binary search of the scan) writes its
-// descriptor, a thread per graph its queue.  32 transport blocks, 155 code blocks:
+// descriptor, a thread per graph its queue.  32 transport blocks, 109 code blocks:
 // 25.7 us with a thread per transport block writing all its code blocks and one
 // thread walking the graphs, 8.5 us in this form.
 __global__ void __launch_bounds__(kSegThreads) tb_segment_kernel(const nrldpc_tb_t* __restrict__ tbs, int n,
@@ -234,7 +234,7 @@ struct FinishParams {
 // after the block).  Remainders: a warp per half code block, four positions per
 // lane and step with 16-byte table loads.  The
 // shift is a power of X = x^(bits per block), by squaring, a warp per code block.
-// Bound by latency.  32 transport blocks of up to 24 code blocks: 77 us with a bit
+// Bound by latency.  32 transport blocks of up to 21 code blocks: 77 us with a bit
 // per lane and step, and the powers of x multiplied bit by bit by one lane; 17.3 us
 // in this form.
 constexpr int kFinishThreads = 512;
