@@ -19,9 +19,9 @@
 //    Circulant shifts are resolved as shared-memory word addresses
 //    col*Zc + (V_ij mod Zc + zx) mod Zc.
 //  * Check-to-variable messages live in a per-CTA global scratch that stays
-//    resident in L2: one word per edge for both code blocks of a pair in rows of
-//    up to ten messages, and compressed (two scaled minima, the position of the
-//    minimum, one sign bit per edge: 16 or 20 bytes) in longer rows.
+//    resident in L2: one word per edge for both code blocks of a pair in short rows
+//    (direct_row), and compressed (two scaled minima, the position of the minimum,
+//    one sign bit per edge: 16 or 20 bytes) in longer rows.
 //  * The grid is persistent.  With a block cursor (DecodeParams::cursor: the
 //    queue head and a count of finished CTAs, both zero at launch and rewound
 //    by the last CTA to finish) every int16 half lane takes code blocks from one

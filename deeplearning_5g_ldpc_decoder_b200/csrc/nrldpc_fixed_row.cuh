@@ -112,8 +112,8 @@ __device__ __forceinline__ uint32_t cond_neg16x2(uint32_t v, uint32_t m) { retur
 // so `fresh` (0xFFFF per half that starts its first iteration) clears one
 // block's old message without touching the other's.
 //
-// With the open maximum, rows 4 and up (kPar) end in the edge to a parity column of their own, with
-// shift 0, which no other row touches.  Its belief only ever is rel + message of
+// With parity words, rows 4 and up (kPar) end in the edge to a parity column of
+// their own, with shift 0, which no other row touches.  Its belief only ever is rel + message of
 // this row, so the next extrinsic input is rel again, unless the clip changed the
 // sum: the column's words hold rel itself, and the row neither subtracts an old
 // message there nor writes a belief, about 20 of an edge's 54 instructions on 42
